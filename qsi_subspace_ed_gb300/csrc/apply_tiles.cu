@@ -15,6 +15,7 @@
 // by row and gathers each column's R values with coalesced loads.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 #include <type_traits>
 
@@ -27,20 +28,21 @@ namespace qsi {
 
 struct TileParams {
     BasisView B;
-    const PullTerm* terms;
-    const uint16_t* lit_off;
-    const uint8_t* lits;
-    const PushTerm* dgen;
+    TileTerms T;
     DiagSpec D;
     const double* diag;  // per-row diagonal, precomputed with diag_value
     const float2* diag_ff;  // the same as (hi, lo) float pairs
-    int n_off, n_lits, nwords;
+    int nwords;
     int vchunk;             // vectors per pass of the 16-byte batched kernel (16, 32, 64 or 128; 0 = 128)
     // operator families (family mode kernels only): the terms' coefficients encode their class as +-(class + 1)
     // and fcoef[class * fR + column] is the coefficient of that class in each column's operator
     const double* fcoef = nullptr;
     int fR = 1;
 };
+
+static TileParams tile_params(const qsi_op* op, int vchunk) {
+    return TileParams{op->basis->view(), op->tile, op->diag, op->d_diag, op->d_diag_ff, op->nwords, vchunk};
+}
 
 // Family mode: the coefficient of a hit whose term's coefficient encodes +-(class + 1), for column col.
 __device__ __forceinline__ double fam_coef(const TileParams& P, double enc, int col) {
@@ -151,72 +153,141 @@ __device__ __forceinline__ void ff2_fma(FF2& a, uint64_t ch, uint64_t cn, uint64
     a.lo = add2(a.lo, add2(err, e));
 }
 
-// Shared-memory layout common to both tile kernels.
+// Shared-memory layout common to the tile kernels.
 struct TileSmem {
-    PullTerm* terms;
-    PushTerm* dgen;
+    uint4* x;           // flipped words; .w as the lookup class wants it
+    ulonglong2* z;
+    double* cs;         // or (hi, lo) float pairs
+    uint2* lit8;
+    uint32_t* pair;
     uint16_t* off;
     uint8_t* lit;
     unsigned char* tail;  // per-warp scratch follows
 };
 
-__device__ __forceinline__ TileSmem stage_terms(const TileParams& P, unsigned char* smem) {
+static size_t tile_smem(const TileTerms& T) {
+    size_t used = (size_t)T.n * (16 + (T.z ? 16 : 0) + 8);
+    if (T.lit8) used += (size_t)T.n * 8 + (size_t)(T.n + 31) / 32 * 4;
+    else used += (size_t)(T.n + 1) * 2 + (size_t)T.n_lits;
+    return (used + 15) & ~(size_t)15;
+}
+
+template <class LK>
+__device__ __forceinline__ TileSmem stage_terms(const TileParams& P, const LK& lk, bool ff, unsigned char* smem) {
+    const TileTerms& T = P.T;
     TileSmem S;
-    S.terms = reinterpret_cast<PullTerm*>(smem);
-    S.dgen = reinterpret_cast<PushTerm*>(S.terms + P.n_off);
-    S.off = reinterpret_cast<uint16_t*>(S.dgen + P.D.n_generic);
-    S.lit = reinterpret_cast<uint8_t*>(S.off + P.n_off + 1);
-    size_t used = (size_t)P.n_off * sizeof(PullTerm) + (size_t)P.D.n_generic * sizeof(PushTerm) +
-                  (size_t)(P.n_off + 1) * 2 + (size_t)P.n_lits;
+    S.x = reinterpret_cast<uint4*>(smem);
+    S.z = reinterpret_cast<ulonglong2*>(S.x + T.n);
+    S.cs = reinterpret_cast<double*>(S.z + (T.z ? T.n : 0));
+    S.lit8 = reinterpret_cast<uint2*>(S.cs + T.n);
+    S.pair = reinterpret_cast<uint32_t*>(S.lit8 + T.n);
+    S.off = reinterpret_cast<uint16_t*>(S.cs + T.n);
+    S.lit = reinterpret_cast<uint8_t*>(S.off + T.n + 1);
+    const size_t used = (size_t)T.n * (16 + (T.z ? 16 : 0) + 8) +
+                        (T.lit8 ? (size_t)T.n * 8 + (size_t)(T.n + 31) / 32 * 4 : (size_t)(T.n + 1) * 2 + (size_t)T.n_lits);
     S.tail = smem + ((used + 15) & ~(size_t)15);
-    for (int k = threadIdx.x; k < P.n_off; k += blockDim.x) S.terms[k] = P.terms[k];
-    for (int k = threadIdx.x; k < P.D.n_generic; k += blockDim.x) S.dgen[k] = P.dgen[k];
-    for (int k = threadIdx.x; k <= P.n_off; k += blockDim.x) S.off[k] = P.lit_off[k];
-    for (int k = threadIdx.x; k < P.n_lits; k += blockDim.x) S.lit[k] = P.lits[k];
+    for (int k = threadIdx.x; k < T.n; k += blockDim.x) {
+        const uint4 x = T.x[k];
+        const Word4 w = lk.words((uint64_t)x.y << 32 | x.x, (uint64_t)x.w << 32 | x.z);
+        S.x[k] = make_uint4(w.w0, w.w1, w.w2, w.w3);
+        if (T.z) S.z[k] = T.z[k];
+        S.cs[k] = ff ? reinterpret_cast<const double*>(T.ff)[k] : T.cs[k];
+    }
+    if (T.lit8) {
+        for (int k = threadIdx.x; k < T.n; k += blockDim.x) S.lit8[k] = T.lit8[k];
+        for (int k = threadIdx.x; k < (T.n + 31) / 32; k += blockDim.x) S.pair[k] = T.pair[k];
+    } else {
+        for (int k = threadIdx.x; k <= T.n; k += blockDim.x) S.off[k] = T.lit_off[k];
+        for (int k = threadIdx.x; k < T.n_lits; k += blockDim.x) S.lit[k] = T.lits[k];
+    }
     __syncthreads();
     return S;
 }
 
-// Transposes the tile's states into per-spin words spinw[0 .. 32*nwords).
+// Transposes the tile's states into per-spin words: spinw[i] bit l = spin i of row l, spinw[128 + i] its complement.
+constexpr int kSpinWords = 256;
 __device__ __forceinline__ void tile_spin_words(const state2 s, int nwords, int lane, uint32_t* spinw) {
     const uint32_t w[4] = {(uint32_t)s.x, (uint32_t)(s.x >> 32), (uint32_t)s.y, (uint32_t)(s.y >> 32)};
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        if (k < nwords) spinw[32 * k + lane] = warp_transpose32(w[k], lane);
+        if (k < nwords) {
+            const uint32_t t = warp_transpose32(w[k], lane);
+            spinw[32 * k + lane] = t;
+            spinw[128 + 32 * k + lane] = ~t;
+        }
     __syncwarp();
 }
 
 // Admission bits of terms t0..t0+31 for this lane's row (bit j = term t0+j).
-__device__ __forceinline__ uint32_t tile_admitted(const TileSmem& S, int n_off, int t0, int lane, uint32_t vmask,
-                                                  const uint32_t* spinw) {
+__device__ __forceinline__ uint32_t tile_admitted(const TileSmem& S, const TileTerms& T, int t0, int lane,
+                                                  uint32_t vmask, const uint32_t* spinw) {
     const int t = t0 + lane;
     uint32_t A = 0;
-    if (t < n_off) {
-        A = vmask;
-        const int e = S.off[t + 1];
-        for (int k = S.off[t]; k < e; ++k) {
-            const uint8_t L = S.lit[k];
-            A &= spinw[L & 127] ^ ((L & 128) ? 0xFFFFFFFFu : 0u);
+    if (t < T.n) {
+        if (T.lit8) {
+            const uint2 L = S.lit8[t];
+            uint32_t all = spinw[L.x & 0xff], any = all;
+#pragma unroll
+            for (int k = 1; k < 8; ++k) {
+                if (k >= T.max_lits) break;
+                const uint32_t w = spinw[((k < 4 ? L.x : L.y) >> (8 * (k & 3))) & 0xff];
+                all &= w;
+                any |= w;
+            }
+            if ((S.pair[t0 >> 5] >> lane) & 1) all |= ~any;
+            A = all & vmask;
+        } else {
+            A = vmask;
+            const int e = S.off[t + 1];
+            for (int k = S.off[t]; k < e; ++k) A &= spinw[S.lit[k]];
         }
     }
     return warp_transpose32(A, lane);
 }
 
-__device__ __forceinline__ double term_coeff(const PullTerm& T, const state2 s) {
-    double cs = T.cs;
-    if (T.has_z && ((__popcll(~s.x & T.z0) + __popcll(~s.y & T.z1)) & 1)) cs = -cs;
-    return cs;
+// Whether term t's matrix element on state s carries a minus sign from its Z mask.
+__device__ __forceinline__ bool term_negative(const TileSmem& S, bool has_z, uint32_t t, const state2 s) {
+    if (!has_z) return false;
+    const ulonglong2 z = S.z[t];
+    return (__popcll(~s.x & z.x) + __popcll(~s.y & z.y)) & 1;
+}
+__device__ __forceinline__ double term_coeff(const TileSmem& S, bool has_z, uint32_t t, const state2 s) {
+    const double cs = S.cs[t];
+    return term_negative(S, has_z, t, s) ? -cs : cs;
+}
+
+// The next up to NB admitted terms of this lane's row, in term order across the 32-term rounds: their numbers and
+// the flipped states.  r, a: the round and what is left of its admission word.
+template <int NB>
+__device__ __forceinline__ int next_hits(const TileSmem& S, const Word4& row, const uint32_t* adm, int lane, int n_rounds,
+                                         int& r, uint32_t& a, uint32_t (&tt)[NB], Word4 (&w)[NB]) {
+    int nh = 0;
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+        tt[u] = 0;
+        w[u] = Word4{0, 0, 0, 0};
+        while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
+        if (a) {
+            tt[u] = r * 32 + __ffs(a) - 1;
+            a &= a - 1;
+            const uint4 x = S.x[tt[u]];
+            w[u] = Word4{row.w0 ^ x.x, row.w1 ^ x.y, row.w2 ^ x.z, row.w3 ^ x.w};
+            ++nh;
+        }
+    }
+    return nh;
 }
 
 template <typename XT, typename YT, class LK, bool kFam = false>
 __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P, LK lk, const XT* __restrict__ x,
                                                                  YT* __restrict__ y, int accumulate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const TileSmem S = stage_terms(P, smem_raw);
+    const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int n_rounds = (P.n_off + 31) >> 5;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (128 + 32 * n_rounds);
-    uint32_t* adm = spinw + 128;  // admission words of the tile, one per lane and 32-term round
+    const int n_rounds = (P.T.n + 31) >> 5;
+    const bool has_z = P.T.z != nullptr;
+    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
+    uint32_t* adm = spinw + kSpinWords;  // admission words of the tile, one per lane and 32-term round
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
@@ -224,44 +295,35 @@ __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.n_off, r * 32, lane, vmask, spinw);
+        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
         double acc = valid ? (kFam ? fam_diag(P, s.x, s.y, 0) : P.diag[row]) * (double)x[row] : 0.0;
         const uint64_t cur = lk.cursor(tile, lane);
+        const Word4 rw = lk.words(s.x, s.y);
         int kk = 0;  // admitted terms of this row looked up so far
         int r = 0;
-        uint32_t a = adm[lane];
+        uint32_t a = n_rounds ? adm[lane] : 0;
         while (true) {
             // up to kNB admitted terms at a time (across rounds): lookups and gathers in flight together,
             // contributions added in term order
             constexpr int kNB = LK::kNB;
-            int tt[kNB];
-            uint64_t tl[kNB], th[kNB];
-            int64_t J[kNB];
-            int nh = 0;
-#pragma unroll
-            for (int u = 0; u < kNB; ++u) {
-                tt[u] = 0;
-                tl[u] = th[u] = 0;
-                while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
-                if (a) {
-                    tt[u] = r * 32 + __ffs(a) - 1;
-                    a &= a - 1;
-                    const PullTerm& T = S.terms[tt[u]];
-                    tl[u] = s.x ^ T.x0;
-                    th[u] = s.y ^ T.x1;
-                    ++nh;
-                }
-            }
+            uint32_t tt[kNB], J[kNB];
+            Word4 w[kNB];
+            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
             if (!nh) break;
-            lk.template find_batch<kNB>(tl, th, J, nh, cur, kk);
+            lk.find_batch(w, nh, J, cur, kk);
             kk += nh;
             XT xv[kNB];
 #pragma unroll
-            for (int u = 0; u < kNB; ++u) xv[u] = (u < nh && J[u] >= 0) ? x[J[u]] : (XT)0;
+            for (int u = 0; u < kNB; ++u) xv[u] = (J[u] != kEmpty) ? x[J[u]] : (XT)0;
+            if constexpr (LK::kCheck) {
+#pragma unroll
+                for (int u = 0; u < kNB; ++u)
+                    if (J[u] != kEmpty && !lk.matches(w[u], J[u])) xv[u] = (XT)0;  // outside the basis
+            }
 #pragma unroll
             for (int u = 0; u < kNB; ++u)
-                if (u < nh && J[u] >= 0 && above_tol(xv[u])) {
-                    const double cs = term_coeff(S.terms[tt[u]], s);
+                if (above_tol(xv[u])) {
+                    const double cs = term_coeff(S, has_z, tt[u], s);
                     acc += (kFam ? fam_coef(P, cs, 0) : cs) * (double)xv[u];
                 }
         }
@@ -281,12 +343,13 @@ template <class LK, int RC>
 __global__ void __launch_bounds__(256, RC <= 4 ? 4 : 2) k_apply_tile_cols(TileParams P, LK lk, const double* __restrict__ x,
                                                             double* __restrict__ y, int accumulate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const TileSmem S = stage_terms(P, smem_raw);
+    const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int n_rounds = (P.n_off + 31) >> 5;
+    const int n_rounds = (P.T.n + 31) >> 5;
+    const bool has_z = P.T.z != nullptr;
     const int R = P.fR;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (128 + 32 * n_rounds);
-    uint32_t* adm = spinw + 128;
+    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
+    uint32_t* adm = spinw + kSpinWords;
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
@@ -294,41 +357,27 @@ __global__ void __launch_bounds__(256, RC <= 4 ? 4 : 2) k_apply_tile_cols(TilePa
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.n_off, r * 32, lane, vmask, spinw);
+        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
         double acc[RC];
 #pragma unroll
         for (int c = 0; c < RC; ++c) acc[c] = (valid && c < R) ? fam_diag(P, s.x, s.y, c) * x[row * R + c] : 0.0;
         const uint64_t cur = lk.cursor(tile, lane);
+        const Word4 rw = lk.words(s.x, s.y);
         int kk = 0, r = 0;
-        uint32_t a = adm[lane];
+        uint32_t a = n_rounds ? adm[lane] : 0;
         while (true) {
             constexpr int kNB = 4;
-            int tt[kNB];
-            uint64_t tl[kNB], th[kNB];
-            int64_t J[kNB];
-            int nh = 0;
-#pragma unroll
-            for (int u = 0; u < kNB; ++u) {
-                tt[u] = 0;
-                tl[u] = th[u] = 0;
-                while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
-                if (a) {
-                    tt[u] = r * 32 + __ffs(a) - 1;
-                    a &= a - 1;
-                    const PullTerm& T = S.terms[tt[u]];
-                    tl[u] = s.x ^ T.x0;
-                    th[u] = s.y ^ T.x1;
-                    ++nh;
-                }
-            }
+            uint32_t tt[kNB], J[kNB];
+            Word4 w[kNB];
+            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
             if (!nh) break;
-            lk.template find_batch<kNB>(tl, th, J, nh, cur, kk);
+            lk.find_batch(w, nh, J, cur, kk);
             kk += nh;
 #pragma unroll
             for (int u = 0; u < kNB; ++u) {
-                if (u >= nh || J[u] < 0) continue;
-                const double cs = term_coeff(S.terms[tt[u]], s);
-                const double* xj = x + J[u] * R;
+                if (J[u] == kEmpty || !lk.matches(w[u], J[u])) continue;
+                const double cs = term_coeff(S, has_z, tt[u], s);
+                const double* xj = x + (int64_t)J[u] * R;
                 double xv[RC];
 #pragma unroll
                 for (int c = 0; c < RC; ++c) xv[c] = (c < R) ? xj[c] : 0.0;
@@ -376,13 +425,14 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
                                              int64_t n_blocks, unsigned char* smem_raw,
                                              const float2* __restrict__ ycoef = nullptr) {
     // accumulate: y <- H x + c y per column, c = 1, or the (hi, lo) float pair ycoef[column] (double-float paths)
-    const TileSmem S = stage_terms(P, smem_raw);
+    const TileSmem S = stage_terms(P, lk, kFF, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int n_rounds = (P.n_off + 31) >> 5;
-    // per-warp scratch: spin words (128 u32), admission words (n_rounds*32 u32), hit list
-    unsigned char* mine = S.tail + (size_t)wid * (512 + (size_t)n_rounds * 128 + (size_t)cap * 12);
+    const int n_rounds = (P.T.n + 31) >> 5;
+    const bool has_z = P.T.z != nullptr;
+    // per-warp scratch: spin words, admission words (n_rounds*32 u32), hit list
+    unsigned char* mine = S.tail + (size_t)wid * (4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12);
     uint32_t* spinw = reinterpret_cast<uint32_t*>(mine);
-    uint32_t* adm = spinw + 128;
+    uint32_t* adm = spinw + kSpinWords;
     double* hc = reinterpret_cast<double*>(adm + n_rounds * 32);  // coefficients (8-byte aligned)
     float2* hcf = reinterpret_cast<float2*>(hc);                   // the same slots as (hi, lo) floats
     uint32_t* hJ = reinterpret_cast<uint32_t*>(hc + cap);
@@ -408,7 +458,7 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
         tile_spin_words(s, P.nwords, lane, spinw);
         int cnt = 0;
         for (int r = 0; r < n_rounds; ++r) {
-            const uint32_t a = tile_admitted(S, P.n_off, r * 32, lane, vmask, spinw);
+            const uint32_t a = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
             adm[r * 32 + lane] = a;
             cnt += __popc(a);
         }
@@ -437,45 +487,29 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
                 }
                 // this row's admitted terms in term order, kNB lookups at a time across the 32-term rounds
                 const uint64_t cur = lk.cursor(tile, lane);
+                const Word4 rw = lk.words(s.x, s.y);
                 int kk = 0;
                 int r = 0;
-                uint32_t a = adm[lane];
+                uint32_t a = n_rounds ? adm[lane] : 0;
                 while (true) {
-                    {
-                        constexpr int kNB = v4 ? 6 : 4;
-                        int tt[kNB];
-                        uint64_t tl[kNB], th[kNB];
-                        int64_t J[kNB];
-                        int nh = 0;
+                    constexpr int kNB = v4 ? 4 : 2;
+                    uint32_t tt[kNB], J[kNB];
+                    Word4 w[kNB];
+                    const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
+                    if (!nh) break;
+                    lk.find_batch(w, nh, J, cur, kk);
+                    kk += nh;
 #pragma unroll
-                        for (int u = 0; u < kNB; ++u) {
-                            tt[u] = 0;
-                            tl[u] = th[u] = 0;
-                            while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
-                            if (a) {
-                                tt[u] = r * 32 + __ffs(a) - 1;
-                                a &= a - 1;
-                                tl[u] = s.x ^ S.terms[tt[u]].x0;
-                                th[u] = s.y ^ S.terms[tt[u]].x1;
-                                ++nh;
-                            }
+                    for (int u = 0; u < kNB; ++u) {
+                        if (u >= nh) continue;
+                        hJ[k] = (J[u] != kEmpty && lk.matches(w[u], J[u])) ? J[u] : kEmpty;
+                        if constexpr (kFF) {
+                            const float2 f = reinterpret_cast<const float2*>(S.cs)[tt[u]];
+                            hcf[k] = term_negative(S, has_z, tt[u], s) ? make_float2(-f.x, -f.y) : f;
+                        } else {
+                            hc[k] = term_coeff(S, has_z, tt[u], s);
                         }
-                        if (!nh) break;
-                        lk.template find_batch<kNB>(tl, th, J, nh, cur, kk);
-                        kk += nh;
-#pragma unroll
-                        for (int u = 0; u < kNB; ++u) {
-                            if (u >= nh) continue;
-                            hJ[k] = (J[u] < 0) ? kEmpty : (uint32_t)J[u];
-                            const PullTerm& T = S.terms[tt[u]];
-                            if constexpr (kFF) {
-                                const bool neg = T.has_z && ((__popcll(~s.x & T.z0) + __popcll(~s.y & T.z1)) & 1);
-                                hcf[k] = neg ? make_float2(-T.cs_hi, -T.cs_lo) : make_float2(T.cs_hi, T.cs_lo);
-                            } else {
-                                hc[k] = term_coeff(T, s);
-                            }
-                            ++k;
-                        }
+                        ++k;
                     }
                 }
             }
@@ -713,7 +747,7 @@ __global__ void __launch_bounds__(256, KM <= kVec4 ? 2 : 3) k_apply_tile_batched
 // use them, else bucket-table lookups.
 struct SectorLaunch {
     TileParams P;
-    HashView H;
+    BinView H;
     CacheView C;
     const float* x;
     float* y;
@@ -736,9 +770,9 @@ __global__ void __launch_bounds__(256, KM <= kVec4 ? 2 : 3) k_apply_sectors(cons
     }
     __syncthreads();
     LK lk;
-    if constexpr (std::is_same<LK, LookupHash>::value) lk = LookupHash{L.H};
-    else if constexpr (std::is_same<LK, LookupCache>::value) lk = LookupCache{L.C};
-    else lk = LookupTable{L.P.B};
+    if constexpr (std::is_same<LK, LookupCache>::value) lk = LookupCache{L.C};
+    else if constexpr (std::is_same<LK, LookupTable>::value) lk = LookupTable{L.P.B};
+    else lk = LK{L.H};
     batched_body<float, LK, true, KM>(L.P, lk, L.x, L.y, L.R, accumulate, L.cap, (int64_t)blockIdx.x - L.block_begin,
                                       L.n_blocks, smem_raw, L.ycoef);
 }
@@ -768,58 +802,239 @@ qsi_status build_diag(qsi_op* op) {
 }
 
 // ------------------------------------------------------------------ hash index build
-__global__ void k_hash_clear(HashSlot* slots, uint64_t n_slots) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_slots; i += (uint64_t)gridDim.x * blockDim.x) {
-        slots[i].lo = 0;
-        slots[i].hi = 0;
-        slots[i].idx = kEmpty;
+__global__ void k_largest_bucket(BasisView B, uint32_t* largest) {
+    uint32_t m = 0;
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < B.n_buckets; v += (int64_t)gridDim.x * blockDim.x)
+        m = max(m, B.tab[v].y - B.tab[v].x);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(largest, m);
+}
+
+__device__ __forceinline__ uint32_t state_bin(const BinView& H, const state2 s, uint2& ab, uint32_t& tag) {
+    bool ok;
+    ab = H.B.tab[bucket_of(H.B, s.x, s.y, ok)];
+    uint32_t frac;
+    bin_hash((uint32_t)s.x, (uint32_t)(s.x >> 32), (uint32_t)s.y, frac, tag);
+    tag = slot_tag(tag, H.off_mask);
+    return pick_bin(ab, frac);
+}
+
+// Every state takes the first free slot of its bin; a state that finds it full is left out.
+__global__ void k_bins_insert(BinView H, uint32_t* bins) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < H.B.n; i += (int64_t)gridDim.x * blockDim.x) {
+        uint2 ab;
+        uint32_t tag;
+        uint32_t* p = bins + (size_t)state_bin(H, H.B.states[i], ab, tag) * kBinSlots;
+        for (int k = 0; k < kBinSlots; ++k)
+            if (atomicCAS(p + k, kEmpty, tag | ((uint32_t)i - ab.x)) == kEmpty) break;
     }
 }
 
-__global__ void k_hash_insert(const state2* __restrict__ states, int64_t n, HashView H, HashSlot* slots,
-                              int* overflow) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const state2 s = states[i];
-        const HashSlot* creg;
-        const uint64_t cap = hash_region(H, s.x, s.y, creg);
-        HashSlot* reg = slots + (creg - H.slots);
-        uint64_t off = cap ? region_first(s.x, s.y, cap) : 0;
-        bool done = false;
-        for (uint64_t probe = 0; probe < cap; ++probe) {
-            if (atomicCAS(&reg[off].idx, kEmpty, (uint32_t)i) == kEmpty) {
-                reg[off].lo = s.x;
-                reg[off].hi = (uint32_t)s.y;
-                done = true;
-                break;
-            }
-            off = (off + 1 == cap) ? 0 : off + 1;
-        }
-        if (!done) atomicOr(overflow, 1);
+// Marks the slots that a state of the basis would take for its own though they are not: afterwards a state's first
+// match is itself or a marked slot, or its bin is full and has no match.
+__global__ void k_bins_check(BinView H, uint32_t* bins) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < H.B.n; i += (int64_t)gridDim.x * blockDim.x) {
+        uint2 ab;
+        uint32_t tag, w[kBinSlots];
+        uint32_t* p = bins + (size_t)state_bin(H, H.B.states[i], ab, tag) * kBinSlots;
+        for (int k = 0; k < kBinSlots; ++k) w[k] = *(volatile uint32_t*)(p + k);
+        const uint32_t m = bin_match(w, tag);
+        if (m > H.off_mask || m == (uint32_t)i - ab.x) continue;
+        for (int k = 0; k < kBinSlots; ++k)
+            if ((w[k] ^ tag) <= H.off_mask) atomicOr(p + k, H.off_mask);
     }
 }
 
-// The regional hash index over the basis's current bucket table (built again whenever the table is): 2n slots.
+void drop_hash(qsi_basis* b) {
+    if (b->d_bins) cudaFree(b->d_bins);
+    b->d_bins = nullptr;
+    b->n_bins = 0;
+}
+
+// The bins over the basis's current bucket table (built again whenever the table is).
 qsi_status build_hash(qsi_basis* b) {
     if (b->hb >= 96) return fail(QSI_INVALID_ARG, "hash index needs states of at most 96 bits");
     if (b->n >= ((int64_t)1 << 31)) return fail(QSI_INVALID_ARG, "hash index needs fewer than 2^31 states");
-    const uint64_t n_slots = 2 * (uint64_t)b->n;
-    if (!b->d_hash || b->hash_slots != n_slots) {
-        if (b->d_hash) cudaFree(b->d_hash);
-        b->d_hash = nullptr;
-        b->hash_slots = 0;
-        QSI_CUDA(cudaMalloc(&b->d_hash, n_slots * sizeof(HashSlot)));
-        b->hash_slots = n_slots;
+    const uint64_t n_bins = (uint64_t)bin_of((uint32_t)(b->n - 1)) + 1;
+    if (!b->d_bins || b->n_bins != n_bins) {
+        drop_hash(b);
+        QSI_CUDA(cudaMalloc(&b->d_bins, n_bins * kBinSlots * sizeof(uint32_t)));
+        b->n_bins = n_bins;
     }
-    int* d_over = nullptr;
-    QSI_CUDA(cudaMalloc(&d_over, sizeof(int)));
-    QSI_CUDA(cudaMemset(d_over, 0, sizeof(int)));
-    k_hash_clear<<<grid_for((int64_t)n_slots, 256), 256>>>(b->d_hash, n_slots);
-    k_hash_insert<<<grid_for(b->n, 256), 256>>>(b->d_states, b->n, b->hview(), b->d_hash, d_over);
-    int over = 0;
-    cudaError_t e = cudaMemcpy(&over, d_over, sizeof(int), cudaMemcpyDeviceToHost);
-    cudaFree(d_over);
-    if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "hash build: %s", cudaGetErrorString(e));
-    if (over) return fail(QSI_CUDA_ERROR, "hash build: a state found no slot in its region");
+    auto build = [&]() -> qsi_status {
+        uint32_t largest = 0;
+        QSI_CUDA(cudaMemset(b->d_bins, 0, sizeof(uint32_t)));  // the maximum's accumulator, before the bins are cleared
+        k_largest_bucket<<<grid_for(b->n_buckets, 256), 256>>>(b->view(), b->d_bins);
+        QSI_CUDA(cudaMemcpy(&largest, b->d_bins, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+        b->off_mask = 15;
+        while (b->off_mask < largest) b->off_mask = 2 * b->off_mask + 1;
+        QSI_CUDA(cudaMemset(b->d_bins, 0xFF, n_bins * kBinSlots * sizeof(uint32_t)));
+        k_bins_insert<<<grid_for(b->n, 256), 256>>>(b->bview(), b->d_bins);
+        k_bins_check<<<grid_for(b->n, 256), 256>>>(b->bview(), b->d_bins);
+        QSI_CUDA(cudaGetLastError());
+        QSI_CUDA(cudaStreamSynchronize(nullptr));
+        return QSI_OK;
+    };
+    const qsi_status s = build();
+    if (s != QSI_OK) drop_hash(b);
+    return s;
+}
+
+// ------------------------------------------------------------------ term tables
+qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull) {
+    std::vector<const PullTerm*> kept;
+    std::vector<uint32_t> pair((pull.size() + 31) / 32 + 1, 0);
+    std::vector<std::vector<uint8_t>> lits(pull.size());
+    bool short_lists = true, any_z = false;
+    for (size_t k = 0; k < pull.size(); ++k) {
+        const PullTerm& t = pull[k];
+        const uint64_t um[2] = {t.up0, t.up1}, dm[2] = {t.dn0, t.dn1};
+        for (int bit = 0; bit < 128; ++bit) {
+            if ((um[bit >> 6] >> (bit & 63)) & 1) lits[k].push_back((uint8_t)bit);
+            if ((dm[bit >> 6] >> (bit & 63)) & 1) lits[k].push_back((uint8_t)(0x80 | bit));
+        }
+        short_lists = short_lists && !lits[k].empty() && lits[k].size() <= 8;
+        any_z = any_z || t.has_z;
+    }
+    std::vector<std::vector<uint8_t>*> klits;
+    for (size_t k = 0; k < pull.size(); ++k) {
+        const PullTerm& t = pull[k];
+        klits.push_back(&lits[k]);
+        kept.push_back(&t);
+        if (short_lists && k + 1 < pull.size()) {
+            const PullTerm& c = pull[k + 1];
+            if (c.x0 == t.x0 && c.x1 == t.x1 && c.z0 == t.z0 && c.z1 == t.z1 && c.cs == t.cs && c.up0 == t.dn0 &&
+                c.up1 == t.dn1 && c.dn0 == t.up0 && c.dn1 == t.up1) {
+                pair[(kept.size() - 1) >> 5] |= 1u << ((kept.size() - 1) & 31);
+                ++k;
+            }
+        }
+    }
+    TileTerms& T = op->tile;
+    T = TileTerms{};
+    T.n = (int)kept.size();
+    std::vector<uint4> x;
+    std::vector<double> cs;
+    std::vector<float2> ff;
+    std::vector<ulonglong2> z;
+    std::vector<uint2> lit8;
+    std::vector<uint16_t> off{0};
+    std::vector<uint8_t> flat;
+    for (int k = 0; k < T.n; ++k) {
+        const PullTerm& t = *kept[k];
+        const std::vector<uint8_t>& l = *klits[k];
+        x.push_back(make_uint4((uint32_t)t.x0, (uint32_t)(t.x0 >> 32), (uint32_t)t.x1, (uint32_t)(t.x1 >> 32)));
+        cs.push_back(t.cs);
+        ff.push_back(make_float2(t.cs_hi, t.cs_lo));
+        if (any_z) z.push_back(make_ulonglong2(t.z0, t.z1));
+        if (short_lists) {
+            uint32_t w[2] = {0, 0};
+            for (int j = 0; j < 8; ++j) w[j >> 2] |= (uint32_t)l[std::min<size_t>(j, l.size() - 1)] << (8 * (j & 3));
+            lit8.push_back(make_uint2(w[0], w[1]));
+            T.max_lits = std::max(T.max_lits, (int)l.size());
+        } else {
+            flat.insert(flat.end(), l.begin(), l.end());
+            if (flat.size() > 65535) return fail(QSI_INVALID_ARG, "qsi_op_create: more than 65535 literals in the term list");
+            off.push_back((uint16_t)flat.size());
+        }
+    }
+    T.n_lits = (int)flat.size();
+    size_t total = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 15) & ~(size_t)15;
+        return at;
+    };
+    const size_t n = (size_t)T.n, o_x = place(n * 16), o_cs = place(n * 8), o_ff = place(n * 8), o_z = place(z.size() * 16),
+                 o_l8 = place(lit8.size() * 8), o_p = place(pair.size() * 4), o_off = place(off.size() * 2),
+                 o_lit = place(flat.size());
+    std::vector<unsigned char> host(total + 16, 0);
+    auto put = [&](size_t at, const void* src, size_t bytes) {
+        if (bytes) std::memcpy(host.data() + at, src, bytes);
+    };
+    put(o_x, x.data(), n * 16);
+    put(o_cs, cs.data(), n * 8);
+    put(o_ff, ff.data(), n * 8);
+    put(o_z, z.data(), z.size() * 16);
+    put(o_l8, lit8.data(), lit8.size() * 8);
+    put(o_p, pair.data(), pair.size() * 4);
+    put(o_off, off.data(), off.size() * 2);
+    put(o_lit, flat.data(), flat.size());
+    QSI_CUDA(cudaMalloc(&op->d_tile_terms, host.size()));
+    QSI_CUDA(cudaMemcpy(op->d_tile_terms, host.data(), host.size(), cudaMemcpyHostToDevice));
+    unsigned char* d = op->d_tile_terms;
+    T.x = reinterpret_cast<const uint4*>(d + o_x);
+    T.cs = reinterpret_cast<const double*>(d + o_cs);
+    T.ff = reinterpret_cast<const float2*>(d + o_ff);
+    T.z = any_z ? reinterpret_cast<const ulonglong2*>(d + o_z) : nullptr;
+    T.lit8 = (short_lists && n) ? reinterpret_cast<const uint2*>(d + o_l8) : nullptr;
+    T.pair = reinterpret_cast<const uint32_t*>(d + o_p);
+    T.lit_off = reinterpret_cast<const uint16_t*>(d + o_off);
+    T.lits = reinterpret_cast<const uint8_t*>(d + o_lit);
+    return QSI_OK;
+}
+
+// *missed = 1 when an admitted term of some row leaves the basis.
+template <class LK>
+__global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, int* __restrict__ missed) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const TileSmem S = stage_terms(P, lk, false, smem_raw);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int n_rounds = (P.T.n + 31) >> 5;
+    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
+    uint32_t* adm = spinw + kSpinWords;
+    const int64_t ntiles = (P.B.n + 31) >> 5;
+    for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
+        if (*(volatile int*)missed) break;
+        const int64_t row = tile * 32 + lane;
+        const bool valid = row < P.B.n;
+        const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
+        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
+        tile_spin_words(s, P.nwords, lane, spinw);
+        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
+        const Word4 rw = lk.words(s.x, s.y);
+        int r = 0;
+        uint32_t a = n_rounds ? adm[lane] : 0;
+        bool miss = false;
+        while (true) {
+            constexpr int kNB = 4;
+            uint32_t tt[kNB], J[kNB];
+            Word4 w[kNB];
+            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
+            if (!nh) break;
+            lk.find_batch(w, nh, J);
+#pragma unroll
+            for (int u = 0; u < kNB; ++u) miss = miss || (u < nh && (J[u] == kEmpty || !lk.matches(w[u], J[u])));
+        }
+        if (miss) *(volatile int*)missed = 1;
+        __syncwarp();
+    }
+}
+
+// Determines op->closed: with a hash index, one pass of compared lookups (about 0.8 of an apply; a first miss ends it).
+// Applies of a closed operator take a tag match for the state itself, which saves each of their lookups the 16-byte
+// load of the state at the index found.
+qsi_status find_closed(qsi_op* op) {
+    op->closed = 0;
+    if (!op->basis->d_bins) return QSI_OK;
+    const TileParams P = tile_params(op, 0);
+    cudaStream_t st = op->stream;
+    int* d_missed = nullptr;
+    QSI_CUDA(cudaMallocAsync(&d_missed, sizeof(int), st));
+    cudaError_t e = cudaMemsetAsync(d_missed, 0, sizeof(int), st);
+    const int64_t ntiles = (P.B.n + 31) / 32;
+    const size_t smem = tile_smem(P.T) + 8 * (4 * kSpinWords + (size_t)(P.T.n + 31) / 32 * 128);
+    const LookupBins<false> lk{op->basis->bview()};
+    auto k = k_find_miss<LookupBins<false>>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k<<<grid_for(ntiles, 8), 256, smem, st>>>(P, lk, d_missed);
+    int missed = 1;
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&missed, d_missed, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFreeAsync(d_missed, st);
+    if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "qsi_op_create (closure): %s", cudaGetErrorString(e));
+    op->closed = !missed;
     return QSI_OK;
 }
 
@@ -829,13 +1044,13 @@ qsi_status build_hash(qsi_basis* b) {
 // admission order of the tile kernels) with coefficient +-cs of the entry's term and the entry's sign, the same
 // sums in the same order as k_apply_tile, so the result is bitwise the matrix-free one.
 template <typename XT, typename YT, typename TT>
-__global__ void __launch_bounds__(256) k_apply_cached(const PullTerm* __restrict__ terms, int n_off,
+__global__ void __launch_bounds__(256) k_apply_cached(const double* __restrict__ coef, int n_off,
                                                       const double* __restrict__ diag, CacheView C,
                                                       const TT* __restrict__ tids, int64_t n, const XT* __restrict__ x,
                                                       YT* __restrict__ y, int accumulate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* cs = reinterpret_cast<double*>(smem_raw);
-    for (int k = threadIdx.x; k < n_off; k += blockDim.x) cs[k] = terms[k].cs;
+    for (int k = threadIdx.x; k < n_off; k += blockDim.x) cs[k] = coef[k];
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int64_t ntiles = (n + 31) >> 5;
@@ -887,7 +1102,7 @@ static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, 
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int bps = op->tune[0].grid_bps > 0 ? op->tune[0].grid_bps : 8;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * bps));
-    const size_t smem = (size_t)std::max(op->n_pull, 1) * 8;
+    const size_t smem = (size_t)std::max(op->tile.n, 1) * 8;
     const CacheView C{op->d_cache_cols, op->d_cache_off};
     auto go = [&](auto xt, auto yt, auto tt) {
         using XT = decltype(xt);
@@ -895,7 +1110,7 @@ static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, 
         using TT = decltype(tt);
         auto k = k_apply_cached<XT, YT, TT>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, block, smem, st>>>(op->d_pull, op->n_pull, op->d_diag, C, (const TT*)op->d_cache_tid, n,
+        k<<<grid, block, smem, st>>>(op->tile.cs, op->tile.n, op->d_diag, C, (const TT*)op->d_cache_tid, n,
                                      (const XT*)x, (YT*)y, accumulate);
     };
     auto by_tid = [&](auto xt, auto yt) {
@@ -914,10 +1129,10 @@ static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, 
 // Admitted terms of the tile's widest row: the tile's number of cache lines.
 __global__ void __launch_bounds__(256) k_cache_widths(TileParams P, uint64_t* __restrict__ width) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const TileSmem S = stage_terms(P, smem_raw);
+    const TileSmem S = stage_terms(P, LookupTable{P.B}, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int n_rounds = (P.n_off + 31) >> 5;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * 128;
+    const int n_rounds = (P.T.n + 31) >> 5;
+    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * kSpinWords;
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
@@ -926,7 +1141,7 @@ __global__ void __launch_bounds__(256) k_cache_widths(TileParams P, uint64_t* __
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         tile_spin_words(s, P.nwords, lane, spinw);
         int cnt = 0;
-        for (int r = 0; r < n_rounds; ++r) cnt += __popc(tile_admitted(S, P.n_off, r * 32, lane, vmask, spinw));
+        for (int r = 0; r < n_rounds; ++r) cnt += __popc(tile_admitted(S, P.T, r * 32, lane, vmask, spinw));
 #pragma unroll
         for (int o = 16; o; o >>= 1) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, o));
         if (lane == 0) width[tile] = (uint64_t)cnt;
@@ -940,11 +1155,12 @@ template <class LK, typename TT>
 __global__ void __launch_bounds__(256) k_cache_fill(TileParams P, LK lk, const uint64_t* __restrict__ off,
                                                     uint32_t* __restrict__ cols, TT* __restrict__ tids) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const TileSmem S = stage_terms(P, smem_raw);
+    const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int n_rounds = (P.n_off + 31) >> 5;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (128 + 32 * n_rounds);
-    uint32_t* adm = spinw + 128;
+    const int n_rounds = (P.T.n + 31) >> 5;
+    const bool has_z = P.T.z != nullptr;
+    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
+    uint32_t* adm = spinw + kSpinWords;
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
@@ -952,40 +1168,26 @@ __global__ void __launch_bounds__(256) k_cache_fill(TileParams P, LK lk, const u
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.n_off, r * 32, lane, vmask, spinw);
+        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
         uint32_t* out = cols + off[tile] * 32 + lane;
         TT* tout = tids + off[tile] * 32 + lane;
+        const Word4 rw = lk.words(s.x, s.y);
         int kk = 0, r = 0;
-        uint32_t a = adm[lane];
+        uint32_t a = n_rounds ? adm[lane] : 0;
         while (true) {
             constexpr int kNB = 4;
-            int tt[kNB];
-            uint64_t tl[kNB], th[kNB];
-            int64_t J[kNB];
-            int nh = 0;
-#pragma unroll
-            for (int u = 0; u < kNB; ++u) {
-                tt[u] = 0;
-                tl[u] = th[u] = 0;
-                while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
-                if (a) {
-                    tt[u] = r * 32 + __ffs(a) - 1;
-                    const PullTerm& T = S.terms[tt[u]];
-                    a &= a - 1;
-                    tl[u] = s.x ^ T.x0;
-                    th[u] = s.y ^ T.x1;
-                    ++nh;
-                }
-            }
+            uint32_t tt[kNB], J[kNB];
+            Word4 w[kNB];
+            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
             if (!nh) break;
-            lk.template find_batch<kNB>(tl, th, J, nh);
+            lk.find_batch(w, nh, J);
 #pragma unroll
             for (int u = 0; u < kNB; ++u)
                 if (u < nh) {
                     // the column, with the sign of the term's matrix element on this row in the top bit
-                    const PullTerm& T = S.terms[tt[u]];
-                    const bool neg = T.has_z && ((__popcll(~s.x & T.z0) + __popcll(~s.y & T.z1)) & 1);
-                    out[(uint64_t)(kk + u) * 32] = (J[u] < 0) ? kEmpty : ((uint32_t)J[u] | (neg ? kCacheNeg : 0u));
+                    const bool in = J[u] != kEmpty && lk.matches(w[u], J[u]);
+                    out[(uint64_t)(kk + u) * 32] =
+                        in ? (J[u] | (term_negative(S, has_z, tt[u], s) ? kCacheNeg : 0u)) : kEmpty;
                     tout[(uint64_t)(kk + u) * 32] = (TT)tt[u];
                 }
             kk += nh;
@@ -995,11 +1197,7 @@ __global__ void __launch_bounds__(256) k_cache_fill(TileParams P, LK lk, const u
 }
 
 // ------------------------------------------------------------------ launchers
-static size_t term_smem(const qsi_op* op) {
-    size_t used = (size_t)op->n_pull * sizeof(PullTerm) + (size_t)op->n_diag_generic * sizeof(PushTerm) +
-                  (size_t)(op->n_pull + 1) * 2 + (size_t)op->n_lits;
-    return (used + 15) & ~(size_t)15;
-}
+static size_t term_smem(const qsi_op* op) { return tile_smem(op->tile); }
 
 template <class K>
 static void set_smem(K kernel, size_t smem) {
@@ -1023,13 +1221,12 @@ template <class LK>
 static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int R, int xdtype, int ydtype,
                                   int accumulate, cudaStream_t st) {
     const qsi_tuning& T = op->tune[R > 1];
-    TileParams P{op->basis->view(), op->d_pull, op->d_lit_off, op->d_lits, op->d_diag_generic, op->diag,
-                 op->d_diag, op->d_diag_ff, op->n_pull, op->n_lits, op->nwords, T.vec_chunk};
+    TileParams P = tile_params(op, T.vec_chunk);
     const int block = 256, nw = block / 32;
     const int64_t ntiles = (P.B.n + 31) / 32;
     if (R == 1) {
         // several waves of blocks: measured faster than one wave for the single-vector kernel
-        const size_t smem = term_smem(op) + (size_t)nw * (512 + (size_t)(op->n_pull + 31) / 32 * 128);
+        const size_t smem = term_smem(op) + (size_t)nw * (4 * kSpinWords + (size_t)(op->tile.n + 31) / 32 * 128);
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1049,9 +1246,9 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
             k<<<grid, block, smem, st>>>(P, lk, (const float*)x, (float*)y, accumulate);
         }
     } else {
-        const int cap = (std::max(T.list_cap, op->n_pull + 1) + 7) & ~7;  // a row: diagonal + terms, padded to 8
-        const int n_rounds = (op->n_pull + 31) / 32;
-        const size_t per_warp = 512 + (size_t)n_rounds * 128 + (size_t)cap * 12;
+        const int cap = (std::max(T.list_cap, op->tile.n + 1) + 7) & ~7;  // a row: diagonal + terms, padded to 8
+        const int n_rounds = (op->tile.n + 31) / 32;
+        const size_t per_warp = 4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12;
         const size_t smem = term_smem(op) + (size_t)nw * per_warp;
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "batched apply: %zu bytes of shared memory needed", smem);
         auto go = [&](auto km) -> void {
@@ -1096,6 +1293,7 @@ qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float*
     plan.vec8 = true;
     plan.vec16 = true;
     plan.hash = true;
+    plan.closed = true;
     plan.cache = true;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -1107,14 +1305,14 @@ qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float*
     for (int s = 0; s < n; ++s) {
         qsi_op* op = ops[s];
         if (op->kernel != 1) return fail(QSI_INVALID_ARG, "sector launch needs the tile kernels");
-        plan.hash = plan.hash && op->basis->d_hash && op->tune[1].use_hash;
+        plan.hash = plan.hash && op->basis->d_bins && op->tune[1].use_hash;
+        plan.closed = plan.closed && op->closed;
         plan.cache = plan.cache && op->d_cache_cols;
-        const int cap = (std::max(op->tune[1].list_cap, op->n_pull + 1) + 7) & ~7;  // a row: diagonal + terms
-        const int n_rounds = (op->n_pull + 31) / 32;
-        smem = std::max(smem, term_smem(op) + (size_t)nw * (512 + (size_t)n_rounds * 128 + (size_t)cap * 12));
-        L[s].P = TileParams{op->basis->view(), op->d_pull, op->d_lit_off, op->d_lits, op->d_diag_generic, op->diag,
-                            op->d_diag, op->d_diag_ff, op->n_pull, op->n_lits, op->nwords, op->tune[1].vec_chunk};
-        L[s].H = op->basis->hview();
+        const int cap = (std::max(op->tune[1].list_cap, op->tile.n + 1) + 7) & ~7;  // a row: diagonal + terms
+        const int n_rounds = (op->tile.n + 31) / 32;
+        smem = std::max(smem, term_smem(op) + (size_t)nw * (4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12));
+        L[s].P = tile_params(op, op->tune[1].vec_chunk);
+        L[s].H = op->basis->bview();
         L[s].C = CacheView{op->d_cache_cols, op->d_cache_off};
         L[s].x = X[s];
         L[s].y = Y[s];
@@ -1153,7 +1351,8 @@ qsi_status launch_sectors(const void* d_records, const SectorPlan& plan, int acc
     auto go = [&](auto km) {
         constexpr int KM = decltype(km)::value;
         auto k = plan.cache ? k_apply_sectors<KM, LookupCache>
-                 : plan.hash ? k_apply_sectors<KM, LookupHash>
+                 : plan.hash && plan.closed ? k_apply_sectors<KM, LookupBins<true>>
+                 : plan.hash ? k_apply_sectors<KM, LookupBins<false>>
                              : k_apply_sectors<KM, LookupTable>;
         set_smem(k, plan.smem);
         k<<<plan.grid, 256, plan.smem, st>>>((const SectorLaunch*)d_records, plan.n, accumulate);
@@ -1174,7 +1373,8 @@ qsi_status preload_apply_f64_rows();  // operator.cu: the row-per-thread kernel
 
 qsi_status preload_apply_f64() {
     cudaFuncAttributes a;
-    QSI_CUDA(cudaFuncGetAttributes(&a, k_apply_tile<double, double, LookupHash>));
+    QSI_CUDA(cudaFuncGetAttributes(&a, k_apply_tile<double, double, LookupBins<true>>));
+    QSI_CUDA(cudaFuncGetAttributes(&a, k_apply_tile<double, double, LookupBins<false>>));
     QSI_CUDA(cudaFuncGetAttributes(&a, k_apply_tile<double, double, LookupTable>));
     return preload_apply_f64_rows();
 }
@@ -1186,12 +1386,13 @@ template <class LK>
 static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double* y, int R, const double* fcoef,
                                    int accumulate, cudaStream_t st) {
     const qsi_tuning& T = tmpl->tune[0];
-    TileParams P{tmpl->basis->view(), tmpl->d_pull, tmpl->d_lit_off, tmpl->d_lits, tmpl->d_diag_generic, tmpl->diag,
-                 tmpl->d_diag, tmpl->d_diag_ff, tmpl->n_pull, tmpl->n_lits, tmpl->nwords, 0, fcoef, R};
+    TileParams P = tile_params(tmpl, 0);
+    P.fcoef = fcoef;
+    P.fR = R;
     const int block = 256, nw = block / 32;
     const int64_t ntiles = (P.B.n + 31) / 32;
     if (R == 1) {
-        const size_t smem = term_smem(tmpl) + (size_t)nw * (512 + (size_t)(tmpl->n_pull + 31) / 32 * 128);
+        const size_t smem = term_smem(tmpl) + (size_t)nw * (4 * kSpinWords + (size_t)(tmpl->tile.n + 31) / 32 * 128);
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1201,7 +1402,7 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
         set_smem(k, smem);
         k<<<grid, block, smem, st>>>(P, lk, x, y, accumulate);
     } else if (R <= 8) {  // a few columns: every lane sums all columns of its row
-        const size_t smem = term_smem(tmpl) + (size_t)nw * (512 + (size_t)(tmpl->n_pull + 31) / 32 * 128);
+        const size_t smem = term_smem(tmpl) + (size_t)nw * (4 * kSpinWords + (size_t)(tmpl->tile.n + 31) / 32 * 128);
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1210,9 +1411,9 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
         set_smem(k, smem);
         k<<<grid, block, smem, st>>>(P, lk, x, y, accumulate);
     } else {
-        const int cap = (std::max(tmpl->tune[1].list_cap, tmpl->n_pull + 1) + 7) & ~7;
-        const int n_rounds = (tmpl->n_pull + 31) / 32;
-        const size_t smem = term_smem(tmpl) + (size_t)nw * (512 + (size_t)n_rounds * 128 + (size_t)cap * 12);
+        const int cap = (std::max(tmpl->tune[1].list_cap, tmpl->tile.n + 1) + 7) & ~7;
+        const int n_rounds = (tmpl->tile.n + 31) / 32;
+        const size_t smem = term_smem(tmpl) + (size_t)nw * (4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12);
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "family apply: %zu bytes of shared memory needed", smem);
         auto go = [&](auto km) {
             constexpr int KM = decltype(km)::value;
@@ -1232,8 +1433,11 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
 qsi_status launch_family(qsi_op* tmpl, const double* x, double* y, int R, const double* fcoef, int accumulate,
                          cudaStream_t st) {
     if (R < 1 || R > 128) return fail(QSI_INVALID_ARG, "family apply: %d columns (1..128)", R);
-    if (tmpl->basis->d_hash && tmpl->tune[R > 1].use_hash)
-        return launch_family_lk(tmpl, LookupHash{tmpl->basis->hview()}, x, y, R, fcoef, accumulate, st);
+    if (tmpl->basis->d_bins && tmpl->tune[R > 1].use_hash) {
+        if (tmpl->closed)
+            return launch_family_lk(tmpl, LookupBins<true>{tmpl->basis->bview()}, x, y, R, fcoef, accumulate, st);
+        return launch_family_lk(tmpl, LookupBins<false>{tmpl->basis->bview()}, x, y, R, fcoef, accumulate, st);
+    }
     return launch_family_lk(tmpl, LookupTable{tmpl->basis->view()}, x, y, R, fcoef, accumulate, st);
 }
 
@@ -1244,7 +1448,11 @@ qsi_status launch_apply_tiles(qsi_op* op, const void* x, void* y, int R, int xdt
         return launch_tiles_lk(op, LookupCache{CacheView{op->d_cache_cols, op->d_cache_off}}, x, y, R, xdtype, ydtype,
                                accumulate, st);
     }
-    if (op->basis->d_hash && op->tune[R > 1].use_hash) return launch_tiles_lk(op, LookupHash{op->basis->hview()}, x, y, R, xdtype, ydtype, accumulate, st);
+    if (op->basis->d_bins && op->tune[R > 1].use_hash) {
+        if (op->closed)
+            return launch_tiles_lk(op, LookupBins<true>{op->basis->bview()}, x, y, R, xdtype, ydtype, accumulate, st);
+        return launch_tiles_lk(op, LookupBins<false>{op->basis->bview()}, x, y, R, xdtype, ydtype, accumulate, st);
+    }
     return launch_tiles_lk(op, LookupTable{op->basis->view()}, x, y, R, xdtype, ydtype, accumulate, st);
 }
 
@@ -1261,10 +1469,9 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         if (op->kernel != 1) return fail(QSI_INVALID_ARG, "qsi_op_materialise: the cache serves the tile kernels (kernel 1)");
         cudaStream_t st = op->stream;
         const int64_t ntiles = (op->basis->n + 31) / 32;
-        TileParams P{op->basis->view(), op->d_pull, op->d_lit_off, op->d_lits, op->d_diag_generic, op->diag,
-                     op->d_diag, op->d_diag_ff, op->n_pull, op->n_lits, op->nwords, 0};
+        TileParams P = tile_params(op, 0);
         const int block = 256, nw = block / 32;
-        const int n_rounds = (op->n_pull + 31) / 32;
+        const int n_rounds = (op->tile.n + 31) / 32;
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1290,7 +1497,7 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         if (e == cudaSuccess) e = cudaMallocAsync(&op->d_cache_off, (size_t)(ntiles + 1) * 8, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(width + ntiles, 0, 8, st);
         if (e != cudaSuccess) return fail_partial(e, "tile offsets");
-        const size_t smem_w = term_smem(op) + (size_t)nw * 512;
+        const size_t smem_w = term_smem(op) + (size_t)nw * 4 * kSpinWords;
         set_smem(k_cache_widths, smem_w);
         k_cache_widths<<<grid, block, smem_w, st>>>(P, width);
         size_t tmp_bytes = 0;
@@ -1303,7 +1510,7 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         if (e != cudaSuccess) return fail_partial(e, "tile widths");
         scratch_free();
         const size_t n_entries = (size_t)lines * 32;
-        op->cache_tid_bytes = op->n_pull <= 256 ? 1 : 2;
+        op->cache_tid_bytes = op->tile.n <= 256 ? 1 : 2;
         e = cudaMalloc(&op->d_cache_cols, std::max<size_t>(n_entries, 1) * 4);
         if (e == cudaSuccess) e = cudaMalloc(&op->d_cache_tid, std::max<size_t>(n_entries, 1) * op->cache_tid_bytes);
         if (e != cudaSuccess) {
@@ -1328,15 +1535,16 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         e = cudaMemsetAsync(op->d_cache_cols, 0xFF, n_entries * 4, st);  // the lanes below their tile's width
         if (e == cudaSuccess) e = cudaMemsetAsync(op->d_cache_tid, 0, n_entries * op->cache_tid_bytes, st);
         if (e != cudaSuccess) return drop_cache(e);
-        const size_t smem_f = term_smem(op) + (size_t)nw * (512 + (size_t)n_rounds * 128);
+        const size_t smem_f = term_smem(op) + (size_t)nw * (4 * kSpinWords + (size_t)n_rounds * 128);
         auto fill = [&](auto lk, auto* tids) {
             auto k = k_cache_fill<decltype(lk), std::remove_pointer_t<decltype(tids)>>;
             set_smem(k, smem_f);
             k<<<grid, block, smem_f, st>>>(P, lk, op->d_cache_off, op->d_cache_cols, tids);
         };
-        if (op->basis->d_hash) {
-            if (op->cache_tid_bytes == 1) fill(LookupHash{op->basis->hview()}, (uint8_t*)op->d_cache_tid);
-            else fill(LookupHash{op->basis->hview()}, (uint16_t*)op->d_cache_tid);
+        if (op->basis->d_bins) {
+            const LookupBins<false> lk{op->basis->bview()};
+            if (op->cache_tid_bytes == 1) fill(lk, (uint8_t*)op->d_cache_tid);
+            else fill(lk, (uint16_t*)op->d_cache_tid);
         } else {
             if (op->cache_tid_bytes == 1) fill(LookupTable{op->basis->view()}, (uint8_t*)op->d_cache_tid);
             else fill(LookupTable{op->basis->view()}, (uint16_t*)op->d_cache_tid);

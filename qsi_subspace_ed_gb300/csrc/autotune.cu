@@ -151,7 +151,7 @@ extern "C" qsi_status qsi_op_autotune(qsi_op* op, const void* x, void* y, int32_
         if (s == QSI_OK && (flags & (QSI_TUNE_INDEX | QSI_TUNE_LOOKUP))) {
             qsi_basis* b = op->basis;
             const int b0 = b->bits;
-            const bool can_hash = b->d_hash != nullptr;
+            const bool can_hash = b->d_bins != nullptr;
             const int hash0 = cfg.use_hash && can_hash ? 1 : 0;
             int best_code = 2 * b0 + hash0;
             std::vector<int> codes;

@@ -294,7 +294,7 @@ extern "C" qsi_status qsi_family_member(qsi_family* f, const double* p, qsi_op**
         std::vector<qsi_term> tt(f->terms);
         for (size_t t = 0; t < tt.size(); ++t) tt[t].c = p[f->cls[t]];
         qsi_op* op = nullptr;
-        qsi_status s = qsi_op_create(f->basis, tt.data(), (int32_t)tt.size(), &op);
+        qsi_status s = create_op(f->basis, tt.data(), (int32_t)tt.size(), false, &op);  // its FP64 applies run the template's terms
         if (s != QSI_OK) return s;
         op->fcoef.assign(p, p + f->n_cls);
         cudaError_t e = cudaMalloc(&op->d_fcoef, (size_t)f->n_cls * sizeof(double));

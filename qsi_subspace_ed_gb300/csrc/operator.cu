@@ -30,29 +30,21 @@ __global__ void k_check_sorted(const state2* s, int64_t n, int* bad) {
     }
 }
 
-// bstart[v] = first index whose bucket >= v, for v in [0, nb].
-__global__ void k_fill_buckets(BasisView B, uint32_t* bstart) {
+// tab[v] = [first, end) of the states in bucket v; the table starts zeroed, and each bucket's first and last state
+// write their side of it.
+__global__ void k_fill_buckets(BasisView B, uint2* tab) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    for (; i <= B.n; i += (int64_t)gridDim.x * blockDim.x) {
+    for (; i < B.n; i += (int64_t)gridDim.x * blockDim.x) {
         bool ok;
-        int64_t cur = (i < B.n) ? (int64_t)bucket_of(B, B.states[i].x, B.states[i].y, ok) : (int64_t)B.n_buckets;
-        int64_t prev = (i > 0) ? (int64_t)bucket_of(B, B.states[i - 1].x, B.states[i - 1].y, ok) : -1;
-        for (int64_t v = prev + 1; v <= cur; ++v) bstart[v] = (uint32_t)i;
+        const uint64_t cur = bucket_of(B, B.states[i].x, B.states[i].y, ok);
+        if (i == 0 || bucket_of(B, B.states[i - 1].x, B.states[i - 1].y, ok) != cur) tab[cur].x = (uint32_t)i;
+        if (i + 1 == B.n || bucket_of(B, B.states[i + 1].x, B.states[i + 1].y, ok) != cur) tab[cur].y = (uint32_t)(i + 1);
     }
 }
 
-__global__ void k_fill_u32(uint32_t* p, int64_t n, uint32_t v) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
-}
-
-// Entries of a bucket table of nb buckets: bstart[0 .. nb] rounded up to whole groups of four, plus one group, so
-// that bucket_bounds' 16-byte reads stay inside the allocation.
-size_t bucket_table_entries(uint32_t nb) { return ((size_t)nb + 1 + 3) / 4 * 4 + 4; }
-
 qsi_status build_buckets(qsi_basis* b) {
-    k_fill_buckets<<<grid_for(b->n + 1, 256), 256>>>(b->view(), b->d_bstart);
-    const int64_t pad = (int64_t)bucket_table_entries(b->n_buckets) - ((int64_t)b->n_buckets + 1);
-    k_fill_u32<<<1, 32>>>(b->d_bstart + b->n_buckets + 1, pad, (uint32_t)b->n);
+    QSI_CUDA(cudaMemset(b->d_tab, 0, (size_t)b->n_buckets * sizeof(uint2)));
+    k_fill_buckets<<<grid_for(b->n, 256), 256>>>(b->view(), b->d_tab);
     QSI_CUDA(cudaGetLastError());
     return QSI_OK;
 }
@@ -278,10 +270,10 @@ static qsi_status prune_pull_terms(qsi_basis* b, std::vector<PullTerm>& pull) {
     if (e == cudaSuccess) {
         const size_t smem = (size_t)n * sizeof(int);
         const int grid = grid_for(b->n, 256);
-        if (b->d_hash) {
-            auto k = k_pull_term_hits<LookupHash>;
+        if (b->d_bins) {
+            auto k = k_pull_term_hits<LookupBins<false>>;
             if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            k<<<grid, 256, smem>>>(b->view(), LookupHash{b->hview()}, d_terms, n, d_hit);
+            k<<<grid, 256, smem>>>(b->view(), LookupBins<false>{b->bview()}, d_terms, n, d_hit);
         } else {
             auto k = k_pull_term_hits<LookupTable>;
             if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -345,7 +337,7 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
         b->shift = hb + 1 - bits;
         b->n_buckets = 1u << bits;
         cudaError_t e = cudaMalloc(&b->d_states, (size_t)n * sizeof(state2));
-        if (e == cudaSuccess) e = cudaMalloc(&b->d_bstart, bucket_table_entries(b->n_buckets) * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMalloc(&b->d_tab, (size_t)b->n_buckets * sizeof(uint2));
         if (e != cudaSuccess) {
             qsi_basis_destroy(b);
             return fail(e == cudaErrorMemoryAllocation ? QSI_OOM : QSI_CUDA_ERROR, "qsi_basis_create: %s", cudaGetErrorString(e));
@@ -370,9 +362,7 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
         // hash index for states of at most 96 bits (skipped, not fatal, when it does not fit in memory)
         if (hb < 96) {
             if (build_hash(b) != QSI_OK) {
-                if (b->d_hash) cudaFree(b->d_hash);
-                b->d_hash = nullptr;
-                b->hash_slots = 0;
+                drop_hash(b);
                 cudaGetLastError();
             }
         }
@@ -384,8 +374,8 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
 extern "C" qsi_status qsi_basis_destroy(qsi_basis* b) {
     if (!b) return QSI_OK;
     if (b->d_states) cudaFree(b->d_states);
-    if (b->d_bstart) cudaFree(b->d_bstart);
-    if (b->d_hash) cudaFree(b->d_hash);
+    if (b->d_tab) cudaFree(b->d_tab);
+    if (b->d_bins) cudaFree(b->d_bins);
     delete b;
     return QSI_OK;
 }
@@ -426,6 +416,10 @@ extern "C" qsi_status qsi_basis_search(qsi_basis* b, const uint64_t* states_lohi
 
 // ------------------------------------------------------------------ C-ABI: operator
 extern "C" qsi_status qsi_op_create(qsi_basis* b, const qsi_term* terms, int32_t n_terms, qsi_op** out) {
+    return create_op(b, terms, n_terms, true, out);
+}
+
+qsi_status qsi::create_op(qsi_basis* b, const qsi_term* terms, int32_t n_terms, bool check_closed, qsi_op** out) {
     return guarded([&]() -> qsi_status {
         if (!b || !out || n_terms < 0 || (n_terms > 0 && !terms)) return fail(QSI_INVALID_ARG, "qsi_op_create: bad argument");
         auto* op = new qsi_op();
@@ -545,33 +539,17 @@ extern "C" qsi_status qsi_op_create(qsi_basis* b, const qsi_term* terms, int32_t
             return fail(QSI_INVALID_ARG, "qsi_op_create: %zu terms exceed the shared-memory term table", pull.size());
         }
         op->smem_bytes = smem;
-        // literal lists for the bit-sliced admission test
-        std::vector<uint16_t> lit_off{0};
-        std::vector<uint8_t> lits;
         int maxbit = b->hb;
-        for (const PullTerm& t : pull) {
-            const uint64_t um[2] = {t.up0, t.up1}, dm[2] = {t.dn0, t.dn1}, xm[2] = {t.x0, t.x1};
+        for (const PullTerm& t : pull)
             for (int w = 0; w < 2; ++w) {
-                for (int bit = 0; bit < 64; ++bit) {
-                    if ((um[w] >> bit) & 1) lits.push_back((uint8_t)(64 * w + bit));
-                    if ((dm[w] >> bit) & 1) lits.push_back((uint8_t)(0x80 | (64 * w + bit)));
-                    if (((um[w] | dm[w] | xm[w]) >> bit) & 1) maxbit = std::max(maxbit, 64 * w + bit);
-                }
+                const uint64_t used = w ? (t.up1 | t.dn1 | t.x1) : (t.up0 | t.dn0 | t.x0);
+                if (used) maxbit = std::max(maxbit, 64 * w + 63 - __builtin_clzll(used));
             }
-            if (lits.size() > 65535) {
-                qsi_op_destroy(op);
-                return fail(QSI_INVALID_ARG, "qsi_op_create: more than 65535 literals in the term list");
-            }
-            lit_off.push_back((uint16_t)lits.size());
-        }
-        op->n_lits = (int)lits.size();
         op->nwords = maxbit / 32 + 1;
-        if (lits.empty()) lits.push_back(0);
-        e = upload((void**)&op->d_lit_off, lit_off.data(), lit_off.size() * 2);
-        if (e == cudaSuccess) e = upload((void**)&op->d_lits, lits.data(), lits.size());
-        if (e != cudaSuccess) {
+        qsi_status us = upload_tile_terms(op, pull);
+        if (us != QSI_OK) {
             qsi_op_destroy(op);
-            return fail(e == cudaErrorMemoryAllocation ? QSI_OOM : QSI_CUDA_ERROR, "qsi_op_create: %s", cudaGetErrorString(e));
+            return us;
         }
         qsi_status ds = build_diag(op);
         if (ds != QSI_OK) {
@@ -579,6 +557,11 @@ extern "C" qsi_status qsi_op_create(qsi_basis* b, const qsi_term* terms, int32_t
             return ds;
         }
         cudaGetDevice(&op->device);
+        if (check_closed) ds = find_closed(op);
+        if (ds != QSI_OK) {
+            qsi_op_destroy(op);
+            return ds;
+        }
         // Device memory that qsi_op_apply_static relies on is reserved here, while allocation is allowed: its
         // staging arrays and the code of the kernels it launches (both are loaded lazily otherwise, at first use).
         // A failure leaves that entry point unavailable on this device and the operator usable.
@@ -597,11 +580,10 @@ extern "C" qsi_status qsi_op_destroy(qsi_op* op) {
     cudaFree(op->d_push_off);
     cudaFree(op->d_push_diag);
     cudaFree(op->d_diag_generic);
-    cudaFree(op->d_lit_off);
+    cudaFree(op->d_tile_terms);
     if (op->d_diag) cudaFreeAsync(op->d_diag, op->stream);
     if (op->d_diag_ff) cudaFreeAsync(op->d_diag_ff, op->stream);
     if (op->stream) cudaStreamSynchronize(op->stream);
-    cudaFree(op->d_lits);
     cudaFree(op->d_x);
     cudaFree(op->d_y);
     cudaFree(op->d_cache_cols);
@@ -813,32 +795,24 @@ extern "C" qsi_status qsi_basis_index(qsi_basis* b, int32_t use_hash, int32_t bu
         if (!b) return fail(QSI_INVALID_ARG, "qsi_basis_index: null basis");
         if (bucket_bits > 0 && bucket_bits != b->bits) {
             int bits = std::min<int>(bucket_bits, std::min(31, b->hb + 1));
-            uint32_t* nb = nullptr;
-            QSI_CUDA(cudaMalloc(&nb, bucket_table_entries(1u << bits) * sizeof(uint32_t)));
-            cudaFree(b->d_bstart);
-            b->d_bstart = nb;
+            uint2* nt = nullptr;
+            QSI_CUDA(cudaMalloc(&nt, ((size_t)1 << bits) * sizeof(uint2)));
+            cudaFree(b->d_tab);
+            b->d_tab = nt;
             b->bits = bits;
             b->shift = b->hb + 1 - bits;
             b->n_buckets = 1u << bits;
             qsi_status bs = build_buckets(b);
             if (bs != QSI_OK) return bs;
             QSI_CUDA(cudaDeviceSynchronize());
-            if (b->d_hash) {  // the hash's regions are the table's buckets
-                if (!use_hash) {
-                    cudaFree(b->d_hash);
-                    b->d_hash = nullptr;
-                    b->hash_slots = 0;
-                    return QSI_OK;
-                }
-                return build_hash(b);
+            if (b->d_bins) {  // the hash's bins are laid out by the table's buckets
+                if (use_hash) return build_hash(b);
+                drop_hash(b);
+                return QSI_OK;
             }
         }
-        if (use_hash && !b->d_hash) return build_hash(b);
-        if (!use_hash && b->d_hash) {
-            cudaFree(b->d_hash);
-            b->d_hash = nullptr;
-            b->hash_slots = 0;
-        }
+        if (use_hash && !b->d_bins) return build_hash(b);
+        if (!use_hash) drop_hash(b);
         return QSI_OK;
     });
 }
@@ -846,10 +820,9 @@ extern "C" qsi_status qsi_basis_index(qsi_basis* b, int32_t use_hash, int32_t bu
 extern "C" qsi_status qsi_basis_info(const qsi_basis* b, int32_t* bucket_bits, int32_t* has_hash, int64_t* index_bytes) {
     if (!b) return fail(QSI_INVALID_ARG, "qsi_basis_info: null basis");
     if (bucket_bits) *bucket_bits = b->bits;
-    if (has_hash) *has_hash = b->d_hash != nullptr;
+    if (has_hash) *has_hash = b->d_bins != nullptr;
     if (index_bytes)
-        *index_bytes = (int64_t)(bucket_table_entries(b->n_buckets) * 4 +
-                                 (b->d_hash ? b->hash_slots * sizeof(HashSlot) : 0));
+        *index_bytes = (int64_t)b->n_buckets * 8 + (b->d_bins ? (int64_t)b->n_bins * kBinSlots * 4 : 0);
     return QSI_OK;
 }
 

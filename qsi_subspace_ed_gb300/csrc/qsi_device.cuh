@@ -32,6 +32,22 @@ struct PushTerm {
     int32_t pad;
 };
 
+// The off-diagonal terms as the tile kernels stage them in shared memory.  Two consecutive terms with the same flip, Z
+// mask and coefficient and opposite requirements (an operator and its conjugate) are one entry with its pair bit set:
+// a row admits at most one of the two, so its hits and their order are those of the separate terms, at half the
+// admission tests.  Literals are spin + 128 when the spin must be down.
+struct TileTerms {
+    const uint4* x;           // flipped bits, four words
+    const double* cs;         // coefficient, and as a (hi, lo) float pair
+    const float2* ff;
+    const ulonglong2* z;      // Z masks (nullptr: no term has one)
+    const uint2* lit8;        // up to eight literals, the last repeated, max_lits of them used (nullptr: lits)
+    const uint32_t* pair;     // pair bits, 32 terms per word
+    const uint16_t* lit_off;  // literal lists of any length, when some term has none or more than eight
+    const uint8_t* lits;
+    int n, n_lits, max_lits;
+};
+
 // Diagonal part: single-site pure-z terms grouped by weight w into masks,
 // contributing w * (2 * popcount(s & M) - popcount(M)); remaining diagonal
 // terms are evaluated one by one.
@@ -45,33 +61,18 @@ struct DiagSpec {
 };
 
 // Sorted basis with a direct bucket table over the top `bits` bits below
-// `shift`: bucket(s) = s >> shift; bstart[v] .. bstart[v+1] is the index
-// range of states in bucket v.
+// `shift`: bucket(s) = s >> shift; tab[v] = [first, end) is the index range of
+// the states in bucket v ({0, 0} for an empty bucket), so one 8-byte load
+// gives a lookup both bounds.
 struct BasisView {
     const state2* states;
-    const uint32_t* bstart;
+    const uint2* tab;
     int64_t n;
     int shift;
     uint32_t n_buckets;
 };
 
-// Slot of the basis hash index (states of at most 96 bits): {low word, high 32 bits, position in the sorted
-// basis}; idx == kEmpty marks a free slot.
-struct HashSlot {
-    uint64_t lo;
-    uint32_t hi;
-    uint32_t idx;
-};
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
-
-__host__ __device__ __forceinline__ uint64_t state_mix(uint64_t lo, uint64_t hi) {
-    uint64_t h = lo * 0x9E3779B97F4A7C15ULL ^ (hi + 0x632BE59BD9B4E019ULL) * 0xC2B2AE3D27D4EB4FULL;
-    h ^= h >> 31;
-    h *= 0xBF58476D1CE4E5B9ULL;
-    h ^= h >> 29;
-    return h;
-}
-
 
 __device__ __forceinline__ bool less128(uint64_t alo, uint64_t ahi, uint64_t blo, uint64_t bhi) {
     return ahi < bhi || (ahi == bhi && alo < blo);
@@ -92,35 +93,17 @@ __device__ __forceinline__ uint64_t bucket_of(const BasisView& B, uint64_t lo, u
     return v;
 }
 
-// Bounds [a, b) of bucket v: one 16-byte load of the aligned group of four table entries holding bstart[v]
-// (the table is 16-byte aligned and padded to a multiple of four entries plus four), a second load only when v is
-// the last of its group.  The apply kernels are bound by the throughput of their uncoalesced loads, so every load
-// saved per lookup counts.
-__device__ __forceinline__ void bucket_bounds(const BasisView& B, uint64_t v, uint32_t& a, uint32_t& b) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(B.bstart + (v & ~3ULL)));
-    switch ((int)(v & 3)) {
-        case 0: a = q.x, b = q.y; break;
-        case 1: a = q.y, b = q.z; break;
-        case 2: a = q.z, b = q.w; break;
-        default: a = q.w, b = __ldg(B.bstart + v + 1); break;
-    }
-}
-
-// Exact index of state (lo, hi) in the basis, or -1.  Lower-bound bisection over the state's bucket; the state at
-// the final position was loaded by the bisection itself whenever that position lies inside the bucket (the last
-// probe that moved the upper end there), and a search that never moved the upper end ends past the bucket, where
-// the state cannot be: no reload either way.
-__device__ __forceinline__ int64_t basis_find(const BasisView& B, uint64_t lo, uint64_t hi) {
-    bool ok;
-    const uint64_t v = bucket_of(B, lo, hi, ok);
-    if (!ok) return -1;
-    uint32_t a, b;
-    bucket_bounds(B, v, a, b);
+// Exact index of state (lo, hi) in [a, b), or -1: lower-bound bisection.  The state at the final position was loaded
+// by the bisection itself whenever that position lies inside the range (the last probe that moved the upper end
+// there), and a search that never moved the upper end ends past the range, where the state cannot be: no reload
+// either way.
+__device__ __forceinline__ int64_t range_find(const state2* __restrict__ states, uint32_t a, uint32_t b, uint64_t lo,
+                                              uint64_t hi) {
     state2 e = make_ulonglong2(0, 0);
     bool seen = false;  // e holds states[b]
     while (a < b) {
-        const uint32_t m = (a + b) >> 1;
-        const state2 t = __ldg(B.states + m);
+        const uint32_t m = a + ((b - a) >> 1);
+        const state2 t = __ldg(states + m);
         if (less128(t.x, t.y, lo, hi)) {
             a = m + 1;
         } else {
@@ -132,122 +115,157 @@ __device__ __forceinline__ int64_t basis_find(const BasisView& B, uint64_t lo, u
     return (seen && e.x == lo && e.y == hi) ? (int64_t)a : -1;
 }
 
-// Regional hash index of the basis: bucket v of the top-bits table owns the slots [2 bstart[v], 2 bstart[v+1])
-// of a table of 2n slots.  A state's probe starts at a hash of the state scaled to its bucket's slots and
-// continues linearly, wrapping inside them.  The regions keep the locality of the sorted basis (the columns of
-// neighbouring rows fall in the same few regions, whose slots stay in L2), and at the fixed load factor of 1/2 a
-// lookup takes about 1.5 probes whatever its bucket's size, where a bisection takes log2 of it (the buckets of
-// spin-ice bases are very uneven: on the 96-spin 12.12.12.12 sector a state's 30-bit bucket holds 18.7 states on
-// average).  One 16-byte load of the table gives the region, as for the bisection.
-struct HashView {
-    const HashSlot* slots;
-    BasisView B;
-};
-
-// First probe of (lo, hi) in a region of cap slots.
-__device__ __forceinline__ uint32_t region_first(uint64_t lo, uint64_t hi, uint64_t cap) {
-    return (uint32_t)(((state_mix(lo, hi) >> 32) * cap) >> 32);
-}
-
-// Region of (lo, hi): its first slot and size (0: the state's bucket is empty or out of range, or the state has
-// more than 96 bits, so it is not in the basis).
-__device__ __forceinline__ uint64_t hash_region(const HashView& Hv, uint64_t lo, uint64_t hi, const HashSlot*& reg) {
-    reg = Hv.slots;
-    if (hi >> 32) return 0;
+// Exact index of state (lo, hi) in the basis, or -1: bisection over the state's bucket.
+__device__ __forceinline__ int64_t basis_find(const BasisView& B, uint64_t lo, uint64_t hi) {
     bool ok;
-    const uint64_t v = bucket_of(Hv.B, lo, hi, ok);
-    if (!ok) return 0;
-    uint32_t a, b;
-    bucket_bounds(Hv.B, v, a, b);
-    reg = Hv.slots + 2 * (uint64_t)a;
-    return 2 * (uint64_t)(b - a);
+    const uint64_t v = bucket_of(B, lo, hi, ok);
+    if (!ok) return -1;
+    const uint2 ab = __ldg(B.tab + v);
+    return range_find(B.states, ab.x, ab.y, lo, hi);
 }
 
-__device__ __forceinline__ bool slot_holds(const uint4& e, uint64_t lo, uint64_t hi) {
-    return e.x == (uint32_t)lo && e.y == (uint32_t)(lo >> 32) && e.z == (uint32_t)hi;
+// Hash index of the basis: a direct-mapped cache of bucket searches in bins of eight 4-byte slots (one 32-byte
+// sector, one load instruction).  The states of a bucket [a, b) share the bins bin_of(a) .. bin_of(b - 1), one bin per
+// 3.2 states of the basis, so neighbouring states' bins are neighbours too; a hash of the state picks its bin and a
+// tag, and its slot holds the tag in the upper bits and the state's offset from a in the lower off_bits.  A lookup is
+// three dependent loads and no loop: the bucket's bounds, its bin, and what it was looked up for.
+//
+// The bins decide nothing alone.  A state that finds its bin full is left out (0.1-0.3% of the states measured), and
+// a state whose tag another state of its bin carries too has both slots marked with offset off_mask (k_bins_check),
+// so for a state of the basis its first match is itself, marked, or absent with a full bin; the last two are settled
+// by bisecting the bucket.  A state outside the basis may match a tag by chance: callers that can meet one compare
+// the state found (kClosed = false).
+//
+// Why bins: a table of 16-byte {state, index} slots with linear probing (load 1/2, 1.5 probes on average) made a
+// warp wait for its unluckiest lane, four to six dependent loads per lookup, and spent 340 warp instructions per 32
+// lookups in hash arithmetic and probe loops; it also took 32 bytes per state where the bins take 10.  FP64 apply of
+// the 64-spin Q=0 basis (2.9 M states): 615 us with that table, 321 with the bins; 96-spin 12.12.12.12 sector (196 M):
+// 69.4 -> 37.1 ms.
+struct BinView {
+    BasisView B;
+    const uint32_t* bins;
+    uint32_t off_mask;
+};
+constexpr int kBinSlots = 8;
+
+__host__ __device__ __forceinline__ uint32_t bin_of(uint32_t i) { return (i >> 2) + (i >> 4); }
+
+// Bin selector (a 32-bit fraction) and tag bits of a state of at most 96 bits: a multilinear hash of its words, its
+// 64-bit sum folded once for the bin and once more for the tag.
+__device__ __forceinline__ void bin_hash(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t& frac, uint32_t& tag) {
+    const uint64_t h = (uint64_t)w0 * 0x9E3779B1u + (uint64_t)w1 * 0x85EBCA6Bu + (uint64_t)w2 * 0xC2B2AE35u;
+    frac = (uint32_t)(h >> 32) * 0x9E3779B1u + (uint32_t)h;
+    tag = (frac ^ (frac >> 15)) * 0x85EBCA6Bu + (uint32_t)h;
+}
+// The tag in a slot's upper bits; the all-ones tag belongs to free slots (kEmpty).
+__device__ __forceinline__ uint32_t slot_tag(uint32_t tag, uint32_t off_mask) {
+    const uint32_t t = tag & ~off_mask;
+    return t == ~off_mask ? 0u : t;
+}
+__device__ __forceinline__ uint32_t pick_bin(uint2 ab, uint32_t frac) {
+    const uint32_t f0 = bin_of(ab.x);
+    return f0 + __umulhi(frac, bin_of(ab.y - 1) - f0 + 1);
+}
+__device__ __forceinline__ void load_bin(const uint32_t* p, uint32_t (&w)[kBinSlots]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(p));
+}
+// Smallest slot ^ tag of a bin: below off_mask it is the offset of the slot that carries the tag (an offset beyond the
+// bucket's size belongs to a neighbouring bucket that shares the bin), off_mask a marked slot, above it no slot
+// carries the tag.
+__device__ __forceinline__ uint32_t bin_match(const uint32_t (&w)[kBinSlots], uint32_t tag) {
+    uint32_t m = w[0] ^ tag;
+#pragma unroll
+    for (int k = 1; k < kBinSlots; ++k) m = min(m, w[k] ^ tag);
+    return m;
 }
 
-// Exact position of (lo, hi) through the hash index, or -1.  A region is never full (load 1/2), so the probes
-// end at a free slot at the latest.
-__device__ __forceinline__ int64_t hash_find(const HashView& Hv, uint64_t lo, uint64_t hi) {
-    const HashSlot* reg;
-    const uint64_t cap = hash_region(Hv, lo, hi, reg);
-    if (!cap) return -1;
-    uint64_t off = region_first(lo, hi, cap);
-    for (uint64_t probe = 0; probe < cap; ++probe) {
-        const uint4 e = __ldg(reinterpret_cast<const uint4*>(reg + off));
-        if (e.w == kEmpty) return -1;
-        if (slot_holds(e, lo, hi)) return (int64_t)e.w;
-        off = (off + 1 == cap) ? 0 : off + 1;
-    }
-    return -1;
+// Column lookups.  Every class takes the admitted rows' states as 32-bit words with the bucket number (see
+// term_words) and returns a candidate index per state, kEmpty when the state is not in the basis; a candidate of a
+// class with kCheck set has to be compared with the state at that index (matches()).  For the materialised
+// operator's cache, cursor(tile, lane) is where the row's entries start, once per tile, and k0 the admission ordinal
+// of the batch's first term.
+struct Word4 {
+    uint32_t w0, w1, w2, w3;  // w3: the bucket number for BinView lookups, bits 96..127 otherwise
+};
+__device__ __forceinline__ Word4 split_state(uint64_t lo, uint64_t hi) {
+    return Word4{(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
 }
 
-// Lookups of up to NB states at once.  The hash variant issues the first
-// probe of every state before resolving any (independent loads in flight);
-// further probes, needed after a collision, follow one by one.
-// Every lookup class takes the states to look up and, for the materialised operator's cache, where the row's
-// entries start (cursor(tile, lane), once per tile) and the admission ordinal of the batch's first term.
 struct LookupTable {
     BasisView B;
     static constexpr int kNB = 4, kMinBlocks = 3;  // lookups per batch per lane, resident 256-thread blocks
+    static constexpr bool kCheck = false;
     __device__ __forceinline__ int64_t find(uint64_t lo, uint64_t hi) const { return basis_find(B, lo, hi); }
+    __device__ __forceinline__ Word4 words(uint64_t lo, uint64_t hi) const { return split_state(lo, hi); }
     __device__ __forceinline__ uint64_t cursor(int64_t, int) const { return 0; }
+    __device__ __forceinline__ bool matches(const Word4&, uint32_t) const { return true; }
     template <int NB>
-    __device__ __forceinline__ void find_batch(const uint64_t* lo, const uint64_t* hi, int64_t* J, int n,
-                                               uint64_t = 0, int = 0) const {
+    __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], uint64_t = 0, int = 0) const {
 #pragma unroll
-        for (int u = 0; u < NB; ++u)
-            if (u < n) J[u] = basis_find(B, lo[u], hi[u]);
+        for (int u = 0; u < NB; ++u) {
+            J[u] = kEmpty;
+            if (u < n)
+                J[u] = (uint32_t)basis_find(B, (uint64_t)s[u].w1 << 32 | s[u].w0, (uint64_t)s[u].w3 << 32 | s[u].w2);
+        }
     }
 };
 
-struct LookupHash {
-    HashView H;
-    // 4 resident blocks (64 registers, a 64-byte spill): 66.9 ms against 74-75 ms at 3 (80 registers) on the
-    // 96-spin sector, whose single-vector apply is bound by the latency of its dependent lookups
-    static constexpr int kNB = 4, kMinBlocks = 4;
-    __device__ __forceinline__ int64_t find(uint64_t lo, uint64_t hi) const { return hash_find(H, lo, hi); }
+// kClosed: every state looked up is in the basis (qsi_op::closed), so a match needs no comparison.  Bucket numbers
+// are linear over XOR, so a row's number XOR a term's is the flipped state's; terms that flip a bit above the basis's
+// highest never land in it and are pruned before they get here.
+template <bool kClosed>
+struct LookupBins {
+    BinView H;
+    // two lookups in flight per lane at 64 registers: 318 us on the 64-spin Q=0 basis, against 397 / 390 / 506 with
+    // one, three or four (the last two spill), and 412 at three resident blocks
+    static constexpr int kNB = 2, kMinBlocks = 4;
+    static constexpr bool kCheck = !kClosed;
+    __device__ __forceinline__ Word4 words(uint64_t lo, uint64_t hi) const {
+        bool ok;
+        Word4 s = split_state(lo, hi);
+        s.w3 = (uint32_t)bucket_of(H.B, lo, hi, ok);
+        return s;
+    }
     __device__ __forceinline__ uint64_t cursor(int64_t, int) const { return 0; }
-    // every state's region (one table load each), then every first probe, before resolving any
+    __device__ __forceinline__ bool matches(const Word4& s, uint32_t J) const {
+        if (kClosed) return true;
+        const uint4 e = __ldg(reinterpret_cast<const uint4*>(H.B.states + J));
+        return e.x == s.w0 && e.y == s.w1 && e.z == s.w2 && e.w == 0;
+    }
     template <int NB>
-    __device__ __forceinline__ void find_batch(const uint64_t* lo, const uint64_t* hi, int64_t* J, int n,
-                                               uint64_t = 0, int = 0) const {
-        const HashSlot* reg[NB];
-        uint32_t cap[NB], off[NB];
-        uint4 e[NB];
+    __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], uint64_t = 0, int = 0) const {
+        uint2 ab[NB];
+#pragma unroll
+        for (int u = 0; u < NB; ++u) ab[u] = (u < n) ? __ldg(H.B.tab + s[u].w3) : make_uint2(0, 0);
+        uint32_t w[NB][kBinSlots], tag[NB];
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
-            cap[u] = 0;
-            reg[u] = H.slots;
-            if (u < n) cap[u] = (uint32_t)hash_region(H, lo[u], hi[u], reg[u]);
+            uint32_t frac;
+            bin_hash(s[u].w0, s[u].w1, s[u].w2, frac, tag[u]);
+            tag[u] = slot_tag(tag[u], H.off_mask);
+            if (ab[u].x != ab[u].y) load_bin(H.bins + (size_t)pick_bin(ab[u], frac) * kBinSlots, w[u]);
         }
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
-            off[u] = 0;
-            e[u] = make_uint4(0, 0, 0, kEmpty);
-            if (cap[u]) {
-                off[u] = region_first(lo[u], hi[u], cap[u]);
-                e[u] = __ldg(reinterpret_cast<const uint4*>(reg[u] + off[u]));
-            }
+            J[u] = kEmpty;
+            if (ab[u].x == ab[u].y) continue;
+            const uint32_t m = bin_match(w[u], tag[u]);
+            if (m < ab[u].y - ab[u].x) J[u] = ab[u].x + m;
+            else if (kClosed || m == H.off_mask || w[u][kBinSlots - 1] != kEmpty)
+                J[u] = (uint32_t)range_find(H.B.states, ab[u].x, ab[u].y, (uint64_t)s[u].w1 << 32 | s[u].w0, s[u].w2);
         }
-#pragma unroll
-        for (int u = 0; u < NB; ++u) {
-            if (u >= n) continue;
-            int64_t r = -1;
-            uint32_t o = off[u];
-            uint4 v = e[u];
-            for (uint32_t probe = 0; probe < cap[u]; ++probe) {
-                if (v.w == kEmpty) break;
-                if (slot_holds(v, lo[u], hi[u])) {
-                    r = (int64_t)v.w;
-                    break;
-                }
-                o = (o + 1 == cap[u]) ? 0 : o + 1;
-                v = __ldg(reinterpret_cast<const uint4*>(reg[u] + o));
-            }
-            J[u] = r;
-        }
+    }
+    // One state of any width.
+    __device__ __forceinline__ int64_t find(uint64_t lo, uint64_t hi) const {
+        bool ok;
+        bucket_of(H.B, lo, hi, ok);
+        if (!ok || (hi >> 32)) return -1;
+        const Word4 s[1] = {words(lo, hi)};
+        uint32_t J[1];
+        find_batch<1>(s, 1, J);
+        return (J[0] != kEmpty && matches(s[0], J[0])) ? (int64_t)J[0] : -1;
     }
 };
 
@@ -265,16 +283,20 @@ struct CacheView {
 struct LookupCache {
     CacheView C;
     static constexpr int kNB = 8, kMinBlocks = 3;
+    static constexpr bool kCheck = false;
+    __device__ __forceinline__ Word4 words(uint64_t, uint64_t) const { return Word4{0, 0, 0, 0}; }
     __device__ __forceinline__ uint64_t cursor(int64_t tile, int lane) const { return C.off[tile] * 32 + lane; }
+    __device__ __forceinline__ bool matches(const Word4&, uint32_t) const { return true; }
     template <int NB>
-    __device__ __forceinline__ void find_batch(const uint64_t*, const uint64_t*, int64_t* J, int n, uint64_t cur,
-                                               int k0) const {
+    __device__ __forceinline__ void find_batch(const Word4 (&)[NB], int n, uint32_t (&J)[NB], uint64_t cur, int k0) const {
 #pragma unroll
-        for (int u = 0; u < NB; ++u)
+        for (int u = 0; u < NB; ++u) {
+            J[u] = kEmpty;
             if (u < n) {
                 const uint32_t c = __ldg(C.cols + cur + (uint64_t)(k0 + u) * 32);
-                J[u] = (c == kEmpty) ? -1 : (int64_t)(c & ~kCacheNeg);
+                J[u] = (c == kEmpty) ? kEmpty : (c & ~kCacheNeg);
             }
+        }
     }
 };
 

@@ -10,12 +10,13 @@ struct qsi_basis {
     int bits = 0, shift = 0;
     uint32_t n_buckets = 0;
     qsi::state2* d_states = nullptr;
-    uint32_t* d_bstart = nullptr;
-    int hb = 0;                        // highest bit used by any state
-    qsi::HashSlot* d_hash = nullptr;   // optional regional hash index over the bucket table (states <= 96 bits)
-    uint64_t hash_slots = 0;           // 2n
-    qsi::BasisView view() const { return qsi::BasisView{d_states, d_bstart, n, shift, n_buckets}; }
-    qsi::HashView hview() const { return qsi::HashView{d_hash, view()}; }
+    uint2* d_tab = nullptr;
+    int hb = 0;                      // highest bit used by any state
+    uint32_t* d_bins = nullptr;      // optional hash index over the bucket table (states <= 96 bits)
+    uint64_t n_bins = 0;
+    uint32_t off_mask = 0;           // offset field of a slot: wide enough for the largest bucket
+    qsi::BasisView view() const { return qsi::BasisView{d_states, d_tab, n, shift, n_buckets}; }
+    qsi::BinView bview() const { return qsi::BinView{view(), d_bins, off_mask}; }
 };
 
 // Launch settings of one class of applies (single vector, batched).  None of them changes results.
@@ -42,10 +43,9 @@ struct qsi_op {
     int n_pull_pruned = 0;                  // transposed terms removed because they map no row into the basis
     qsi::DiagSpec diag{};
     size_t smem_bytes = 0;
-    // bit-sliced admission tests: per pull term, literals (spin | 0x80 when the spin must be down)
-    uint16_t* d_lit_off = nullptr;  // n_pull + 1 offsets
-    uint8_t* d_lits = nullptr;
-    int n_lits = 0;
+    unsigned char* d_tile_terms = nullptr;  // the tile kernels' term tables, one block (see TileTerms)
+    qsi::TileTerms tile{};                  // views into it
+    int closed = 0;                 // every admitted term of every row lands in the basis (find_closed)
     int nwords = 4;                 // 32-bit words that hold any basis or term bit
     int kernel = 1;                 // 0 = row-per-thread / warp-per-row, 1 = bit-sliced tiles
     int ff_accumulate = 1;          // FP32 batched applies accumulate rows in double-float (else FP64)
@@ -79,10 +79,15 @@ qsi_status family_apply(qsi_op* op, const double* x, double* y, int accumulate, 
 // Called by qsi_op_destroy for a family member.
 void family_release_member(qsi_op* op);
 qsi_status build_hash(qsi_basis* b);
+void drop_hash(qsi_basis* b);
+// qsi_op_create; check_closed: determine op->closed (one pass of lookups over the basis), else it stays 0.
+qsi_status create_op(qsi_basis* b, const qsi_term* terms, int32_t n_terms, bool check_closed, qsi_op** out);
+// Builds op->tile from the transposed terms; sets op->closed.
+qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull);
+qsi_status find_closed(qsi_op* op);
 // Builds (enable) or frees an operator's lookup cache (qsi_op_materialise); *bytes: its size in device memory.
 qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes);
-// Bucket table of a basis at its current width (b->bits, b->shift, b->n_buckets), allocated with padding for the
-// 16-byte reads of bucket_bounds.
+// Fills the bucket table of a basis at its current width (b->bits, b->shift, b->n_buckets).
 qsi_status build_buckets(qsi_basis* b);
 // Loads the single-vector FP64 apply kernels on the current device (CUDA loads device code lazily, on first use).
 qsi_status preload_apply_f64();
@@ -97,6 +102,7 @@ struct SectorPlan {
     bool vec8 = true;  // ... of 8 vectors per lane, and every sector's batched applies are set to them
     bool vec16 = true; // ... of 16 vectors per lane, likewise
     bool hash = true;  // every sector's batched applies look columns up through the hash index
+    bool closed = true; // ... and no admitted term leaves any sector's basis
     bool cache = true; // every sector is materialised (qsi_op_materialise): columns come from the lookup caches
 };
 qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float* const* Y, const int* R,

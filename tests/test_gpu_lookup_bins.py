@@ -1,0 +1,102 @@
+"""The bin index and the tile kernels' term tables where they can go wrong: full bins and shared tags (settled by
+bisection), lookups that leave the basis, conjugate pairs stored as one entry, terms without literals, with more than
+eight, and with Z factors.  Every apply against the oracle's push loop and, bitwise, the row-per-thread kernel, which
+shares neither the index nor the tables."""
+import numpy as np
+import pytest
+
+import qsi_subspace_ed_gb300 as q
+from oracle import oracle as O
+from qsi_subspace_ed_gb300 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def opsum(specs):
+    H = q.SymbolicOpSum()
+    for c, s in specs:
+        H.add_term(c, q.SymbolicPMROperator(s))
+    return H
+
+
+def integers(n, lo_shift=0, hi_shift=None):
+    """States 0 .. n-1 with their low ten bits at lo_shift and the others higher (in the high word when given)."""
+    i = np.arange(n, dtype=np.uint64)
+    low, high = (i & np.uint64(1023)) << np.uint64(lo_shift), i >> np.uint64(10)
+    out = np.zeros((n, 2), dtype=np.uint64)
+    out[:, 0] = low if hi_shift is not None else low | (high << np.uint64(lo_shift + 10))
+    if hi_shift is not None:
+        out[:, 1] = high << np.uint64(hi_shift)
+    return out
+
+
+FLIPS = [(0.3 * (k + 1), f"{k}x") for k in range(10)]  # no literals: every row admits them
+MIXED = [(0.7, "0+ 1-"), (0.7, "0- 1+"), (-0.4, "2+ 3- 4z"), (-0.4, "2- 3+ 4z"), (0.2, "5+ 6-"), (0.9, "5- 6+"),
+         (0.1, "0+ 1- 2+ 3- 4+ 5- 6+ 7- 8+ 9-"), (0.1, "0- 1+ 2- 3+ 4- 5+ 6- 7+ 8- 9+"), (0.05, "1z"), (0.6, "7+")]
+PAIRS = [(0.7, "0+ 1-"), (0.7, "0- 1+"), (0.7, "0+ 1-"), (0.2, "2+ 3-"), (0.2, "2- 3+"), (0.5, "4+ 5- 6+ 7- 8+ 9-"),
+         (0.5, "4- 5+ 6- 7+ 8- 9+"), (0.3, "4+ 5- 6+ 7- 8+ 9-")]
+
+
+def check(lohi, H, bits):
+    n = len(lohi)
+    x = np.random.default_rng(3).standard_normal(n)
+    x[::7] = 0.0
+    x[3::11] = 1e-15  # not above the apply tolerance
+    ref = O.apply_port(lohi, H.specs(), x, threads=1)
+    b = q.ZBasis(lohi)
+    op = q.LazyOpSum(b, H)
+    op.set_kernel(0)
+    row = np.zeros(n)
+    op.evaluate(x, row)
+    # one rounding per term and row at most, 18 terms
+    np.testing.assert_allclose(row, ref, rtol=0, atol=40 * 2.3e-16 * max(np.abs(ref).max(), 1.0))
+    X = np.stack([x] * 3, axis=1)
+    for use in (1, 0):
+        for w in bits:
+            b.set_index(use_hash=True, bucket_bits=w)
+            assert b.index_info()["hash"]
+            op.set_kernel(1, use)
+            y = np.full(n, 7.0)
+            op.evaluate(x, y)
+            assert np.array_equal(y, row), (use, w)
+            Y = np.full_like(X, 7.0)
+            op.apply_batched(X, Y)
+            assert all(np.array_equal(Y[:, k], row) for k in range(3)), (use, w)
+            op.materialise(True)
+            y = np.full(n, 7.0)
+            op.evaluate(x, y)
+            assert np.array_equal(y, row), (use, w)
+            op.materialise(False)
+
+
+# 1023, 1024: the last states' flips leave the basis or not; 200,000 states in two buckets: 15-bit tags, shared ones
+# in the thousands of bins, and bins that overflow
+@pytest.mark.parametrize("n,bits", [(1, (1,)), (31, (1, 5)), (1023, (1, 8, 10)), (1024, (1, 8, 10)), (200_000, (1, 9, 18))])
+@pytest.mark.parametrize("terms", ["flips", "mixed", "pairs"])
+@pytest.mark.parametrize("place", [(0, None), (3, None), (0, 0), (0, 21)])
+def test_applies_on_integer_bases(n, bits, terms, place):
+    lo_shift, hi_shift = place
+    if hi_shift == 21 and n < 1024:
+        hi_shift = 0
+    specs = {"flips": FLIPS, "mixed": MIXED, "pairs": PAIRS}[terms]
+    if lo_shift:
+        specs = [(c, " ".join(f"{int(t[:-1]) + lo_shift}{t[-1]}" for t in s.split())) for c, s in specs]
+    check(integers(n, lo_shift, hi_shift), opsum(specs), bits)
+
+
+@pytest.mark.parametrize("pairs", [0, 1, 2])
+def test_applies_on_spinon_bases(pairs):
+    """Closed (no pairs), and hopping whose images leave the basis (one and two pairs)."""
+    lat = workloads.lattice("pyro_1x2x1")
+    g, B = workloads.ring_zeeman_params(5)
+    lohi = q.enumerate_basis(lat, n_spinon_pairs=pairs)
+    check(lohi, q.build_ring_zeeman(lat, g, B, Jpm=0.05 if pairs else 0.0), (4, 14))
+
+
+def test_one_sided_terms():
+    """Rings without their conjugates: a non-symmetric operator, nothing to pair."""
+    lat = workloads.lattice("pyro_1x2x1")
+    H = q.SymbolicOpSum()
+    for k, op in enumerate(q.get_ring_ops(lat)[0]):
+        H.add_term(0.1 * (k + 1), op)
+    check(q.enumerate_basis(lat), H, (6, 14))
