@@ -155,7 +155,7 @@ __device__ __forceinline__ void ff2_fma(FF2& a, uint64_t ch, uint64_t cn, uint64
 
 // Shared-memory layout common to the tile kernels.
 struct TileSmem {
-    uint4* x;           // flipped words; .w as the lookup class wants it
+    uint4* x;           // the terms' flips as the lookup class describes them
     ulonglong2* z;
     double* cs;         // or (hi, lo) float pairs
     uint2* lit8;
@@ -187,9 +187,7 @@ __device__ __forceinline__ TileSmem stage_terms(const TileParams& P, const LK& l
                         (T.lit8 ? (size_t)T.n * 8 + (size_t)(T.n + 31) / 32 * 4 : (size_t)(T.n + 1) * 2 + (size_t)T.n_lits);
     S.tail = smem + ((used + 15) & ~(size_t)15);
     for (int k = threadIdx.x; k < T.n; k += blockDim.x) {
-        const uint4 x = T.x[k];
-        const Word4 w = lk.words((uint64_t)x.y << 32 | x.x, (uint64_t)x.w << 32 | x.z);
-        S.x[k] = make_uint4(w.w0, w.w1, w.w2, w.w3);
+        S.x[k] = lk.term_words(T.x[k]);
         if (T.z) S.z[k] = T.z[k];
         S.cs[k] = ff ? reinterpret_cast<const double*>(T.ff)[k] : T.cs[k];
     }
@@ -218,7 +216,7 @@ __device__ __forceinline__ void tile_spin_words(const state2 s, int nwords, int 
     __syncwarp();
 }
 
-// Admission bits of terms t0..t0+31 for this lane's row (bit j = term t0+j).
+// Rows that admit term t0 + lane (bit l = row l).
 __device__ __forceinline__ uint32_t tile_admitted(const TileSmem& S, const TileTerms& T, int t0, int lane,
                                                   uint32_t vmask, const uint32_t* spinw) {
     const int t = t0 + lane;
@@ -242,7 +240,7 @@ __device__ __forceinline__ uint32_t tile_admitted(const TileSmem& S, const TileT
             for (int k = S.off[t]; k < e; ++k) A &= spinw[S.lit[k]];
         }
     }
-    return warp_transpose32(A, lane);
+    return A;
 }
 
 // Whether term t's matrix element on state s carries a minus sign from its Z mask.
@@ -256,28 +254,156 @@ __device__ __forceinline__ double term_coeff(const TileSmem& S, bool has_z, uint
     return term_negative(S, has_z, t, s) ? -cs : cs;
 }
 
-// The next up to NB admitted terms of this lane's row, in term order across the 32-term rounds: their numbers and
-// the flipped states.  r, a: the round and what is left of its admission word.
-template <int NB>
-__device__ __forceinline__ int next_hits(const TileSmem& S, const Word4& row, const uint32_t* adm, int lane, int n_rounds,
-                                         int& r, uint32_t& a, uint32_t (&tt)[NB], Word4 (&w)[NB]) {
-    int nh = 0;
-#pragma unroll
-    for (int u = 0; u < NB; ++u) {
-        tt[u] = 0;
-        w[u] = Word4{0, 0, 0, 0};
-        while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
-        if (a) {
-            tt[u] = r * 32 + __ffs(a) - 1;
-            a &= a - 1;
-            const uint4 x = S.x[tt[u]];
-            w[u] = Word4{row.w0 ^ x.x, row.w1 ^ x.y, row.w2 ^ x.z, row.w3 ^ x.w};
-            ++nh;
-        }
-    }
-    return nh;
+// Per-warp scratch in shared memory of the matrix-free kernels, rounds = 32-term rounds:
+//   spin words, then (they are done with once the tile's admission is known) the rows' flippable words and list bases;
+//   adm[rounds * 32]: admission word of row l in round r at r * 32 + l;
+//   ts[rounds * 32]: {rows that admit term t, t's first position in the hit list};
+//   list: the hits of the tile (or of as many of its rows as fit), term by term.
+struct WarpScratch {
+    uint32_t* spinw;
+    Word4* rows;
+    uint32_t* base;
+    uint32_t* adm;
+    uint2* ts;
+    unsigned char* list;
+};
+__host__ __device__ constexpr size_t scratch_bytes(int rounds) { return 4 * kSpinWords + (size_t)rounds * (128 + 256); }
+__device__ __forceinline__ WarpScratch warp_scratch(unsigned char* p, int rounds) {
+    WarpScratch W;
+    W.spinw = reinterpret_cast<uint32_t*>(p);
+    W.rows = reinterpret_cast<Word4*>(p);
+    W.base = reinterpret_cast<uint32_t*>(p + 32 * sizeof(Word4));
+    W.ts = reinterpret_cast<uint2*>(p + 4 * kSpinWords);
+    W.adm = reinterpret_cast<uint32_t*>(W.ts + rounds * 32);
+    W.list = reinterpret_cast<unsigned char*>(W.adm + rounds * 32);
+    return W;
 }
 
+// A hit in the list: its term (an operator's term table holds at most 2,327), its row in the tile and its ordinal
+// among the row's hits.
+__device__ __forceinline__ uint32_t pack_hit(uint32_t t, uint32_t l, uint32_t k) { return t << 19 | l << 14 | k; }
+__device__ __forceinline__ uint32_t hit_term(uint32_t e) { return e >> 19; }
+__device__ __forceinline__ uint32_t hit_row(uint32_t e) { return (e >> 14) & 31; }
+__device__ __forceinline__ uint32_t hit_ordinal(uint32_t e) { return e & 0x3fff; }
+
+// Admission of the tile's rows: fills adm, the rows of ts and rows; returns this lane's number of hits.
+template <class LK>
+__device__ __forceinline__ int tile_admit(const TileSmem& S, const TileParams& P, const LK& lk, const WarpScratch& W,
+                                          const state2 s, int64_t row, int n_rounds, int lane) {
+    const uint32_t vmask = __ballot_sync(0xffffffffu, row < P.B.n);
+    const Word4 words = lk.row_words(row, s);
+    tile_spin_words(s, P.nwords, lane, W.spinw);
+    int cnt = 0;
+    for (int r = 0; r < n_rounds; ++r) {
+        const uint32_t A = tile_admitted(S, P.T, r * 32, lane, vmask, W.spinw);
+        const uint32_t a = warp_transpose32(A, lane);
+        W.ts[r * 32 + lane].x = A;
+        W.adm[r * 32 + lane] = a;
+        cnt += __popc(a);
+    }
+    __syncwarp();
+    W.rows[lane] = words;
+    return cnt;
+}
+
+// Rows [row_start, row_end) whose list slots (per_row each) fit cap, at least one row; *base: this lane's first slot.
+__device__ __forceinline__ int chunk_rows(int row_start, int per_row, int cap, int lane, int& base) {
+    const int c = (lane >= row_start) ? per_row : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    base = incl - c;
+    return 32 - __clz(__ballot_sync(0xffffffffu, lane >= row_start && (incl <= cap || lane == row_start)));
+}
+__device__ __forceinline__ uint32_t row_mask(int row_start, int row_end) {
+    return (0xffffffffu >> (32 - row_end)) & (0xffffffffu << row_start);
+}
+
+// Lists the hits of the rows in mask, term by term and by row inside a term (slot i at list + i * stride), and returns
+// their number.  Neighbouring rows flipped by one term land on neighbouring states, so a warp that takes 32
+// consecutive hits of this order touches 0.49 sectors per load and lane where one hit of each row takes 0.75 (64-spin
+// Q=0 basis), and all its lanes have work, where rows of 10.5 hits on average wait for the tile's longest of 14.3 and
+// the rows outside a chunk for the chunk.  FP32 batched apply, 30.8 M states: R = 64 45.4 -> 38.7 ms, R = 16 23.0 ->
+// 18.1 ms against lookups row by row.
+__device__ __forceinline__ int list_hits(const WarpScratch& W, uint32_t mask, int n_rounds, int lane, int stride) {
+    int total = 0;
+    for (int r = 0; r < n_rounds; ++r) {
+        const int c = __popc(W.ts[r * 32 + lane].x & mask);
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        W.ts[r * 32 + lane].y = (uint32_t)(total + incl - c);
+        total += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    __syncwarp();
+    if ((mask >> lane) & 1) {
+        const uint32_t below = mask & ((1u << lane) - 1);
+        uint32_t k = 0;
+        for (int r = 0; r < n_rounds; ++r)
+            for (uint32_t a = W.adm[r * 32 + lane]; a; a &= a - 1) {
+                const uint32_t t = r * 32 + __ffs(a) - 1;
+                const uint2 p = W.ts[t];
+                *reinterpret_cast<uint32_t*>(W.list + (size_t)(p.y + __popc(p.x & below)) * stride) = pack_hit(t, lane, k++);
+            }
+    }
+    __syncwarp();
+    return total;
+}
+
+// State of row `row` flipped by term t.
+__device__ __forceinline__ state2 flipped_state(const TileParams& P, int64_t row, uint32_t t) {
+    const state2 s = __ldg(P.B.states + row);
+    const uint4 x = __ldg(P.T.x + t);
+    return make_ulonglong2(s.x ^ ((uint64_t)x.y << 32 | x.x), s.y ^ ((uint64_t)x.w << 32 | x.z));
+}
+
+// Looks the list's hits up, NB per lane at a time: f(i, n, hits, indices) with the lane's first slot i and number of
+// hits n <= NB; index kEmpty for a state outside the basis.
+template <int NB, class LK, class F>
+__device__ __forceinline__ void look_up_hits(const TileSmem& S, const TileParams& P, const WarpScratch& W, const LK& lk,
+                                             int64_t tile, int total, int lane, int stride, F&& f) {
+    for (int i0 = lane; i0 < total; i0 += 32 * NB) {
+        uint32_t e[NB], J[NB];
+        Word4 w[NB];
+        int n = 0;
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            e[u] = 0;
+            w[u] = Word4{0, 0, 0, 0};
+            if (i0 + 32 * u < total) {
+                e[u] = *reinterpret_cast<const uint32_t*>(W.list + (size_t)(i0 + 32 * u) * stride);
+                w[u] = flip_words(W.rows[hit_row(e[u])], S.x[hit_term(e[u])]);
+                ++n;
+            }
+        }
+        lk.find_batch(w, n, J, [&](int u) { return flipped_state(P, tile * 32 + hit_row(e[u]), hit_term(e[u])); });
+        f(i0, n, e, J);
+    }
+}
+
+// Calls f(term, slot) for this lane's hits in term order; slot: the hit's position in the list.
+template <class F>
+__device__ __forceinline__ void for_row_hits(const WarpScratch& W, uint32_t mask, int n_rounds, int lane, F&& f) {
+    const uint32_t below = mask & ((1u << lane) - 1);
+    for (int r = 0; r < n_rounds; ++r)
+        for (uint32_t a = W.adm[r * 32 + lane]; a; a &= a - 1) {
+            const uint32_t t = r * 32 + __ffs(a) - 1;
+            const uint2 p = W.ts[t];
+            f(t, p.y + __popc(p.x & below));
+        }
+}
+
+// Single vector: every lane looks its own row's hits up, gathers x and adds, kNB hits at a time in step with the other
+// lanes.  Bound by the L1's data pipe (76% busy), which serves one sector per cycle of the scattered loads, 2.26 per
+// hit, then by latency.  The hit list of the batched kernel below needs a third fewer sectors, but the list's own
+// shared-memory traffic and instructions cost more than that saves where a hit brings one value: 351 us against 282
+// on the 64-spin Q=0 basis.
 template <typename XT, typename YT, class LK, bool kFam = false>
 __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P, LK lk, const XT* __restrict__ x,
                                                                  YT* __restrict__ y, int accumulate) {
@@ -287,39 +413,44 @@ __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P
     const int n_rounds = (P.T.n + 31) >> 5;
     const bool has_z = P.T.z != nullptr;
     uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
-    uint32_t* adm = spinw + kSpinWords;  // admission words of the tile, one per lane and 32-term round
+    uint32_t* adm = spinw + kSpinWords;
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
+        const Word4 rw = lk.row_words(row, s);
+        double acc = valid ? (kFam ? fam_diag(P, s.x, s.y, 0) : P.diag[row]) * (double)x[row] : 0.0;
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
-        double acc = valid ? (kFam ? fam_diag(P, s.x, s.y, 0) : P.diag[row]) * (double)x[row] : 0.0;
-        const uint64_t cur = lk.cursor(tile, lane);
-        const Word4 rw = lk.words(s.x, s.y);
-        int kk = 0;  // admitted terms of this row looked up so far
+        int cnt = 0;
+        for (int r = 0; r < n_rounds; ++r) {
+            const uint32_t a = warp_transpose32(tile_admitted(S, P.T, r * 32, lane, vmask, spinw), lane);
+            adm[r * 32 + lane] = a;
+            cnt += __popc(a);
+        }
+        const int width = __reduce_max_sync(0xffffffffu, cnt);
         int r = 0;
         uint32_t a = n_rounds ? adm[lane] : 0;
-        while (true) {
-            // up to kNB admitted terms at a time (across rounds): lookups and gathers in flight together,
-            // contributions added in term order
+        for (int k0 = 0; k0 < width; k0 += LK::kNB) {  // up to kNB hits of every row, summed in term order
             constexpr int kNB = LK::kNB;
             uint32_t tt[kNB], J[kNB];
             Word4 w[kNB];
-            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
-            if (!nh) break;
-            lk.find_batch(w, nh, J, cur, kk);
-            kk += nh;
+#pragma unroll
+            for (int u = 0; u < kNB; ++u) {
+                while (!a && r + 1 < n_rounds) a = adm[++r * 32 + lane];
+                tt[u] = 0;
+                w[u] = rw;
+                if (a) {
+                    tt[u] = r * 32 + 31 - __clz(a & -a);
+                    a &= a - 1;
+                    w[u] = flip_words(rw, S.x[tt[u]]);
+                }
+            }
+            lk.find_batch(w, min(max(cnt - k0, 0), kNB), J, [&](int u) { return flipped_state(P, row, tt[u]); });
             XT xv[kNB];
 #pragma unroll
             for (int u = 0; u < kNB; ++u) xv[u] = (J[u] != kEmpty) ? x[J[u]] : (XT)0;
-            if constexpr (LK::kCheck) {
-#pragma unroll
-                for (int u = 0; u < kNB; ++u)
-                    if (J[u] != kEmpty && !lk.matches(w[u], J[u])) xv[u] = (XT)0;  // outside the basis
-            }
 #pragma unroll
             for (int u = 0; u < kNB; ++u)
                 if (above_tol(xv[u])) {
@@ -335,56 +466,58 @@ __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P
     }
 }
 
-// Family mode with a few columns (FP64 [row][R], 2 <= R <= RC): the single-vector tile kernel with each lane
-// summing all R columns of its row, the R values of a hit gathered from one place.  Each column's sum is the one
-// k_apply_tile forms for that column alone (same terms in the same order, same coefficients and tests), so a
-// member's result does not depend on the batch it ran in.
+// Family mode with a few columns (FP64 [row][R], 2 <= R <= RC): as the single-vector tile kernel, with the hits'
+// columns left in the list and each lane summing all R columns of its row, the R values of a hit gathered from one
+// place.  Each column's sum is the one k_apply_tile forms for that column alone (same terms in the same order, same
+// coefficients and tests), so a member's result does not depend on the batch it ran in.
 template <class LK, int RC>
 __global__ void __launch_bounds__(256, RC <= 4 ? 4 : 2) k_apply_tile_cols(TileParams P, LK lk, const double* __restrict__ x,
-                                                            double* __restrict__ y, int accumulate) {
+                                                            double* __restrict__ y, int accumulate, int cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
     const bool has_z = P.T.z != nullptr;
     const int R = P.fR;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
-    uint32_t* adm = spinw + kSpinWords;
+    const WarpScratch W = warp_scratch(S.tail + wid * (scratch_bytes(n_rounds) + (size_t)cap * 4), n_rounds);
+    uint32_t* js = reinterpret_cast<uint32_t*>(W.list);
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
-        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-        tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
         double acc[RC];
 #pragma unroll
         for (int c = 0; c < RC; ++c) acc[c] = (valid && c < R) ? fam_diag(P, s.x, s.y, c) * x[row * R + c] : 0.0;
-        const uint64_t cur = lk.cursor(tile, lane);
-        const Word4 rw = lk.words(s.x, s.y);
-        int kk = 0, r = 0;
-        uint32_t a = n_rounds ? adm[lane] : 0;
-        while (true) {
-            constexpr int kNB = 4;
-            uint32_t tt[kNB], J[kNB];
-            Word4 w[kNB];
-            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
-            if (!nh) break;
-            lk.find_batch(w, nh, J, cur, kk);
-            kk += nh;
+        const int cnt = tile_admit(S, P, lk, W, s, row, n_rounds, lane);
+        for (int row_start = 0; row_start < 32;) {
+            int base;
+            const int row_end = chunk_rows(row_start, cnt, cap, lane, base);
+            const uint32_t mask = row_mask(row_start, row_end);
+            const int total = list_hits(W, mask, n_rounds, lane, 4);
+            constexpr int kNB = 2;
+            look_up_hits<kNB>(S, P, W, lk, tile, total, lane, 4,
+                              [&](int i0, int n, const uint32_t (&)[kNB], const uint32_t (&J)[kNB]) {
 #pragma unroll
-            for (int u = 0; u < kNB; ++u) {
-                if (J[u] == kEmpty || !lk.matches(w[u], J[u])) continue;
-                const double cs = term_coeff(S, has_z, tt[u], s);
-                const double* xj = x + (int64_t)J[u] * R;
-                double xv[RC];
+                for (int u = 0; u < kNB; ++u)
+                    if (u < n) js[i0 + 32 * u] = J[u];
+            });
+            __syncwarp();
+            if ((mask >> lane) & 1)
+                for_row_hits(W, mask, n_rounds, lane, [&](uint32_t t, uint32_t slot) {
+                    const uint32_t J = js[slot];
+                    if (J == kEmpty) return;
+                    const double cs = term_coeff(S, has_z, t, s);
+                    const double* xj = x + (int64_t)J * R;
+                    double xv[RC];
 #pragma unroll
-                for (int c = 0; c < RC; ++c) xv[c] = (c < R) ? xj[c] : 0.0;
+                    for (int c = 0; c < RC; ++c) xv[c] = (c < R) ? xj[c] : 0.0;
 #pragma unroll
-                for (int c = 0; c < RC; ++c)
-                    if (c < R && above_tol(xv[c])) acc[c] += fam_coef(P, cs, c) * xv[c];
-            }
+                    for (int c = 0; c < RC; ++c)
+                        if (c < R && above_tol(xv[c])) acc[c] += fam_coef(P, cs, c) * xv[c];
+                });
+            __syncwarp();
+            row_start = row_end;
         }
         if (valid) {
 #pragma unroll
@@ -395,7 +528,6 @@ __global__ void __launch_bounds__(256, RC <= 4 ? 4 : 2) k_apply_tile_cols(TilePa
                 y[row * R + c] = v;
             }
         }
-        __syncwarp();
     }
 }
 
@@ -429,13 +561,15 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
     const bool has_z = P.T.z != nullptr;
-    // per-warp scratch: spin words, admission words (n_rounds*32 u32), hit list
-    unsigned char* mine = S.tail + (size_t)wid * (4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12);
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(mine);
-    uint32_t* adm = spinw + kSpinWords;
-    double* hc = reinterpret_cast<double*>(adm + n_rounds * 32);  // coefficients (8-byte aligned)
-    float2* hcf = reinterpret_cast<float2*>(hc);                   // the same slots as (hi, lo) floats
+    // per-warp scratch, then the rows' slots in row order (coefficients, columns)
+    constexpr bool kCached = std::is_same<LK, LookupCache>::value;
+    unsigned char* mine = S.tail + (size_t)wid * (scratch_bytes(n_rounds) + (size_t)cap * 16);
+    const WarpScratch W = warp_scratch(mine, n_rounds);
+    double* hc = reinterpret_cast<double*>(W.list);  // coefficients (8-byte aligned)
+    float2* hcf = reinterpret_cast<float2*>(hc);     // the same slots as (hi, lo) floats
     uint32_t* hJ = reinterpret_cast<uint32_t*>(hc + cap);
+    WarpScratch WL = W;  // with the hits in list order behind them
+    WL.list = reinterpret_cast<unsigned char*>(hJ + cap);
     // KM == kVec4 / kVec8 (FP32, R accepted by vec4_ok / vec8_ok): 16-byte gathers.  A lane owns VPL = 4 or 8
     // consecutive vectors, lpc lanes cover one column's vectors (up to 32*VPL per pass), and the warp's
     // cpw = 32/lpc lane groups sum cpw rows at once.  Otherwise a lane owns KM vectors and the warp sums one
@@ -453,65 +587,65 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
     for (int64_t tile = block_id * nw + wid; tile < ntiles; tile += n_blocks * nw) {
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
-        const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
-        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-        tile_spin_words(s, P.nwords, lane, spinw);
-        int cnt = 0;
-        for (int r = 0; r < n_rounds; ++r) {
-            const uint32_t a = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
-            adm[r * 32 + lane] = a;
-            cnt += __popc(a);
+        state2 s = make_ulonglong2(0, 0);
+        int cnt = 0, width = 0;
+        uint64_t cur = 0;
+        if constexpr (kCached) {  // the row's entries are read from the cache, misses left out
+            cur = lk.cursor(tile, lane);
+            width = (int)((lk.cursor(tile + 1, lane) - cur) >> 5);
+            for (int k = 0; k < width; ++k) cnt += __ldg(lk.C.cols + cur + (uint64_t)k * 32) != kEmpty;
+            if constexpr (kFam) s = valid ? P.B.states[row] : s;
+        } else {
+            if (valid) s = P.B.states[row];
+            cnt = tile_admit(S, P, lk, W, s, row, n_rounds, lane);
         }
         const int pc = v4 ? cnt + 1 : cnt;  // list slots of this row: (the diagonal,) the hits
         const double d = valid ? P.diag[row] : 0.0;
-        int row_start = 0;
-        while (row_start < 32) {
+        for (int row_start = 0; row_start < 32;) {
             // rows [row_start, row_end) whose slots fit the list (at least one row; cap >= a row's slots)
-            int c = (lane >= row_start) ? pc : 0;
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            const bool in_chunk = lane >= row_start && (incl <= cap || lane == row_start);
-            const uint32_t cm = __ballot_sync(0xffffffffu, in_chunk);
-            const int row_end = 32 - __clz(cm);
-            int base = incl - c;
-            if (in_chunk) {
-                int k = base;
-                if constexpr (v4) {  // the diagonal leads the row's list (gathered like a hit, no tolerance test)
-                    hJ[k] = valid ? (uint32_t)row | kDiagSlot : kEmpty;
-                    hcf[k] = valid ? P.diag_ff[row] : make_float2(0.f, 0.f);
-                    ++k;
+            int base;
+            const int row_end = chunk_rows(row_start, pc, cap, lane, base);
+            const bool in_chunk = lane >= row_start && lane < row_end;
+            if constexpr (v4) {  // the diagonal leads the row's list (gathered like a hit, no tolerance test)
+                if (in_chunk) {
+                    hJ[base] = valid ? (uint32_t)row | kDiagSlot : kEmpty;
+                    hcf[base] = valid ? P.diag_ff[row] : make_float2(0.f, 0.f);
                 }
-                // this row's admitted terms in term order, kNB lookups at a time across the 32-term rounds
-                const uint64_t cur = lk.cursor(tile, lane);
-                const Word4 rw = lk.words(s.x, s.y);
-                int kk = 0;
-                int r = 0;
-                uint32_t a = n_rounds ? adm[lane] : 0;
-                while (true) {
-                    constexpr int kNB = v4 ? 4 : 2;
-                    uint32_t tt[kNB], J[kNB];
-                    Word4 w[kNB];
-                    const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
-                    if (!nh) break;
-                    lk.find_batch(w, nh, J, cur, kk);
-                    kk += nh;
-#pragma unroll
-                    for (int u = 0; u < kNB; ++u) {
-                        if (u >= nh) continue;
-                        hJ[k] = (J[u] != kEmpty && lk.matches(w[u], J[u])) ? J[u] : kEmpty;
-                        if constexpr (kFF) {
-                            const float2 f = reinterpret_cast<const float2*>(S.cs)[tt[u]];
-                            hcf[k] = term_negative(S, has_z, tt[u], s) ? make_float2(-f.x, -f.y) : f;
-                        } else {
-                            hc[k] = term_coeff(S, has_z, tt[u], s);
-                        }
-                        ++k;
+            }
+            auto put = [&](uint32_t slot, uint32_t J, uint32_t t, bool neg) {
+                hJ[slot] = J;
+                if constexpr (kFF) {
+                    const float2 f = reinterpret_cast<const float2*>(S.cs)[t];
+                    hcf[slot] = neg ? make_float2(-f.x, -f.y) : f;
+                } else {
+                    const double c = S.cs[t];
+                    hc[slot] = neg ? -c : c;
+                }
+            };
+            if constexpr (kCached) {
+                if (in_chunk) {
+                    int k = base + (v4 ? 1 : 0);
+                    for (int e = 0; e < width; ++e) {
+                        const uint64_t at = cur + (uint64_t)e * 32;
+                        const uint32_t c = __ldg(lk.C.cols + at);
+                        if (c != kEmpty) put(k++, c & ~kCacheNeg, lk.term(at), c & kCacheNeg);
                     }
                 }
+            } else {
+                W.base[lane] = base + (v4 ? 1 : 0);
+                const int total = list_hits(WL, row_mask(row_start, row_end), n_rounds, lane, 4);
+                constexpr int kNB = v4 ? 4 : 2;
+                look_up_hits<kNB>(S, P, WL, lk, tile, total, lane, 4,
+                                  [&](int, int n, const uint32_t (&e)[kNB], const uint32_t (&J)[kNB]) {
+#pragma unroll
+                    for (int u = 0; u < kNB; ++u) {
+                        if (u >= n) continue;
+                        const uint32_t t = hit_term(e[u]), l = hit_row(e[u]);
+                        bool neg = false;
+                        if (has_z) neg = term_negative(S, true, t, P.B.states[tile * 32 + l]);
+                        put(W.base[l] + hit_ordinal(e[u]), J[u], t, neg);
+                    }
+                });
             }
             __syncwarp();
             if constexpr (kFF) {
@@ -802,31 +936,43 @@ qsi_status build_diag(qsi_op* op) {
 }
 
 // ------------------------------------------------------------------ hash index build
-__global__ void k_largest_bucket(BasisView B, uint32_t* largest) {
-    uint32_t m = 0;
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < B.n_buckets; v += (int64_t)gridDim.x * blockDim.x)
-        m = max(m, B.tab[v].y - B.tab[v].x);
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(largest, m);
+// The keys of the states (of at most 96 bits), by tables of the twelve bytes' keys.
+__global__ void __launch_bounds__(256) k_state_keys(BasisView B, uint2* __restrict__ keys) {
+    __shared__ uint2 part[12][256];
+    for (int e = threadIdx.x; e < 12 * 256; e += blockDim.x) {
+        const int byte = e >> 8;
+        const uint64_t v = (uint64_t)(e & 255) << (8 * (byte & 7));
+        part[byte][e & 255] = byte < 8 ? state_key(v, 0) : state_key(0, v);
+    }
+    __syncthreads();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < B.n; i += (int64_t)gridDim.x * blockDim.x) {
+        const state2 s = B.states[i];
+        uint2 k = make_uint2(0, 0);
+#pragma unroll
+        for (int byte = 0; byte < 12; ++byte) {
+            const uint2 p = part[byte][((byte < 8 ? s.x : s.y) >> (8 * (byte & 7))) & 255];
+            k.x ^= p.x;
+            k.y ^= p.y;
+        }
+        keys[i] = k;
+    }
 }
 
-__device__ __forceinline__ uint32_t state_bin(const BinView& H, const state2 s, uint2& ab, uint32_t& tag) {
+__device__ __forceinline__ uint32_t* state_bin(const BinView& H, uint32_t* bins, int64_t i, uint32_t& offset, uint32_t& tag) {
     bool ok;
-    ab = H.B.tab[bucket_of(H.B, s.x, s.y, ok)];
-    uint32_t frac;
-    bin_hash((uint32_t)s.x, (uint32_t)(s.x >> 32), (uint32_t)s.y, frac, tag);
-    tag = slot_tag(tag, H.off_mask);
-    return pick_bin(ab, frac);
+    const uint2 bucket = H.B.tab[bucket_of(H.B, H.B.states[i].x, H.B.states[i].y, ok)], key = H.keys[i];
+    offset = (uint32_t)i - bucket.x;
+    tag = key.y & ~H.off_mask;
+    return bins + (size_t)pick_bin(bucket, key.x, key.y) * kBinSlots;
 }
 
 // Every state takes the first free slot of its bin; a state that finds it full is left out.
 __global__ void k_bins_insert(BinView H, uint32_t* bins) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < H.B.n; i += (int64_t)gridDim.x * blockDim.x) {
-        uint2 ab;
-        uint32_t tag;
-        uint32_t* p = bins + (size_t)state_bin(H, H.B.states[i], ab, tag) * kBinSlots;
+        uint32_t offset, tag;
+        uint32_t* p = state_bin(H, bins, i, offset, tag);
         for (int k = 0; k < kBinSlots; ++k)
-            if (atomicCAS(p + k, kEmpty, tag | ((uint32_t)i - ab.x)) == kEmpty) break;
+            if (atomicCAS(p + k, kEmpty, tag | offset) == kEmpty) break;
     }
 }
 
@@ -834,20 +980,21 @@ __global__ void k_bins_insert(BinView H, uint32_t* bins) {
 // match is itself or a marked slot, or its bin is full and has no match.
 __global__ void k_bins_check(BinView H, uint32_t* bins) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < H.B.n; i += (int64_t)gridDim.x * blockDim.x) {
-        uint2 ab;
-        uint32_t tag, w[kBinSlots];
-        uint32_t* p = bins + (size_t)state_bin(H, H.B.states[i], ab, tag) * kBinSlots;
+        uint32_t offset, tag, w[kBinSlots];
+        uint32_t* p = state_bin(H, bins, i, offset, tag);
         for (int k = 0; k < kBinSlots; ++k) w[k] = *(volatile uint32_t*)(p + k);
         const uint32_t m = bin_match(w, tag);
-        if (m > H.off_mask || m == (uint32_t)i - ab.x) continue;
+        if (m >= H.off_mask || m == offset) continue;
         for (int k = 0; k < kBinSlots; ++k)
-            if ((w[k] ^ tag) <= H.off_mask) atomicOr(p + k, H.off_mask);
+            if (w[k] != kEmpty && (w[k] ^ tag) < H.off_mask) atomicOr(p + k, H.off_mask);
     }
 }
 
 void drop_hash(qsi_basis* b) {
     if (b->d_bins) cudaFree(b->d_bins);
+    if (b->d_keys) cudaFree(b->d_keys);
     b->d_bins = nullptr;
+    b->d_keys = nullptr;
     b->n_bins = 0;
 }
 
@@ -855,20 +1002,19 @@ void drop_hash(qsi_basis* b) {
 qsi_status build_hash(qsi_basis* b) {
     if (b->hb >= 96) return fail(QSI_INVALID_ARG, "hash index needs states of at most 96 bits");
     if (b->n >= ((int64_t)1 << 31)) return fail(QSI_INVALID_ARG, "hash index needs fewer than 2^31 states");
-    const uint64_t n_bins = (uint64_t)bin_of((uint32_t)(b->n - 1)) + 1;
-    if (!b->d_bins || b->n_bins != n_bins) {
-        drop_hash(b);
-        QSI_CUDA(cudaMalloc(&b->d_bins, n_bins * kBinSlots * sizeof(uint32_t)));
-        b->n_bins = n_bins;
-    }
     auto build = [&]() -> qsi_status {
-        uint32_t largest = 0;
-        QSI_CUDA(cudaMemset(b->d_bins, 0, sizeof(uint32_t)));  // the maximum's accumulator, before the bins are cleared
-        k_largest_bucket<<<grid_for(b->n_buckets, 256), 256>>>(b->view(), b->d_bins);
-        QSI_CUDA(cudaMemcpy(&largest, b->d_bins, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+        if (!b->d_keys) {
+            QSI_CUDA(cudaMalloc(&b->d_keys, (size_t)b->n * sizeof(uint2)));
+            k_state_keys<<<std::min(grid_for(b->n, 256), 608), 256>>>(b->view(), b->d_keys);
+        }
+        if (!b->d_bins) {
+            // a bucket's last bin: first_bin(a) + first_bin(m) <= first_bin(n)
+            b->n_bins = (uint64_t)first_bin((uint32_t)b->n) + 1;
+            QSI_CUDA(cudaMalloc(&b->d_bins, b->n_bins * kBinSlots * sizeof(uint32_t)));
+        }
         b->off_mask = 15;
-        while (b->off_mask < largest) b->off_mask = 2 * b->off_mask + 1;
-        QSI_CUDA(cudaMemset(b->d_bins, 0xFF, n_bins * kBinSlots * sizeof(uint32_t)));
+        while (b->off_mask < b->largest_bucket) b->off_mask = 2 * b->off_mask + 1;
+        QSI_CUDA(cudaMemset(b->d_bins, 0xFF, b->n_bins * kBinSlots * sizeof(uint32_t)));
         k_bins_insert<<<grid_for(b->n, 256), 256>>>(b->bview(), b->d_bins);
         k_bins_check<<<grid_for(b->n, 256), 256>>>(b->bview(), b->d_bins);
         QSI_CUDA(cudaGetLastError());
@@ -976,39 +1122,53 @@ qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull) {
 
 // *missed = 1 when an admitted term of some row leaves the basis.
 template <class LK>
-__global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, int* __restrict__ missed) {
+__global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, int* __restrict__ missed, int cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
-    uint32_t* adm = spinw + kSpinWords;
+    const WarpScratch W = warp_scratch(S.tail + wid * (scratch_bytes(n_rounds) + (size_t)cap * 4), n_rounds);
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         if (*(volatile int*)missed) break;
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
-        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-        tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
-        const Word4 rw = lk.words(s.x, s.y);
-        int r = 0;
-        uint32_t a = n_rounds ? adm[lane] : 0;
+        const int cnt = tile_admit(S, P, lk, W, s, row, n_rounds, lane);
         bool miss = false;
-        while (true) {
-            constexpr int kNB = 4;
-            uint32_t tt[kNB], J[kNB];
-            Word4 w[kNB];
-            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
-            if (!nh) break;
-            lk.find_batch(w, nh, J);
+        for (int row_start = 0; row_start < 32;) {
+            int base;
+            const int row_end = chunk_rows(row_start, cnt, cap, lane, base);
+            const int total = list_hits(W, row_mask(row_start, row_end), n_rounds, lane, 4);
+            constexpr int kNB = 2;
+            look_up_hits<kNB>(S, P, W, lk, tile, total, lane, 4,
+                              [&](int, int n, const uint32_t (&)[kNB], const uint32_t (&J)[kNB]) {
 #pragma unroll
-            for (int u = 0; u < kNB; ++u) miss = miss || (u < nh && (J[u] == kEmpty || !lk.matches(w[u], J[u])));
+                for (int u = 0; u < kNB; ++u) miss = miss || (u < n && J[u] == kEmpty);
+            });
+            __syncwarp();
+            row_start = row_end;
         }
         if (miss) *(volatile int*)missed = 1;
-        __syncwarp();
     }
+}
+
+// Block, shared memory and list capacity of a matrix-free tile kernel whose list slots take slot_bytes (0: no list): a
+// list holds want hits or a row of all terms; blocks have eight warps, fewer where a long term list leaves no room.
+struct TileLaunch {
+    int block, cap;
+    size_t smem;
+};
+constexpr int kListCap = 512;
+static TileLaunch tile_launch(const qsi_op* op, size_t slot_bytes, int want) {
+    TileLaunch L;
+    L.cap = (std::max(want, op->tile.n + 1) + 7) & ~7;  // a batched row: the diagonal and every term
+    const int rounds = (op->tile.n + 31) / 32;
+    const size_t per_warp = slot_bytes ? scratch_bytes(rounds) + (size_t)L.cap * slot_bytes : 4 * kSpinWords + (size_t)rounds * 128;
+    for (L.block = 256; L.block > 32; L.block /= 2)
+        if (tile_smem(op->tile) + L.block / 32 * per_warp <= 227 * 1024) break;
+    L.smem = tile_smem(op->tile) + L.block / 32 * per_warp;
+    return L;
 }
 
 // Determines op->closed: with a hash index, one pass of compared lookups (about 0.8 of an apply; a first miss ends it).
@@ -1023,11 +1183,11 @@ qsi_status find_closed(qsi_op* op) {
     QSI_CUDA(cudaMallocAsync(&d_missed, sizeof(int), st));
     cudaError_t e = cudaMemsetAsync(d_missed, 0, sizeof(int), st);
     const int64_t ntiles = (P.B.n + 31) / 32;
-    const size_t smem = tile_smem(P.T) + 8 * (4 * kSpinWords + (size_t)(P.T.n + 31) / 32 * 128);
     const LookupBins<false> lk{op->basis->bview()};
     auto k = k_find_miss<LookupBins<false>>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<grid_for(ntiles, 8), 256, smem, st>>>(P, lk, d_missed);
+    const TileLaunch L = tile_launch(op, 4, kListCap);
+    if (L.smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+    k<<<grid_for(ntiles, L.block / 32), L.block, L.smem, st>>>(P, lk, d_missed, L.cap);
     int missed = 1;
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&missed, d_missed, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -1092,6 +1252,10 @@ __global__ void __launch_bounds__(256) k_apply_cached(const double* __restrict__
     }
 }
 
+static CacheView cache_view(const qsi_op* op) {
+    return CacheView{op->d_cache_cols, op->d_cache_off, op->d_cache_tid, op->cache_tid_bytes};
+}
+
 static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, int ydtype, int accumulate,
                                 cudaStream_t st) {
     const int64_t n = op->basis->n;
@@ -1103,7 +1267,7 @@ static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, 
     const int bps = op->tune[0].grid_bps > 0 ? op->tune[0].grid_bps : 8;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * bps));
     const size_t smem = (size_t)std::max(op->tile.n, 1) * 8;
-    const CacheView C{op->d_cache_cols, op->d_cache_off};
+    const CacheView C = cache_view(op);
     auto go = [&](auto xt, auto yt, auto tt) {
         using XT = decltype(xt);
         using YT = decltype(yt);
@@ -1132,16 +1296,13 @@ __global__ void __launch_bounds__(256) k_cache_widths(TileParams P, uint64_t* __
     const TileSmem S = stage_terms(P, LookupTable{P.B}, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * kSpinWords;
+    const WarpScratch W = warp_scratch(S.tail + wid * scratch_bytes(n_rounds), n_rounds);
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
-        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-        tile_spin_words(s, P.nwords, lane, spinw);
-        int cnt = 0;
-        for (int r = 0; r < n_rounds; ++r) cnt += __popc(tile_admitted(S, P.T, r * 32, lane, vmask, spinw));
+        int cnt = tile_admit(S, P, LookupTable{P.B}, W, s, row, n_rounds, lane);
 #pragma unroll
         for (int o = 16; o; o >>= 1) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, o));
         if (lane == 0) width[tile] = (uint64_t)cnt;
@@ -1153,52 +1314,45 @@ __global__ void __launch_bounds__(256) k_cache_widths(TileParams P, uint64_t* __
 // LookupCache reads them from.
 template <class LK, typename TT>
 __global__ void __launch_bounds__(256) k_cache_fill(TileParams P, LK lk, const uint64_t* __restrict__ off,
-                                                    uint32_t* __restrict__ cols, TT* __restrict__ tids) {
+                                                    uint32_t* __restrict__ cols, TT* __restrict__ tids, int cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
     const bool has_z = P.T.z != nullptr;
-    uint32_t* spinw = reinterpret_cast<uint32_t*>(S.tail) + wid * (kSpinWords + 32 * n_rounds);
-    uint32_t* adm = spinw + kSpinWords;
+    const WarpScratch W = warp_scratch(S.tail + wid * (scratch_bytes(n_rounds) + (size_t)cap * 4), n_rounds);
     const int64_t ntiles = (P.B.n + 31) >> 5;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
-        const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-        tile_spin_words(s, P.nwords, lane, spinw);
-        for (int r = 0; r < n_rounds; ++r) adm[r * 32 + lane] = tile_admitted(S, P.T, r * 32, lane, vmask, spinw);
-        uint32_t* out = cols + off[tile] * 32 + lane;
-        TT* tout = tids + off[tile] * 32 + lane;
-        const Word4 rw = lk.words(s.x, s.y);
-        int kk = 0, r = 0;
-        uint32_t a = n_rounds ? adm[lane] : 0;
-        while (true) {
-            constexpr int kNB = 4;
-            uint32_t tt[kNB], J[kNB];
-            Word4 w[kNB];
-            const int nh = next_hits(S, rw, adm, lane, n_rounds, r, a, tt, w);
-            if (!nh) break;
-            lk.find_batch(w, nh, J);
+        const int cnt = tile_admit(S, P, lk, W, s, row, n_rounds, lane);
+        const uint64_t o0 = off[tile] * 32;
+        for (int row_start = 0; row_start < 32;) {
+            int base;
+            const int row_end = chunk_rows(row_start, cnt, cap, lane, base);
+            const int total = list_hits(W, row_mask(row_start, row_end), n_rounds, lane, 4);
+            constexpr int kNB = 2;
+            look_up_hits<kNB>(S, P, W, lk, tile, total, lane, 4,
+                              [&](int, int n, const uint32_t (&e)[kNB], const uint32_t (&J)[kNB]) {
 #pragma unroll
-            for (int u = 0; u < kNB; ++u)
-                if (u < nh) {
+                for (int u = 0; u < kNB; ++u) {
+                    if (u >= n) continue;
                     // the column, with the sign of the term's matrix element on this row in the top bit
-                    const bool in = J[u] != kEmpty && lk.matches(w[u], J[u]);
-                    out[(uint64_t)(kk + u) * 32] =
-                        in ? (J[u] | (term_negative(S, has_z, tt[u], s) ? kCacheNeg : 0u)) : kEmpty;
-                    tout[(uint64_t)(kk + u) * 32] = (TT)tt[u];
+                    const uint32_t t = hit_term(e[u]), l = hit_row(e[u]);
+                    const bool neg = has_z && term_negative(S, true, t, P.B.states[tile * 32 + l]);
+                    const uint64_t at = o0 + (uint64_t)hit_ordinal(e[u]) * 32 + l;
+                    cols[at] = J[u] != kEmpty ? (J[u] | (neg ? kCacheNeg : 0u)) : kEmpty;
+                    tids[at] = (TT)t;
                 }
-            kk += nh;
+            });
+            __syncwarp();
+            row_start = row_end;
         }
-        __syncwarp();
     }
 }
 
 // ------------------------------------------------------------------ launchers
-static size_t term_smem(const qsi_op* op) { return tile_smem(op->tile); }
-
 template <class K>
 static void set_smem(K kernel, size_t smem) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1217,39 +1371,40 @@ static int one_wave(K kernel, int block, size_t smem, int64_t ntiles, int bps = 
     return (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + block / 32 - 1) / (block / 32), (int64_t)sms * per_sm));
 }
 
+// Grid of the single-vector tile kernels: several waves of blocks measured faster than one.
+static int tile_grid(int64_t ntiles, int block, int bps) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int nw = block / 32;
+    return (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * (bps > 0 ? bps : 8)));
+}
+
 template <class LK>
 static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int R, int xdtype, int ydtype,
                                   int accumulate, cudaStream_t st) {
     const qsi_tuning& T = op->tune[R > 1];
     TileParams P = tile_params(op, T.vec_chunk);
-    const int block = 256, nw = block / 32;
     const int64_t ntiles = (P.B.n + 31) / 32;
     if (R == 1) {
-        // several waves of blocks: measured faster than one wave for the single-vector kernel
-        const size_t smem = term_smem(op) + (size_t)nw * (4 * kSpinWords + (size_t)(op->tile.n + 31) / 32 * 128);
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = (int)std::max<int64_t>(
-            1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * (T.grid_bps > 0 ? T.grid_bps : 8)));
-        if (xdtype == QSI_F64) {
-            auto k = k_apply_tile<double, double, LK>;
-            set_smem(k, smem);
-            k<<<grid, block, smem, st>>>(P, lk, (const double*)x, (double*)y, accumulate);
-        } else if (ydtype == QSI_F64) {
-            auto k = k_apply_tile<float, double, LK>;
-            set_smem(k, smem);
-            k<<<grid, block, smem, st>>>(P, lk, (const float*)x, (double*)y, accumulate);
-        } else {
-            auto k = k_apply_tile<float, float, LK>;
-            set_smem(k, smem);
-            k<<<grid, block, smem, st>>>(P, lk, (const float*)x, (float*)y, accumulate);
+        if constexpr (std::is_same<LK, LookupCache>::value) return fail(QSI_INVALID_ARG, "tile apply: no cached form");
+        else {
+            auto go = [&](auto xt, auto yt) {
+                using XT = decltype(xt);
+                using YT = decltype(yt);
+                auto k = k_apply_tile<XT, YT, LK>;
+                const TileLaunch L = tile_launch(op, 0, 0);
+                set_smem(k, L.smem);
+                k<<<tile_grid(ntiles, L.block, T.grid_bps), L.block, L.smem, st>>>(P, lk, (const XT*)x, (YT*)y, accumulate);
+            };
+            if (xdtype == QSI_F64) go(double{}, double{});
+            else if (ydtype == QSI_F64) go(float{}, double{});
+            else go(float{}, float{});
         }
     } else {
-        const int cap = (std::max(T.list_cap, op->tile.n + 1) + 7) & ~7;  // a row: diagonal + terms, padded to 8
-        const int n_rounds = (op->tile.n + 31) / 32;
-        const size_t per_warp = 4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12;
-        const size_t smem = term_smem(op) + (size_t)nw * per_warp;
+        const TileLaunch L = tile_launch(op, 16, T.list_cap);
+        const int block = L.block, cap = L.cap;
+        const size_t smem = L.smem;
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "batched apply: %zu bytes of shared memory needed", smem);
         auto go = [&](auto km) -> void {
             constexpr int KM = decltype(km)::value;
@@ -1298,7 +1453,9 @@ qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float*
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int nw = 8;
+    int block = 256;  // the largest that every sector's term list leaves room for
+    for (int s = 0; s < n; ++s) block = std::min(block, tile_launch(ops[s], 16, ops[s]->tune[1].list_cap).block);
+    const int nw = block / 32;
     size_t smem = 0;
     int maxR = 1;
     double work_total = 0;
@@ -1308,12 +1465,11 @@ qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float*
         plan.hash = plan.hash && op->basis->d_bins && op->tune[1].use_hash;
         plan.closed = plan.closed && op->closed;
         plan.cache = plan.cache && op->d_cache_cols;
-        const int cap = (std::max(op->tune[1].list_cap, op->tile.n + 1) + 7) & ~7;  // a row: diagonal + terms
-        const int n_rounds = (op->tile.n + 31) / 32;
-        smem = std::max(smem, term_smem(op) + (size_t)nw * (4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12));
+        const int cap = tile_launch(op, 16, op->tune[1].list_cap).cap;
+        smem = std::max(smem, tile_smem(op->tile) + nw * (scratch_bytes((op->tile.n + 31) / 32) + (size_t)cap * 16));
         L[s].P = tile_params(op, op->tune[1].vec_chunk);
         L[s].H = op->basis->bview();
-        L[s].C = CacheView{op->d_cache_cols, op->d_cache_off};
+        L[s].C = cache_view(op);
         L[s].x = X[s];
         L[s].y = Y[s];
         L[s].ycoef = ycoef ? ycoef[s] : nullptr;
@@ -1343,6 +1499,7 @@ qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float*
     plan.smem = smem;
     plan.maxR = maxR;
     plan.grid = begin;
+    plan.block = block;
     plan.n = n;
     return QSI_OK;
 }
@@ -1355,7 +1512,7 @@ qsi_status launch_sectors(const void* d_records, const SectorPlan& plan, int acc
                  : plan.hash ? k_apply_sectors<KM, LookupBins<false>>
                              : k_apply_sectors<KM, LookupTable>;
         set_smem(k, plan.smem);
-        k<<<plan.grid, 256, plan.smem, st>>>((const SectorLaunch*)d_records, plan.n, accumulate);
+        k<<<plan.grid, plan.block, plan.smem, st>>>((const SectorLaunch*)d_records, plan.n, accumulate);
     };
     if (plan.vec16) go(std::integral_constant<int, kVec16>{});
     else if (plan.vec8) go(std::integral_constant<int, kVec8>{});
@@ -1389,31 +1546,21 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
     TileParams P = tile_params(tmpl, 0);
     P.fcoef = fcoef;
     P.fR = R;
-    const int block = 256, nw = block / 32;
     const int64_t ntiles = (P.B.n + 31) / 32;
     if (R == 1) {
-        const size_t smem = term_smem(tmpl) + (size_t)nw * (4 * kSpinWords + (size_t)(tmpl->tile.n + 31) / 32 * 128);
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = (int)std::max<int64_t>(
-            1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * (T.grid_bps > 0 ? T.grid_bps : 8)));
+        const TileLaunch L = tile_launch(tmpl, 0, 0);
         auto k = k_apply_tile<double, double, LK, true>;
-        set_smem(k, smem);
-        k<<<grid, block, smem, st>>>(P, lk, x, y, accumulate);
+        set_smem(k, L.smem);
+        k<<<tile_grid(ntiles, L.block, T.grid_bps), L.block, L.smem, st>>>(P, lk, x, y, accumulate);
     } else if (R <= 8) {  // a few columns: every lane sums all columns of its row
-        const size_t smem = term_smem(tmpl) + (size_t)nw * (4 * kSpinWords + (size_t)(tmpl->tile.n + 31) / 32 * 128);
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * 8));
+        const TileLaunch L = tile_launch(tmpl, 4, kListCap);
         auto k = (R <= 2) ? k_apply_tile_cols<LK, 2> : (R <= 4) ? k_apply_tile_cols<LK, 4> : k_apply_tile_cols<LK, 8>;
-        set_smem(k, smem);
-        k<<<grid, block, smem, st>>>(P, lk, x, y, accumulate);
+        set_smem(k, L.smem);
+        k<<<tile_grid(ntiles, L.block, 0), L.block, L.smem, st>>>(P, lk, x, y, accumulate, L.cap);
     } else {
-        const int cap = (std::max(tmpl->tune[1].list_cap, tmpl->tile.n + 1) + 7) & ~7;
-        const int n_rounds = (tmpl->tile.n + 31) / 32;
-        const size_t smem = term_smem(tmpl) + (size_t)nw * (4 * kSpinWords + (size_t)n_rounds * 128 + (size_t)cap * 12);
+        const TileLaunch L = tile_launch(tmpl, 16, tmpl->tune[1].list_cap);
+        const int block = L.block, cap = L.cap;
+        const size_t smem = L.smem;
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "family apply: %zu bytes of shared memory needed", smem);
         auto go = [&](auto km) {
             constexpr int KM = decltype(km)::value;
@@ -1445,7 +1592,7 @@ qsi_status launch_apply_tiles(qsi_op* op, const void* x, void* y, int R, int xdt
                               cudaStream_t st) {
     if (op->d_cache_cols) {
         if (R == 1) return launch_cached(op, x, y, xdtype, ydtype, accumulate, st);
-        return launch_tiles_lk(op, LookupCache{CacheView{op->d_cache_cols, op->d_cache_off}}, x, y, R, xdtype, ydtype,
+        return launch_tiles_lk(op, LookupCache{cache_view(op)}, x, y, R, xdtype, ydtype,
                                accumulate, st);
     }
     if (op->basis->d_bins && op->tune[R > 1].use_hash) {
@@ -1470,12 +1617,8 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         cudaStream_t st = op->stream;
         const int64_t ntiles = (op->basis->n + 31) / 32;
         TileParams P = tile_params(op, 0);
-        const int block = 256, nw = block / 32;
-        const int n_rounds = (op->tile.n + 31) / 32;
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * 8));
+        const TileLaunch L = tile_launch(op, 4, kListCap);
+        const int grid = tile_grid(ntiles, L.block, 8);
         // widths, their exclusive scan (tile offsets in cache lines), then the columns
         // the scratch arrays are freed, and a failure leaves no partial cache behind, on every path out
         uint64_t* width = nullptr;
@@ -1497,9 +1640,8 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         if (e == cudaSuccess) e = cudaMallocAsync(&op->d_cache_off, (size_t)(ntiles + 1) * 8, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(width + ntiles, 0, 8, st);
         if (e != cudaSuccess) return fail_partial(e, "tile offsets");
-        const size_t smem_w = term_smem(op) + (size_t)nw * 4 * kSpinWords;
-        set_smem(k_cache_widths, smem_w);
-        k_cache_widths<<<grid, block, smem_w, st>>>(P, width);
+        set_smem(k_cache_widths, L.smem);
+        k_cache_widths<<<grid, L.block, L.smem, st>>>(P, width);
         size_t tmp_bytes = 0;
         e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, width, op->d_cache_off, ntiles + 1, st);
         if (e == cudaSuccess) e = cudaMallocAsync(&tmp, tmp_bytes, st);
@@ -1535,11 +1677,10 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         e = cudaMemsetAsync(op->d_cache_cols, 0xFF, n_entries * 4, st);  // the lanes below their tile's width
         if (e == cudaSuccess) e = cudaMemsetAsync(op->d_cache_tid, 0, n_entries * op->cache_tid_bytes, st);
         if (e != cudaSuccess) return drop_cache(e);
-        const size_t smem_f = term_smem(op) + (size_t)nw * (4 * kSpinWords + (size_t)n_rounds * 128);
         auto fill = [&](auto lk, auto* tids) {
             auto k = k_cache_fill<decltype(lk), std::remove_pointer_t<decltype(tids)>>;
-            set_smem(k, smem_f);
-            k<<<grid, block, smem_f, st>>>(P, lk, op->d_cache_off, op->d_cache_cols, tids);
+            set_smem(k, L.smem);
+            k<<<grid, L.block, L.smem, st>>>(P, lk, op->d_cache_off, op->d_cache_cols, tids, L.cap);
         };
         if (op->basis->d_bins) {
             const LookupBins<false> lk{op->basis->bview()};

@@ -30,22 +30,43 @@ __global__ void k_check_sorted(const state2* s, int64_t n, int* bad) {
     }
 }
 
-// tab[v] = [first, end) of the states in bucket v; the table starts zeroed, and each bucket's first and last state
-// write their side of it.
+// tab[v] = {first, size} of the states in bucket v: the table starts zeroed, each bucket's first state writes its
+// index, then each bucket's last state the size.
 __global__ void k_fill_buckets(BasisView B, uint2* tab) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     for (; i < B.n; i += (int64_t)gridDim.x * blockDim.x) {
         bool ok;
         const uint64_t cur = bucket_of(B, B.states[i].x, B.states[i].y, ok);
         if (i == 0 || bucket_of(B, B.states[i - 1].x, B.states[i - 1].y, ok) != cur) tab[cur].x = (uint32_t)i;
-        if (i + 1 == B.n || bucket_of(B, B.states[i + 1].x, B.states[i + 1].y, ok) != cur) tab[cur].y = (uint32_t)(i + 1);
     }
+}
+// ... and the largest bucket.
+__global__ void k_size_buckets(BasisView B, uint2* tab, uint32_t* largest) {
+    uint32_t most = 0;
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (; i < B.n; i += (int64_t)gridDim.x * blockDim.x) {
+        bool ok;
+        const uint64_t cur = bucket_of(B, B.states[i].x, B.states[i].y, ok);
+        if (i + 1 != B.n && bucket_of(B, B.states[i + 1].x, B.states[i + 1].y, ok) == cur) continue;
+        const uint32_t m = (uint32_t)(i + 1) - tab[cur].x;
+        tab[cur].y = m;
+        most = max(most, m);
+    }
+    for (int o = 16; o; o >>= 1) most = max(most, __shfl_down_sync(0xffffffffu, most, o));
+    if ((threadIdx.x & 31) == 0 && most) atomicMax(largest, most);
 }
 
 qsi_status build_buckets(qsi_basis* b) {
-    QSI_CUDA(cudaMemset(b->d_tab, 0, (size_t)b->n_buckets * sizeof(uint2)));
+    uint32_t* d_largest = nullptr;
+    QSI_CUDA(cudaMalloc(&d_largest, sizeof(uint32_t)));
+    cudaError_t e = cudaMemset(d_largest, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(b->d_tab, 0, (size_t)b->n_buckets * sizeof(uint2));
     k_fill_buckets<<<grid_for(b->n, 256), 256>>>(b->view(), b->d_tab);
-    QSI_CUDA(cudaGetLastError());
+    k_size_buckets<<<grid_for(b->n, 256), 256>>>(b->view(), b->d_tab, d_largest);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(&b->largest_bucket, d_largest, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+    cudaFree(d_largest);
+    if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "bucket table: %s", cudaGetErrorString(e));
     return QSI_OK;
 }
 
@@ -230,8 +251,7 @@ __global__ void k_count_connectivity(BasisView B, const PushTerm* __restrict__ o
 // hit[t] = 1 when transposed term t maps some row's state onto a basis state.  A block stops once every term
 // is known to hit (terms that hit usually do so within the first rows); terms that never hit are tested on
 // every row they admit.
-template <class LK>
-__global__ void k_pull_term_hits(BasisView B, LK lk, const PullTerm* __restrict__ terms, int n, int* __restrict__ hit) {
+__global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms, int n, int* __restrict__ hit) {
     extern __shared__ int known[];
     __shared__ int n_known;
     if (threadIdx.x == 0) n_known = 0;
@@ -248,7 +268,7 @@ __global__ void k_pull_term_hits(BasisView B, LK lk, const PullTerm* __restrict_
             if (((volatile int*)known)[t]) continue;
             const PullTerm& T = terms[t];
             const bool ok = ((s.x & T.dn0) | (s.y & T.dn1)) == 0 && (s.x & T.up0) == T.up0 && (s.y & T.up1) == T.up1;
-            if (ok && lk.find(s.x ^ T.x0, s.y ^ T.x1) >= 0 && atomicExch(known + t, 1) == 0) {
+            if (ok && basis_find(B, s.x ^ T.x0, s.y ^ T.x1) >= 0 && atomicExch(known + t, 1) == 0) {
                 atomicAdd(&n_known, 1);
                 hit[t] = 1;
             }
@@ -270,15 +290,9 @@ static qsi_status prune_pull_terms(qsi_basis* b, std::vector<PullTerm>& pull) {
     if (e == cudaSuccess) {
         const size_t smem = (size_t)n * sizeof(int);
         const int grid = grid_for(b->n, 256);
-        if (b->d_bins) {
-            auto k = k_pull_term_hits<LookupBins<false>>;
-            if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            k<<<grid, 256, smem>>>(b->view(), LookupBins<false>{b->bview()}, d_terms, n, d_hit);
-        } else {
-            auto k = k_pull_term_hits<LookupTable>;
-            if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            k<<<grid, 256, smem>>>(b->view(), LookupTable{b->view()}, d_terms, n, d_hit);
-        }
+        auto k = k_pull_term_hits;
+        if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k<<<grid, 256, smem>>>(b->view(), d_terms, n, d_hit);
         e = cudaGetLastError();
     }
     std::vector<int> hit(n, 1);
@@ -329,7 +343,9 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
         if (bits <= 0) {
             int lg = 0;
             while ((1LL << lg) < n) ++lg;
-            bits = std::min(28, std::max(8, lg + 2));
+            // two to four states per bucket on average: wider tables measured the same or slower (64-spin Q=0 basis:
+            // 278 us at 21 bits, 284 at 22, 300 at 24; 96-spin 8.8.16.16: 4.88 ms at 24, 4.83 at 25, 4.89 at 27)
+            bits = std::min(28, std::max(8, lg - 1));
         }
         bits = std::min(bits, std::min(31, hb + 1));
         b->bits = bits;
@@ -376,6 +392,7 @@ extern "C" qsi_status qsi_basis_destroy(qsi_basis* b) {
     if (b->d_states) cudaFree(b->d_states);
     if (b->d_tab) cudaFree(b->d_tab);
     if (b->d_bins) cudaFree(b->d_bins);
+    if (b->d_keys) cudaFree(b->d_keys);
     delete b;
     return QSI_OK;
 }
@@ -822,7 +839,7 @@ extern "C" qsi_status qsi_basis_info(const qsi_basis* b, int32_t* bucket_bits, i
     if (bucket_bits) *bucket_bits = b->bits;
     if (has_hash) *has_hash = b->d_bins != nullptr;
     if (index_bytes)
-        *index_bytes = (int64_t)b->n_buckets * 8 + (b->d_bins ? (int64_t)b->n_bins * kBinSlots * 4 : 0);
+        *index_bytes = (int64_t)b->n_buckets * 8 + (b->d_bins ? (int64_t)b->n_bins * kBinSlots * 4 + b->n * 8 : 0);
     return QSI_OK;
 }
 

@@ -61,7 +61,7 @@ struct DiagSpec {
 };
 
 // Sorted basis with a direct bucket table over the top `bits` bits below
-// `shift`: bucket(s) = s >> shift; tab[v] = [first, end) is the index range of
+// `shift`: bucket(s) = s >> shift; tab[v] = {first, size} is the index range of
 // the states in bucket v ({0, 0} for an empty bucket), so one 8-byte load
 // gives a lookup both bounds.
 struct BasisView {
@@ -120,51 +120,59 @@ __device__ __forceinline__ int64_t basis_find(const BasisView& B, uint64_t lo, u
     bool ok;
     const uint64_t v = bucket_of(B, lo, hi, ok);
     if (!ok) return -1;
-    const uint2 ab = __ldg(B.tab + v);
-    return range_find(B.states, ab.x, ab.y, lo, hi);
+    const uint2 t = __ldg(B.tab + v);
+    return range_find(B.states, t.x, t.x + t.y, lo, hi);
 }
 
 // Hash index of the basis: a direct-mapped cache of bucket searches in bins of eight 4-byte slots (one 32-byte
-// sector, one load instruction).  The states of a bucket [a, b) share the bins bin_of(a) .. bin_of(b - 1), one bin per
-// 3.2 states of the basis, so neighbouring states' bins are neighbours too; a hash of the state picks its bin and a
-// tag, and its slot holds the tag in the upper bits and the state's offset from a in the lower off_bits.  A lookup is
-// three dependent loads and no loop: the bucket's bounds, its bin, and what it was looked up for.
+// sector, one load instruction).  The states of a bucket {a, m} share the bins first_bin(a) .. first_bin(a) +
+// first_bin(m), one bin per two states of the basis, so neighbouring states' bins are neighbours too.  (One per 3.2
+// or 2.7 states leaves more states out, and one lookup in the slow path holds its warp: 5.37 and 5.02 ms against
+// 4.93 for the apply of the 96-spin 8.8.16.16 sector.)  A state's
+// key, a 64-bit hash, picks its bin with the upper word and gives a tag with the lower; its slot holds the tag in the
+// upper bits and the state's offset from a in the lower off_bits.  A lookup is three dependent loads and no loop: the
+// bucket's bounds, its bin, and what it was looked up for.
 //
-// The bins decide nothing alone.  A state that finds its bin full is left out (0.1-0.3% of the states measured), and
+// Keys are linear over XOR (each spin has a 64-bit word, a state's key is the XOR of its up spins'), and so are bucket
+// numbers: the key and the bucket of a flipped state are those of the row XOR those of the term's flips, three XORs per
+// lookup, with the rows' keys stored (8 bytes per state) and the terms' computed when they are staged.
+//
+// The bins decide nothing alone.  A state that finds its bin full is left out (few in a thousand), and
 // a state whose tag another state of its bin carries too has both slots marked with offset off_mask (k_bins_check),
 // so for a state of the basis its first match is itself, marked, or absent with a full bin; the last two are settled
-// by bisecting the bucket.  A state outside the basis may match a tag by chance: callers that can meet one compare
-// the state found (kClosed = false).
+// by bisecting the bucket.  (The all-ones tag meets the free slots' kEmpty as a mark.)  A state outside the basis may
+// match a tag by chance: callers that can meet one compare the state found (kClosed = false).
 //
 // Why bins: a table of 16-byte {state, index} slots with linear probing (load 1/2, 1.5 probes on average) made a
 // warp wait for its unluckiest lane, four to six dependent loads per lookup, and spent 340 warp instructions per 32
-// lookups in hash arithmetic and probe loops; it also took 32 bytes per state where the bins take 10.  FP64 apply of
-// the 64-spin Q=0 basis (2.9 M states): 615 us with that table, 321 with the bins; 96-spin 12.12.12.12 sector (196 M):
-// 69.4 -> 37.1 ms.
+// lookups in hash arithmetic and probe loops.  FP64 apply of the 64-spin Q=0 basis (2.9 M states): 615 us with that
+// table, 321 with bins of a multilinear hash per lookup, 280 with linear keys.
 struct BinView {
     BasisView B;
     const uint32_t* bins;
+    const uint2* keys;  // per state: {bin fraction, tag bits}
     uint32_t off_mask;
 };
 constexpr int kBinSlots = 8;
 
-__host__ __device__ __forceinline__ uint32_t bin_of(uint32_t i) { return (i >> 2) + (i >> 4); }
+__host__ __device__ __forceinline__ uint32_t first_bin(uint32_t i) { return i >> 1; }
 
-// Bin selector (a 32-bit fraction) and tag bits of a state of at most 96 bits: a multilinear hash of its words, its
-// 64-bit sum folded once for the bin and once more for the tag.
-__device__ __forceinline__ void bin_hash(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t& frac, uint32_t& tag) {
-    const uint64_t h = (uint64_t)w0 * 0x9E3779B1u + (uint64_t)w1 * 0x85EBCA6Bu + (uint64_t)w2 * 0xC2B2AE35u;
-    frac = (uint32_t)(h >> 32) * 0x9E3779B1u + (uint32_t)h;
-    tag = (frac ^ (frac >> 15)) * 0x85EBCA6Bu + (uint32_t)h;
+__device__ __forceinline__ uint2 state_key(uint64_t lo, uint64_t hi) {
+    uint64_t k = 0;
+    for (int w = 0; w < 2; ++w)
+        for (uint64_t rest = w ? hi : lo; rest; rest &= rest - 1) {
+            uint64_t z = (uint64_t)(64 * w + __ffsll((long long)rest)) * 0x9E3779B97F4A7C15ULL;  // splitmix64
+            z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+            z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+            k ^= z ^ (z >> 31);
+        }
+    return make_uint2((uint32_t)(k >> 32), (uint32_t)k);
 }
-// The tag in a slot's upper bits; the all-ones tag belongs to free slots (kEmpty).
-__device__ __forceinline__ uint32_t slot_tag(uint32_t tag, uint32_t off_mask) {
-    const uint32_t t = tag & ~off_mask;
-    return t == ~off_mask ? 0u : t;
-}
-__device__ __forceinline__ uint32_t pick_bin(uint2 ab, uint32_t frac) {
-    const uint32_t f0 = bin_of(ab.x);
-    return f0 + __umulhi(frac, bin_of(ab.y - 1) - f0 + 1);
+// The bin of a key: a multiplication breaks the linearity, which would send whole families of states that differ by a
+// few independent flips to one bin (at one bin per 3.2 states, bins of up to 34 states and 1.0% of the 96-spin
+// 8.8.16.16 basis left out instead of 0.4%).
+__device__ __forceinline__ uint32_t pick_bin(uint2 bucket, uint32_t k0, uint32_t k1) {
+    return first_bin(bucket.x) + __umulhi(__umulhi(k0, 0x9E3779B1u) ^ k1, first_bin(bucket.y) + 1);
 }
 __device__ __forceinline__ void load_bin(const uint32_t* p, uint32_t (&w)[kBinSlots]) {
     asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -181,28 +189,25 @@ __device__ __forceinline__ uint32_t bin_match(const uint32_t (&w)[kBinSlots], ui
     return m;
 }
 
-// Column lookups.  Every class takes the admitted rows' states as 32-bit words with the bucket number (see
-// term_words) and returns a candidate index per state, kEmpty when the state is not in the basis; a candidate of a
-// class with kCheck set has to be compared with the state at that index (matches()).  For the materialised
-// operator's cache, cursor(tile, lane) is where the row's entries start, once per tile, and k0 the admission ordinal
-// of the batch's first term.
+// Column lookups.  Every class describes rows and terms by four words whose XOR describes the flipped state, and
+// returns for flipped states an index, kEmpty when the state is not in the basis.  state(u) gives the whole flipped
+// state u where the words do not settle a lookup.
 struct Word4 {
-    uint32_t w0, w1, w2, w3;  // w3: the bucket number for BinView lookups, bits 96..127 otherwise
+    uint32_t w0, w1, w2, w3;
 };
-__device__ __forceinline__ Word4 split_state(uint64_t lo, uint64_t hi) {
-    return Word4{(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
+__device__ __forceinline__ Word4 flip_words(const Word4& a, const uint4& x) {
+    return Word4{a.w0 ^ x.x, a.w1 ^ x.y, a.w2 ^ x.z, a.w3 ^ x.w};
 }
 
 struct LookupTable {
     BasisView B;
     static constexpr int kNB = 4, kMinBlocks = 3;  // lookups per batch per lane, resident 256-thread blocks
-    static constexpr bool kCheck = false;
-    __device__ __forceinline__ int64_t find(uint64_t lo, uint64_t hi) const { return basis_find(B, lo, hi); }
-    __device__ __forceinline__ Word4 words(uint64_t lo, uint64_t hi) const { return split_state(lo, hi); }
-    __device__ __forceinline__ uint64_t cursor(int64_t, int) const { return 0; }
-    __device__ __forceinline__ bool matches(const Word4&, uint32_t) const { return true; }
-    template <int NB>
-    __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], uint64_t = 0, int = 0) const {
+    __device__ __forceinline__ Word4 row_words(int64_t, const state2 s) const {
+        return Word4{(uint32_t)s.x, (uint32_t)(s.x >> 32), (uint32_t)s.y, (uint32_t)(s.y >> 32)};
+    }
+    __device__ __forceinline__ uint4 term_words(const uint4 x) const { return x; }
+    template <int NB, class F>
+    __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], F&&) const {
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
             J[u] = kEmpty;
@@ -212,60 +217,50 @@ struct LookupTable {
     }
 };
 
-// kClosed: every state looked up is in the basis (qsi_op::closed), so a match needs no comparison.  Bucket numbers
-// are linear over XOR, so a row's number XOR a term's is the flipped state's; terms that flip a bit above the basis's
-// highest never land in it and are pruned before they get here.
+// kClosed: every state looked up is in the basis (qsi_op::closed), so a match needs no comparison.  Terms that flip a
+// bit above the basis's highest never land in it and are pruned before they get here.
 template <bool kClosed>
 struct LookupBins {
     BinView H;
-    // two lookups in flight per lane at 64 registers: 318 us on the 64-spin Q=0 basis, against 397 / 390 / 506 with
-    // one, three or four (the last two spill), and 412 at three resident blocks
+    // two lookups in flight per lane at 64 registers: 282 us on the 64-spin Q=0 basis, against 373 with one (at 48
+    // registers), 317 with three and 342 with four at three resident blocks
     static constexpr int kNB = 2, kMinBlocks = 4;
-    static constexpr bool kCheck = !kClosed;
-    __device__ __forceinline__ Word4 words(uint64_t lo, uint64_t hi) const {
+    __device__ __forceinline__ Word4 row_words(int64_t row, const state2 s) const {
         bool ok;
-        Word4 s = split_state(lo, hi);
-        s.w3 = (uint32_t)bucket_of(H.B, lo, hi, ok);
-        return s;
+        const uint2 k = row < H.B.n ? __ldg(H.keys + row) : make_uint2(0, 0);
+        return Word4{(uint32_t)bucket_of(H.B, s.x, s.y, ok), k.x, k.y, 0};
     }
-    __device__ __forceinline__ uint64_t cursor(int64_t, int) const { return 0; }
-    __device__ __forceinline__ bool matches(const Word4& s, uint32_t J) const {
-        if (kClosed) return true;
-        const uint4 e = __ldg(reinterpret_cast<const uint4*>(H.B.states + J));
-        return e.x == s.w0 && e.y == s.w1 && e.z == s.w2 && e.w == 0;
+    __device__ __forceinline__ uint4 term_words(const uint4 x) const {
+        bool ok;
+        const uint64_t lo = (uint64_t)x.y << 32 | x.x, hi = (uint64_t)x.w << 32 | x.z;
+        const uint2 k = state_key(lo, hi);
+        return make_uint4((uint32_t)bucket_of(H.B, lo, hi, ok), k.x, k.y, 0);
     }
-    template <int NB>
-    __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], uint64_t = 0, int = 0) const {
-        uint2 ab[NB];
+    template <int NB, class F>
+    __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], F&& state) const {
+        uint2 bucket[NB];
 #pragma unroll
-        for (int u = 0; u < NB; ++u) ab[u] = (u < n) ? __ldg(H.B.tab + s[u].w3) : make_uint2(0, 0);
-        uint32_t w[NB][kBinSlots], tag[NB];
+        for (int u = 0; u < NB; ++u) bucket[u] = (u < n) ? __ldg(H.B.tab + s[u].w0) : make_uint2(0, 0);
+        uint32_t w[NB][kBinSlots];
 #pragma unroll
-        for (int u = 0; u < NB; ++u) {
-            uint32_t frac;
-            bin_hash(s[u].w0, s[u].w1, s[u].w2, frac, tag[u]);
-            tag[u] = slot_tag(tag[u], H.off_mask);
-            if (ab[u].x != ab[u].y) load_bin(H.bins + (size_t)pick_bin(ab[u], frac) * kBinSlots, w[u]);
-        }
+        for (int u = 0; u < NB; ++u)
+            if (kClosed ? u < n : bucket[u].y != 0) load_bin(H.bins + (size_t)pick_bin(bucket[u], s[u].w1, s[u].w2) * kBinSlots, w[u]);
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
             J[u] = kEmpty;
-            if (ab[u].x == ab[u].y) continue;
-            const uint32_t m = bin_match(w[u], tag[u]);
-            if (m < ab[u].y - ab[u].x) J[u] = ab[u].x + m;
-            else if (kClosed || m == H.off_mask || w[u][kBinSlots - 1] != kEmpty)
-                J[u] = (uint32_t)range_find(H.B.states, ab[u].x, ab[u].y, (uint64_t)s[u].w1 << 32 | s[u].w0, s[u].w2);
+            if (kClosed ? u >= n : bucket[u].y == 0) continue;
+            const uint32_t m = bin_match(w[u], s[u].w2 & ~H.off_mask);
+            if (m < bucket[u].y) {
+                J[u] = bucket[u].x + m;
+                if (!kClosed) {
+                    const state2 t = state(u), e = __ldg(H.B.states + J[u]);
+                    if (e.x != t.x || e.y != t.y) J[u] = kEmpty;
+                }
+            } else if (kClosed || m == H.off_mask || w[u][kBinSlots - 1] != kEmpty) {
+                const state2 t = state(u);
+                J[u] = (uint32_t)range_find(H.B.states, bucket[u].x, bucket[u].x + bucket[u].y, t.x, t.y);
+            }
         }
-    }
-    // One state of any width.
-    __device__ __forceinline__ int64_t find(uint64_t lo, uint64_t hi) const {
-        bool ok;
-        bucket_of(H.B, lo, hi, ok);
-        if (!ok || (hi >> 32)) return -1;
-        const Word4 s[1] = {words(lo, hi)};
-        uint32_t J[1];
-        find_batch<1>(s, 1, J);
-        return (J[0] != kEmpty && matches(s[0], J[0])) ? (int64_t)J[0] : -1;
     }
 };
 
@@ -279,24 +274,15 @@ constexpr uint32_t kCacheNeg = 0x80000000u;
 struct CacheView {
     const uint32_t* cols;
     const uint64_t* off;
+    const void* tids;  // term of every entry: uint8, or uint16 beyond 256 terms
+    int tid_bytes;
 };
 struct LookupCache {
     CacheView C;
-    static constexpr int kNB = 8, kMinBlocks = 3;
-    static constexpr bool kCheck = false;
-    __device__ __forceinline__ Word4 words(uint64_t, uint64_t) const { return Word4{0, 0, 0, 0}; }
+    __device__ __forceinline__ uint4 term_words(const uint4 x) const { return x; }
     __device__ __forceinline__ uint64_t cursor(int64_t tile, int lane) const { return C.off[tile] * 32 + lane; }
-    __device__ __forceinline__ bool matches(const Word4&, uint32_t) const { return true; }
-    template <int NB>
-    __device__ __forceinline__ void find_batch(const Word4 (&)[NB], int n, uint32_t (&J)[NB], uint64_t cur, int k0) const {
-#pragma unroll
-        for (int u = 0; u < NB; ++u) {
-            J[u] = kEmpty;
-            if (u < n) {
-                const uint32_t c = __ldg(C.cols + cur + (uint64_t)(k0 + u) * 32);
-                J[u] = (c == kEmpty) ? kEmpty : (c & ~kCacheNeg);
-            }
-        }
+    __device__ __forceinline__ uint32_t term(uint64_t at) const {
+        return C.tid_bytes == 1 ? __ldg((const uint8_t*)C.tids + at) : __ldg((const uint16_t*)C.tids + at);
     }
 };
 

@@ -14,9 +14,11 @@ struct qsi_basis {
     int hb = 0;                      // highest bit used by any state
     uint32_t* d_bins = nullptr;      // optional hash index over the bucket table (states <= 96 bits)
     uint64_t n_bins = 0;
+    uint2* d_keys = nullptr;         // ... and the states' keys
+    uint32_t largest_bucket = 0;
     uint32_t off_mask = 0;           // offset field of a slot: wide enough for the largest bucket
     qsi::BasisView view() const { return qsi::BasisView{d_states, d_tab, n, shift, n_buckets}; }
-    qsi::BinView bview() const { return qsi::BinView{view(), d_bins, off_mask}; }
+    qsi::BinView bview() const { return qsi::BinView{view(), d_bins, d_keys, off_mask}; }
 };
 
 // Launch settings of one class of applies (single vector, batched).  None of them changes results.
@@ -97,7 +99,7 @@ qsi_status build_diag(qsi_op* op);
 struct SectorPlan {
     std::vector<unsigned char> records;  // one launch record per sector, to be copied to device memory
     size_t smem = 0;
-    int maxR = 1, grid = 0, n = 0;
+    int maxR = 1, grid = 0, block = 256, n = 0;
     bool vec4 = true;  // every sector's R and vectors take 16-byte gathers
     bool vec8 = true;  // ... of 8 vectors per lane, and every sector's batched applies are set to them
     bool vec16 = true; // ... of 16 vectors per lane, likewise
