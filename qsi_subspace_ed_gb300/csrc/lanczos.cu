@@ -353,118 +353,135 @@ __global__ void __launch_bounds__(128) k_ritz_vectors(const VT* __restrict__ V, 
 }
 
 // ------------------------------------------------------------------ small dense symmetric eigensolver
-// Cyclic Jacobi with round-robin pair ordering, one thread block per matrix.
-// A (M x M, row-major, M even, M <= 128) is read from global, diagonalised in
-// shared memory; eigenvalues ascending to evals, eigenvectors as columns of
-// evecs (row-major M x M).  Padding rows/columns of zeros stay decoupled.
+// Cyclic Jacobi, one thread block per matrix: A (M x M, row-major, M even, M <= 128) is diagonalised in shared memory;
+// eigenvalues ascending to evals, eigenvectors as columns of evecs (row-major M x M).  Padding rows/columns of zeros
+// stay decoupled.  A round rotates M/2 disjoint pairs (round-robin order) at once: the angles, then every 2 x 2 block
+// of A from both sides and every row of the eigenvectors (in shared memory when both fit), so a round has two barriers.
+// A pair is left alone when its off-diagonal element is below 1e-17 of the matrix's norm, a rotated one's is set to
+// zero, and a sweep without rotations ends the iteration: 6-8 sweeps.  (A test on the whole off-diagonal mass never
+// passed for elements that are left at rounding size: every call took all 60 sweeps, 5.6 ms for a 24 x 24 matrix
+// against 0.3 ms.)
 __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, int M, double* __restrict__ evals,
-                                                double* __restrict__ evecs, int max_sweeps) {
+                                                double* __restrict__ evecs, int max_sweeps, int v_shared) {
     extern __shared__ double sm[];
-    double* A = sm;                 // M*M
-    double* cs = A + M * M;         // M/2 cosines
-    double* sn = cs + M / 2;        // M/2 sines
-    int* pp = (int*)(sn + M / 2);   // M/2 p indices
-    int* qq = pp + M / 2;           // M/2 q indices
-    int* perm = qq + M / 2;         // M positions
+    const int H = M / 2;
+    double* A = sm;          // M*M
+    double* cs = A + M * M;  // M/2 cosines
+    double* sn = cs + H;     // M/2 sines
+    int* pp = (int*)(sn + H);
+    int* qq = pp + H;
+    double* V = v_shared ? sn + H + H : evecs + (int64_t)blockIdx.x * M * M;  // 2 * H ints take H doubles
     __shared__ double red[32];
-    __shared__ int stop;
+    __shared__ double tau;
     const double* Ab = Ain + (int64_t)blockIdx.x * M * M;
     double* Vb = evecs + (int64_t)blockIdx.x * M * M;
     double* eb = evals + (int64_t)blockIdx.x * M;
+    double nrm = 0.0;
     for (int i = threadIdx.x; i < M * M; i += blockDim.x) {
         A[i] = Ab[i];
-        Vb[i] = (i / M == i % M) ? 1.0 : 0.0;
+        V[i] = (i / M == i % M) ? 1.0 : 0.0;
+        nrm += Ab[i] * Ab[i];
     }
-    for (int i = threadIdx.x; i < M; i += blockDim.x) perm[i] = i;
+    nrm = block_sum(nrm, red);
+    if (threadIdx.x == 0) tau = 1e-17 * sqrt(nrm);
     __syncthreads();
-    const int H = M / 2;
+    const int nblk = H * (H + 1) / 2;  // blocks (t, u), t <= u
     for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-        // convergence: off-diagonal mass relative to total
-        double off = 0.0, tot = 0.0;
-        for (int i = threadIdx.x; i < M * M; i += blockDim.x) {
-            double a = A[i] * A[i];
-            tot += a;
-            if (i / M != i % M) off += a;
-        }
-        double offs = block_sum(off, red);
-        double tots = block_sum(tot, red);
-        if (threadIdx.x == 0) stop = !(offs > 1e-32 * tots) || tots == 0.0;
-        __syncthreads();
-        if (stop) break;
+        int rotated = 0;
         for (int round = 0; round < M - 1; ++round) {
-            for (int t = threadIdx.x; t < H; t += blockDim.x) {
-                int p = perm[t], q = perm[M - 1 - t];
+            int any = 0;
+            if (threadIdx.x < H) {
+                // round-robin: player M-1 stays, the others turn
+                const int t = threadIdx.x;
+                int p = (t == 0) ? M - 1 : (round + t) % (M - 1);
+                int q = (t == 0) ? round : (round + M - 1 - t) % (M - 1);
                 if (p > q) {
-                    int tmp = p;
+                    const int tmp = p;
                     p = q;
                     q = tmp;
                 }
                 pp[t] = p;
                 qq[t] = q;
-                double apq = A[p * M + q];
+                const double apq = A[p * M + q];
                 double c = 1.0, s = 0.0;
-                if (apq != 0.0) {
-                    double theta = (A[q * M + q] - A[p * M + p]) / (2.0 * apq);
-                    double tt = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+                if (fabs(apq) > tau) {
+                    const double theta = (A[q * M + q] - A[p * M + p]) / (2.0 * apq);
+                    const double tt = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
                     c = 1.0 / sqrt(tt * tt + 1.0);
                     s = tt * c;
+                    any = 1;
                 }
                 cs[t] = c;
                 sn[t] = s;
             }
-            __syncthreads();
-            // rows: A <- J^T A
-            for (int idx = threadIdx.x; idx < H * M; idx += blockDim.x) {
-                int t = idx / M, col = idx % M;
-                int p = pp[t], q = qq[t];
-                double c = cs[t], s = sn[t];
-                double ap = A[p * M + col], aq = A[q * M + col];
-                A[p * M + col] = c * ap - s * aq;
-                A[q * M + col] = s * ap + c * aq;
+            any = __syncthreads_or(any);
+            if (!any) continue;
+            rotated = 1;
+            for (int idx = threadIdx.x; idx < nblk; idx += blockDim.x) {
+                // block idx of the upper triangle, row by row from the last
+                const int r = (int)((sqrtf(8.0f * (float)idx + 1.0f) - 1.0f) * 0.5f);
+                int t = r, o = idx - r * (r + 1) / 2;
+                if (o < 0) --t, o = idx - t * (t + 1) / 2;
+                else if (o > t) ++t, o = idx - t * (t + 1) / 2;
+                const int u = t, v = o;  // pairs u >= v
+                const double c1 = cs[v], s1 = sn[v], c2 = cs[u], s2 = sn[u];
+                if (s1 == 0.0 && s2 == 0.0) continue;
+                const int p1 = pp[v], q1 = qq[v], p2 = pp[u], q2 = qq[u];
+                const double app = A[p1 * M + p2], apq = A[p1 * M + q2], aqp = A[q1 * M + p2], aqq = A[q1 * M + q2];
+                // rows p1, q1 then columns p2, q2
+                const double bpp = c1 * app - s1 * aqp, bpq = c1 * apq - s1 * aqq;
+                const double bqp = s1 * app + c1 * aqp, bqq = s1 * apq + c1 * aqq;
+                double dpp = c2 * bpp - s2 * bpq, dpq = s2 * bpp + c2 * bpq;
+                double dqp = c2 * bqp - s2 * bqq, dqq = s2 * bqp + c2 * bqq;
+                if (u == v) dpq = dqp = 0.0;
+                A[p1 * M + p2] = dpp;
+                A[p1 * M + q2] = dpq;
+                A[q1 * M + p2] = dqp;
+                A[q1 * M + q2] = dqq;
+                if (u != v) {
+                    A[p2 * M + p1] = dpp;
+                    A[q2 * M + p1] = dpq;
+                    A[p2 * M + q1] = dqp;
+                    A[q2 * M + q1] = dqq;
+                }
             }
-            __syncthreads();
-            // columns: A <- A J, V <- V J
             for (int idx = threadIdx.x; idx < H * M; idx += blockDim.x) {
-                int t = idx / M, row = idx % M;
-                int p = pp[t], q = qq[t];
-                double c = cs[t], s = sn[t];
-                double ap = A[row * M + p], aq = A[row * M + q];
-                A[row * M + p] = c * ap - s * aq;
-                A[row * M + q] = s * ap + c * aq;
-                double vp = Vb[row * M + p], vq = Vb[row * M + q];
-                Vb[row * M + p] = c * vp - s * vq;
-                Vb[row * M + q] = s * vp + c * vq;
-            }
-            __syncthreads();
-            // rotate positions 1..M-1 (position 0 fixed)
-            if (threadIdx.x == 0) {
-                int last = perm[M - 1];
-                for (int i = M - 1; i > 1; --i) perm[i] = perm[i - 1];
-                perm[1] = last;
+                const int t = idx % H, row = idx / H;
+                const double c = cs[t], s = sn[t];
+                if (s == 0.0) continue;
+                const int p = pp[t], q = qq[t];
+                const double vp = V[row * M + p], vq = V[row * M + q];
+                V[row * M + p] = c * vp - s * vq;
+                V[row * M + q] = s * vp + c * vq;
             }
             __syncthreads();
         }
+        if (!rotated) break;
     }
-    // sort ascending (selection sort by one thread; M <= 128), permute columns
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < M; ++i) perm[i] = i;
-        for (int i = 0; i < M; ++i) {
-            int best = i;
-            for (int j = i + 1; j < M; ++j)
-                if (A[perm[j] * M + perm[j]] < A[perm[best] * M + perm[best]]) best = j;
-            int tmp = perm[i];
-            perm[i] = perm[best];
-            perm[best] = tmp;
+    // ascending order by counting, then the eigenvector columns in that order (row by row through the free A when
+    // they are in place in global memory)
+    int* perm = pp;  // M entries: pp and qq
+    __syncthreads();
+    for (int i = threadIdx.x; i < M; i += blockDim.x) {
+        const double d = A[i * M + i];
+        int rank = 0;
+        for (int j = 0; j < M; ++j) {
+            const double e = A[j * M + j];
+            rank += (e < d || (!(e > d) && j < i)) ? 1 : 0;
         }
+        perm[i] = rank;
+        eb[rank] = d;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < M; i += blockDim.x) eb[i] = A[perm[i] * M + perm[i]];
-    // permute eigenvector columns through shared memory row by row
-    for (int row = 0; row < M; ++row) {
-        __syncthreads();
-        for (int j = threadIdx.x; j < M; j += blockDim.x) A[j] = Vb[row * M + perm[j]];
-        __syncthreads();
-        for (int j = threadIdx.x; j < M; j += blockDim.x) Vb[row * M + j] = A[j];
+    if (v_shared) {
+        for (int i = threadIdx.x; i < M * M; i += blockDim.x) Vb[(i / M) * M + perm[i % M]] = V[i];
+    } else {
+        for (int row = 0; row < M; ++row) {
+            for (int j = threadIdx.x; j < M; j += blockDim.x) A[perm[j]] = V[row * M + j];
+            __syncthreads();
+            for (int j = threadIdx.x; j < M; j += blockDim.x) V[row * M + j] = A[j];
+            __syncthreads();
+        }
     }
 }
 
@@ -495,9 +512,11 @@ qsi_status jacobi_eigh(const std::vector<double>& A, int m, int n_mat, std::vect
     QSI_CUDA(cudaMallocAsync(&dw, (size_t)n_mat * M * 8, st));
     QSI_CUDA(cudaMallocAsync(&dV, Ap.size() * 8, st));
     QSI_CUDA(cudaMemcpyAsync(dA, Ap.data(), Ap.size() * 8, cudaMemcpyHostToDevice, st));
-    size_t smem = (size_t)M * M * 8 + (size_t)M * 8 + (size_t)M * 2 * 4 + (size_t)M * 4 + 64;
+    size_t smem = (size_t)M * M * 8 + (size_t)M * 12 + 64;
+    const int v_shared = smem + (size_t)M * M * 8 <= 227 * 1024;
+    if (v_shared) smem += (size_t)M * M * 8;
     cudaFuncSetAttribute(k_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_jacobi<<<n_mat, 256, smem, st>>>(dA, M, dw, dV, 60);
+    k_jacobi<<<n_mat, 256, smem, st>>>(dA, M, dw, dV, 60, v_shared);
     std::vector<double> wp((size_t)n_mat * M), Vp(Ap.size());
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(wp.data(), dw, wp.size() * 8, cudaMemcpyDeviceToHost, st);
