@@ -26,14 +26,15 @@
 
 namespace qsi {
 
-constexpr int kRedBlock = 256;
-constexpr int kRedGrid = 1024;  // fixed partial-sum grid: reduction order independent of the device
-
-template <typename T>
-__device__ __forceinline__ double ld(const T* p, int64_t i) {
-    return (double)p[i];
+// Reductions over the rows run in a fixed order: a grid that depends on the dimension alone (dot_grid), each thread's
+// rows in order, a fixed tree over the block's threads, then the blocks' partial sums in a fixed tree.
+constexpr int kDotBlock = 512;
+constexpr int kDotMaxGrid = 304;  // two blocks on each of the 152 SMs
+static int dot_grid(int64_t n) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>(kDotMaxGrid, (n + 2 * kDotBlock - 1) / (2 * kDotBlock)));
 }
 
+// Sum of v over the block's threads (a power of two, at least 32), valid in thread 0.
 __device__ __forceinline__ double block_sum(double v, double* sh) {
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -43,7 +44,20 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     double r = 0.0;
     if (threadIdx.x == 0)
         for (int k = 0; k < (int)(blockDim.x >> 5); ++k) r += sh[k];
-    return r;  // valid in thread 0
+    return r;
+}
+
+// Sum of count partial sums, the same in every block that computes it: warp 0 adds them lane by lane, then across the
+// lanes; every thread receives it.
+__device__ __forceinline__ double sum_partials(const double* __restrict__ partial, int count, double* sh) {
+    if (threadIdx.x < 32) {
+        double v = 0.0;
+        for (int b = threadIdx.x; b < count; b += 32) v += partial[b];
+        for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (threadIdx.x == 0) *sh = v;
+    }
+    __syncthreads();
+    return *sh;
 }
 
 // Double-float accumulator (two FP32 words, about 2^-46 relative): a += x * (ch + cl), x an FP32 value, with an
@@ -65,105 +79,6 @@ __device__ __forceinline__ void df_split(double v, float& h, float& l) {
     h = (float)v;
     l = (float)(v - (double)h);
 }
-
-// FP32 Krylov vectors: the dots V_i . w of eight vectors per pass over the rows (w, FP64, split into a float pair
-// once per row and pass), accumulated in double-float: GB300's FP64 pipe runs at 1/64 of the FP32 rate, and the
-// FP64 form of these loops is bound by it.  |w|^2 stays an FP64 sum (one FMA per row).
-constexpr int kDotGroup = 8;
-__global__ void __launch_bounds__(kRedBlock) k_multidot_f32(const float* __restrict__ V, int64_t ld_v, int k,
-                                                            const double* __restrict__ w, int64_t n,
-                                                            double* __restrict__ partial) {
-    __shared__ double sh[32];
-    const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t a = blockIdx.x * chunk, b = min(n, a + chunk);
-    for (int g0 = 0; g0 < k; g0 += kDotGroup) {
-        // the group's vectors (the last repeated past k, its sums unused): every load unconditional, so a
-        // row's kDotGroup + 1 loads are in flight together
-        const int nv = min(kDotGroup, k - g0);
-        const float* vp[kDotGroup];
-#pragma unroll
-        for (int u = 0; u < kDotGroup; ++u) vp[u] = V + (int64_t)(g0 + min(u, nv - 1)) * ld_v;
-        DF acc[kDotGroup];
-#pragma unroll
-        for (int u = 0; u < kDotGroup; ++u) acc[u] = DF{0.f, 0.f};
-        for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) {
-            const double wd = __ldg(w + r);
-            float v[kDotGroup];
-#pragma unroll
-            for (int u = 0; u < kDotGroup; ++u) v[u] = __ldg(vp[u] + r);
-            float wh, wl;
-            df_split(wd, wh, wl);
-#pragma unroll
-            for (int u = 0; u < kDotGroup; ++u) df_fma(acc[u], wh, wl, v[u]);
-        }
-        for (int u = 0; u < nv; ++u) {
-            const double s = block_sum(df_value(acc[u]), sh);
-            if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * (k + 1) + g0 + u] = s;
-        }
-    }
-    double acc = 0.0;
-    for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) acc += w[r] * w[r];
-    const double s = block_sum(acc, sh);
-    if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * (k + 1) + k] = s;
-}
-
-// partial[b*(k+1) + i] = sum over this block's rows of V_i . w  (i < k), and
-// partial[b*(k+1) + k] = sum of w^2.
-template <typename VT>
-__global__ void __launch_bounds__(kRedBlock) k_multidot(const VT* __restrict__ V, int64_t ld_v, int k,
-                                                        const double* __restrict__ w, int64_t n,
-                                                        double* __restrict__ partial) {
-    __shared__ double sh[32];
-    const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t a = blockIdx.x * chunk, b = min(n, a + chunk);
-    for (int i = 0; i <= k; ++i) {
-        double acc = 0.0;
-        if (i < k) {
-            const VT* vi = V + (int64_t)i * ld_v;
-            for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) acc += ld(vi, r) * w[r];
-        } else {
-            for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) acc += w[r] * w[r];
-        }
-        double s = block_sum(acc, sh);
-        if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * (k + 1) + i] = s;
-    }
-}
-
-__global__ void k_reduce_partials(const double* __restrict__ partial, int nblocks, int k1, double* __restrict__ out) {
-    __shared__ double sh[32];
-    for (int i = 0; i < k1; ++i) {
-        double acc = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc += partial[(int64_t)b * k1 + i];
-        double s = block_sum(acc, sh);
-        if (threadIdx.x == 0) out[i] = s;
-    }
-}
-
-// w -= sum_i h_i V_i ; partial[b] = this block's sum of the new w^2.
-template <typename VT>
-__global__ void __launch_bounds__(kRedBlock) k_multi_axpy(const VT* __restrict__ V, int64_t ld_v, int k,
-                                                          const double* __restrict__ h, double* __restrict__ w,
-                                                          int64_t n, double* __restrict__ partial) {
-    __shared__ double sh[32];
-    __shared__ double hs[256];
-    for (int i = threadIdx.x; i < k; i += blockDim.x) hs[i] = h[i];
-    __syncthreads();
-    const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t a = blockIdx.x * chunk, b = min(n, a + chunk);
-    double acc = 0.0;
-    for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) {
-        double v = w[r];
-        for (int i = 0; i < k; ++i) v -= hs[i] * ld(V + (int64_t)i * ld_v, r);
-        w[r] = v;
-        acc += v * v;
-    }
-    double s = block_sum(acc, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s;
-}
-
-// The working vector of the FP32 solve as a double-float pair array: split once per Lanczos step, then the
-// reorthogonalisation (dots, updates, norms) and the store of the next Krylov vector run on the FP32 pipe with no
-// FP64 operation per row.
 __device__ __forceinline__ float2 df_sub(float2 a, float2 b) {  // (a - b) in double-float, renormalised
     const float s = a.x - b.x;
     const float bb = s - a.x;
@@ -171,105 +86,252 @@ __device__ __forceinline__ float2 df_sub(float2 a, float2 b) {  // (a - b) in do
     const float hi = s + e;
     return make_float2(hi, e - (hi - s));
 }
-__global__ void k_split_f64(const double* __restrict__ w, float2* __restrict__ wf, int64_t n) {
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        float h, l;
-        df_split(w[r], h, l);
-        wf[r] = make_float2(h, l);
+
+// The vectors of the Krylov kernels.  FP64 vectors (Vec64): the working vector w and every sum in FP64.  FP32 vectors
+// (Vec32): w as a double-float pair array in the buffer that takes the apply's FP64 result, sums in double-float on
+// the FP32 pipe (GB300's FP64 pipe runs at 1/64 of its rate, and FP64 forms of these loops are bound by it).
+struct Vec64 {
+    using V = double;
+    using W = double;
+    using Acc = double;
+    using Coef = double;
+    __device__ static W from_apply(double y) { return y; }
+    __device__ static Coef coef(double h) { return h; }
+    __device__ static Acc zero() { return 0.0; }
+    __device__ static void dot(Acc& a, W w, V v) { a += w * v; }
+    __device__ static void norm(Acc& a, W w) { a += w * w; }
+    __device__ static double value(const Acc& a) { return a; }
+    // w minus a sum of coef * v, the sum carried in up to four parts
+    static constexpr int kParts = 1;
+    __device__ static void part(Acc& s, Coef h, V v) { s += h * v; }
+    __device__ static W minus(W w, const Acc (&s)[1]) { return w - s[0]; }
+    __device__ static V scaled(W w, double inv) { return w * inv; }
+};
+struct Vec32 {
+    using V = float;
+    using W = float2;
+    using Acc = DF;
+    using Coef = float2;
+    __device__ static W from_apply(double y) {
+        float2 w;
+        df_split(y, w.x, w.y);
+        return w;
     }
-}
-// partial[b*(k+1) + i] = V_i . w (i < k) and partial[b*(k+1) + k] = |w|^2 over this block's rows, w a pair array.
-__global__ void __launch_bounds__(kRedBlock) k_multidot_df(const float* __restrict__ V, int64_t ld_v, int k,
-                                                           const float2* __restrict__ wf, int64_t n,
-                                                           double* __restrict__ partial) {
-    __shared__ double sh[32];
-    const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t a = blockIdx.x * chunk, b = min(n, a + chunk);
-    for (int g0 = 0; g0 < k; g0 += kDotGroup) {
-        const int nv = min(kDotGroup, k - g0);
-        const float* vp[kDotGroup];
-#pragma unroll
-        for (int u = 0; u < kDotGroup; ++u) vp[u] = V + (int64_t)(g0 + min(u, nv - 1)) * ld_v;
-        DF acc[kDotGroup];
-#pragma unroll
-        for (int u = 0; u < kDotGroup; ++u) acc[u] = DF{0.f, 0.f};
-        for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) {
-            const float2 wv = __ldg(wf + r);
-            float v[kDotGroup];
-#pragma unroll
-            for (int u = 0; u < kDotGroup; ++u) v[u] = __ldg(vp[u] + r);
-#pragma unroll
-            for (int u = 0; u < kDotGroup; ++u) df_fma(acc[u], wv.x, wv.y, v[u]);
-        }
-        for (int u = 0; u < nv; ++u) {
-            const double t = block_sum(df_value(acc[u]), sh);
-            if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * (k + 1) + g0 + u] = t;
-        }
-    }
-    DF nrm{0.f, 0.f};
-    for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) {
-        const float2 wv = __ldg(wf + r);
-        df_fma(nrm, wv.x, 2.f * wv.y, wv.x);  // hi^2 + 2 hi lo
-    }
-    const double t = block_sum(df_value(nrm), sh);
-    if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * (k + 1) + k] = t;
-}
-// w -= sum_i h_i V_i on the pair array: the sum in double-float with h_i as float pairs (four interleaved partial
-// sums combined in a fixed order, so four loads per row are in flight and the dependent chain is a quarter as
-// long), the subtraction in double-float; partial[b] = this block's |w|^2.
-__global__ void __launch_bounds__(kRedBlock) k_multi_axpy_df(const float* __restrict__ V, int64_t ld_v, int k,
-                                                             const double* __restrict__ h, float2* __restrict__ wf,
-                                                             int64_t n, double* __restrict__ partial) {
-    __shared__ double sh[32];
-    __shared__ float hh[256], hl[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        hh[i] = hl[i] = 0.f;
-        if (i < k) df_split(h[i], hh[i], hl[i]);
-    }
-    __syncthreads();
-    const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t a = blockIdx.x * chunk, b = min(n, a + chunk);
-    const int k4 = (k + 3) & ~3;
-    DF nrm{0.f, 0.f};
-    for (int64_t r = a + threadIdx.x; r < b; r += blockDim.x) {
-        DF s[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-        for (int i = 0; i < k4; i += 4) {
-            float v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = __ldg(V + (int64_t)min(i + u, k - 1) * ld_v + r);  // h = 0 past k
-#pragma unroll
-            for (int u = 0; u < 4; ++u) df_fma(s[u], hh[i + u], hl[i + u], v[u]);
-        }
+    __device__ static Coef coef(double h) { return from_apply(h); }
+    __device__ static Acc zero() { return DF{0.f, 0.f}; }
+    __device__ static void dot(Acc& a, W w, V v) { df_fma(a, w.x, w.y, v); }
+    __device__ static void norm(Acc& a, W w) { df_fma(a, w.x, 2.f * w.y, w.x); }  // hi^2 + 2 hi lo
+    __device__ static double value(const Acc& a) { return df_value(a); }
+    static constexpr int kParts = 4;  // interleaved partial sums: a quarter of the dependent chain
+    __device__ static void part(Acc& s, Coef h, V v) { df_fma(s, h.x, h.y, v); }
+    __device__ static W minus(W w, const Acc (&s)[4]) {
         float2 t = df_sub(make_float2(s[0].hi, s[0].lo), make_float2(-s[1].hi, -s[1].lo));
         t = df_sub(t, make_float2(-s[2].hi, -s[2].lo));
         t = df_sub(t, make_float2(-s[3].hi, -s[3].lo));
-        const float2 wv = df_sub(wf[r], t);
-        wf[r] = wv;
-        df_fma(nrm, wv.x, 2.f * wv.y, wv.x);
+        return df_sub(w, t);
     }
-    const double t = block_sum(df_value(nrm), sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = t;
+    __device__ static V scaled(W w, double inv) {
+        const float2 c = from_apply(inv);
+        const float p = w.x * c.x;
+        return p + (fmaf(w.x, c.x, -p) + (w.x * c.y + w.y * c.x));
+    }
+};
+
+// Rows of this block.
+struct RowRange {
+    int64_t a, b;
+    __device__ explicit RowRange(int64_t n) {
+        const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
+        a = min(n, blockIdx.x * chunk);
+        b = min(n, a + chunk);
+    }
+};
+
+// partial[block] = v . w over the block's rows, w the apply's FP64 result.
+template <class K>
+__global__ void __launch_bounds__(kDotBlock) k_krylov_alpha(const typename K::V* __restrict__ v,
+                                                            const double* __restrict__ w, int64_t n,
+                                                            double* __restrict__ partial) {
+    __shared__ double sh[32];
+    const RowRange R(n);
+    typename K::Acc acc = K::zero();
+#pragma unroll 4
+    for (int64_t r = R.a + threadIdx.x; r < R.b; r += blockDim.x) K::dot(acc, K::from_apply(w[r]), v[r]);
+    const double s = block_sum(K::value(acc), sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
-// out = w / |w| rounded to FP32 (beta_sq: the squared norm on the device).
-__global__ void k_scale_store_df(const float2* __restrict__ wf, const double* __restrict__ beta_sq,
-                                 float* __restrict__ out, int64_t n) {
-    const double inv = 1.0 / sqrt(*beta_sq);
-    float ih, il;
-    df_split(inv, ih, il);
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        const float2 wv = wf[r];
-        const float p = wv.x * ih;
-        out[r] = p + (fmaf(wv.x, ih, -p) + (wv.x * il + wv.y * ih));
+
+// Sums acc[0 .. kDotGroup) over the block's threads into out[0 .. nv): each thread's values go to shared memory and a
+// shrinking set of threads adds them, so every FP64 add has full lanes (as warp shuffles the same sums would take
+// the FP64 pipe five adds per warp and value).
+constexpr int kDotGroup = 8;
+constexpr size_t kDotSmem = (size_t)kDotGroup * kDotBlock * 8;
+__device__ __forceinline__ void group_sums(const double (&acc)[kDotGroup], double* sh, int nv, double* __restrict__ out) {
+    static_assert(kDotBlock == 512, "8 x 8 x 8 threads");
+    const int t = threadIdx.x;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kDotGroup; ++u) sh[u * kDotBlock + t] = acc[u];
+    __syncthreads();
+    // thread t: value u = t / 64, threads t % 64 + 64 k
+    const double* p = sh + (t >> 6) * kDotBlock + (t & 63);
+    double v = p[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) v += p[64 * k];
+    __syncthreads();
+    sh[t] = v;
+    __syncthreads();
+    if (t < 64) {  // value t / 8, eight of its 64 sums
+        v = sh[(t >> 3) * 64 + (t & 7)];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v += sh[(t >> 3) * 64 + (t & 7) + 8 * k];
+        // the eight lanes of a value are neighbours
+#pragma unroll
+        for (int o = 4; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 8);
+        if ((t & 7) == 0 && (t >> 3) < nv) out[t >> 3] = v;
     }
 }
 
-// out = w * (1/beta), converted to the storage type.// out = w * (1/beta), converted to the storage type.
-template <typename VT>
-__global__ void k_scale_store(const double* __restrict__ w, const double* __restrict__ beta, VT* __restrict__ out,
-                              int64_t n) {
-    const double inv = 1.0 / sqrt(*beta);  // beta holds the squared norm
+// One pass over the rows of a Lanczos step: w <- w - alpha V_j - beta V_{j-1} (nloc = 2; 1: without beta; 0: neither;
+// the coefficients from the device, alpha as the sum of k_krylov_alpha's partials), then the dots of V_0 .. V_{k-1}
+// with the new w: partial[block * k + i].  Each group of eight vectors is one sweep over the block's rows with nine
+// loads in flight per thread.  first: w holds the apply's FP64 result, otherwise K::W.
+template <class K>
+__global__ void __launch_bounds__(kDotBlock, 2) k_krylov_dots(const typename K::V* __restrict__ V, int64_t ld, int k,
+                                                           void* __restrict__ wbuf, int first, int nloc,
+                                                           const double* __restrict__ alpha_partial, int n_partial,
+                                                           const double* __restrict__ beta_prev,
+                                                           double* __restrict__ alpha_out, int64_t n,
+                                                           double* __restrict__ partial) {
+    extern __shared__ double sh[];
+    using W = typename K::W;
+    W* w = reinterpret_cast<W*>(wbuf);
+    const double* y = reinterpret_cast<const double*>(wbuf);
+    typename K::Coef ca{}, cb{};
+    const typename K::V *va = V, *vb = V;
+    if (nloc >= 1) {
+        const double a = sum_partials(alpha_partial, n_partial, sh);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *alpha_out = a;
+        ca = K::coef(a);
+        va = V + (int64_t)(k - 1) * ld;
+        if (nloc >= 2) {
+            cb = K::coef(*beta_prev);
+            vb = V + (int64_t)(k - 2) * ld;
+        }
+        __syncthreads();
+    }
+    const RowRange R(n);
+    for (int g0 = 0; g0 < k; g0 += kDotGroup) {
+        const int nv = min(kDotGroup, k - g0);
+        const typename K::V* vg = V + (int64_t)g0 * ld;
+        typename K::Acc acc[kDotGroup];
+#pragma unroll
+        for (int u = 0; u < kDotGroup; ++u) acc[u] = K::zero();
+        const bool update = g0 == 0 && (first || nloc);
+        for (int64_t r = R.a + threadIdx.x; r < R.b; r += blockDim.x) {
+            typename K::V v[kDotGroup];
+            const typename K::V* p = vg + r;
+#pragma unroll
+            for (int u = 0; u < kDotGroup; ++u, p += ld) v[u] = u < nv ? *p : (typename K::V)0;
+            W x;
+            if (update) {
+                x = first ? K::from_apply(y[r]) : w[r];
+                if (nloc) {
+                    typename K::Acc s[K::kParts];
+#pragma unroll
+                    for (int q = 0; q < K::kParts; ++q) s[q] = K::zero();
+                    K::part(s[0], ca, va[r]);
+                    if (nloc >= 2) K::part(s[K::kParts > 1], cb, vb[r]);
+                    x = K::minus(x, s);
+                }
+                w[r] = x;
+            } else {
+                x = w[r];
+            }
+#pragma unroll
+            for (int u = 0; u < kDotGroup; ++u) K::dot(acc[u], x, v[u]);
+        }
+        double val[kDotGroup];
+#pragma unroll
+        for (int u = 0; u < kDotGroup; ++u) val[u] = K::value(acc[u]);
+        group_sums(val, sh, nv, partial + (int64_t)blockIdx.x * k + g0);
+    }
+}
+
+// h[i] = sum over blocks of partial[b * k + i], one block per i; with last (the alpha of the step): *last += h[k-1].
+__global__ void __launch_bounds__(128) k_krylov_reduce(const double* __restrict__ partial, int nblocks, int k,
+                                                       double* __restrict__ h, double* __restrict__ last, int add) {
+    __shared__ double sh[32];
+    const int i = blockIdx.x;
+    double acc = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) acc += partial[(int64_t)b * k + i];
+    const double s = block_sum(acc, sh);
+    if (threadIdx.x == 0) {
+        h[i] = s;
+        if (last && i == k - 1) *last = add ? *last + s : s;
+    }
+}
+
+// w <- w - sum_i h_i V_i; partial[block] = |w|^2 over the block's rows.
+template <class K>
+__global__ void __launch_bounds__(kDotBlock) k_krylov_subtract(const typename K::V* __restrict__ V, int64_t ld, int k,
+                                                               const double* __restrict__ h,
+                                                               typename K::W* __restrict__ w, int64_t n,
+                                                               double* __restrict__ partial) {
+    __shared__ double sh[32];
+    __shared__ typename K::Coef hs[264];
+    const int k8 = (k + 7) & ~7;
+    for (int i = threadIdx.x; i < k8; i += blockDim.x) hs[i] = K::coef(i < k ? h[i] : 0.0);
+    __syncthreads();
+    const RowRange R(n);
+    typename K::Acc nrm = K::zero();
+    for (int64_t r = R.a + threadIdx.x; r < R.b; r += blockDim.x) {
+        typename K::Acc s[K::kParts];
+#pragma unroll
+        for (int q = 0; q < K::kParts; ++q) s[q] = K::zero();
+        for (int i = 0; i < k8; i += 8) {
+            typename K::V v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = V[(int64_t)min(i + u, k - 1) * ld + r];  // h = 0 past k
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i + u < k) K::part(s[u % K::kParts], hs[i + u], v[u]);
+        }
+        const typename K::W x = K::minus(w[r], s);
+        w[r] = x;
+        K::norm(nrm, x);
+    }
+    const double t = block_sum(K::value(nrm), sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = t;
+}
+
+// out = w / |w|, |w|^2 the sum of partial; *beta = |w|.
+template <class K>
+__global__ void __launch_bounds__(256) k_krylov_scale(const typename K::W* __restrict__ w,
+                                                      const double* __restrict__ partial, int n_partial,
+                                                      double* __restrict__ beta, typename K::V* __restrict__ out,
+                                                      int64_t n) {
+    __shared__ double sh;
+    const double nrm = sqrt(fmax(sum_partials(partial, n_partial, &sh), 0.0));
+    if (blockIdx.x == 0 && threadIdx.x == 0) *beta = nrm;
+    const double inv = 1.0 / nrm;
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        out[r] = (VT)(w[r] * inv);
+        out[r] = K::scaled(w[r], inv);
+}
+
+// The apply's FP64 result converted to the working vector's form in place.
+template <class K>
+__global__ void k_krylov_convert(void* __restrict__ wbuf, int64_t n) {
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
+        reinterpret_cast<typename K::W*>(wbuf)[r] = K::from_apply(reinterpret_cast<const double*>(wbuf)[r]);
+}
+
+// out = w * (1/beta) (FP64; beta holds the squared norm).
+__global__ void k_scale_store(const double* __restrict__ w, const double* __restrict__ beta, double* __restrict__ out,
+                              int64_t n) {
+    const double inv = 1.0 / sqrt(*beta);
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
+        out[r] = w[r] * inv;
 }
 
 // Deterministic N(0,1) start vector: counter-based SplitMix64 bits, Box-Muller.
@@ -537,18 +599,21 @@ qsi_status jacobi_eigh(const std::vector<double>& A, int m, int n_mat, std::vect
 }
 
 // ------------------------------------------------------------------ vector toolkit
+// Dots and updates of FP64 vectors for the drivers that need the coefficients on the host.
 struct Vecs {
     int64_t n = 0;
     cudaStream_t st = nullptr;
-    double* partial = nullptr;  // kRedGrid * 257
-    double* red = nullptr;      // 257
-    std::vector<double> hred;
+    int grid = 1;
+    double* partial = nullptr;  // kDotMaxGrid * 257
+    double* red = nullptr;      // 258
     qsi_status init(int64_t n_, cudaStream_t s) {
         n = n_;
         st = s;
-        QSI_CUDA(cudaMallocAsync(&partial, (size_t)kRedGrid * 257 * 8, st));
-        QSI_CUDA(cudaMallocAsync(&red, 257 * 8, st));
-        hred.resize(257);
+        grid = dot_grid(n);
+        cudaFuncSetAttribute(k_krylov_dots<Vec64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDotSmem);
+        cudaFuncSetAttribute(k_krylov_dots<Vec32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDotSmem);
+        QSI_CUDA(cudaMallocAsync(&partial, (size_t)kDotMaxGrid * 257 * 8, st));
+        QSI_CUDA(cudaMallocAsync(&red, 258 * 8, st));
         return QSI_OK;
     }
     ~Vecs() {
@@ -556,40 +621,25 @@ struct Vecs {
         cudaFreeAsync(red, st);
     }
     // h[0..k) = V_i . w and h[k] = |w|^2, copied to host
-    template <typename VT>
-    qsi_status dots(const VT* V, int64_t ldv, int k, const double* w, std::vector<double>& h) {
-        if constexpr (sizeof(VT) == 4) k_multidot_f32<<<kRedGrid, kRedBlock, 0, st>>>(V, ldv, k, w, n, partial);
-        else k_multidot<VT><<<kRedGrid, kRedBlock, 0, st>>>(V, ldv, k, w, n, partial);
-        k_reduce_partials<<<1, 256, 0, st>>>(partial, kRedGrid, k + 1, red);
+    qsi_status dots(const double* V, int64_t ldv, int k, const double* w, std::vector<double>& h) {
+        double* ww = const_cast<double*>(w);  // not written: neither converted nor updated
+        if (k > 0) {
+            k_krylov_dots<Vec64><<<grid, kDotBlock, kDotSmem, st>>>(V, ldv, k, ww, 0, 0, nullptr, 0, nullptr, nullptr, n, partial);
+            k_krylov_reduce<<<k, 128, 0, st>>>(partial, grid, k, red, nullptr, 0);
+        }
+        k_krylov_alpha<Vec64><<<grid, kDotBlock, 0, st>>>(w, w, n, partial + (size_t)kDotMaxGrid * 256);
+        k_krylov_reduce<<<1, 128, 0, st>>>(partial + (size_t)kDotMaxGrid * 256, grid, 1, red + k, nullptr, 0);
+        QSI_CUDA(cudaGetLastError());
         h.resize(k + 1);
         QSI_CUDA(cudaMemcpyAsync(h.data(), red, (size_t)(k + 1) * 8, cudaMemcpyDeviceToHost, st));
-        QSI_CUDA(cudaStreamSynchronize(st));
-        return QSI_OK;
-    }
-    // FP32 Krylov vectors with the working vector as a pair array: h[0..k) = V_i . w, h[k] = |w|^2
-    qsi_status dots_df(const float* V, int64_t ldv, int k, const float2* wf, std::vector<double>& h) {
-        k_multidot_df<<<kRedGrid, kRedBlock, 0, st>>>(V, ldv, k, wf, n, partial);
-        k_reduce_partials<<<1, 256, 0, st>>>(partial, kRedGrid, k + 1, red);
-        h.resize(k + 1);
-        QSI_CUDA(cudaMemcpyAsync(h.data(), red, (size_t)(k + 1) * 8, cudaMemcpyDeviceToHost, st));
-        QSI_CUDA(cudaStreamSynchronize(st));
-        return QSI_OK;
-    }
-    // ... w -= V h; returns |w|^2 (device copy left in red[0])
-    qsi_status axpy_df(const float* V, int64_t ldv, int k, const std::vector<double>& h, float2* wf, double& nrm2) {
-        QSI_CUDA(cudaMemcpyAsync(red + 1, h.data(), (size_t)k * 8, cudaMemcpyHostToDevice, st));
-        k_multi_axpy_df<<<kRedGrid, kRedBlock, 0, st>>>(V, ldv, k, red + 1, wf, n, partial);
-        k_reduce_partials<<<1, 256, 0, st>>>(partial, kRedGrid, 1, red);
-        QSI_CUDA(cudaMemcpyAsync(&nrm2, red, 8, cudaMemcpyDeviceToHost, st));
         QSI_CUDA(cudaStreamSynchronize(st));
         return QSI_OK;
     }
     // w -= V h ; returns |w|^2 (device copy left in red[0])
-    template <typename VT>
-    qsi_status axpy(const VT* V, int64_t ldv, int k, const std::vector<double>& h, double* w, double& nrm2) {
+    qsi_status axpy(const double* V, int64_t ldv, int k, const std::vector<double>& h, double* w, double& nrm2) {
         QSI_CUDA(cudaMemcpyAsync(red + 1, h.data(), (size_t)k * 8, cudaMemcpyHostToDevice, st));
-        k_multi_axpy<VT><<<kRedGrid, kRedBlock, 0, st>>>(V, ldv, k, red + 1, w, n, partial);
-        k_reduce_partials<<<1, 256, 0, st>>>(partial, kRedGrid, 1, red);
+        k_krylov_subtract<Vec64><<<grid, kDotBlock, 0, st>>>(V, ldv, k, red + 1, w, n, partial);
+        k_krylov_reduce<<<1, 128, 0, st>>>(partial, grid, 1, red, nullptr, 0);
         QSI_CUDA(cudaMemcpyAsync(&nrm2, red, 8, cudaMemcpyDeviceToHost, st));
         QSI_CUDA(cudaStreamSynchronize(st));
         return QSI_OK;
@@ -632,18 +682,18 @@ static qsi_status orthonormalise(Vecs& vx, double* X, int k, int64_t n) {
     for (int i = 0; i < k; ++i) {
         double* xi = X + (size_t)i * n;
         for (int pass = 0; pass < 2; ++pass) {
-            qsi_status s = vx.dots<double>(X, n, i, xi, h);
+            qsi_status s = vx.dots(X, n, i, xi, h);
             if (s) return s;
             double nrm2 = h[i];
             if (i > 0) {
                 h.resize(i);
-                s = vx.axpy<double>(X, n, i, h, xi, nrm2);
+                s = vx.axpy(X, n, i, h, xi, nrm2);
                 if (s) return s;
             }
             if (pass == 1) {
                 if (!(nrm2 > 0)) return fail(QSI_NOT_CONVERGED, "polish: Ritz vectors became linearly dependent");
                 QSI_CUDA(cudaMemcpyAsync(vx.red, &nrm2, 8, cudaMemcpyHostToDevice, vx.st));
-                k_scale_store<double><<<grid_for(n, 256), 256, 0, vx.st>>>(xi, vx.red, xi, n);
+                k_scale_store<<<grid_for(n, 256), 256, 0, vx.st>>>(xi, vx.red, xi, n);
             }
         }
     }
@@ -657,7 +707,7 @@ static qsi_status rayleigh_ritz(Vecs& vx, const double* S, const double* HS, int
                                 double* HX, std::vector<double>& theta, cudaStream_t st) {
     std::vector<double> G((size_t)k * k), h;
     for (int j = 0; j < k; ++j) {
-        qsi_status s = vx.dots<double>(S, n, k, HS + (size_t)j * n, h);
+        qsi_status s = vx.dots(S, n, k, HS + (size_t)j * n, h);
         if (s) return s;
         for (int i = 0; i < k; ++i) G[(size_t)i * k + j] = h[i];
     }
@@ -771,10 +821,10 @@ static qsi_status finish_solve(qsi_op* op, const qsi_lanczos_cfg& cfg, Vecs& vx,
         QSI_CUDA(cudaMemcpyAsync(d2.p, th.data(), (size_t)nev * 8, cudaMemcpyHostToDevice, st));
         k_residual<<<grid_for(n, 256), 256, 0, st>>>(HX.p, X.p, d2.p, nev, n, R.p);
         for (int i = 0; i < nev && i < 64; ++i) {
-            s = vx.dots<double>(X.p + (size_t)i * n, n, 1, R.p + (size_t)i * n, h);
+            s = vx.dots(X.p + (size_t)i * n, n, 1, R.p + (size_t)i * n, h);
             if (s) return s;
             std::vector<double> hx;
-            s = vx.dots<double>(X.p, n, 0, X.p + (size_t)i * n, hx);
+            s = vx.dots(X.p, n, 0, X.p + (size_t)i * n, hx);
             if (s) return s;
             rep->residual[i] = std::sqrt(h[1] / std::max(hx[0], 1e-300));
         }
@@ -814,88 +864,91 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     const double tol_req = cfg.tol > 0 ? cfg.tol : 1e-10;
     const double tol = (sizeof(VT) == 4 && cfg.polish_steps >= 2) ? std::max(tol_req, fp32_stop(cfg.polish_steps)) : tol_req;
     const double eps23 = std::pow(2.220446049250313e-16, 2.0 / 3.0);
+    using K = std::conditional_t<sizeof(VT) == 4, Vec32, Vec64>;
     Vecs vx;
     qsi_status s = vx.init(n, st);
     if (s) return s;
     DevBuf<VT> V;
-    DevBuf<double> w, dY;
+    DevBuf<double> w, dY, coef;
     QSI_CUDA(V.alloc((size_t)(m + 1) * n, st));
-    QSI_CUDA(w.alloc((size_t)n, st));
+    QSI_CUDA(w.alloc((size_t)n, st));  // the apply's result, then the working vector in its own form (K::W)
     QSI_CUDA(dY.alloc((size_t)m * m, st));
-    constexpr bool kDF = sizeof(VT) == 4;  // FP32 vectors: reorthogonalise w as a double-float pair array
-    DevBuf<float2> wf;
-    if (kDF) QSI_CUDA(wf.alloc((size_t)n, st));
-    // the reorthogonalisation's dots and updates, on w (FP64) or on its pair array (FP32 vectors)
-    auto rdots = [&](int k, std::vector<double>& hv) -> qsi_status {
-        if constexpr (kDF) return vx.dots_df(reinterpret_cast<const float*>(V.p), n, k, wf.p, hv);
-        else return vx.dots<VT>(V.p, n, k, w.p, hv);
-    };
-    auto raxpy = [&](int k, const std::vector<double>& hv, double& nrm2) -> qsi_status {
-        if constexpr (kDF) return vx.axpy_df(reinterpret_cast<const float*>(V.p), n, k, hv, wf.p, nrm2);
-        else return vx.axpy<VT>(V.p, n, k, hv, w.p, nrm2);
-    };
+    QSI_CUDA(coef.alloc((size_t)2 * m, st));
+    double *d_alpha = coef.p, *d_beta = coef.p + m;
+    typename K::W* wk = reinterpret_cast<typename K::W*>(w.p);
+    const int grid = vx.grid;
+    double* alpha_partial = vx.partial + (size_t)kDotMaxGrid * 256;
     auto vec = [&](int j) { return V.p + (size_t)j * n; };
+    // Orthogonalises w against V_0 .. V_j, coefficients on the device: dots in the same pass as the local update
+    // (nloc) or the conversion of the apply's result (first), then the subtraction with the new norm.  d_alpha[j]
+    // becomes (add: grows by) the coefficient of V_j.
+    auto orth_pass = [&](int j, int first, int nloc, int add) {
+        k_krylov_dots<K><<<grid, kDotBlock, kDotSmem, st>>>(V.p, n, j + 1, w.p, first, nloc, alpha_partial, grid,
+                                                            d_beta + std::max(0, j - 1), d_alpha + j, n, vx.partial);
+        k_krylov_reduce<<<j + 1, 128, 0, st>>>(vx.partial, grid, j + 1, vx.red, d_alpha + j, add);
+        k_krylov_subtract<K><<<grid, kDotBlock, 0, st>>>(V.p, n, j + 1, vx.red, wk, n, vx.partial);
+    };
+    // w = H V_j, alpha_j, beta_j and V_{j+1}, enqueued without waiting: the three-term part first, then one pass of
+    // classical Gram-Schmidt against the whole basis, whose coefficients are the loss of orthogonality alone, so the
+    // second pass that a plain Gram-Schmidt of H V_j needs is left out.  After a restart (j == k > 0) H V_j has
+    // components along every kept vector, and two full passes take them out.
+    auto lanczos_step = [&](int j, int k) -> qsi_status {
+        qsi_status ss = apply_to_w<VT>(op, vec(j), w.p, st);
+        if (ss) return ss;
+        if (j == k && k > 0) {
+            orth_pass(j, 1, 0, 0);
+            orth_pass(j, 0, 0, 1);
+        } else {
+            k_krylov_alpha<K><<<grid, kDotBlock, 0, st>>>(vec(j), w.p, n, alpha_partial);
+            orth_pass(j, 1, j > 0 ? 2 : 1, 1);
+        }
+        k_krylov_scale<K><<<grid_for(n, 256), 256, 0, st>>>(wk, vx.partial, grid, d_beta + j, vec(j + 1), n);
+        QSI_CUDA(cudaGetLastError());
+        return QSI_OK;
+    };
     // start vector N(0,1), normalised (stored)
     k_randn<<<grid_for(n, 256), 256, 0, st>>>(w.p, n, cfg.seed, 0);
-    std::vector<double> h;
-    s = vx.dots<VT>(V.p, n, 0, w.p, h);
-    if (s) return s;
-    QSI_CUDA(cudaMemcpyAsync(vx.red, &h[0], 8, cudaMemcpyHostToDevice, st));
-    k_scale_store<VT><<<grid_for(n, 256), 256, 0, st>>>(w.p, vx.red, vec(0), n);
+    k_krylov_alpha<Vec64><<<grid, kDotBlock, 0, st>>>(w.p, w.p, n, vx.partial);
+    if (sizeof(VT) == 4) k_krylov_convert<K><<<grid_for(n, 256), 256, 0, st>>>(w.p, n);
+    k_krylov_scale<K><<<grid_for(n, 256), 256, 0, st>>>(wk, vx.partial, grid, d_beta, vec(0), n);
     std::vector<double> alpha(m, 0.0), beta(m, 0.0), theta, coup;  // coup[i] = s_i couplings after restart
+    std::vector<double> hcoef((size_t)2 * m);
     int k = 0;
     int64_t applies = 0;
     int restarts = 0, nconv = 0;
     std::vector<double> Tw, TY;
     PhaseClock clk{st, sizeof(VT) == 4 ? "trlan-f32" : "trlan-f64"};
     for (;;) {
-        for (int j = k; j < m; ++j) {
-            clk.mark("setup/host");
-            s = apply_to_w<VT>(op, vec(j), w.p, st);
-            if (s) return s;
-            ++applies;
-            clk.mark("apply");
-            if (kDF) k_split_f64<<<grid_for(n, 256), 256, 0, st>>>(w.p, wf.p, n);
-            // full reorthogonalisation: classical Gram-Schmidt against v_0..v_j, repeated once
-            // when the norm drops by more than 1/sqrt(2) (DGKS criterion)
-            s = rdots(j + 1, h);
-            if (s) return s;
-            double before = h[j + 1];
-            double a = h[j];
-            std::vector<double> hh(h.begin(), h.begin() + j + 1);
-            double nrm2 = 0;
-            s = raxpy(j + 1, hh, nrm2);
-            if (s) return s;
-            if (nrm2 < 0.5 * before) {
-                s = rdots(j + 1, h);
-                if (s) return s;
-                a += h[j];
-                hh.assign(h.begin(), h.begin() + j + 1);
-                s = raxpy(j + 1, hh, nrm2);
+        int done = k;  // steps of this cycle known to be sound
+        while (done < m) {
+            for (int j = done; j < m; ++j) {
+                s = lanczos_step(j, k);
                 if (s) return s;
             }
-            alpha[j] = a;
-            double b = std::sqrt(std::max(nrm2, 0.0));
-            if (!(b > 1e-13 * std::max(1.0, std::fabs(a)))) {
-                // invariant subspace: continue from a fresh random direction orthogonal to V
-                b = 0.0;
-                k_randn<<<grid_for(n, 256), 256, 0, st>>>(w.p, n, cfg.seed + 7919 * (uint64_t)(j + 1 + restarts * m), 0);
-                if (kDF) k_split_f64<<<grid_for(n, 256), 256, 0, st>>>(w.p, wf.p, n);
-                for (int pass = 0; pass < 2; ++pass) {
-                    s = rdots(j + 1, h);
-                    if (s) return s;
-                    hh.assign(h.begin(), h.begin() + j + 1);
-                    s = raxpy(j + 1, hh, nrm2);
-                    if (s) return s;
-                }
+            QSI_CUDA(cudaMemcpyAsync(hcoef.data(), coef.p, (size_t)2 * m * 8, cudaMemcpyDeviceToHost, st));
+            QSI_CUDA(cudaStreamSynchronize(st));
+            clk.mark("steps");
+            int j = done;
+            for (; j < m; ++j) {
+                alpha[j] = hcoef[j];
+                beta[j] = hcoef[m + j];
+                ++applies;
+                if (!(beta[j] > 1e-13 * std::max(1.0, std::fabs(alpha[j])))) break;
             }
-            beta[j] = b;
-            QSI_CUDA(cudaMemcpyAsync(vx.red, &nrm2, 8, cudaMemcpyHostToDevice, st));
-            if constexpr (kDF)
-                k_scale_store_df<<<grid_for(n, 256), 256, 0, st>>>(wf.p, vx.red, reinterpret_cast<float*>(vec(j + 1)), n);
-            else
-                k_scale_store<VT><<<grid_for(n, 256), 256, 0, st>>>(w.p, vx.red, vec(j + 1), n);
-            clk.mark("orthogonalise");
+            if (j == m) break;
+            // invariant subspace at step j: continue from a fresh random direction orthogonal to V (the steps after
+            // j divided by a vanishing norm and are taken again)
+            beta[j] = 0.0;
+            const double zero = 0.0;
+            k_randn<<<grid_for(n, 256), 256, 0, st>>>(w.p, n, cfg.seed + 7919 * (uint64_t)(j + 1 + restarts * m), 0);
+            double kept = alpha[j];
+            orth_pass(j, 1, 0, 0);
+            orth_pass(j, 0, 0, 0);
+            k_krylov_scale<K><<<grid_for(n, 256), 256, 0, st>>>(wk, vx.partial, grid, d_beta + j, vec(j + 1), n);
+            QSI_CUDA(cudaMemcpyAsync(d_alpha + j, &kept, 8, cudaMemcpyHostToDevice, st));
+            QSI_CUDA(cudaMemcpyAsync(d_beta + j, &zero, 8, cudaMemcpyHostToDevice, st));
+            QSI_CUDA(cudaStreamSynchronize(st));
+            done = j + 1;
         }
         // projected matrix: arrowhead (kept Ritz values + couplings) then tridiagonal
         std::vector<double> T((size_t)m * m, 0.0);
@@ -1681,11 +1734,11 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
             if (it > 0) k_axpby<<<grid_for(n, 256), 256, 0, st>>>(u.p, v.p, 0.0, -beta, n);
             s = launch_apply(op, v.p, u.p, 1, QSI_F64, 1, st);
             if (s) return s;
-            s = vx.dots<double>(v.p, n, 1, u.p, h);
+            s = vx.dots(v.p, n, 1, u.p, h);
             if (s) return s;
             double alpha = h[0];
             k_axpby<<<grid_for(n, 256), 256, 0, st>>>(u.p, v.p, -alpha, 1.0, n);
-            s = vx.dots<double>(v.p, n, 0, u.p, h);
+            s = vx.dots(v.p, n, 0, u.p, h);
             if (s) return s;
             beta = std::sqrt(h[0]);
             if (beta < cfg->abs_tol) break;
@@ -1807,7 +1860,7 @@ extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, cons
                 QSI_CUDA(cudaStreamSynchronize(st));
                 s = launch_apply(op, P.p + (size_t)i * n, w, 1, QSI_F64, 0, op->stream);
                 if (s == QSI_OK && cudaStreamSynchronize(op->stream) != cudaSuccess) s = fail(QSI_CUDA_ERROR, "apply");
-                if (s == QSI_OK) s = vx.dots<double>(P.p, n, nvec, w, h);
+                if (s == QSI_OK) s = vx.dots(P.p, n, nvec, w, h);
                 for (int j = 0; j < nvec && s == QSI_OK; ++j) expect[((size_t)l * nvec + i) * nvec + j] = h[j];
             }
             qsi_op_destroy(op);
@@ -1820,7 +1873,7 @@ extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, cons
                     const double* wmj = W.p + (size_t)(m * nvec + j) * n;
                     for (int64_t c0 = 0; c0 < K; c0 += 256) {  // the reduction buffers hold 256 dots
                         const int kc = (int)std::min<int64_t>(256, K - c0);
-                        s = vx.dots<double>(W.p + (size_t)c0 * n, n, kc, wmj, h);
+                        s = vx.dots(W.p + (size_t)c0 * n, n, kc, wmj, h);
                         if (s) return s;
                         std::copy(h.begin(), h.begin() + kc, col.begin() + c0);
                     }
