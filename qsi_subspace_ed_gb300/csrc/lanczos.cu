@@ -1522,10 +1522,57 @@ __global__ void k_tridiag_vector(const double* __restrict__ a, const double* __r
     }
 }
 
-__global__ void k_axpby(double* __restrict__ y, const double* __restrict__ x, double a, double b, int64_t n) {
-    // y = b*y + a*x
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        y[r] = b * y[r] + a * x[r];
+// One three-term step of eigval0 in three passes over the rows, coefficients on the device (alpha[it], beta[it]):
+//   u <- w - beta[it-1] u, with v . u in partial sums (w = H v);
+__global__ void __launch_bounds__(kDotBlock) k_three_term_dot(const double* __restrict__ w, const double* __restrict__ v,
+                                                              double* __restrict__ u, const double* __restrict__ beta_prev,
+                                                              int64_t n, double* __restrict__ partial) {
+    __shared__ double sh[32];
+    const RowRange R(n);
+    const double nb = beta_prev ? -*beta_prev : 0.0;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int64_t r = R.a + threadIdx.x; r < R.b; r += blockDim.x) {
+        const double t = w[r] + nb * u[r];
+        u[r] = t;
+        acc += v[r] * t;
+    }
+    const double s = block_sum(acc, sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+//   u <- u - alpha v, with |u|^2 in partial sums; ev (optional) += y v;
+__global__ void __launch_bounds__(kDotBlock) k_three_term_subtract(const double* __restrict__ v, double* __restrict__ u,
+                                                                   const double* __restrict__ dot_partial, int n_partial,
+                                                                   double* __restrict__ alpha, double* __restrict__ ev,
+                                                                   double y, int64_t n, double* __restrict__ partial) {
+    __shared__ double sh[32];
+    const RowRange R(n);
+    const double a = sum_partials(dot_partial, n_partial, sh);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *alpha = a;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int64_t r = R.a + threadIdx.x; r < R.b; r += blockDim.x) {
+        const double x = v[r], t = u[r] - a * x;
+        u[r] = t;
+        acc += t * t;
+        if (ev) ev[r] += y * x;
+    }
+    const double s = block_sum(acc, sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+//   u <- u / beta, beta = |u|: the next v.
+__global__ void __launch_bounds__(256) k_three_term_scale(double* __restrict__ u, const double* __restrict__ norm_partial,
+                                                          int n_partial, double* __restrict__ beta, int64_t n) {
+    __shared__ double sh;
+    const double b = sqrt(sum_partials(norm_partial, n_partial, &sh));
+    if (blockIdx.x == 0 && threadIdx.x == 0) *beta = b;
+    const double inv = 1.0 / b;
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) u[r] *= inv;
+}
+
+// y += a x
+__global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, double a, int64_t n) {
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) y[r] += a * x[r];
 }
 
 static qsi_status lowest_of_tridiag(const std::vector<double>& al, const std::vector<double>& be, double& e0,
@@ -1639,6 +1686,8 @@ static qsi_status write_eigval0_checkpoint(const char* path, const double* d_v, 
 // (relative); a second identical pass accumulates the Ritz vector.  With a
 // checkpoint, the first pass resumes from it and writes it at the top of an
 // iteration (the state that iteration starts from).
+constexpr int kEig0Batch = 128;
+
 static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigval0Checkpoint* ck, double* e0,
                               double* eigvec, int32_t* iterations) {
     const int64_t n = op->basis->n;
@@ -1656,24 +1705,38 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
     Vecs vx;
     qsi_status s = vx.init(n, st);
     if (s) return s;
-    DevBuf<double> v, u, ev;
+    DevBuf<double> v, u, w, ev, coef;
     QSI_CUDA(v.alloc(n, st));
     QSI_CUDA(u.alloc(n, st));
-    std::vector<double> alphas, betas, ritz, h;
+    QSI_CUDA(w.alloc(n, st));
+    const int max_it = std::max(0, cfg->max_iterations);
+    QSI_CUDA(coef.alloc((size_t)2 * max_it + 2, st));
+    double *d_al = coef.p, *d_be = coef.p + max_it;
+    double *dot_partial = vx.partial, *norm_partial = vx.partial + kDotMaxGrid;
+    // Iterations [it, end) enqueued without waiting; before: iteration `it` starts from v, u and beta[it - 1].
+    auto enqueue = [&](int it, int end, const std::vector<double>* ritz) -> qsi_status {
+        for (; it < end; ++it) {
+            const bool acc = ritz && it < (int)ritz->size();
+            qsi_status ss = launch_apply(op, v.p, w.p, 1, QSI_F64, 0, st);
+            if (ss) return ss;
+            k_three_term_dot<<<vx.grid, kDotBlock, 0, st>>>(w.p, v.p, u.p, it > 0 ? d_be + it - 1 : nullptr, n, dot_partial);
+            k_three_term_subtract<<<vx.grid, kDotBlock, 0, st>>>(v.p, u.p, dot_partial, vx.grid, d_al + it,
+                                                                 acc ? ev.p : nullptr, acc ? (*ritz)[it] : 0.0, n, norm_partial);
+            k_three_term_scale<<<grid_for(n, 256), 256, 0, st>>>(u.p, norm_partial, vx.grid, d_be + it, n);
+            std::swap(v.p, u.p);
+        }
+        QSI_CUDA(cudaGetLastError());
+        return QSI_OK;
+    };
+    std::vector<double> al, be, ritz;
     double eig = 1e308, e0_pass0 = 0.0;
     int its = 0;
     const auto t_start = std::chrono::steady_clock::now();
-    for (int pass = 0; pass < (cfg->calc_eigenvector ? 2 : 1); ++pass) {
-        QSI_CUDA(cudaMemcpyAsync(v.p, v0.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-        QSI_CUDA(cudaMemsetAsync(u.p, 0, (size_t)n * 8, st));
-        if (pass == 1) {
-            QSI_CUDA(ev.alloc(n, st));
-            QSI_CUDA(cudaMemsetAsync(ev.p, 0, (size_t)n * 8, st));
-        }
-        std::vector<double> al, be;
-        double beta = 0.0;
+    QSI_CUDA(cudaMemcpyAsync(v.p, v0.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
+    QSI_CUDA(cudaMemsetAsync(u.p, 0, (size_t)n * 8, st));
+    {
         int it, it0 = 0;
-        if (pass == 0 && ck) {  // resume the first pass from an existing checkpoint of this run
+        if (ck) {  // resume the first pass from an existing checkpoint of this run
             h5::OutDataset dv, du, da, db, dbeta, dit, dseed;
             bool have = false;
             try {
@@ -1696,20 +1759,24 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                     db.data.size() != m * 8 || (int64_t)m != itv || dbeta.data.size() != 8 ||
                     seed32 != (int32_t)(uint32_t)cfg->seed || itv > cfg->max_iterations)
                     return fail(QSI_INVALID_ARG, "eigval0 checkpoint %s: not a checkpoint of this run", ck->path);
-                QSI_CUDA(cudaMemcpyAsync(v.p, dv.data.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-                QSI_CUDA(cudaMemcpyAsync(u.p, du.data.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-                QSI_CUDA(cudaStreamSynchronize(st));
+                double beta = 0.0;
                 al.resize(m);
                 be.resize(m);
                 std::memcpy(al.data(), da.data.data(), m * 8);
                 std::memcpy(be.data(), db.data.data(), m * 8);
                 std::memcpy(&beta, dbeta.data.data(), 8);
+                QSI_CUDA(cudaMemcpyAsync(v.p, dv.data.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
+                QSI_CUDA(cudaMemcpyAsync(u.p, du.data.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
+                if (m > 0) QSI_CUDA(cudaMemcpyAsync(d_be + m - 1, &beta, 8, cudaMemcpyHostToDevice, st));
+                QSI_CUDA(cudaStreamSynchronize(st));
                 it0 = (int)itv;
             }
         }
-        if (pass == 1) eig = 1e308;
-        for (it = it0; it < cfg->max_iterations; ++it) {
-            if (pass == 0 && ck && it > it0) {
+        // The first pass never stops on convergence (lanczos.cpp:163-167 breaks only when a Ritz vector is being
+        // accumulated), so its iterations run in batches that end where something has to be looked at: a vanishing
+        // beta at the latest after kEig0Batch, a checkpoint, a stop, or each iteration under a wall-clock limit.
+        for (it = it0; it < max_it;) {
+            if (ck && it > it0) {
                 const double elapsed =
                     std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
                 const bool stop = (ck->stop_after > 0 && it - it0 >= ck->stop_after) ||
@@ -1721,7 +1788,8 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                         s = lowest_of_tridiag(al, b2, est, st);
                         if (s) return s;
                     }
-                    s = write_eigval0_checkpoint(ck->path, v.p, u.p, n, al, be, beta, it, est, cfg->seed, st);
+                    s = write_eigval0_checkpoint(ck->path, v.p, u.p, n, al, be, be.empty() ? 0.0 : be.back(), it, est,
+                                                 cfg->seed, st);
                     if (s) return s;
                 }
                 if (stop) {
@@ -1729,57 +1797,75 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                     return fail(QSI_TIMEOUT, "eigval0: stopped at iteration %d, checkpoint written to %s", it, ck->path);
                 }
             }
-            if (pass == 1 && it < (int)ritz.size())
-                k_axpby<<<grid_for(n, 256), 256, 0, st>>>(ev.p, v.p, ritz[it], 1.0, n);
-            if (it > 0) k_axpby<<<grid_for(n, 256), 256, 0, st>>>(u.p, v.p, 0.0, -beta, n);
-            s = launch_apply(op, v.p, u.p, 1, QSI_F64, 1, st);
+            int end = std::min(max_it, it + kEig0Batch);
+            if (ck) {
+                if (ck->wall_limit_s > 0) end = it + 1;
+                if (ck->every > 0) end = std::min(end, (it / ck->every + 1) * ck->every);
+                if (ck->stop_after > 0) end = std::min(end, it0 + ck->stop_after);
+            }
+            s = enqueue(it, end, nullptr);
             if (s) return s;
-            s = vx.dots(v.p, n, 1, u.p, h);
+            const int got = end - it;
+            al.resize(it + got);
+            be.resize(it + got);
+            QSI_CUDA(cudaMemcpyAsync(al.data() + it, d_al + it, (size_t)got * 8, cudaMemcpyDeviceToHost, st));
+            QSI_CUDA(cudaMemcpyAsync(be.data() + it, d_be + it, (size_t)got * 8, cudaMemcpyDeviceToHost, st));
+            QSI_CUDA(cudaStreamSynchronize(st));
+            bool vanished = false;
+            for (; it < end && !vanished; ++it)
+                if (be[it] < cfg->abs_tol) {
+                    vanished = true;
+                    break;
+                }
+            al.resize(it);
+            be.resize(it);
+            if (vanished) break;
+        }
+        its = it;
+        std::vector<double> b2(be.begin(), be.empty() ? be.end() : be.end() - 1);
+        s = lowest_of_tridiag(al, b2, eig, st);
+        if (s) return s;
+        e0_pass0 = eig;
+        if (cfg->calc_eigenvector) {
+            const int m = (int)al.size();
+            DevBuf<double> d, work, y;
+            QSI_CUDA(d.alloc((size_t)2 * m, st));
+            QSI_CUDA(work.alloc((size_t)5 * m + 8, st));
+            QSI_CUDA(y.alloc((size_t)m, st));
+            QSI_CUDA(cudaMemcpyAsync(d.p, al.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st));
+            if (m > 1) QSI_CUDA(cudaMemcpyAsync(d.p + m, b2.data(), (size_t)(m - 1) * 8, cudaMemcpyHostToDevice, st));
+            k_tridiag_vector<<<1, 32, 0, st>>>(d.p, d.p + m, m, eig, work.p, y.p);
+            ritz.resize(m);
+            QSI_CUDA(cudaMemcpyAsync(ritz.data(), y.p, (size_t)m * 8, cudaMemcpyDeviceToHost, st));
+            QSI_CUDA(cudaStreamSynchronize(st));
+        }
+    }
+    if (cfg->calc_eigenvector) {
+        // The second pass repeats the first's recurrence, bit for bit, up to the iteration at which it stops, which
+        // the first pass's coefficients therefore tell: the lowest Ritz value changed by less than abs_tol or
+        // rel_tol from min_iterations on, or the first pass's end.
+        QSI_CUDA(ev.alloc(n, st));
+        QSI_CUDA(cudaMemsetAsync(ev.p, 0, (size_t)n * 8, st));
+        int last = std::min(its, max_it - 1);
+        eig = 1e308;
+        for (int it = std::max(0, cfg->min_iterations); it < its; ++it) {
+            const double old = eig;
+            s = lowest_of_tridiag(std::vector<double>(al.begin(), al.begin() + it + 1),
+                                  std::vector<double>(be.begin(), be.begin() + it), eig, st);
             if (s) return s;
-            double alpha = h[0];
-            k_axpby<<<grid_for(n, 256), 256, 0, st>>>(u.p, v.p, -alpha, 1.0, n);
-            s = vx.dots(v.p, n, 0, u.p, h);
-            if (s) return s;
-            beta = std::sqrt(h[0]);
-            if (beta < cfg->abs_tol) break;
-            std::swap(v.p, u.p);
-            k_axpby<<<grid_for(n, 256), 256, 0, st>>>(v.p, v.p, 0.0, 1.0 / beta, n);
-            al.push_back(alpha);
-            be.push_back(beta);
-            // The first pass never stops on convergence (lanczos.cpp:163-167 breaks
-            // only when a Ritz vector is being accumulated); the second pass does.
-            if (pass == 1 && it >= cfg->min_iterations) {
-                double old = eig;
-                std::vector<double> b2(be.begin(), be.end() - 1);
-                s = lowest_of_tridiag(al, b2, eig, st);
-                if (s) return s;
-                double err = std::fabs(eig - old);
-                double rel = err / std::max(std::fabs(eig), 1e-10);
-                if (err < cfg->abs_tol || rel < cfg->rel_tol) break;
+            const double err = std::fabs(eig - old);
+            const double rel = err / std::max(std::fabs(eig), 1e-10);
+            if (err < cfg->abs_tol || rel < cfg->rel_tol) {
+                last = it;
+                break;
             }
         }
-        if (pass == 0) {
-            its = it;
-            alphas = al;
-            betas = be;
-            std::vector<double> b2(be.begin(), be.empty() ? be.end() : be.end() - 1);
-            s = lowest_of_tridiag(al, b2, eig, st);
-            if (s) return s;
-            e0_pass0 = eig;
-            if (cfg->calc_eigenvector) {
-                const int m = (int)al.size();
-                DevBuf<double> d, work, y;
-                QSI_CUDA(d.alloc((size_t)2 * m, st));
-                QSI_CUDA(work.alloc((size_t)5 * m + 8, st));
-                QSI_CUDA(y.alloc((size_t)m, st));
-                QSI_CUDA(cudaMemcpyAsync(d.p, al.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st));
-                if (m > 1) QSI_CUDA(cudaMemcpyAsync(d.p + m, b2.data(), (size_t)(m - 1) * 8, cudaMemcpyHostToDevice, st));
-                k_tridiag_vector<<<1, 32, 0, st>>>(d.p, d.p + m, m, eig, work.p, y.p);
-                ritz.resize(m);
-                QSI_CUDA(cudaMemcpyAsync(ritz.data(), y.p, (size_t)m * 8, cudaMemcpyDeviceToHost, st));
-                QSI_CUDA(cudaStreamSynchronize(st));
-            }
-        }
+        // iterations 0 .. last accumulate ritz[it] v_it; the last needs no step of its own
+        QSI_CUDA(cudaMemcpyAsync(v.p, v0.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
+        QSI_CUDA(cudaMemsetAsync(u.p, 0, (size_t)n * 8, st));
+        s = enqueue(0, last, &ritz);
+        if (s) return s;
+        if (last < (int)ritz.size()) k_axpy<<<grid_for(n, 256), 256, 0, st>>>(ev.p, v.p, ritz[last], n);
     }
     *e0 = e0_pass0;
     if (iterations) *iterations = its;
