@@ -537,9 +537,15 @@ __global__ void __launch_bounds__(256, RC <= 4 ? 4 : 2) k_apply_tile_cols(TilePa
 constexpr int kVec4 = 0;
 constexpr int kVec8 = -1;
 constexpr int kVec16 = -2;
+// A few vectors (R <= kGroupMax) without 16-byte gathers: the warp sums 32 / lpc rows at once, lpc = R rounded up to a
+// power of two lanes each.  (With one row per warp the lanes beyond R idle, and GB300's FP64 pipe takes 17 cycles per
+// instruction however few of its lanes work.)
+constexpr int kGroup = -3;
+constexpr int kGroupMax = 16;
 constexpr uint32_t kDiagSlot = 0x80000000u;
+constexpr int min_blocks(int km) { return km == kGroup || km > 0 ? 3 : 2; }
 inline bool vec4_ok(int64_t n, int R, const void* x, const void* y) {
-    return n < (int64_t)kDiagSlot - 1 && R >= 16 && (R & 3) == 0 &&
+    return n < (int64_t)kDiagSlot - 1 && R >= 4 && (R & 3) == 0 &&
            (R <= 128 ? (R & (R - 1)) == 0 : (R & 127) == 0) &&
            ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
 }
@@ -648,7 +654,70 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
                 });
             }
             __syncwarp();
-            if constexpr (kFF) {
+            if constexpr (KM == kGroup) {
+                int lpc = 1;
+                while (lpc < R) lpc *= 2;
+                const int g = lane / lpc, c = lane % lpc;
+                constexpr int kU = 8;  // column gathers in flight per lane
+                for (int l0 = row_start; l0 < row_end; l0 += 32 / lpc) {
+                    const int l = l0 + g;
+                    const int64_t rl = tile * 32 + l;
+                    const bool mine = l < row_end && rl < P.B.n;
+                    const int kb = __shfl_sync(0xffffffffu, base, l & 31);
+                    int nl = __shfl_sync(0xffffffffu, cnt, l & 31);
+                    if (!mine) nl = 0;
+                    const int steps = __reduce_max_sync(0xffffffffu, nl);
+                    const bool on = mine && c < R;
+                    std::conditional_t<kFF, FF, double> acc{};
+                    if (on) {
+                        const XT xd = x[rl * R + c];
+                        if constexpr (kFF) {
+                            const float2 dd = P.diag_ff[rl];
+                            ff_fma(acc, dd.x, dd.y, (float)xd);
+                        } else {
+                            double dl;
+                            if constexpr (kFam) {
+                                const state2 t = P.B.states[rl];
+                                dl = fam_diag(P, t.x, t.y, c);
+                            } else {
+                                dl = P.diag[rl];
+                            }
+                            acc = dl * (double)xd;
+                        }
+                    }
+                    for (int s0 = 0; s0 < steps; s0 += kU) {
+                        XT xv[kU];
+#pragma unroll
+                        for (int u = 0; u < kU; ++u) {
+                            const uint32_t J = (s0 + u < nl) ? hJ[kb + s0 + u] : kEmpty;
+                            xv[u] = (on && J != kEmpty) ? x[(int64_t)J * R + c] : (XT)0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < kU; ++u) {
+                            if (!above_tol(xv[u])) continue;
+                            if constexpr (kFF) {
+                                const float2 ck = hcf[kb + s0 + u];
+                                ff_fma(acc, ck.x, ck.y, (float)xv[u]);
+                            } else {
+                                const double ck = hc[kb + s0 + u];
+                                acc += (kFam ? fam_coef(P, ck, c) : ck) * (double)xv[u];
+                            }
+                        }
+                    }
+                    if (on) {
+                        if constexpr (kFF) {
+                            if (accumulate) {
+                                const float2 yc = ycoef ? ycoef[c] : make_float2(1.0f, 0.0f);
+                                ff_fma(acc, yc.x, yc.y, (float)y[rl * R + c]);
+                            }
+                            y[rl * R + c] = (XT)(acc.hi + acc.lo);
+                        } else {
+                            if (accumulate) acc += (double)y[rl * R + c];
+                            y[rl * R + c] = (XT)acc;
+                        }
+                    }
+                }
+            } else if constexpr (kFF) {
                 // FP32 storage, double-float accumulation, no FP64 instruction.  The chunk's hit list
                 // is walked in order across row boundaries with kU column gathers in flight.
                 static_assert(std::is_same<XT, float>::value, "double-float accumulation is for FP32 vectors");
@@ -867,7 +936,7 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
 }
 
 template <typename XT, class LK, bool kFF, int KM, bool kFam = false>
-__global__ void __launch_bounds__(256, KM <= kVec4 ? 2 : 3) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
+__global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
                                                             XT* __restrict__ y, int R, int accumulate, int cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     batched_body<XT, LK, kFF, KM, kFam>(P, lk, x, y, R, accumulate, cap, blockIdx.x, gridDim.x, smem_raw);
@@ -893,7 +962,7 @@ struct SectorLaunch {
 };
 
 template <int KM, class LK>
-__global__ void __launch_bounds__(256, KM <= kVec4 ? 2 : 3) k_apply_sectors(const SectorLaunch* __restrict__ secs, int n_secs,
+__global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_sectors(const SectorLaunch* __restrict__ secs, int n_secs,
                                                           int accumulate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SectorLaunch L;
@@ -1428,7 +1497,8 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
                                                                          accumulate, cap);
             }
         };
-        if (R <= 32) go(std::integral_constant<int, 1>{});
+        if (R <= kGroupMax) go(std::integral_constant<int, kGroup>{});
+        else if (R <= 32) go(std::integral_constant<int, 1>{});
         else if (R <= 64) go(std::integral_constant<int, 2>{});
         else go(std::integral_constant<int, 4>{});
     }
@@ -1517,6 +1587,7 @@ qsi_status launch_sectors(const void* d_records, const SectorPlan& plan, int acc
     if (plan.vec16) go(std::integral_constant<int, kVec16>{});
     else if (plan.vec8) go(std::integral_constant<int, kVec8>{});
     else if (plan.vec4) go(std::integral_constant<int, kVec4>{});
+    else if (plan.maxR <= kGroupMax) go(std::integral_constant<int, kGroup>{});
     else if (plan.maxR <= 32) go(std::integral_constant<int, 1>{});
     else if (plan.maxR <= 64) go(std::integral_constant<int, 2>{});
     else go(std::integral_constant<int, 4>{});
@@ -1569,7 +1640,8 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
             k<<<one_wave(k, block, smem, ntiles, tmpl->tune[1].grid_bps), block, smem, st>>>(P, lk, x, y, R, accumulate,
                                                                                              cap);
         };
-        if (R <= 32) go(std::integral_constant<int, 1>{});
+        if (R <= kGroupMax) go(std::integral_constant<int, kGroup>{});
+        else if (R <= 32) go(std::integral_constant<int, 1>{});
         else if (R <= 64) go(std::integral_constant<int, 2>{});
         else go(std::integral_constant<int, 4>{});
     }

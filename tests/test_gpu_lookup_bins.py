@@ -37,7 +37,7 @@ PAIRS = [(0.7, "0+ 1-"), (0.7, "0- 1+"), (0.7, "0+ 1-"), (0.2, "2+ 3-"), (0.2, "
          (0.5, "4- 5+ 6- 7+ 8- 9+"), (0.3, "4+ 5- 6+ 7- 8+ 9-")]
 
 
-def check(lohi, H, bits):
+def check(lohi, H, bits, terms=18):
     n = len(lohi)
     x = np.random.default_rng(3).standard_normal(n)
     x[::7] = 0.0
@@ -48,8 +48,8 @@ def check(lohi, H, bits):
     op.set_kernel(0)
     row = np.zeros(n)
     op.evaluate(x, row)
-    # one rounding per term and row at most, 18 terms
-    np.testing.assert_allclose(row, ref, rtol=0, atol=40 * 2.3e-16 * max(np.abs(ref).max(), 1.0))
+    # two roundings per term and row (product, sum), in another order
+    np.testing.assert_allclose(row, ref, rtol=0, atol=2 * terms * 2.3e-16 * max(np.abs(ref).max(), 1.0))
     X = np.stack([x] * 3, axis=1)
     for use in (1, 0):
         for w in bits:
@@ -100,3 +100,49 @@ def test_one_sided_terms():
     for k, op in enumerate(q.get_ring_ops(lat)[0]):
         H.add_term(0.1 * (k + 1), op)
     check(q.enumerate_basis(lat), H, (6, 14))
+
+
+def xor_terms(n_bits, most):
+    """A term flipping each non-empty set of bits, up to `most` of them, every one with its own coefficient."""
+    return [(0.01 * (m + 1), " ".join(f"{k}x" for k in range(n_bits) if (m >> k) & 1)) for m in range(1, min(most + 1, 1 << n_bits))]
+
+
+# 30, 31, 32 distinct coefficients: 16- and 32-bit cache slots; 64, 65 terms on every row: lists of 2,048 and 2,080
+# hits, around a slot's 11 bits of position; 1,023 terms: a list that no block's shared memory holds
+@pytest.mark.parametrize("n", [40, 1000, 1024])
+@pytest.mark.parametrize("most", [30, 31, 32, 64, 65, 1023])
+def test_long_lists_and_many_coefficients(n, most):
+    bits = max(6, (n - 1).bit_length())
+    if most >= 1 << bits:
+        pytest.skip("more terms than sets of bits")
+    check(integers(n), opsum(xor_terms(bits, most)), (1, 8), terms=most)
+
+
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 20, 33])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("pairs", [0, 2])
+def test_few_vectors(R, dtype, pairs):
+    """Rows summed several at a time (R <= 16), with 16-byte gathers (FP32, 4 and 8) and one at a time: every column
+    bitwise the one of a 33-column apply, plain and accumulating, for short lists, and materialised."""
+    if R == 1 and dtype == np.float32:
+        pytest.skip("one FP32 vector is summed in FP64, not double-float")
+    lat = workloads.lattice("pyro_1x2x1")
+    g, B = workloads.ring_zeeman_params(5)
+    lohi = q.enumerate_basis(lat, n_spinon_pairs=pairs)[:20_011]  # cut off: some lookups leave the basis
+    op = q.LazyOpSum(q.ZBasis(lohi), q.build_ring_zeeman(lat, g, B, Jpm=0.05))
+    rng = np.random.default_rng(R)
+    n = len(lohi)
+    wide = rng.standard_normal((n, 33)).astype(dtype)
+    wide[::5, ::3] = 0
+    wide0 = rng.standard_normal((n, 33)).astype(dtype)
+    for acc in (False, True):
+        ref = wide0.copy()
+        op.apply_batched(wide, ref, accumulate=acc)
+        for cap in (8, 256):
+            op.set_kernel(1, 1, list_cap=cap)
+            for cached in (False, True):
+                op.materialise(cached)
+                X, Y = wide[:, :R].copy(), wide0[:, :R].copy()
+                op.apply_batched(X, Y, accumulate=acc)
+                assert np.array_equal(Y, ref[:, :R]), (acc, cap, cached)
+            op.materialise(False)
