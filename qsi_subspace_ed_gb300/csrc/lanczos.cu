@@ -1898,10 +1898,123 @@ extern "C" qsi_status qsi_eigval0_checkpointed(qsi_op* op, const qsi_eigval0_cfg
 }
 
 // ------------------------------------------------------------------ expectation values
+namespace qsi {
+
+// W[(l - l0) * nvec + i][j] = (O_l psi_i)[j] for operators of off-diagonal terms only, terms in transposed form: one
+// thread per row and operator, blockIdx.y = l - l0, the sums of LazyOpSum's apply (terms in order, sources with
+// |x| <= 1e-15 skipped, misses dropped).  Columns are looked up by bisection: an observable admits a few rows in a
+// hundred, and building an operator per observable, as an apply needs one, took 1.2 ms each.
+__global__ void __launch_bounds__(256) k_observables(BasisView B, const PullTerm* __restrict__ terms,
+                                                     const int* __restrict__ first, const double* __restrict__ psi,
+                                                     int nvec, double* __restrict__ W) {
+    const int l = blockIdx.y, t0 = first[l], t1 = first[l + 1];
+    double* out = W + (int64_t)l * nvec * B.n;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < B.n; j += (int64_t)gridDim.x * blockDim.x) {
+        const state2 s = B.states[j];
+        bool any = false;
+        for (int t = t0; t < t1; ++t) {
+            const PullTerm& T = terms[t];
+            if (((s.x & T.dn0) | (s.y & T.dn1)) != 0) continue;
+            if ((((s.x & T.up0) ^ T.up0) | ((s.y & T.up1) ^ T.up1)) != 0) continue;
+            const int64_t J = basis_find(B, s.x ^ T.x0, s.y ^ T.x1);
+            if (J < 0) continue;
+            const double cs = (T.has_z && ((__popcll(~s.x & T.z0) + __popcll(~s.y & T.z1)) & 1)) ? -T.cs : T.cs;
+            for (int i = 0; i < nvec; ++i) {
+                const double x = psi[(int64_t)i * B.n + J];
+                const double w = any ? out[(int64_t)i * B.n + j] : 0.0 * psi[(int64_t)i * B.n + j];
+                out[(int64_t)i * B.n + j] = fabs(x) > 1e-15 ? w + cs * x : w;
+            }
+            any = true;
+        }
+        if (!any)
+            for (int i = 0; i < nvec; ++i) out[(int64_t)i * B.n + j] = 0.0 * psi[(int64_t)i * B.n + j];  // no diagonal
+    }
+}
+
+// Gram matrix of two sets of vectors, A (ka of them) and C (kc), all of length n: partial[chunk][a][c] over the rows
+// of chunk blockIdx.y, in kGramTile x kGramTile tiles (blockIdx.x; symmetric: the tiles on and above the diagonal of
+// A = C only).  A thread holds a 4 x 4 square of sums, two FP64 multiply-adds per shared-memory value: bound by the
+// FP64 pipe, where a dot per vector pair read both vectors for each multiply-add.
+constexpr int kGramTile = 64, kGramRows = 16;
+__global__ void __launch_bounds__(256) k_gram(const double* __restrict__ A, int ka, const double* __restrict__ C, int kc,
+                                              int symmetric, int64_t n, double* __restrict__ partial) {
+    __shared__ double ta[kGramRows][kGramTile + 2], tc[kGramRows][kGramTile + 2];
+    const int tiles_c = (kc + kGramTile - 1) / kGramTile;
+    const int bi = blockIdx.x / tiles_c, bj = blockIdx.x % tiles_c;
+    if (symmetric && bj < bi) return;
+    const int a0 = bi * kGramTile, c0 = bj * kGramTile;
+    const int64_t chunk = ((n + gridDim.y - 1) / gridDim.y + kGramRows - 1) / kGramRows * kGramRows;
+    const int64_t r0 = min(n, blockIdx.y * chunk), r1 = min(n, r0 + chunk);
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // vectors tx + 16 u of C, ty + 16 u of A
+    double acc[4][4] = {};
+    for (int64_t r = r0; r < r1; r += kGramRows) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < kGramRows * kGramTile; e += 256) {
+            const int row = e % kGramRows, v = e / kGramRows;
+            const bool in = r + row < r1;
+            ta[row][v] = in && a0 + v < ka ? A[(int64_t)(a0 + v) * n + r + row] : 0.0;
+            tc[row][v] = in && c0 + v < kc ? C[(int64_t)(c0 + v) * n + r + row] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int row = 0; row < kGramRows; ++row) {
+            double av[4], cv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) av[u] = ta[row][ty + 16 * u], cv[u] = tc[row][tx + 16 * u];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int w = 0; w < 4; ++w) acc[u][w] += av[u] * cv[w];
+        }
+    }
+    double* out = partial + (int64_t)blockIdx.y * ka * kc;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const int a = a0 + ty + 16 * u, c = c0 + tx + 16 * w;
+            if (a < ka && c < kc) out[(int64_t)a * kc + c] = acc[u][w];
+        }
+}
+__global__ void k_gram_reduce(const double* __restrict__ partial, int chunks, int64_t count, double* __restrict__ out) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
+        double t = 0.0;
+        for (int b = 0; b < chunks; ++b) t += partial[(int64_t)b * count + e];
+        out[e] = t;
+    }
+}
+
+// h (host, ka x kc) = A^T C.
+static qsi_status gram(const double* A, int ka, const double* C, int kc, int64_t n, cudaStream_t st, std::vector<double>& h) {
+    const int symmetric = A == C && ka == kc;
+    const int tiles_a = (ka + kGramTile - 1) / kGramTile, tiles_c = (kc + kGramTile - 1) / kGramTile;
+    const int tiles = tiles_a * tiles_c, busy = symmetric ? tiles_a * (tiles_a + 1) / 2 : tiles;
+    const int64_t count = (int64_t)ka * kc;
+    // two blocks per SM over the tiles that work, each with at least 256 rows, and at most 256 MiB of partial sums
+    int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(304 / busy, (n + 255) / 256));
+    chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, ((int64_t)1 << 25) / count));
+    DevBuf<double> partial, out;
+    QSI_CUDA(partial.alloc((size_t)(chunks * count), st));
+    QSI_CUDA(out.alloc((size_t)count, st));
+    if (symmetric) QSI_CUDA(cudaMemsetAsync(partial.p, 0, (size_t)(chunks * count) * 8, st));
+    k_gram<<<dim3(tiles, (unsigned)chunks), 256, 0, st>>>(A, ka, C, kc, symmetric, n, partial.p);
+    k_gram_reduce<<<grid_for(count, 256), 256, 0, st>>>(partial.p, (int)chunks, count, out.p);
+    QSI_CUDA(cudaGetLastError());
+    h.resize((size_t)count);
+    QSI_CUDA(cudaMemcpyAsync(h.data(), out.p, (size_t)count * 8, cudaMemcpyDeviceToHost, st));
+    QSI_CUDA(cudaStreamSynchronize(st));
+    if (symmetric)
+        for (int a = 0; a < ka; ++a)
+            for (int c = 0; c < a / kGramTile * kGramTile; ++c) h[(size_t)a * kc + c] = h[(size_t)c * kc + a];
+    return QSI_OK;
+}
+
+}  // namespace qsi
+
 // compute_all_expectations / compute_cross_correlation (src/expectation_eval.cpp:27-110) on the device:
-// expect[l][i][j] = psi_j . (O_l psi_i), cross[l][m][i][j] = (O_l psi_i) . (O_m psi_j).  Each operator l
-// (terms[off[l] .. off[l+1])) is bound to the basis in turn; W_{l,i} = O_l psi_i is one FP64 apply.  The
-// dots are the fixed-order FP64 reductions of the Lanczos drivers.
+// expect[l][i][j] = psi_j . (O_l psi_i), cross[l][m][i][j] = (O_l psi_i) . (O_m psi_j).  The images W_{l,i} = O_l psi_i
+// of as many operators as a GiB holds (of all, for cross) come from one launch, those of operators with diagonal
+// terms from an apply each; their products with psi and with one another are Gram matrices, FP64 in a fixed order.
 extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, const int32_t* op_offsets, int32_t n_ops,
                                        const double* psi, int32_t nvec, double* expect, double* cross) {
     return guarded([&]() -> qsi_status {
@@ -1912,6 +2025,7 @@ extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, cons
                 return fail(QSI_INVALID_ARG, "qsi_expectations: operator offsets must not decrease");
         const int64_t n = b->n;
         const int64_t K = (int64_t)n_ops * nvec;  // vectors W_{l,i}, index l*nvec + i
+        if (K > INT32_MAX) return fail(QSI_INVALID_ARG, "qsi_expectations: %lld vectors", (long long)K);
         cudaStream_t st = nullptr;
         QSI_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         struct StreamGuard {
@@ -1929,44 +2043,64 @@ extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, cons
                 return fail(QSI_OOM, "qsi_expectations: %lld vectors of %lld states exceed device memory",
                             (long long)K, (long long)n);
         }
-        Vecs vx;
-        qsi_status s = vx.init(n, st);
-        if (s) return s;
+        // the operators' terms in transposed form (as qsi_op_create makes them; terms that vanish are left out)
+        std::vector<PullTerm> pull;
+        std::vector<int> first{0};
+        std::vector<char> direct(n_ops, 1);
+        for (int l = 0; l < n_ops; ++l) {
+            for (int t = op_offsets[l]; t < op_offsets[l + 1]; ++t) {
+                if ((terms[t].x[0] | terms[t].x[1]) == 0) direct[l] = 0;
+                else if (terms[t].sign != 0) pull.push_back(transposed_term(terms[t]));
+            }
+            first.push_back((int)pull.size());
+        }
+        DevBuf<PullTerm> d_pull;
+        DevBuf<int> d_first;
         DevBuf<double> P, W;
+        QSI_CUDA(d_pull.alloc(pull.size(), st));
+        QSI_CUDA(d_first.alloc(first.size(), st));
+        QSI_CUDA(cudaMemcpyAsync(d_pull.p, pull.data(), pull.size() * sizeof(PullTerm), cudaMemcpyHostToDevice, st));
+        QSI_CUDA(cudaMemcpyAsync(d_first.p, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         QSI_CUDA(P.alloc((size_t)n * nvec, st));
         QSI_CUDA(cudaMemcpyAsync(P.p, psi, (size_t)n * nvec * 8, cudaMemcpyHostToDevice, st));
-        QSI_CUDA(W.alloc((size_t)n * (cross ? K : 1), st));
+        const int per = cross ? n_ops : (int)std::max<int64_t>(1, std::min<int64_t>(n_ops, ((int64_t)1 << 27) / (n * nvec)));
+        QSI_CUDA(W.alloc((size_t)n * nvec * per, st));
         std::vector<double> h;
-        for (int l = 0; l < n_ops; ++l) {
-            qsi_op* op = nullptr;
-            s = qsi_op_create(b, terms + op_offsets[l], op_offsets[l + 1] - op_offsets[l], &op);
-            if (s) return s;
-            for (int i = 0; i < nvec && s == QSI_OK; ++i) {
-                double* w = W.p + (cross ? (size_t)(l * nvec + i) * n : 0);
+        for (int l0 = 0; l0 < n_ops; l0 += per) {
+            const int nl = std::min(per, n_ops - l0);
+            for (int y0 = 0; y0 < nl; y0 += 32768)
+                k_observables<<<dim3(grid_for(n, 256), std::min(32768, nl - y0)), 256, 0, st>>>(
+                    b->view(), d_pull.p, d_first.p + l0 + y0, P.p, nvec, W.p + (size_t)y0 * nvec * n);
+            QSI_CUDA(cudaGetLastError());
+            for (int l = l0; l < l0 + nl; ++l) {
+                if (direct[l]) continue;
+                qsi_op* op = nullptr;
+                qsi_status s = create_op(b, terms + op_offsets[l], op_offsets[l + 1] - op_offsets[l], false, &op);
+                if (s) return s;
                 QSI_CUDA(cudaStreamSynchronize(st));
-                s = launch_apply(op, P.p + (size_t)i * n, w, 1, QSI_F64, 0, op->stream);
+                for (int i = 0; i < nvec && s == QSI_OK; ++i)
+                    s = launch_apply(op, P.p + (size_t)i * n, W.p + ((size_t)(l - l0) * nvec + i) * n, 1, QSI_F64, 0, op->stream);
                 if (s == QSI_OK && cudaStreamSynchronize(op->stream) != cudaSuccess) s = fail(QSI_CUDA_ERROR, "apply");
-                if (s == QSI_OK) s = vx.dots(P.p, n, nvec, w, h);
-                for (int j = 0; j < nvec && s == QSI_OK; ++j) expect[((size_t)l * nvec + i) * nvec + j] = h[j];
+                qsi_op_destroy(op);
+                if (s) return s;
             }
-            qsi_op_destroy(op);
+            qsi_status s = gram(W.p, nl * nvec, P.p, nvec, n, st, h);
             if (s) return s;
+            std::copy(h.begin(), h.end(), expect + (size_t)l0 * nvec * nvec);
         }
         if (cross) {
-            std::vector<double> col((size_t)K);
-            for (int m = 0; m < n_ops; ++m)
-                for (int j = 0; j < nvec; ++j) {
-                    const double* wmj = W.p + (size_t)(m * nvec + j) * n;
-                    for (int64_t c0 = 0; c0 < K; c0 += 256) {  // the reduction buffers hold 256 dots
-                        const int kc = (int)std::min<int64_t>(256, K - c0);
-                        s = vx.dots(W.p + (size_t)c0 * n, n, kc, wmj, h);
-                        if (s) return s;
-                        std::copy(h.begin(), h.begin() + kc, col.begin() + c0);
-                    }
-                    for (int l = 0; l < n_ops; ++l)
+            const int panel = std::max(1, 2048 / nvec);  // operators per Gram matrix: all of them (symmetric) or a panel
+            for (int l0 = 0; l0 < n_ops; l0 += panel) {
+                const int nl = std::min(panel, n_ops - l0);
+                qsi_status s = gram(W.p + (size_t)l0 * nvec * n, nl * nvec, W.p, (int)K, n, st, h);
+                if (s) return s;
+                for (int l = 0; l < nl; ++l)
+                    for (int m = 0; m < n_ops; ++m)
                         for (int i = 0; i < nvec; ++i)
-                            cross[(((size_t)l * n_ops + m) * nvec + i) * nvec + j] = col[(size_t)l * nvec + i];
-                }
+                            for (int j = 0; j < nvec; ++j)
+                                cross[(((size_t)(l0 + l) * n_ops + m) * nvec + i) * nvec + j] =
+                                    h[((size_t)l * nvec + i) * K + (size_t)m * nvec + j];
+            }
         }
         return QSI_OK;
     });

@@ -320,6 +320,23 @@ int grid_for(int64_t n, int block) {
     return (int)std::max<int64_t>(1, std::min(g, cap));
 }
 
+PullTerm transposed_term(const qsi_term& t) {
+    PullTerm q{};
+    q.x0 = t.x[0], q.x1 = t.x[1], q.z0 = t.z[0], q.z1 = t.z[1];
+    // transpose: bits flipped by X swap their up/down requirement
+    q.up0 = (t.up[0] & ~t.x[0]) | (t.down[0] & t.x[0]);
+    q.up1 = (t.up[1] & ~t.x[1]) | (t.down[1] & t.x[1]);
+    q.dn0 = (t.down[0] & ~t.x[0]) | (t.up[0] & t.x[0]);
+    q.dn1 = (t.down[1] & ~t.x[1]) | (t.up[1] & t.x[1]);
+    // the element is evaluated on the row (pre-image) state: same sign as the
+    // reference's evaluation on the image state, see operator.hpp:246-253
+    q.cs = t.c * (double)t.sign;
+    q.has_z = (t.z[0] | t.z[1]) != 0;
+    q.cs_hi = (float)q.cs;
+    q.cs_lo = (float)(q.cs - (double)q.cs_hi);
+    return q;
+}
+
 static bool is_single_site_z(const qsi_term& t) {
     if (t.x[0] | t.x[1] | t.up[0] | t.up[1] | t.down[0] | t.down[1]) return false;
     return __builtin_popcountll(t.z[0]) + __builtin_popcountll(t.z[1]) == 1;
@@ -466,20 +483,7 @@ qsi_status qsi::create_op(qsi_basis* b, const qsi_term* terms, int32_t n_terms, 
             }
             push_off.push_back(p);
             if (t.sign == 0) continue;
-            PullTerm q{};
-            q.x0 = t.x[0], q.x1 = t.x[1], q.z0 = t.z[0], q.z1 = t.z[1];
-            // transpose: bits flipped by X swap their up/down requirement
-            q.up0 = (t.up[0] & ~t.x[0]) | (t.down[0] & t.x[0]);
-            q.up1 = (t.up[1] & ~t.x[1]) | (t.down[1] & t.x[1]);
-            q.dn0 = (t.down[0] & ~t.x[0]) | (t.up[0] & t.x[0]);
-            q.dn1 = (t.down[1] & ~t.x[1]) | (t.up[1] & t.x[1]);
-            // the element is evaluated on the row (pre-image) state: same sign as the
-            // reference's evaluation on the image state, see operator.hpp:246-253
-            q.cs = t.c * (double)t.sign;
-            q.has_z = (t.z[0] | t.z[1]) != 0;
-            q.cs_hi = (float)q.cs;
-            q.cs_lo = (float)(q.cs - (double)q.cs_hi);
-            pull.push_back(q);
+            pull.push_back(transposed_term(t));
         }
         const int n_pull_given = (int)pull.size();
         {

@@ -84,7 +84,9 @@ qsi_status build_hash(qsi_basis* b);
 void drop_hash(qsi_basis* b);
 // qsi_op_create; check_closed: determine op->closed (one pass of lookups over the basis), else it stays 0.
 qsi_status create_op(qsi_basis* b, const qsi_term* terms, int32_t n_terms, bool check_closed, qsi_op** out);
-// Builds op->tile from the transposed terms; sets op->closed.
+// An off-diagonal term in the pull form of the applies.
+PullTerm transposed_term(const qsi_term& t);
+// Builds op->tile from the transposed terms.
 qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull);
 qsi_status find_closed(qsi_op* op);
 // Builds (enable) or frees an operator's lookup cache (qsi_op_materialise); *bytes: its size in device memory.
