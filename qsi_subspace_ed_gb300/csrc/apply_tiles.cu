@@ -556,13 +556,12 @@ inline bool vec16_ok(int64_t n, int R, const void* x, const void* y) {
     return vec4_ok(n, R, x, y) && R >= 64 && (R <= 512 ? (R & (R - 1)) == 0 : (R & 511) == 0);
 }
 
-// Body of the batched tile kernel for one block (block_id of n_blocks working on this operator).
 template <typename XT, class LK, bool kFF, int KM, bool kFam = false>
-__device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, const XT* __restrict__ x,
-                                             XT* __restrict__ y, int R, int accumulate, int cap, int64_t block_id,
-                                             int64_t n_blocks, unsigned char* smem_raw,
-                                             const float2* __restrict__ ycoef = nullptr) {
+__global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
+                                                            XT* __restrict__ y, int R, int accumulate, int cap,
+                                                            const float2* __restrict__ ycoef) {
     // accumulate: y <- H x + c y per column, c = 1, or the (hi, lo) float pair ycoef[column] (double-float paths)
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const TileSmem S = stage_terms(P, lk, kFF, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
@@ -590,7 +589,7 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
         cpw = 32 / lpc;
     }
     const int64_t ntiles = (P.B.n + 31) >> 5;
-    for (int64_t tile = block_id * nw + wid; tile < ntiles; tile += n_blocks * nw) {
+    for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         state2 s = make_ulonglong2(0, 0);
@@ -933,51 +932,6 @@ __device__ __forceinline__ void batched_body(const TileParams& P, const LK& lk, 
             row_start = row_end;
         }
     }
-}
-
-template <typename XT, class LK, bool kFF, int KM, bool kFam = false>
-__global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
-                                                            XT* __restrict__ y, int R, int accumulate, int cap) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    batched_body<XT, LK, kFF, KM, kFam>(P, lk, x, y, R, accumulate, cap, blockIdx.x, gridDim.x, smem_raw);
-}
-
-// Several operators (sectors) in one launch: the grid is partitioned into
-// per-sector block ranges in proportion to each sector's rows x vectors;
-// each block stages its own sector's terms and works through that sector's
-// tiles.  FP32 storage, double-float accumulation; the lookup caches when every
-// sector is materialised, else hash lookups when every sector's batched applies
-// use them, else bucket-table lookups.
-struct SectorLaunch {
-    TileParams P;
-    BinView H;
-    CacheView C;
-    const float* x;
-    float* y;
-    const float2* ycoef;  // accumulating launches: y <- H x + ycoef[c] y per column (nullptr: coefficient 1)
-    int R;
-    int cap;
-    int block_begin;
-    int n_blocks;
-};
-
-template <int KM, class LK>
-__global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_sectors(const SectorLaunch* __restrict__ secs, int n_secs,
-                                                          int accumulate) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SectorLaunch L;
-    if (threadIdx.x == 0) {
-        int s = 0;
-        while (s + 1 < n_secs && (int)blockIdx.x >= secs[s + 1].block_begin) ++s;
-        L = secs[s];
-    }
-    __syncthreads();
-    LK lk;
-    if constexpr (std::is_same<LK, LookupCache>::value) lk = LookupCache{L.C};
-    else if constexpr (std::is_same<LK, LookupTable>::value) lk = LookupTable{L.P.B};
-    else lk = LK{L.H};
-    batched_body<float, LK, true, KM>(L.P, lk, L.x, L.y, L.R, accumulate, L.cap, (int64_t)blockIdx.x - L.block_begin,
-                                      L.n_blocks, smem_raw, L.ycoef);
 }
 
 // Per-row diagonal, evaluated once per operator with the same arithmetic as
@@ -1451,11 +1405,11 @@ static int tile_grid(int64_t ntiles, int block, int bps) {
 
 template <class LK>
 static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int R, int xdtype, int ydtype,
-                                  int accumulate, cudaStream_t st) {
-    const qsi_tuning& T = op->tune[R > 1];
+                                  int accumulate, cudaStream_t st, bool batched, const float2* ycoef) {
+    const qsi_tuning& T = op->tune[batched];
     TileParams P = tile_params(op, T.vec_chunk);
     const int64_t ntiles = (P.B.n + 31) / 32;
-    if (R == 1) {
+    if (!batched) {
         if constexpr (std::is_same<LK, LookupCache>::value) return fail(QSI_INVALID_ARG, "tile apply: no cached form");
         else {
             auto go = [&](auto xt, auto yt) {
@@ -1481,7 +1435,7 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
                 auto k = k_apply_tile_batched<double, LK, false, KM>;
                 set_smem(k, smem);
                 k<<<one_wave(k, block, smem, ntiles, T.grid_bps), block, smem, st>>>(P, lk, (const double*)x, (double*)y, R,
-                                                                         accumulate, cap);
+                                                                         accumulate, cap, ycoef);
             } else if (op->ff_accumulate) {
                 auto k = (T.vec_width == 16 && vec16_ok(P.B.n, R, x, y)) ? k_apply_tile_batched<float, LK, true, kVec16>
                          : (T.vec_width == 8 && vec8_ok(P.B.n, R, x, y))  ? k_apply_tile_batched<float, LK, true, kVec8>
@@ -1489,12 +1443,12 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
                                                                           : k_apply_tile_batched<float, LK, true, KM>;
                 set_smem(k, smem);
                 k<<<one_wave(k, block, smem, ntiles, T.grid_bps), block, smem, st>>>(P, lk, (const float*)x, (float*)y, R,
-                                                                         accumulate, cap);
+                                                                         accumulate, cap, ycoef);
             } else {
                 auto k = k_apply_tile_batched<float, LK, false, KM>;
                 set_smem(k, smem);
                 k<<<one_wave(k, block, smem, ntiles, T.grid_bps), block, smem, st>>>(P, lk, (const float*)x, (float*)y, R,
-                                                                         accumulate, cap);
+                                                                         accumulate, cap, ycoef);
             }
         };
         if (R <= kGroupMax) go(std::integral_constant<int, kGroup>{});
@@ -1506,96 +1460,6 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
     if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "tile apply launch: %s", cudaGetErrorString(e));
     return QSI_OK;
 }
-
-// Several sectors in one launch (FP32 batched, double-float), in two steps: plan_sectors builds the per-sector
-// launch records on the host (block ranges in proportion to weights, e.g. each sector's measured apply time, or
-// else to rows x vectors; shared memory for the largest sector); the caller copies plan.records to device memory once, and launch_sectors enqueues the
-// kernel (capturable into a CUDA graph: it does no host-to-device copy).
-qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float* const* Y, const int* R,
-                        SectorPlan& plan, const double* weights, const float2* const* ycoef) {
-    std::vector<SectorLaunch> L(n);
-    plan.vec4 = true;
-    plan.vec8 = true;
-    plan.vec16 = true;
-    plan.hash = true;
-    plan.closed = true;
-    plan.cache = true;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int block = 256;  // the largest that every sector's term list leaves room for
-    for (int s = 0; s < n; ++s) block = std::min(block, tile_launch(ops[s], 16, ops[s]->tune[1].list_cap).block);
-    const int nw = block / 32;
-    size_t smem = 0;
-    int maxR = 1;
-    double work_total = 0;
-    for (int s = 0; s < n; ++s) {
-        qsi_op* op = ops[s];
-        if (op->kernel != 1) return fail(QSI_INVALID_ARG, "sector launch needs the tile kernels");
-        plan.hash = plan.hash && op->basis->d_bins && op->tune[1].use_hash;
-        plan.closed = plan.closed && op->closed;
-        plan.cache = plan.cache && op->d_cache_cols;
-        const int cap = tile_launch(op, 16, op->tune[1].list_cap).cap;
-        smem = std::max(smem, tile_smem(op->tile) + nw * (scratch_bytes((op->tile.n + 31) / 32) + (size_t)cap * 16));
-        L[s].P = tile_params(op, op->tune[1].vec_chunk);
-        L[s].H = op->basis->bview();
-        L[s].C = cache_view(op);
-        L[s].x = X[s];
-        L[s].y = Y[s];
-        L[s].ycoef = ycoef ? ycoef[s] : nullptr;
-        L[s].R = R[s];
-        L[s].cap = cap;
-        maxR = std::max(maxR, R[s]);
-        plan.vec4 = plan.vec4 && vec4_ok(op->basis->n, R[s], X[s], Y[s]);
-        plan.vec8 = plan.vec8 && op->tune[1].vec_width == 8 && vec8_ok(op->basis->n, R[s], X[s], Y[s]);
-        plan.vec16 = plan.vec16 && op->tune[1].vec_width == 16 && vec16_ok(op->basis->n, R[s], X[s], Y[s]);
-        work_total += weights ? weights[s] : (double)op->basis->n * R[s];
-    }
-    if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "sector launch: %zu bytes of shared memory needed", smem);
-    // one wave of the kernel's resident blocks per SM, or the first sector's tuned blocks per SM
-    const int bps = ops[0]->tune[1].grid_bps;
-    const int total = sms * (bps > 0 ? bps : plan.vec4 ? 2 : 3);
-    int begin = 0;
-    for (int s = 0; s < n; ++s) {
-        const int64_t tiles = (ops[s]->basis->n + 31) / 32;
-        const double work = weights ? weights[s] : (double)ops[s]->basis->n * R[s];
-        int b = (int)std::llround(total * work / std::max(work_total, 1e-30));
-        b = (int)std::max<int64_t>(1, std::min<int64_t>(b, (tiles + nw - 1) / nw));
-        L[s].block_begin = begin;
-        L[s].n_blocks = b;
-        begin += b;
-    }
-    plan.records.assign((const unsigned char*)L.data(), (const unsigned char*)(L.data() + n));
-    plan.smem = smem;
-    plan.maxR = maxR;
-    plan.grid = begin;
-    plan.block = block;
-    plan.n = n;
-    return QSI_OK;
-}
-
-qsi_status launch_sectors(const void* d_records, const SectorPlan& plan, int accumulate, cudaStream_t st) {
-    auto go = [&](auto km) {
-        constexpr int KM = decltype(km)::value;
-        auto k = plan.cache ? k_apply_sectors<KM, LookupCache>
-                 : plan.hash && plan.closed ? k_apply_sectors<KM, LookupBins<true>>
-                 : plan.hash ? k_apply_sectors<KM, LookupBins<false>>
-                             : k_apply_sectors<KM, LookupTable>;
-        set_smem(k, plan.smem);
-        k<<<plan.grid, plan.block, plan.smem, st>>>((const SectorLaunch*)d_records, plan.n, accumulate);
-    };
-    if (plan.vec16) go(std::integral_constant<int, kVec16>{});
-    else if (plan.vec8) go(std::integral_constant<int, kVec8>{});
-    else if (plan.vec4) go(std::integral_constant<int, kVec4>{});
-    else if (plan.maxR <= kGroupMax) go(std::integral_constant<int, kGroup>{});
-    else if (plan.maxR <= 32) go(std::integral_constant<int, 1>{});
-    else if (plan.maxR <= 64) go(std::integral_constant<int, 2>{});
-    else go(std::integral_constant<int, 4>{});
-    QSI_CUDA(cudaGetLastError());
-    return QSI_OK;
-}
-
-size_t sector_launch_bytes() { return sizeof(SectorLaunch); }
 
 qsi_status preload_apply_f64_rows();  // operator.cu: the row-per-thread kernel
 
@@ -1638,7 +1502,7 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
             auto k = k_apply_tile_batched<double, LK, false, KM, true>;
             set_smem(k, smem);
             k<<<one_wave(k, block, smem, ntiles, tmpl->tune[1].grid_bps), block, smem, st>>>(P, lk, x, y, R, accumulate,
-                                                                                             cap);
+                                                                                             cap, nullptr);
         };
         if (R <= kGroupMax) go(std::integral_constant<int, kGroup>{});
         else if (R <= 32) go(std::integral_constant<int, 1>{});
@@ -1660,19 +1524,26 @@ qsi_status launch_family(qsi_op* tmpl, const double* x, double* y, int R, const 
     return launch_family_lk(tmpl, LookupTable{tmpl->basis->view()}, x, y, R, fcoef, accumulate, st);
 }
 
+static qsi_status launch_tiles(qsi_op* op, const void* x, void* y, int R, int xdtype, int ydtype, int accumulate,
+                               cudaStream_t st, bool batched, const float2* ycoef) {
+    auto go = [&](auto lk) { return launch_tiles_lk(op, lk, x, y, R, xdtype, ydtype, accumulate, st, batched, ycoef); };
+    if (op->d_cache_cols) return go(LookupCache{cache_view(op)});
+    if (op->basis->d_bins && op->tune[batched].use_hash) {
+        if (op->closed) return go(LookupBins<true>{op->basis->bview()});
+        return go(LookupBins<false>{op->basis->bview()});
+    }
+    return go(LookupTable{op->basis->view()});
+}
+
 qsi_status launch_apply_tiles(qsi_op* op, const void* x, void* y, int R, int xdtype, int ydtype, int accumulate,
                               cudaStream_t st) {
-    if (op->d_cache_cols) {
-        if (R == 1) return launch_cached(op, x, y, xdtype, ydtype, accumulate, st);
-        return launch_tiles_lk(op, LookupCache{cache_view(op)}, x, y, R, xdtype, ydtype,
-                               accumulate, st);
-    }
-    if (op->basis->d_bins && op->tune[R > 1].use_hash) {
-        if (op->closed)
-            return launch_tiles_lk(op, LookupBins<true>{op->basis->bview()}, x, y, R, xdtype, ydtype, accumulate, st);
-        return launch_tiles_lk(op, LookupBins<false>{op->basis->bview()}, x, y, R, xdtype, ydtype, accumulate, st);
-    }
-    return launch_tiles_lk(op, LookupTable{op->basis->view()}, x, y, R, xdtype, ydtype, accumulate, st);
+    if (R == 1 && op->d_cache_cols) return launch_cached(op, x, y, xdtype, ydtype, accumulate, st);
+    return launch_tiles(op, x, y, R, xdtype, ydtype, accumulate, st, R > 1, nullptr);
+}
+
+qsi_status launch_apply_ff(qsi_op* op, const float* x, float* y, int R, int accumulate, const float2* ycoef,
+                           cudaStream_t st) {
+    return launch_tiles(op, x, y, R, QSI_F32, QSI_F32, accumulate, st, true, ycoef);
 }
 
 // Builds (enable) or frees the operator's lookup cache; *bytes: its size.

@@ -2258,14 +2258,29 @@ __global__ void __launch_bounds__(256) k_col_dots(const VT* __restrict__ a, cons
     col_block_sum<VW>(L, res, R, sh, partial);
 }
 
+// Sum over blocks of partial[b][r] in block order, sixteen loads ahead of the adds: the adds are a chain (their order
+// fixes the recurrences' rounding), the loads need not be.
+__device__ __forceinline__ double col_sum(const double* __restrict__ partial, int nblocks, int R, int r) {
+    double t = 0.0;
+    int b = 0;
+    for (; b + 16 <= nblocks; b += 16) {
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = __ldg(partial + (int64_t)(b + u) * R + r);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) t += v[u];
+    }
+    for (; b < nblocks; ++b) t += partial[(int64_t)b * R + r];
+    return t;
+}
+
 // out[r] = sum over blocks of partial[b][r] (its square root with sqrt_out, and then also the column's
 // scale 1/out[r] for k_col_scale: FP64 and as a (hi, lo) float pair).
 __global__ void k_col_reduce(const double* __restrict__ partial, int nblocks, int R, double* __restrict__ out,
                              int sqrt_out, double* __restrict__ inv = nullptr, float2* __restrict__ inv_ff = nullptr,
                              float2* __restrict__ neg_ff = nullptr) {
     for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        double t = 0.0;
-        for (int b = 0; b < nblocks; ++b) t += partial[(int64_t)b * R + r];
+        const double t = col_sum(partial, nblocks, R, r);
         out[r] = sqrt_out ? sqrt(t) : t;
         if (inv) {
             const double v = out[r] > 0 ? 1.0 / out[r] : 1.0;
@@ -2460,12 +2475,8 @@ __global__ void k_ftlm_coef3(const double* __restrict__ partial, int nblocks, in
                              float2* __restrict__ neg_ff) {
     const int64_t stride = (int64_t)nblocks * R;
     for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        double cp = 0.0, pp = 0.0, cc = 0.0;
-        for (int b = 0; b < nblocks; ++b) {
-            cp += partial[(int64_t)b * R + r];
-            pp += partial[stride + (int64_t)b * R + r];
-            cc += partial[2 * stride + (int64_t)b * R + r];
-        }
+        const double cp = col_sum(partial, nblocks, R, r), pp = col_sum(partial + stride, nblocks, R, r),
+                     cc = col_sum(partial + 2 * stride, nblocks, R, r);
         const double a = cp;
         const double b2 = pp - 2.0 * a * cp + a * a * cc;
         const double b = b2 > 0.0 ? sqrt(b2) : 0.0;
@@ -2533,33 +2544,74 @@ struct FtlmSector {
     DevBuf<float2> inv_ff, nbeta_ff;
 };
 
-// All sectors advance together: per step one apply launch covering every sector
-// (FP32 storage with hash indexes) or one per sector, then the per-sector
-// recurrence kernels.  The whole M-step run is captured into one CUDA graph.
+// The sectors' recurrences do not touch one another: the whole run is one CUDA graph with a branch per sector (at most
+// kFtlmBranches), so one sector's reductions (a chain of FP64 adds on one SM) and the tail of its apply overlap with
+// another's work, and every apply is the kernel that suits its sector.  One apply launch for all sectors, its blocks
+// shared out by measured times, ran the lookups of every sector as the least favourable one needs them and waited for
+// the slowest block of each step: 6.2 ms for three sectors (64-spin Q=0, one pair; 32-spin two pairs) whose applies
+// take 1.0, 2.5 and 0.7 ms, beside 1.4 ms of column passes one after another.
 //
 // Three blocks of R vectors per sector (prev P, current C, W = H C):
 //   W = H C;  alpha = <C, W>;  P <- W - alpha C - beta_prev P;  beta = |P|;  P /= beta;  swap(P, C).
 // Two blocks (blocks == 2, or blocks == 0 when three do not fit in free device memory), the in-place
 // recurrence with P holding q_prev at the start of a step:
 //   P <- H C - beta_prev P;  alpha = <C, P>;  P <- P - alpha C;  beta = |P|;  P /= beta;  swap(P, C).
-// The one-launch sector apply takes -beta_prev per column as its accumulate coefficient (double-float), and its
-// column work is two passes (k_col_dots3: <C, P>, |P|^2 and |C|^2 in one read; k_ftlm_update_scaled:
-// P <- (P - alpha C) / beta), so a step moves 6 blocks beyond the apply's gathers against 9 for three blocks,
-// though the accumulating apply is slower on small sectors: three blocks are taken when they fit.  The
-// per-sector launches instead have the column pass also scale C by -beta for the next step.
+// The double-float apply takes -beta_prev per column as its accumulate coefficient, and its column work is two passes
+// (k_col_dots3: <C, P>, |P|^2 and |C|^2 in one read; k_ftlm_update_scaled: P <- (P - alpha C) / beta), so a step moves
+// 6 blocks beyond the apply's gathers against 9 for three blocks, though the accumulating apply is slower on small
+// sectors: three blocks are taken when they fit.  The other applies instead have the column pass also scale C by
+// -beta for the next step.
+constexpr int kFtlmBranches = 8;
+
+// Streams and events of the graph's branches: the first is the run's own stream.
+struct Branches {
+    std::vector<cudaStream_t> st;
+    std::vector<cudaEvent_t> ev;
+    qsi_status init(int n, cudaStream_t own) {
+        st.assign(1, own);
+        for (int b = 0; b < n; ++b) {
+            cudaEvent_t e = nullptr;
+            QSI_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            ev.push_back(e);
+            if (b == 0) continue;
+            cudaStream_t s = nullptr;
+            QSI_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            st.push_back(s);
+        }
+        return QSI_OK;
+    }
+    cudaError_t fork() {
+        cudaError_t e = cudaEventRecord(ev[0], st[0]);
+        for (size_t b = 1; b < st.size() && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(st[b], ev[0], 0);
+        return e;
+    }
+    cudaError_t join() {
+        cudaError_t e = cudaSuccess;
+        for (size_t b = 1; b < st.size() && e == cudaSuccess; ++b) {
+            e = cudaEventRecord(ev[b], st[b]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(st[0], ev[b], 0);
+        }
+        return e;
+    }
+    ~Branches() {
+        for (size_t b = 1; b < st.size(); ++b) cudaStreamDestroy(st[b]);
+        for (cudaEvent_t e : ev) cudaEventDestroy(e);
+    }
+};
+
 template <typename VT>
 static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint64_t seed, double* alphas,
                            double* betas, int blocks) {
     cudaStream_t st = ops[0]->stream;
     std::vector<FtlmSector<VT>> S(ns);
-    bool one_launch = (sizeof(VT) == 4);
+    std::vector<char> ff(ns);  // sectors whose FP32 applies sum in double-float
     size_t block_bytes = 0;
     for (int s = 0; s < ns; ++s) {
         const int R = Rs[s];
         if (R <= 0 || R > 256 || (R & (R - 1))) return fail(QSI_INVALID_ARG, "ftlm: R must be a power of two in [1,256]");
         if (ops[s]->basis->n < 1) return fail(QSI_INVALID_ARG, "ftlm: empty sector");
         block_bytes += (size_t)ops[s]->basis->n * R * sizeof(VT);
-        one_launch = one_launch && ops[s]->kernel == 1 && ops[s]->ff_accumulate;
+        ff[s] = sizeof(VT) == 4 && ops[s]->kernel == 1 && ops[s]->ff_accumulate;
     }
     if (blocks == 0) {  // three blocks when they fit with 4 GiB to spare, else two
         size_t free_b = 0, total_b = 0;
@@ -2586,81 +2638,37 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
     }
     std::vector<VT*> prev(ns), cur(ns);
     for (int s = 0; s < ns; ++s) prev[s] = S[s].P.p, cur[s] = S[s].C.p;
-    // one-launch plans for even steps (input C) and odd steps (input P), uploaded before capture
-    SectorPlan plan[2];
-    DevBuf<unsigned char> d_plan[2];
-    if (one_launch) {
-        std::vector<qsi_op*> opv(ops, ops + ns);
-        // Blocks are shared out in proportion to each sector's apply time alone (rows, vectors, hits and lookup
-        // misses all count): one warm-up and one timed apply per sector, W = H C on the run's own buffers.
-        std::vector<double> weight(ns, 1.0);
-        if (ns > 1) {
-            cudaEvent_t e0 = nullptr, e1 = nullptr;
-            QSI_CUDA(cudaEventCreate(&e0));
-            QSI_CUDA(cudaEventCreate(&e1));
-            qsi_status ts = QSI_OK;
-            for (int s = 0; s < ns && ts == QSI_OK; ++s) {
-                VT* out = two ? S[s].P.p : S[s].W.p;  // P is zeroed again below
-                ts = launch_apply(ops[s], S[s].C.p, out, S[s].R, QSI_F32, 0, st);
-                if (ts == QSI_OK && cudaEventRecord(e0, st) != cudaSuccess) ts = QSI_CUDA_ERROR;
-                if (ts == QSI_OK) ts = launch_apply(ops[s], S[s].C.p, out, S[s].R, QSI_F32, 0, st);
-                float ms = 0.f;
-                if (ts == QSI_OK && (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-                                     cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess))
-                    ts = fail(QSI_CUDA_ERROR, "ftlm: sector timing failed");
-                weight[s] = std::max(1e-3, (double)ms);
-            }
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
-            if (ts != QSI_OK) return ts;
-            if (two)
-                for (int s = 0; s < ns; ++s)
-                    QSI_CUDA(cudaMemsetAsync(S[s].P.p, 0, (size_t)S[s].n * S[s].R * sizeof(VT), st));
-        }
-        for (int parity = 0; parity < 2; ++parity) {
-            std::vector<const float*> X(ns);
-            std::vector<float*> Y(ns);
-            for (int s = 0; s < ns; ++s) {
-                X[s] = (const float*)(parity ? S[s].P.p : S[s].C.p);
-                Y[s] = (float*)(two ? (parity ? S[s].C.p : S[s].P.p) : S[s].W.p);
-            }
-            // two blocks: the accumulating apply scales the previous block by -beta_prev itself
-            std::vector<const float2*> yc(ns);
-            for (int s = 0; s < ns; ++s) yc[s] = S[s].nbeta_ff.p;
-            qsi_status ps = plan_sectors(opv.data(), ns, X.data(), Y.data(), Rs, plan[parity], weight.data(),
-                                         two ? yc.data() : nullptr);
-            if (ps != QSI_OK) return ps;
-            QSI_CUDA(d_plan[parity].alloc(plan[parity].records.size(), st));
-            QSI_CUDA(cudaMemcpyAsync(d_plan[parity].p, plan[parity].records.data(), plan[parity].records.size(),
-                                     cudaMemcpyHostToDevice, st));
-        }
+    Branches br;
+    {
+        const qsi_status bs = br.init(std::min(ns, kFtlmBranches), st);
+        if (bs != QSI_OK) return bs;
     }
     QSI_CUDA(cudaStreamSynchronize(st));
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     QSI_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    qsi_status status = QSI_OK;
+    qsi_status status = br.fork() == cudaSuccess ? QSI_OK : fail(QSI_CUDA_ERROR, "ftlm: graph branches");
     const int blk = 256;
-    for (int j = 0; j < M && status == QSI_OK; ++j) {
-        // two blocks: the apply accumulates into prev, which holds q_prev (zero at the first step) and is scaled
-        // by -beta_prev on the way: inside the sector launch, else by the previous step's column pass
-        if (one_launch) {
-            status = launch_sectors(d_plan[j & 1].p, plan[j & 1], two ? 1 : 0, st);
-        } else {
-            for (int s = 0; s < ns && status == QSI_OK; ++s)
-                status = launch_apply(ops[s], cur[s], two ? prev[s] : S[s].W.p, S[s].R,
-                                      sizeof(VT) == 4 ? QSI_F32 : QSI_F64, two ? 1 : 0, st);
-        }
-        for (int s = 0; s < ns; ++s) {
-            FtlmSector<VT>& F = S[s];
-            double* dA = F.ab.p;
-            double* dB = F.ab.p + (size_t)M * F.R;
+    for (int s = 0; s < ns && status == QSI_OK; ++s) {
+        FtlmSector<VT>& F = S[s];
+        cudaStream_t st = br.st[s % br.st.size()];  // this sector's branch
+        double* dA = F.ab.p;
+        double* dB = F.ab.p + (size_t)M * F.R;
+        for (int j = 0; j < M && status == QSI_OK; ++j) {
+            // two blocks: the apply accumulates into prev, which holds q_prev (zero at the first step) and is scaled
+            // by -beta_prev on the way: inside the double-float apply, else by the previous step's column pass
+            VT* out = two ? prev[s] : F.W.p;
+            if (ff[s])
+                status = launch_apply_ff(ops[s], reinterpret_cast<const float*>(cur[s]), reinterpret_cast<float*>(out), F.R,
+                                         two ? 1 : 0, two ? F.nbeta_ff.p : nullptr, st);
+            else
+                status = launch_apply(ops[s], cur[s], out, F.R, sizeof(VT) == 4 ? QSI_F32 : QSI_F64, two ? 1 : 0, st);
             const double* bprev = j ? dB + (size_t)(j - 1) * F.R : nullptr;
             double* beta = dB + (size_t)j * F.R;
             auto col_step = [&](auto vw) {
                 constexpr int VW = decltype(vw)::value;
                 if constexpr (sizeof(VT) == 4) {
-                    if (one_launch && two) {  // two passes: three dots, then (P - alpha C) / beta
+                    if (ff[s] && two) {  // two passes: three dots, then (P - alpha C) / beta
                         const float* c = reinterpret_cast<const float*>(cur[s]);
                         float* p = reinterpret_cast<float*>(prev[s]);
                         k_col_dots3<VW><<<kColGrid, blk, 0, st>>>(c, p, F.n, F.R, F.partial.p);
@@ -2682,7 +2690,7 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
                 k_col_reduce<<<1, 256, 0, st>>>(F.partial.p, kColGrid, F.R, beta, 1, F.inv.p, F.inv_ff.p,
                                                 two ? F.nbeta_ff.p : nullptr);
                 k_col_scale<VT, VW><<<grid_for(F.n * F.R / VW, 256), 256, 0, st>>>(
-                    prev[s], F.inv.p, F.inv_ff.p, F.n, F.R, (two && !one_launch) ? cur[s] : nullptr, beta,
+                    prev[s], F.inv.p, F.inv_ff.p, F.n, F.R, (two && !ff[s]) ? cur[s] : nullptr, beta,
                     F.nbeta_ff.p);
             };
             constexpr int kVW = 16 / sizeof(VT);  // 16-byte accesses when R allows
@@ -2691,6 +2699,7 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
             std::swap(prev[s], cur[s]);
         }
     }
+    if (br.join() != cudaSuccess && status == QSI_OK) status = fail(QSI_CUDA_ERROR, "ftlm: graph branches");
     cudaError_t ce = cudaStreamEndCapture(st, &graph);
     if (status != QSI_OK) {
         if (graph) cudaGraphDestroy(graph);

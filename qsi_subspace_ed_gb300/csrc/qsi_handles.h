@@ -98,19 +98,9 @@ qsi_status preload_apply_f64();
 // Looks the static staging arrays of qsi_op_apply_static up on the current device (once per device).
 qsi_status static_stage_prepare();
 qsi_status build_diag(qsi_op* op);
-struct SectorPlan {
-    std::vector<unsigned char> records;  // one launch record per sector, to be copied to device memory
-    size_t smem = 0;
-    int maxR = 1, grid = 0, block = 256, n = 0;
-    bool vec4 = true;  // every sector's R and vectors take 16-byte gathers
-    bool vec8 = true;  // ... of 8 vectors per lane, and every sector's batched applies are set to them
-    bool vec16 = true; // ... of 16 vectors per lane, likewise
-    bool hash = true;  // every sector's batched applies look columns up through the hash index
-    bool closed = true; // ... and no admitted term leaves any sector's basis
-    bool cache = true; // every sector is materialised (qsi_op_materialise): columns come from the lookup caches
-};
-qsi_status plan_sectors(qsi_op* const* ops, int n, const float* const* X, float* const* Y, const int* R,
-                        SectorPlan& plan, const double* weights = nullptr, const float2* const* ycoef = nullptr);
-qsi_status launch_sectors(const void* d_records, const SectorPlan& plan, int accumulate, cudaStream_t st);
+// Y <- H X + c Y for R FP32 vectors [row][R] summed in double-float (the tile kernels, also for R = 1): c = 0
+// (accumulate = 0), 1, or per column the (hi, lo) float pair ycoef[column].
+qsi_status launch_apply_ff(qsi_op* op, const float* x, float* y, int R, int accumulate, const float2* ycoef,
+                           cudaStream_t st);
 qsi_status jacobi_eigh(const std::vector<double>& A, int m, int n_mat, std::vector<double>& w, std::vector<double>& V, cudaStream_t st);
 }  // namespace qsi
