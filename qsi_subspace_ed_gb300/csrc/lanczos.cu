@@ -34,7 +34,11 @@ static int dot_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(kDotMaxGrid, (n + 2 * kDotBlock - 1) / (2 * kDotBlock)));
 }
 
-// Sum of v over the block's threads (a power of two, at least 32), valid in thread 0.
+// Blocks of 256 threads for a scaling pass whose blocks each work out the factor first.
+static int scale_grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(912, (n + 1023) / 1024)); }
+
+// Sum of v over the block's threads (whole warps), valid in thread 0: a dependent FP64 add takes 65 cycles here, so both
+// levels are trees.
 __device__ __forceinline__ double block_sum(double v, double* sh) {
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -42,22 +46,34 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     if (l == 0) sh[w] = v;
     __syncthreads();
     double r = 0.0;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) r += sh[k];
+    if (w == 0) {
+        r = l < (int)(blockDim.x >> 5) ? sh[l] : 0.0;
+        for (int o = 16; o; o >>= 1)
+            if (o < (int)(blockDim.x >> 5)) r += __shfl_down_sync(0xffffffffu, r, o);
+    }
     return r;
 }
 
-// Sum of count partial sums, the same in every block that computes it: warp 0 adds them lane by lane, then across the
-// lanes; every thread receives it.
-__device__ __forceinline__ double sum_partials(const double* __restrict__ partial, int count, double* sh) {
+// f(sum of count partial sums), the same in every block that computes it: four sums per lane of warp 0, then a tree;
+// every thread receives it.  One thread evaluates f: an FP64 square root and division by all threads of all blocks
+// took the FP64 pipe longer than the scaling they are for (27.8 us at 2.9 M rows).
+template <class F>
+__device__ __forceinline__ double of_partials(const double* __restrict__ partial, int count, double* sh, F&& f) {
     if (threadIdx.x < 32) {
-        double v = 0.0;
-        for (int b = threadIdx.x; b < count; b += 32) v += partial[b];
-        for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) *sh = v;
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int b = threadIdx.x; b < count; b += 128)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (b + 32 * u < count) v[u] += partial[b + 32 * u];
+        double t = (v[0] + v[1]) + (v[2] + v[3]);
+        for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) *sh = f(t);
     }
     __syncthreads();
     return *sh;
+}
+__device__ __forceinline__ double sum_partials(const double* __restrict__ partial, int count, double* sh) {
+    return of_partials(partial, count, sh, [](double t) { return t; });
 }
 
 // Double-float accumulator (two FP32 words, about 2^-46 relative): a += x * (ch + cl), x an FP32 value, with an
@@ -312,9 +328,11 @@ __global__ void __launch_bounds__(256) k_krylov_scale(const typename K::W* __res
                                                       double* __restrict__ beta, typename K::V* __restrict__ out,
                                                       int64_t n) {
     __shared__ double sh;
-    const double nrm = sqrt(fmax(sum_partials(partial, n_partial, &sh), 0.0));
-    if (blockIdx.x == 0 && threadIdx.x == 0) *beta = nrm;
-    const double inv = 1.0 / nrm;
+    const double inv = of_partials(partial, n_partial, &sh, [&](double t) {
+        const double nrm = sqrt(fmax(t, 0.0));
+        if (blockIdx.x == 0) *beta = nrm;
+        return 1.0 / nrm;
+    });
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
         out[r] = K::scaled(w[r], inv);
 }
@@ -419,10 +437,26 @@ __global__ void __launch_bounds__(128) k_ritz_vectors(const VT* __restrict__ V, 
 // eigenvalues ascending to evals, eigenvectors as columns of evecs (row-major M x M).  Padding rows/columns of zeros
 // stay decoupled.  A round rotates M/2 disjoint pairs (round-robin order) at once: the angles, then every 2 x 2 block
 // of A from both sides and every row of the eigenvectors (in shared memory when both fit), so a round has two barriers.
-// A pair is left alone when its off-diagonal element is below 1e-17 of the matrix's norm, a rotated one's is set to
-// zero, and a sweep without rotations ends the iteration: 6-8 sweeps.  (A test on the whole off-diagonal mass never
+// A pair is left alone when its off-diagonal element is below 1e-17 of the matrix's norm, and a sweep without rotations
+// ends the iteration: 6-9 sweeps.  (A test on the whole off-diagonal mass never
 // passed for elements that are left at rounding size: every call took all 60 sweeps, 5.6 ms for a 24 x 24 matrix
 // against 0.3 ms.)
+// Cosine and sine of a rotation that all but clears apq (to about 1e-7 of it; the next sweep finds the rest): the
+// tangent in FP32, from elements scaled into its range, and c = 1 / sqrt(1 + t^2) in FP64 by Newton's iteration from the
+// FP32 value, so the rotation is orthogonal to rounding whatever the tangent's error.  An FP64 division takes 446
+// cycles and a square root 691; three and two of them in a chain were most of a round.
+__device__ __forceinline__ void rotation(double app, double aqq, double apq, double scale, double& c, double& s) {
+    const float d = (float)((aqq - app) * scale), o = (float)(apq * scale);
+    const float theta = d / (2.0f * o);
+    const float tf = (theta >= 0.f ? 1.0f : -1.0f) / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
+    const double t = (double)tf, x = fma(t, t, 1.0);
+    double y = (double)rsqrtf((float)x);  // 1 <= x <= 2
+    y = fma(y, fma(-0.5 * x * y, y, 0.5), y);
+    y = fma(y, fma(-0.5 * x * y, y, 0.5), y);
+    c = y;
+    s = t * y;
+}
+
 __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, int M, double* __restrict__ evals,
                                                 double* __restrict__ evecs, int max_sweeps, int v_shared) {
     extern __shared__ double sm[];
@@ -434,7 +468,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
     int* qq = pp + H;
     double* V = v_shared ? sn + H + H : evecs + (int64_t)blockIdx.x * M * M;  // 2 * H ints take H doubles
     __shared__ double red[32];
-    __shared__ double tau;
+    __shared__ double tau, inv_norm;
     const double* Ab = Ain + (int64_t)blockIdx.x * M * M;
     double* Vb = evecs + (int64_t)blockIdx.x * M * M;
     double* eb = evals + (int64_t)blockIdx.x * M;
@@ -445,8 +479,12 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
         nrm += Ab[i] * Ab[i];
     }
     nrm = block_sum(nrm, red);
-    if (threadIdx.x == 0) tau = 1e-17 * sqrt(nrm);
+    if (threadIdx.x == 0) {
+        tau = nrm > 0.0 ? 1e-17 * sqrt(nrm) : 1e300;
+        inv_norm = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
+    }
     __syncthreads();
+    const double scale = inv_norm;
     const int nblk = H * (H + 1) / 2;  // blocks (t, u), t <= u
     for (int sweep = 0; sweep < max_sweeps; ++sweep) {
         int rotated = 0;
@@ -467,10 +505,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
                 const double apq = A[p * M + q];
                 double c = 1.0, s = 0.0;
                 if (fabs(apq) > tau) {
-                    const double theta = (A[q * M + q] - A[p * M + p]) / (2.0 * apq);
-                    const double tt = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                    c = 1.0 / sqrt(tt * tt + 1.0);
-                    s = tt * c;
+                    rotation(A[p * M + p], A[q * M + q], apq, scale, c, s);
                     any = 1;
                 }
                 cs[t] = c;
@@ -493,9 +528,10 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
                 // rows p1, q1 then columns p2, q2
                 const double bpp = c1 * app - s1 * aqp, bpq = c1 * apq - s1 * aqq;
                 const double bqp = s1 * app + c1 * aqp, bqq = s1 * apq + c1 * aqq;
-                double dpp = c2 * bpp - s2 * bpq, dpq = s2 * bpp + c2 * bpq;
-                double dqp = c2 * bqp - s2 * bqq, dqq = s2 * bqp + c2 * bqq;
-                if (u == v) dpq = dqp = 0.0;
+                const double dpp = c2 * bpp - s2 * bpq, dpq = s2 * bpp + c2 * bpq;
+                double dqp = c2 * bqp - s2 * bqq;
+                const double dqq = s2 * bqp + c2 * bqq;
+                if (u == v) dqp = dpq;
                 A[p1 * M + p2] = dpp;
                 A[p1 * M + q2] = dpq;
                 A[q1 * M + p2] = dqp;
@@ -902,7 +938,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
             k_krylov_alpha<K><<<grid, kDotBlock, 0, st>>>(vec(j), w.p, n, alpha_partial);
             orth_pass(j, 1, j > 0 ? 2 : 1, 1);
         }
-        k_krylov_scale<K><<<grid_for(n, 256), 256, 0, st>>>(wk, vx.partial, grid, d_beta + j, vec(j + 1), n);
+        k_krylov_scale<K><<<scale_grid(n), 256, 0, st>>>(wk, vx.partial, grid, d_beta + j, vec(j + 1), n);
         QSI_CUDA(cudaGetLastError());
         return QSI_OK;
     };
@@ -910,7 +946,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     k_randn<<<grid_for(n, 256), 256, 0, st>>>(w.p, n, cfg.seed, 0);
     k_krylov_alpha<Vec64><<<grid, kDotBlock, 0, st>>>(w.p, w.p, n, vx.partial);
     if (sizeof(VT) == 4) k_krylov_convert<K><<<grid_for(n, 256), 256, 0, st>>>(w.p, n);
-    k_krylov_scale<K><<<grid_for(n, 256), 256, 0, st>>>(wk, vx.partial, grid, d_beta, vec(0), n);
+    k_krylov_scale<K><<<scale_grid(n), 256, 0, st>>>(wk, vx.partial, grid, d_beta, vec(0), n);
     std::vector<double> alpha(m, 0.0), beta(m, 0.0), theta, coup;  // coup[i] = s_i couplings after restart
     std::vector<double> hcoef((size_t)2 * m);
     int k = 0;
@@ -944,7 +980,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
             double kept = alpha[j];
             orth_pass(j, 1, 0, 0);
             orth_pass(j, 0, 0, 0);
-            k_krylov_scale<K><<<grid_for(n, 256), 256, 0, st>>>(wk, vx.partial, grid, d_beta + j, vec(j + 1), n);
+            k_krylov_scale<K><<<scale_grid(n), 256, 0, st>>>(wk, vx.partial, grid, d_beta + j, vec(j + 1), n);
             QSI_CUDA(cudaMemcpyAsync(d_alpha + j, &kept, 8, cudaMemcpyHostToDevice, st));
             QSI_CUDA(cudaMemcpyAsync(d_beta + j, &zero, 8, cudaMemcpyHostToDevice, st));
             QSI_CUDA(cudaStreamSynchronize(st));
@@ -1564,9 +1600,11 @@ __global__ void __launch_bounds__(kDotBlock) k_three_term_subtract(const double*
 __global__ void __launch_bounds__(256) k_three_term_scale(double* __restrict__ u, const double* __restrict__ norm_partial,
                                                           int n_partial, double* __restrict__ beta, int64_t n) {
     __shared__ double sh;
-    const double b = sqrt(sum_partials(norm_partial, n_partial, &sh));
-    if (blockIdx.x == 0 && threadIdx.x == 0) *beta = b;
-    const double inv = 1.0 / b;
+    const double inv = of_partials(norm_partial, n_partial, &sh, [&](double t) {
+        const double b = sqrt(t);
+        if (blockIdx.x == 0) *beta = b;
+        return 1.0 / b;
+    });
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) u[r] *= inv;
 }
 
@@ -1722,7 +1760,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
             k_three_term_dot<<<vx.grid, kDotBlock, 0, st>>>(w.p, v.p, u.p, it > 0 ? d_be + it - 1 : nullptr, n, dot_partial);
             k_three_term_subtract<<<vx.grid, kDotBlock, 0, st>>>(v.p, u.p, dot_partial, vx.grid, d_al + it,
                                                                  acc ? ev.p : nullptr, acc ? (*ritz)[it] : 0.0, n, norm_partial);
-            k_three_term_scale<<<grid_for(n, 256), 256, 0, st>>>(u.p, norm_partial, vx.grid, d_be + it, n);
+            k_three_term_scale<<<scale_grid(n), 256, 0, st>>>(u.p, norm_partial, vx.grid, d_be + it, n);
             std::swap(v.p, u.p);
         }
         QSI_CUDA(cudaGetLastError());
