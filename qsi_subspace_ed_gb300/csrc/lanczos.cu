@@ -1970,47 +1970,54 @@ __global__ void __launch_bounds__(256) k_observables(BasisView B, const PullTerm
 }
 
 // Gram matrix of two sets of vectors, A (ka of them) and C (kc), all of length n: partial[chunk][a][c] over the rows
-// of chunk blockIdx.y, in kGramTile x kGramTile tiles (blockIdx.x; symmetric: the tiles on and above the diagonal of
-// A = C only).  A thread holds a 4 x 4 square of sums, two FP64 multiply-adds per shared-memory value: bound by the
-// FP64 pipe, where a dot per vector pair read both vectors for each multiply-add.
+// of chunk blockIdx.y, in tiles of kGramTile vectors of A and 16 TW or (TW = 0) 4 of C (blockIdx.x; symmetric, A = C:
+// on and above the diagonal).  A thread holds 4 x TW sums (TW = 0: one), two FP64 multiply-adds per shared-memory
+// value: bound by the FP64 pipe, where a dot per pair of vectors read both for each multiply-add.
 constexpr int kGramTile = 64, kGramRows = 16;
+template <int TW>
 __global__ void __launch_bounds__(256) k_gram(const double* __restrict__ A, int ka, const double* __restrict__ C, int kc,
                                               int symmetric, int64_t n, double* __restrict__ partial) {
-    __shared__ double ta[kGramRows][kGramTile + 2], tc[kGramRows][kGramTile + 2];
-    const int tiles_c = (kc + kGramTile - 1) / kGramTile;
-    const int bi = blockIdx.x / tiles_c, bj = blockIdx.x % tiles_c;
-    if (symmetric && bj < bi) return;
-    const int a0 = bi * kGramTile, c0 = bj * kGramTile;
+    constexpr int kTileC = TW ? 16 * TW : 4, kTx = TW ? 16 : 4, kTy = 256 / kTx, kU = kGramTile / kTy, kW = TW ? TW : 1;
+    __shared__ double ta[kGramRows][kGramTile + 2], tc[kGramRows][kTileC + 2];
+    const int tiles_c = (kc + kTileC - 1) / kTileC;
+    const int a0 = blockIdx.x / tiles_c * kGramTile, c0 = blockIdx.x % tiles_c * kTileC;
+    if (symmetric && c0 < a0) return;
+    const bool diagonal = symmetric && c0 == a0;
     const int64_t chunk = ((n + gridDim.y - 1) / gridDim.y + kGramRows - 1) / kGramRows * kGramRows;
     const int64_t r0 = min(n, blockIdx.y * chunk), r1 = min(n, r0 + chunk);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // vectors tx + 16 u of C, ty + 16 u of A
-    double acc[4][4] = {};
+    const int tx = threadIdx.x % kTx, ty = threadIdx.x / kTx;  // vectors tx + kTx w of C, ty + kTy u of A
+    double acc[kU][kW] = {};
     for (int64_t r = r0; r < r1; r += kGramRows) {
         __syncthreads();
         for (int e = threadIdx.x; e < kGramRows * kGramTile; e += 256) {
             const int row = e % kGramRows, v = e / kGramRows;
-            const bool in = r + row < r1;
-            ta[row][v] = in && a0 + v < ka ? A[(int64_t)(a0 + v) * n + r + row] : 0.0;
-            tc[row][v] = in && c0 + v < kc ? C[(int64_t)(c0 + v) * n + r + row] : 0.0;
+            ta[row][v] = r + row < r1 && a0 + v < ka ? A[(int64_t)(a0 + v) * n + r + row] : 0.0;
+        }
+        for (int e = threadIdx.x; e < kGramRows * kTileC; e += 256) {
+            const int row = e % kGramRows, v = e / kGramRows;
+            tc[row][v] = r + row < r1 && c0 + v < kc ? C[(int64_t)(c0 + v) * n + r + row] : 0.0;
         }
         __syncthreads();
 #pragma unroll 4
         for (int row = 0; row < kGramRows; ++row) {
-            double av[4], cv[4];
+            double av[kU], cv[kW];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) av[u] = ta[row][ty + 16 * u], cv[u] = tc[row][tx + 16 * u];
+            for (int u = 0; u < kU; ++u) av[u] = ta[row][ty + kTy * u];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int w = 0; w < kW; ++w) cv[w] = tc[row][tx + kTx * w];
 #pragma unroll
-                for (int w = 0; w < 4; ++w) acc[u][w] += av[u] * cv[w];
+            for (int u = 0; u < kU; ++u)
+#pragma unroll
+                for (int w = 0; w < kW; ++w)
+                    if (TW != 4 || u <= w || !diagonal) acc[u][w] += av[u] * cv[w];  // u > w: below the diagonal
         }
     }
     double* out = partial + (int64_t)blockIdx.y * ka * kc;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < kU; ++u)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const int a = a0 + ty + 16 * u, c = c0 + tx + 16 * w;
+        for (int w = 0; w < kW; ++w) {
+            const int a = a0 + ty + kTy * u, c = c0 + tx + kTx * w;
             if (a < ka && c < kc) out[(int64_t)a * kc + c] = acc[u][w];
         }
 }
@@ -2025,17 +2032,20 @@ __global__ void k_gram_reduce(const double* __restrict__ partial, int chunks, in
 // h (host, ka x kc) = A^T C.
 static qsi_status gram(const double* A, int ka, const double* C, int kc, int64_t n, cudaStream_t st, std::vector<double>& h) {
     const int symmetric = A == C && ka == kc;
-    const int tiles_a = (ka + kGramTile - 1) / kGramTile, tiles_c = (kc + kGramTile - 1) / kGramTile;
+    // tiles of 4, 16 or 64 vectors of C (symmetric: square ones)
+    auto k = symmetric || kc > 32 ? k_gram<4> : kc > 4 ? k_gram<1> : k_gram<0>;
+    const int wide = symmetric || kc > 32 ? 64 : kc > 4 ? 16 : 4;
+    const int tiles_a = (ka + kGramTile - 1) / kGramTile, tiles_c = (kc + wide - 1) / wide;
     const int tiles = tiles_a * tiles_c, busy = symmetric ? tiles_a * (tiles_a + 1) / 2 : tiles;
     const int64_t count = (int64_t)ka * kc;
-    // two blocks per SM over the tiles that work, each with at least 256 rows, and at most 256 MiB of partial sums
-    int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(304 / busy, (n + 255) / 256));
+    // four blocks per SM over the tiles that work, each with at least 128 rows, and at most 256 MiB of partial sums
+    int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(608 / busy, (n + 127) / 128));
     chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, ((int64_t)1 << 25) / count));
     DevBuf<double> partial, out;
     QSI_CUDA(partial.alloc((size_t)(chunks * count), st));
     QSI_CUDA(out.alloc((size_t)count, st));
     if (symmetric) QSI_CUDA(cudaMemsetAsync(partial.p, 0, (size_t)(chunks * count) * 8, st));
-    k_gram<<<dim3(tiles, (unsigned)chunks), 256, 0, st>>>(A, ka, C, kc, symmetric, n, partial.p);
+    k<<<dim3(tiles, (unsigned)chunks), 256, 0, st>>>(A, ka, C, kc, symmetric, n, partial.p);
     k_gram_reduce<<<grid_for(count, 256), 256, 0, st>>>(partial.p, (int)chunks, count, out.p);
     QSI_CUDA(cudaGetLastError());
     h.resize((size_t)count);
@@ -2043,7 +2053,7 @@ static qsi_status gram(const double* A, int ka, const double* C, int kc, int64_t
     QSI_CUDA(cudaStreamSynchronize(st));
     if (symmetric)
         for (int a = 0; a < ka; ++a)
-            for (int c = 0; c < a / kGramTile * kGramTile; ++c) h[(size_t)a * kc + c] = h[(size_t)c * kc + a];
+            for (int c = 0; c < a; ++c) h[(size_t)a * kc + c] = h[(size_t)c * kc + a];
     return QSI_OK;
 }
 
