@@ -1226,8 +1226,13 @@ qsi_status find_closed(qsi_op* op) {
 // admission test): lane l of tile t sums row 32 t + l as the diagonal, then its entries in cache order (the
 // admission order of the tile kernels) with coefficient +-cs of the entry's term and the entry's sign, the same
 // sums in the same order as k_apply_tile, so the result is bitwise the matrix-free one.
+//
+// Latency-bound: six entries in flight per lane at 40 registers and six resident blocks.  With eight (64 registers, four
+// blocks, and 11.5 entries per tile padded to 16) the 64-spin Q=0 basis takes 166 us against 93, the 96-spin 8.8.16.16
+// sector 2.34 ms against 1.29; four entries at eight blocks 95 us and 1.38 ms.
+constexpr int kCachedBlocks = 6;
 template <typename XT, typename YT, typename TT>
-__global__ void __launch_bounds__(256) k_apply_cached(const double* __restrict__ coef, int n_off,
+__global__ void __launch_bounds__(256, kCachedBlocks) k_apply_cached(const double* __restrict__ coef, int n_off,
                                                       const double* __restrict__ diag, CacheView C,
                                                       const TT* __restrict__ tids, int64_t n, const XT* __restrict__ x,
                                                       YT* __restrict__ y, int accumulate) {
@@ -1245,7 +1250,7 @@ __global__ void __launch_bounds__(256) k_apply_cached(const double* __restrict__
         double acc = valid ? diag[row] * (double)x[row] : 0.0;
         const uint32_t* cp = C.cols + o0 * 32 + lane;
         const TT* tp = tids + o0 * 32 + lane;
-        constexpr int kU = 8;  // entries in flight per lane
+        constexpr int kU = 6;  // entries in flight per lane
         for (int k0 = 0; k0 < width; k0 += kU) {
             uint32_t c[kU];
             TT t[kU];
@@ -1287,7 +1292,8 @@ static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, 
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int bps = op->tune[0].grid_bps > 0 ? op->tune[0].grid_bps : 8;
+    // four waves of the resident blocks: 8 blocks per SM, one wave and a third, took 114 us on the 64-spin Q=0 basis
+    const int bps = op->tune[0].grid_bps > 0 ? op->tune[0].grid_bps : 4 * kCachedBlocks;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * bps));
     const size_t smem = (size_t)std::max(op->tile.n, 1) * 8;
     const CacheView C = cache_view(op);
