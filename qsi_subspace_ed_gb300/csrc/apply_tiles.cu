@@ -543,7 +543,6 @@ constexpr int kVec16 = -2;
 constexpr int kGroup = -3;
 constexpr int kGroupMax = 16;
 constexpr uint32_t kDiagSlot = 0x80000000u;
-constexpr int min_blocks(int km) { return km == kGroup || km > 0 ? 3 : 2; }
 inline bool vec4_ok(int64_t n, int R, const void* x, const void* y) {
     return n < (int64_t)kDiagSlot - 1 && R >= 4 && (R & 3) == 0 &&
            (R <= 128 ? (R & (R - 1)) == 0 : (R & 127) == 0) &&
@@ -557,7 +556,7 @@ inline bool vec16_ok(int64_t n, int R, const void* x, const void* y) {
 }
 
 template <typename XT, class LK, bool kFF, int KM, bool kFam = false>
-__global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
+__global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
                                                             XT* __restrict__ y, int R, int accumulate, int cap,
                                                             const float2* __restrict__ ycoef) {
     // accumulate: y <- H x + c y per column, c = 1, or the (hi, lo) float pair ycoef[column] (double-float paths)
@@ -639,7 +638,7 @@ __global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_tile_batched(Tile
             } else {
                 W.base[lane] = base + (v4 ? 1 : 0);
                 const int total = list_hits(WL, row_mask(row_start, row_end), n_rounds, lane, 4);
-                constexpr int kNB = v4 ? 4 : 2;
+                constexpr int kNB = 2;
                 look_up_hits<kNB>(S, P, WL, lk, tile, total, lane, 4,
                                   [&](int, int n, const uint32_t (&e)[kNB], const uint32_t (&J)[kNB]) {
 #pragma unroll
@@ -720,7 +719,12 @@ __global__ void __launch_bounds__(256, min_blocks(KM)) k_apply_tile_batched(Tile
                 // FP32 storage, double-float accumulation, no FP64 instruction.  The chunk's hit list
                 // is walked in order across row boundaries with kU column gathers in flight.
                 static_assert(std::is_same<XT, float>::value, "double-float accumulation is for FP32 vectors");
-                constexpr int kU = 32 / VPL;  // column gathers in flight per lane (kU * VPL = 32 floats)
+                // Column gathers in flight per lane.  With 16-byte gathers 24 floats are in flight at 80 registers and
+                // three blocks per SM; bound by the gathers' latency, 64 vectors take, with the look-ups / materialised:
+                //   floats, blocks          32, 2        32, 3        24, 3        20, 3        16, 3
+                //   96-spin 8.8.16.16 ms  40.1 / 38.9  40.4 / 30.2  37.7 / 28.5  38.5 / 29.8  45.9 / 31.4
+                //   64-spin Q=0 ms        2.48 / 2.30  2.62 / 1.87  2.38 / 1.78  2.38 / 1.84  2.73 / 1.91
+                constexpr int kU = v4 ? 24 / VPL : 8;
                 const int kbeg = __shfl_sync(0xffffffffu, base, row_start);
                 const int last = row_end - 1;
                 const int kend = __shfl_sync(0xffffffffu, base + pc, last);
