@@ -216,9 +216,11 @@ __device__ __forceinline__ void tile_spin_words(const state2 s, int nwords, int 
     __syncwarp();
 }
 
-// Rows that admit term t0 + lane (bit l = row l).
+// Rows that admit term t0 + lane (bit l = row l).  kForward: of a pair only the rows that admit its first operator, with
+// *skew the number of rows that admit the first less those that admit the second.
+template <bool kForward = false>
 __device__ __forceinline__ uint32_t tile_admitted(const TileSmem& S, const TileTerms& T, int t0, int lane,
-                                                  uint32_t vmask, const uint32_t* spinw) {
+                                                  uint32_t vmask, const uint32_t* spinw, int* skew = nullptr) {
     const int t = t0 + lane;
     uint32_t A = 0;
     if (t < T.n) {
@@ -232,7 +234,10 @@ __device__ __forceinline__ uint32_t tile_admitted(const TileSmem& S, const TileT
                 all &= w;
                 any |= w;
             }
-            if ((S.pair[t0 >> 5] >> lane) & 1) all |= ~any;
+            if ((S.pair[t0 >> 5] >> lane) & 1) {
+                if constexpr (kForward) *skew += __popc(all & vmask) - __popc(~any & vmask);
+                else all |= ~any;
+            }
             A = all & vmask;
         } else {
             A = vmask;
@@ -287,15 +292,15 @@ __device__ __forceinline__ uint32_t hit_row(uint32_t e) { return (e >> 14) & 31;
 __device__ __forceinline__ uint32_t hit_ordinal(uint32_t e) { return e & 0x3fff; }
 
 // Admission of the tile's rows: fills adm, the rows of ts and rows; returns this lane's number of hits.
-template <class LK>
+template <bool kForward = false, class LK>
 __device__ __forceinline__ int tile_admit(const TileSmem& S, const TileParams& P, const LK& lk, const WarpScratch& W,
-                                          const state2 s, int64_t row, int n_rounds, int lane) {
+                                          const state2 s, int64_t row, int n_rounds, int lane, int* skew = nullptr) {
     const uint32_t vmask = __ballot_sync(0xffffffffu, row < P.B.n);
     const Word4 words = lk.row_words(row, s);
     tile_spin_words(s, P.nwords, lane, W.spinw);
     int cnt = 0;
     for (int r = 0; r < n_rounds; ++r) {
-        const uint32_t A = tile_admitted(S, P.T, r * 32, lane, vmask, W.spinw);
+        const uint32_t A = tile_admitted<kForward>(S, P.T, r * 32, lane, vmask, W.spinw, skew);
         const uint32_t a = warp_transpose32(A, lane);
         W.ts[r * 32 + lane].x = A;
         W.adm[r * 32 + lane] = a;
@@ -1058,7 +1063,7 @@ qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull) {
     std::vector<const PullTerm*> kept;
     std::vector<uint32_t> pair((pull.size() + 31) / 32 + 1, 0);
     std::vector<std::vector<uint8_t>> lits(pull.size());
-    bool short_lists = true, any_z = false;
+    bool short_lists = true, any_z = false, reversible = true;
     for (size_t k = 0; k < pull.size(); ++k) {
         const PullTerm& t = pull[k];
         const uint64_t um[2] = {t.up0, t.up1}, dm[2] = {t.dn0, t.dn1};
@@ -1079,6 +1084,7 @@ qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull) {
             if (c.x0 == t.x0 && c.x1 == t.x1 && c.z0 == t.z0 && c.z1 == t.z1 && c.cs == t.cs && c.up0 == t.dn0 &&
                 c.up1 == t.dn1 && c.dn0 == t.up0 && c.dn1 == t.up1) {
                 pair[(kept.size() - 1) >> 5] |= 1u << ((kept.size() - 1) & 31);
+                reversible = reversible && !((t.up0 | t.dn0) & ~t.x0) && !((t.up1 | t.dn1) & ~t.x1);
                 ++k;
             }
         }
@@ -1112,6 +1118,7 @@ qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull) {
         }
     }
     T.n_lits = (int)flat.size();
+    T.reversible = reversible;
     size_t total = 0;
     auto place = [&](size_t bytes) {
         const size_t at = total;
@@ -1147,21 +1154,34 @@ qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull) {
     return QSI_OK;
 }
 
-// *missed = 1 when an admitted term of some row leaves the basis.
-template <class LK>
-__global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, int* __restrict__ missed, int cap) {
+// What find_closed reads: missed != 0 when an admitted term of some row leaves the basis; with kForward also the sum over
+// all rows and pairs of tile_admitted's skew.
+struct Closure {
+    unsigned long long skew;
+    int missed;
+};
+
+// kForward (every pair is reversible): only the first operator of a pair is looked up.  It maps the rows that admit it one
+// to one onto states that admit the second, so when none of them leaves the basis, at least as many rows admit the
+// second; when the sum over all pairs says that no more do, each row that admits a second operator is the image of
+// one that admits the first and is mapped back onto it, inside the basis.
+template <bool kForward, class LK>
+__global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, Closure* __restrict__ out, int cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const TileSmem S = stage_terms(P, lk, false, smem_raw);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n_rounds = (P.T.n + 31) >> 5;
     const WarpScratch W = warp_scratch(S.tail + wid * (scratch_bytes(n_rounds) + (size_t)cap * 4), n_rounds);
     const int64_t ntiles = (P.B.n + 31) >> 5;
+    long long skew = 0;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
-        if (*(volatile int*)missed) break;
+        if (*(volatile int*)&out->missed) break;
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
-        const int cnt = tile_admit(S, P, lk, W, s, row, n_rounds, lane);
+        int here = 0;
+        const int cnt = tile_admit<kForward>(S, P, lk, W, s, row, n_rounds, lane, &here);
+        skew += here;
         bool miss = false;
         for (int row_start = 0; row_start < 32;) {
             int base;
@@ -1176,7 +1196,12 @@ __global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, int* __r
             __syncwarp();
             row_start = row_end;
         }
-        if (miss) *(volatile int*)missed = 1;
+        if (miss) *(volatile int*)&out->missed = 1;
+    }
+    if constexpr (kForward) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) skew += __shfl_down_sync(0xffffffffu, skew, o);
+        if (lane == 0 && skew) atomicAdd(&out->skew, (unsigned long long)skew);
     }
 }
 
@@ -1198,30 +1223,31 @@ static TileLaunch tile_launch(const qsi_op* op, size_t slot_bytes, int want) {
     return L;
 }
 
-// Determines op->closed: with a hash index, one pass of compared lookups (about 0.8 of an apply; a first miss ends it).
-// Applies of a closed operator take a tag match for the state itself, which saves each of their lookups the 16-byte
+// Determines op->closed: with a hash index, one pass of compared lookups; a first miss ends it.  With one operator of
+// each pair it takes 209 us on the 64-spin Q=0 basis and 3.2 ms on the 96-spin 8.8.16.16 sector, 305 us and 5.8 ms with
+// both.  Applies of a closed operator take a tag match for the state itself, which saves each of their lookups the 16-byte
 // load of the state at the index found.
 qsi_status find_closed(qsi_op* op) {
     op->closed = 0;
     if (!op->basis->d_bins) return QSI_OK;
     const TileParams P = tile_params(op, 0);
     cudaStream_t st = op->stream;
-    int* d_missed = nullptr;
-    QSI_CUDA(cudaMallocAsync(&d_missed, sizeof(int), st));
-    cudaError_t e = cudaMemsetAsync(d_missed, 0, sizeof(int), st);
+    Closure* d_out = nullptr;
+    QSI_CUDA(cudaMallocAsync(&d_out, sizeof(Closure), st));
+    cudaError_t e = cudaMemsetAsync(d_out, 0, sizeof(Closure), st);
     const int64_t ntiles = (P.B.n + 31) / 32;
     const LookupBins<false> lk{op->basis->bview()};
-    auto k = k_find_miss<LookupBins<false>>;
+    auto k = op->tile.reversible ? k_find_miss<true, LookupBins<false>> : k_find_miss<false, LookupBins<false>>;
     const TileLaunch L = tile_launch(op, 4, kListCap);
     if (L.smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
-    k<<<grid_for(ntiles, L.block / 32), L.block, L.smem, st>>>(P, lk, d_missed, L.cap);
-    int missed = 1;
+    k<<<grid_for(ntiles, L.block / 32), L.block, L.smem, st>>>(P, lk, d_out, L.cap);
+    Closure c{0, 1};
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&missed, d_missed, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&c, d_out, sizeof(c), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFreeAsync(d_missed, st);
+    cudaFreeAsync(d_out, st);
     if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "qsi_op_create (closure): %s", cudaGetErrorString(e));
-    op->closed = !missed;
+    op->closed = !c.missed && !c.skew;
     return QSI_OK;
 }
 

@@ -250,8 +250,9 @@ __global__ void k_count_connectivity(BasisView B, const PushTerm* __restrict__ o
 
 // hit[t] = 1 when transposed term t maps some row's state onto a basis state.  A block stops once every term
 // is known to hit (terms that hit usually do so within the first rows); terms that never hit are tested on
-// every row they admit.
-__global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms, int n, int* __restrict__ hit) {
+// every row they admit.  Rows 0, stride, 2 stride, ... are tested.
+__global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms, int n, int64_t stride,
+                                 int* __restrict__ hit) {
     extern __shared__ int known[];
     __shared__ int n_known;
     if (threadIdx.x == 0) n_known = 0;
@@ -261,10 +262,12 @@ __global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms
         if (known[t]) atomicAdd(&n_known, 1);
     }
     __syncthreads();
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < B.n; j += (int64_t)gridDim.x * blockDim.x) {
+    const int t0 = (int)((int64_t)(threadIdx.x >> 5) * n / (blockDim.x >> 5));  // the warps search for different terms
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i * stride < B.n;
+         i += (int64_t)gridDim.x * blockDim.x) {
         if (*(volatile int*)&n_known == n) break;
-        const state2 s = B.states[j];
-        for (int t = 0; t < n; ++t) {
+        const state2 s = B.states[i * stride];
+        for (int k = 0, t = t0; k < n; ++k, t = t + 1 < n ? t + 1 : 0) {
             if (((volatile int*)known)[t]) continue;
             const PullTerm& T = terms[t];
             const bool ok = ((s.x & T.dn0) | (s.y & T.dn1)) == 0 && (s.x & T.up0) == T.up0 && (s.y & T.up1) == T.up1;
@@ -278,6 +281,7 @@ __global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms
 
 // Removes the transposed terms that map no row into the basis (their contributions are all dropped misses), keeping
 // the order of the others: an exact reduction of the lookups the apply issues.
+constexpr int kSampleRows = 8192;
 static qsi_status prune_pull_terms(qsi_basis* b, std::vector<PullTerm>& pull) {
     const int n = (int)pull.size();
     if (n == 0 || b->n == 0) return QSI_OK;
@@ -289,10 +293,14 @@ static qsi_status prune_pull_terms(qsi_basis* b, std::vector<PullTerm>& pull) {
     if (e == cudaSuccess) e = cudaMemset(d_hit, 0, n * sizeof(int));
     if (e == cudaSuccess) {
         const size_t smem = (size_t)n * sizeof(int);
-        const int grid = grid_for(b->n, 256);
         auto k = k_pull_term_hits;
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, 256, smem>>>(b->view(), d_terms, n, d_hit);
+        // A sample of rows first: every block of a launch finds each term by itself, so a full grid repeats that
+        // work thousands of times; after the sample its blocks mostly have nothing left to find (64-spin Q=0 basis:
+        // 311 -> 78 us, 96-spin 8.8.16.16 sector: 946 -> 147 us).
+        const int64_t stride = b->n / kSampleRows;
+        if (stride > 1) k<<<kSampleRows / 256, 256, smem>>>(b->view(), d_terms, n, stride, d_hit);
+        k<<<grid_for(b->n, 256), 256, smem>>>(b->view(), d_terms, n, 1, d_hit);
         e = cudaGetLastError();
     }
     std::vector<int> hit(n, 1);

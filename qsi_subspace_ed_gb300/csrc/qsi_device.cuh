@@ -46,6 +46,7 @@ struct TileTerms {
     const uint16_t* lit_off;  // literal lists of any length, when some term has none or more than eight
     const uint8_t* lits;
     int n, n_lits, max_lits;
+    int reversible;           // every pair's requirements are on spins it flips: each operator undoes the other
 };
 
 // Diagonal part: single-site pure-z terms grouped by weight w into masks,

@@ -146,3 +146,13 @@ def test_few_vectors(R, dtype, pairs):
                 op.apply_batched(X, Y, accumulate=acc)
                 assert np.array_equal(Y, ref[:, :R]), (acc, cap, cached)
             op.materialise(False)
+
+
+@pytest.mark.parametrize("kept", [1, 2])
+def test_pairs_that_leave_one_way(kept):
+    """A third of the states that admit one operator of the pair on spins 0 and 1 are missing, so that only the other's
+    images leave the basis, first or second in the pair; shared tags, so a lookup that takes a match for the state errs."""
+    lohi = integers(200_000)
+    i = np.arange(200_000)
+    lohi = lohi[~(((i & 3) == 3 - kept) & ((i >> 10) % 3 == 0))]
+    check(lohi, opsum(PAIRS[:2] + PAIRS[3:7]), (1, 9))
