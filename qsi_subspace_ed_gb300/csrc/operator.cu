@@ -370,7 +370,10 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
             while ((1LL << lg) < n) ++lg;
             // two to four states per bucket on average: wider tables measured the same or slower (64-spin Q=0 basis:
             // 278 us at 21 bits, 284 at 22, 300 at 24; 96-spin 8.8.16.16: 4.88 ms at 24, 4.83 at 25, 4.89 at 27)
-            bits = std::min(28, std::max(8, lg - 1));
+            // Without bins the table is what every lookup starts from (the 64-spin Q=0 basis spread over 126 bits: 566 us
+            // at 21 bits, 551 at 24; row-per-thread kernel 1153 and 1002).
+            const bool bins = hb < 96 && n < ((int64_t)1 << 31);
+            bits = std::min(28, std::max(8, bins ? lg - 1 : lg + 1));
         }
         bits = std::min(bits, std::min(31, hb + 1));
         b->bits = bits;
