@@ -1582,15 +1582,26 @@ qsi_status launch_apply_ff(qsi_op* op, const float* x, float* y, int R, int accu
     return launch_tiles(op, x, y, R, QSI_F32, QSI_F32, accumulate, st, true, ycoef);
 }
 
-// Builds (enable) or frees the operator's lookup cache; *bytes: its size.
-qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
-    cudaFree(op->d_cache_cols);
-    cudaFree(op->d_cache_off);
-    cudaFree(op->d_cache_tid);
+// Allocates and frees the operator's lookup cache: a solve's own (cache_pooled) in the order of the operator's stream, so
+// that solves overlap, a handle's behind the applies of every stream (cudaFree waits for them).
+static cudaError_t cache_alloc(qsi_op* op, void** p, size_t bytes) {
+    return op->cache_pooled ? cudaMallocAsync(p, bytes, op->stream) : cudaMalloc(p, bytes);
+}
+static void drop_cache(qsi_op* op) {
+    for (void* p : {(void*)op->d_cache_cols, (void*)op->d_cache_off, op->d_cache_tid}) {
+        if (op->cache_pooled) cudaFreeAsync(p, op->stream);
+        else cudaFree(p);
+    }
     op->d_cache_cols = nullptr;
     op->d_cache_off = nullptr;
     op->d_cache_tid = nullptr;
     op->cache_entries = 0;
+}
+
+// Builds (enable) or frees the operator's lookup cache; *bytes: its size.  A cache of more than `most` bytes is not
+// built (QSI_OK, 0 bytes).
+qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes, size_t most) {
+    drop_cache(op);
     if (enable) {
         if (op->kernel != 1) return fail(QSI_INVALID_ARG, "qsi_op_materialise: the cache serves the tile kernels (kernel 1)");
         cudaStream_t st = op->stream;
@@ -1610,13 +1621,12 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         };
         auto fail_partial = [&](cudaError_t e, const char* what) {
             scratch_free();
-            cudaFree(op->d_cache_off);
-            op->d_cache_off = nullptr;
+            drop_cache(op);
             return fail(e == cudaErrorMemoryAllocation ? QSI_OOM : QSI_CUDA_ERROR, "qsi_op_materialise: %s: %s", what,
                         cudaGetErrorString(e));
         };
         cudaError_t e = cudaMallocAsync(&width, (size_t)(ntiles + 1) * 8, st);
-        if (e == cudaSuccess) e = cudaMallocAsync(&op->d_cache_off, (size_t)(ntiles + 1) * 8, st);
+        if (e == cudaSuccess) e = cache_alloc(op, (void**)&op->d_cache_off, (size_t)(ntiles + 1) * 8);
         if (e == cudaSuccess) e = cudaMemsetAsync(width + ntiles, 0, 8, st);
         if (e != cudaSuccess) return fail_partial(e, "tile offsets");
         set_smem(k_cache_widths, L.smem);
@@ -1632,46 +1642,41 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
         scratch_free();
         const size_t n_entries = (size_t)lines * 32;
         op->cache_tid_bytes = op->tile.n <= 256 ? 1 : 2;
-        e = cudaMalloc(&op->d_cache_cols, std::max<size_t>(n_entries, 1) * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&op->d_cache_tid, std::max<size_t>(n_entries, 1) * op->cache_tid_bytes);
+        if (n_entries * (4 + op->cache_tid_bytes) > most) {
+            drop_cache(op);
+            if (bytes) *bytes = 0;
+            return QSI_OK;
+        }
+        e = cache_alloc(op, (void**)&op->d_cache_cols, std::max<size_t>(n_entries, 1) * 4);
+        if (e == cudaSuccess) e = cache_alloc(op, &op->d_cache_tid, std::max<size_t>(n_entries, 1) * op->cache_tid_bytes);
         if (e != cudaSuccess) {
-            cudaFree(op->d_cache_off);
-            cudaFree(op->d_cache_cols);
-            op->d_cache_off = nullptr;
-            op->d_cache_cols = nullptr;
-            op->d_cache_tid = nullptr;
+            drop_cache(op);
             return fail(e == cudaErrorMemoryAllocation ? QSI_OOM : QSI_CUDA_ERROR,
                         "qsi_op_materialise: %zu bytes for the cache: %s", n_entries * (4 + op->cache_tid_bytes),
                         cudaGetErrorString(e));
         }
-        auto drop_cache = [&](cudaError_t err) {  // a cache that was not filled completely is never used
-            cudaFree(op->d_cache_cols);
-            cudaFree(op->d_cache_tid);
-            cudaFree(op->d_cache_off);
-            op->d_cache_cols = nullptr;
-            op->d_cache_tid = nullptr;
-            op->d_cache_off = nullptr;
+        auto unfilled = [&](cudaError_t err) {  // a cache that was not filled completely is never used
+            drop_cache(op);
             return fail(QSI_CUDA_ERROR, "qsi_op_materialise: %s", cudaGetErrorString(err));
         };
         e = cudaMemsetAsync(op->d_cache_cols, 0xFF, n_entries * 4, st);  // the lanes below their tile's width
         if (e == cudaSuccess) e = cudaMemsetAsync(op->d_cache_tid, 0, n_entries * op->cache_tid_bytes, st);
-        if (e != cudaSuccess) return drop_cache(e);
+        if (e != cudaSuccess) return unfilled(e);
         auto fill = [&](auto lk, auto* tids) {
             auto k = k_cache_fill<decltype(lk), std::remove_pointer_t<decltype(tids)>>;
             set_smem(k, L.smem);
             k<<<grid, L.block, L.smem, st>>>(P, lk, op->d_cache_off, op->d_cache_cols, tids, L.cap);
         };
-        if (op->basis->d_bins) {
-            const LookupBins<false> lk{op->basis->bview()};
+        auto by_tid = [&](auto lk) {
             if (op->cache_tid_bytes == 1) fill(lk, (uint8_t*)op->d_cache_tid);
             else fill(lk, (uint16_t*)op->d_cache_tid);
-        } else {
-            if (op->cache_tid_bytes == 1) fill(LookupTable{op->basis->view()}, (uint8_t*)op->d_cache_tid);
-            else fill(LookupTable{op->basis->view()}, (uint16_t*)op->d_cache_tid);
-        }
+        };
+        if (!op->basis->d_bins) by_tid(LookupTable{op->basis->view()});
+        else if (op->closed) by_tid(LookupBins<true>{op->basis->bview()});
+        else by_tid(LookupBins<false>{op->basis->bview()});
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) return drop_cache(e);
+        if (e != cudaSuccess) return unfilled(e);
         op->cache_entries = n_entries;
     }
     if (bytes)
@@ -1679,6 +1684,34 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes) {
                                               ((op->basis->n + 31) / 32 + 1) * 8)
                                   : 0;
     return QSI_OK;
+}
+
+// Rows from which a solve builds its own cache, and applies after which it does: those that pay for the building and the
+// release.  2.9 M rows (64-spin Q=0 basis): 276 -> 93 us per apply against 0.78 ms; 31 M (96-spin 8.8.16.16 sector): 4.8 ->
+// 1.3 ms against 8.5 ms; 221,628: 36 -> 12.5 us against 0.37 ms; 15,528: 14.7 -> 8.0 us against 0.08 ms; 3,618 rows
+// (10.4 -> 7.9 us) are launch-bound, and a solve of 115 applies takes 5.25 ms instead of 5.18.
+constexpr int64_t kCacheMinRows = 8192;
+static int64_t applies_for_cache(int64_t n) { return n >= (1 << 20) ? 6 : 16; }
+
+void SolveOp::plan(int64_t applies) {
+    const int64_t n = op_->basis->n;
+    if (tried_ || op_->kernel != 1 || op_->family || op_->d_cache_cols || n < kCacheMinRows ||
+        n >= ((int64_t)1 << 31) - 1 || applies < applies_for_cache(n))
+        return;
+    tried_ = true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+        view_ = *op_;
+        view_.cache_pooled = true;
+        materialise(&view_, true, nullptr, free_b / 4);
+    }
+    cudaGetLastError();  // without a cache the solve applies the operator as it is
+}
+
+bool SolveOp::drop() {
+    if (!view_.d_cache_cols) return false;
+    drop_cache(&view_);
+    return true;
 }
 
 }  // namespace qsi

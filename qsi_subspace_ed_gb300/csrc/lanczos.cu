@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <map>
 #include <random>
 #include <string>
@@ -803,25 +804,23 @@ struct PhaseClock {
 
 // FP64 polish of the Ritz block X (nev FP64 vectors, vector-major, Ritz values th): Rayleigh-Ritz on X, then
 // `rounds - 1` Rayleigh-Ritz steps on [X, HX - X theta]; then the residual report and the solver's outputs.
-static qsi_status finish_solve(qsi_op* op, const qsi_lanczos_cfg& cfg, Vecs& vx, DevBuf<double>& X, DevBuf<double>& HX,
+static qsi_status finish_solve(SolveOp& A, int64_t n, cudaStream_t st, const qsi_lanczos_cfg& cfg, Vecs& vx, DevBuf<double>& X, DevBuf<double>& HX,
                                std::vector<double>& th, int nev, int rounds, int64_t applies, int nconv, int restarts,
                                bool exhausted, std::chrono::steady_clock::time_point t0, double* evals, double* evecs,
                                qsi_report* rep) {
-    const int64_t n = op->basis->n;
-    cudaStream_t st = op->stream;
     qsi_status s = QSI_OK;
     std::vector<double> h;
     // FP64 polish: Rayleigh-Ritz on the Ritz block, then optional residual-augmented rounds
     DevBuf<double> S, HS, dth;
     if (rounds > 0) {
-        QSI_CUDA(S.alloc((size_t)2 * nev * n, st));
-        QSI_CUDA(HS.alloc((size_t)2 * nev * n, st));
+        QSI_CUDA(A.alloc(S, (size_t)2 * nev * n));
+        QSI_CUDA(A.alloc(HS, (size_t)2 * nev * n));
         QSI_CUDA(dth.alloc((size_t)nev, st));
         QSI_CUDA(cudaMemcpyAsync(S.p, X.p, (size_t)nev * n * 8, cudaMemcpyDeviceToDevice, st));
         s = orthonormalise(vx, S.p, nev, n);
         if (s) return s;
         for (int i = 0; i < nev; ++i) {
-            s = launch_apply(op, S.p + (size_t)i * n, HS.p + (size_t)i * n, 1, QSI_F64, 0, st);
+            s = launch_apply(A.get(), S.p + (size_t)i * n, HS.p + (size_t)i * n, 1, QSI_F64, 0, st);
             if (s) return s;
             ++applies;
         }
@@ -835,7 +834,7 @@ static qsi_status finish_solve(qsi_op* op, const qsi_lanczos_cfg& cfg, Vecs& vx,
             s = orthonormalise(vx, S.p, 2 * nev, n);
             if (s) return s;
             for (int i = 0; i < 2 * nev; ++i) {
-                s = launch_apply(op, S.p + (size_t)i * n, HS.p + (size_t)i * n, 1, QSI_F64, 0, st);
+                s = launch_apply(A.get(), S.p + (size_t)i * n, HS.p + (size_t)i * n, 1, QSI_F64, 0, st);
                 if (s) return s;
                 ++applies;
             }
@@ -844,7 +843,7 @@ static qsi_status finish_solve(qsi_op* op, const qsi_lanczos_cfg& cfg, Vecs& vx,
         }
     } else {
         for (int i = 0; i < nev; ++i) {
-            s = launch_apply(op, X.p + (size_t)i * n, HX.p + (size_t)i * n, 1, QSI_F64, 0, st);
+            s = launch_apply(A.get(), X.p + (size_t)i * n, HX.p + (size_t)i * n, 1, QSI_F64, 0, st);
             if (s) return s;
             ++applies;
         }
@@ -852,7 +851,7 @@ static qsi_status finish_solve(qsi_op* op, const qsi_lanczos_cfg& cfg, Vecs& vx,
     // residual norms ||H x - theta x|| / ||x||
     if (rep) {
         DevBuf<double> R, d2;
-        QSI_CUDA(R.alloc((size_t)nev * n, st));
+        QSI_CUDA(A.alloc(R, (size_t)nev * n));
         QSI_CUDA(d2.alloc((size_t)nev, st));
         QSI_CUDA(cudaMemcpyAsync(d2.p, th.data(), (size_t)nev * 8, cudaMemcpyHostToDevice, st));
         k_residual<<<grid_for(n, 256), 256, 0, st>>>(HX.p, X.p, d2.p, nev, n, R.p);
@@ -904,6 +903,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     Vecs vx;
     qsi_status s = vx.init(n, st);
     if (s) return s;
+    SolveOp A(op);
     DevBuf<VT> V;
     DevBuf<double> w, dY, coef;
     QSI_CUDA(V.alloc((size_t)(m + 1) * n, st));
@@ -929,7 +929,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     // second pass that a plain Gram-Schmidt of H V_j needs is left out.  After a restart (j == k > 0) H V_j has
     // components along every kept vector, and two full passes take them out.
     auto lanczos_step = [&](int j, int k) -> qsi_status {
-        qsi_status ss = apply_to_w<VT>(op, vec(j), w.p, st);
+        qsi_status ss = apply_to_w<VT>(A.get(), vec(j), w.p, st);
         if (ss) return ss;
         if (j == k && k > 0) {
             orth_pass(j, 1, 0, 0);
@@ -955,6 +955,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     std::vector<double> Tw, TY;
     PhaseClock clk{st, sizeof(VT) == 4 ? "trlan-f32" : "trlan-f64"};
     for (;;) {
+        A.plan(applies + m - k);
         int done = k;  // steps of this cycle known to be sound
         while (done < m) {
             for (int j = done; j < m; ++j) {
@@ -1029,8 +1030,8 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     }
     // Ritz vectors in FP64
     DevBuf<double> X, HX;
-    QSI_CUDA(X.alloc((size_t)nev * n, st));
-    QSI_CUDA(HX.alloc((size_t)nev * n, st));
+    QSI_CUDA(A.alloc(X, (size_t)nev * n));
+    QSI_CUDA(A.alloc(HX, (size_t)nev * n));
     {
         std::vector<double> Yk((size_t)m * nev);
         for (int i = 0; i < m; ++i)
@@ -1045,7 +1046,7 @@ static qsi_status trlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, d
     // free the Krylov basis before polishing
     V.release();
     clk.mark("ritz vectors");
-    s = finish_solve(op, cfg, vx, X, HX, th, nev, std::max(cfg.polish_steps, sizeof(VT) == 4 ? 1 : 0), applies, nconv,
+    s = finish_solve(A, n, st, cfg, vx, X, HX, th, nev, std::max(cfg.polish_steps, sizeof(VT) == 4 ? 1 : 0), applies, nconv,
                      restarts, m >= n, t0, evals, evecs, rep);
     clk.mark("polish");
     return s;
@@ -1296,6 +1297,7 @@ struct BlockSolver {
 // Block thick-restart Lanczos, FP32 Krylov blocks of kBlk vectors (see above), then the FP64 polish.
 static qsi_status btrlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, double* evecs, qsi_report* rep) {
     auto t0 = std::chrono::steady_clock::now();
+    SolveOp A(op);
     BlockSolver B{op};
     qsi_status s = B.init();
     if (s) return s;
@@ -1334,9 +1336,10 @@ static qsi_status btrlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, 
     int restarts = 0, nconv = 0;
     uint64_t breakdowns = 0;
     for (;;) {
+        A.plan(applies / kBlk + nblk - k0);
         for (int j = k0; j < nblk; ++j) {
             clk.mark("setup/host");
-            s = launch_apply(op, Q[j], W, kBlk, QSI_F32, 0, st);
+            s = launch_apply(A.get(), Q[j], W, kBlk, QSI_F32, 0, st);
             if (s) return s;
             applies += kBlk;
             clk.mark("apply");
@@ -1424,8 +1427,8 @@ static qsi_status btrlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, 
     }
     // FP64 Ritz vectors (vector-major) for the polish
     DevBuf<double> X, HX;
-    QSI_CUDA(X.alloc((size_t)nev * n, st));
-    QSI_CUDA(HX.alloc((size_t)nev * n, st));
+    QSI_CUDA(A.alloc(X, (size_t)nev * n));
+    QSI_CUDA(A.alloc(HX, (size_t)nev * n));
     {
         const int nout = (nev + kBlk - 1) / kBlk;
         std::vector<double> Yn((size_t)m * nout * kBlk, 0.0);
@@ -1440,7 +1443,7 @@ static qsi_status btrlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, 
     s = vx.init(n, st);
     if (s) return s;
     clk.mark("ritz vectors");
-    s = finish_solve(op, cfg, vx, X, HX, th, nev, std::max(cfg.polish_steps, 1), applies, nconv, restarts, false, t0,
+    s = finish_solve(A, n, st, cfg, vx, X, HX, th, nev, std::max(cfg.polish_steps, 1), applies, nconv, restarts, false, t0,
                      evals, evecs, rep);
     clk.mark("polish");
     return s;
@@ -1743,6 +1746,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
     Vecs vx;
     qsi_status s = vx.init(n, st);
     if (s) return s;
+    SolveOp A(op);
     DevBuf<double> v, u, w, ev, coef;
     QSI_CUDA(v.alloc(n, st));
     QSI_CUDA(u.alloc(n, st));
@@ -1755,7 +1759,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
     auto enqueue = [&](int it, int end, const std::vector<double>* ritz) -> qsi_status {
         for (; it < end; ++it) {
             const bool acc = ritz && it < (int)ritz->size();
-            qsi_status ss = launch_apply(op, v.p, w.p, 1, QSI_F64, 0, st);
+            qsi_status ss = launch_apply(A.get(), v.p, w.p, 1, QSI_F64, 0, st);
             if (ss) return ss;
             k_three_term_dot<<<vx.grid, kDotBlock, 0, st>>>(w.p, v.p, u.p, it > 0 ? d_be + it - 1 : nullptr, n, dot_partial);
             k_three_term_subtract<<<vx.grid, kDotBlock, 0, st>>>(v.p, u.p, dot_partial, vx.grid, d_al + it,
@@ -1841,6 +1845,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                 if (ck->every > 0) end = std::min(end, (it / ck->every + 1) * ck->every);
                 if (ck->stop_after > 0) end = std::min(end, it0 + ck->stop_after);
             }
+            A.plan(it + (ck && ck->stop_after > 0 ? end - it : max_it - it));
             s = enqueue(it, end, nullptr);
             if (s) return s;
             const int got = end - it;
@@ -1882,7 +1887,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         // The second pass repeats the first's recurrence, bit for bit, up to the iteration at which it stops, which
         // the first pass's coefficients therefore tell: the lowest Ritz value changed by less than abs_tol or
         // rel_tol from min_iterations on, or the first pass's end.
-        QSI_CUDA(ev.alloc(n, st));
+        QSI_CUDA(A.alloc(ev, n));
         QSI_CUDA(cudaMemsetAsync(ev.p, 0, (size_t)n * 8, st));
         int last = std::min(its, max_it - 1);
         eig = 1e308;
@@ -2684,6 +2689,8 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
         QSI_CUDA(cudaMemsetAsync(S[s].nbeta_ff.p, 0, (size_t)R * sizeof(float2), st));
         k_ftlm_init<VT><<<grid_for(S[s].n * R, 256), 256, 0, st>>>(S[s].C.p, S[s].P.p, S[s].n, R, seed + (uint64_t)s);
     }
+    std::deque<SolveOp> A;  // destroyed before the vectors, after the run
+    for (int s = 0; s < ns; ++s) A.emplace_back(ops[s]).plan(M);
     std::vector<VT*> prev(ns), cur(ns);
     for (int s = 0; s < ns; ++s) prev[s] = S[s].P.p, cur[s] = S[s].C.p;
     Branches br;
@@ -2707,10 +2714,10 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
             // by -beta_prev on the way: inside the double-float apply, else by the previous step's column pass
             VT* out = two ? prev[s] : F.W.p;
             if (ff[s])
-                status = launch_apply_ff(ops[s], reinterpret_cast<const float*>(cur[s]), reinterpret_cast<float*>(out), F.R,
+                status = launch_apply_ff(A[s].get(), reinterpret_cast<const float*>(cur[s]), reinterpret_cast<float*>(out), F.R,
                                          two ? 1 : 0, two ? F.nbeta_ff.p : nullptr, st);
             else
-                status = launch_apply(ops[s], cur[s], out, F.R, sizeof(VT) == 4 ? QSI_F32 : QSI_F64, two ? 1 : 0, st);
+                status = launch_apply(A[s].get(), cur[s], out, F.R, sizeof(VT) == 4 ? QSI_F32 : QSI_F64, two ? 1 : 0, st);
             const double* bprev = j ? dB + (size_t)(j - 1) * F.R : nullptr;
             double* beta = dB + (size_t)j * F.R;
             auto col_step = [&](auto vw) {

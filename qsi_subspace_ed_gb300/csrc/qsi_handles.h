@@ -1,6 +1,8 @@
 // Handle layouts behind the opaque qsi_basis / qsi_op pointers of the C-ABI.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <cstdint>
 #include <vector>
 
 #include "qsi_device.cuh"
@@ -59,6 +61,7 @@ struct qsi_op {
     void* d_cache_tid = nullptr;       // the term index of every entry (uint8, or uint16 beyond 256 terms)
     int cache_tid_bytes = 1;
     size_t cache_entries = 0;
+    bool cache_pooled = false;         // from the stream-ordered allocator (SolveOp)
     cudaStream_t stream = nullptr;
     int device = 0;        // the device current at qsi_op_create (owner of every buffer and of the stream)
     void* d_x = nullptr;   // staging for host-pointer applies
@@ -89,8 +92,41 @@ PullTerm transposed_term(const qsi_term& t);
 // Builds op->tile from the transposed terms.
 qsi_status upload_tile_terms(qsi_op* op, const std::vector<PullTerm>& pull);
 qsi_status find_closed(qsi_op* op);
-// Builds (enable) or frees an operator's lookup cache (qsi_op_materialise); *bytes: its size in device memory.
-qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes);
+// Builds (enable) or frees an operator's lookup cache (qsi_op_materialise); *bytes: its size in device memory.  A cache of
+// more than `most` bytes is not built (QSI_OK, 0 bytes).
+qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes, size_t most = SIZE_MAX);
+
+// An operator as one solve applies it: with a lookup cache of the solve's own, in a copy of the handle, once enough
+// applies are known to use it and if it takes no more than a quarter of the free device memory; the results are
+// bitwise those of the operator without it.  A family's members apply in their family's batches and get none.
+class SolveOp {
+   public:
+    explicit SolveOp(qsi_op* op) : op_(op) {}
+    ~SolveOp() { drop(); }
+    SolveOp(const SolveOp&) = delete;
+    SolveOp& operator=(const SolveOp&) = delete;
+    // applies: those done so far and those sure to follow.
+    void plan(int64_t applies);
+    qsi_op* get() { return view_.d_cache_cols ? &view_ : op_; }
+    // Frees the cache behind the applies enqueued on the operator's stream; whether there was one.
+    bool drop();
+    // An allocation on the operator's stream that comes before the cache when both don't fit.
+    template <class Buf>
+    cudaError_t alloc(Buf& b, size_t count) {
+        cudaError_t e = b.alloc(count, op_->stream);
+        if (e == cudaErrorMemoryAllocation && drop()) {
+            cudaGetLastError();
+            cudaStreamSynchronize(op_->stream);
+            e = b.alloc(count, op_->stream);
+        }
+        return e;
+    }
+
+   private:
+    qsi_op* op_;
+    qsi_op view_;
+    bool tried_ = false;
+};
 // Fills the bucket table of a basis at its current width (b->bits, b->shift, b->n_buckets).
 qsi_status build_buckets(qsi_basis* b);
 // Loads the single-vector FP64 apply kernels on the current device (CUDA loads device code lazily, on first use).

@@ -1,11 +1,12 @@
 """The Krylov drivers' device kernels at the edges of their tiles and batches: the Jacobi eigensolver with its
 eigenvectors in shared and in global memory, Krylov bases around groups of eight vectors, invariant subspaces inside a
-cycle, and eigval0 around its batches of iterations."""
+cycle, eigval0 around its batches of iterations, and solves that materialise the operator for themselves."""
 import numpy as np
 import pytest
 
 import qsi_subspace_ed_gb300 as q
 from oracle import oracle as O
+from qsi_subspace_ed_gb300 import workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -155,3 +156,27 @@ def test_expectations_tiles(nvec, n):
     np.testing.assert_allclose(expect, np.einsum("lni,nj->lij", W, psi), rtol=0, atol=8 * EPS * scale)
     np.testing.assert_allclose(cross, np.einsum("lni,mnj->lmij", W, W), rtol=0, atol=8 * EPS * scale)
     assert none is None and np.array_equal(only, expect)
+
+
+# 8,191 / 8,192 rows: without and with a solve's own lookup cache; cut-off bases: some cached entries are empty
+@pytest.mark.parametrize("pairs,n", [(0, 3618), (2, 8191), (2, 8192), (2, 20_011)])
+def test_solves_with_their_own_cache(pairs, n):
+    """Bitwise those of the row-per-thread kernel, which has no cache: the materialised sums are the same."""
+    lat = workloads.lattice("pyro_1x2x1")
+    g, B = workloads.ring_zeeman_params(5)
+    lohi = q.enumerate_basis(lat, n_spinon_pairs=pairs)[:n]
+    assert len(lohi) == n
+    op = q.LazyOpSum(q.ZBasis(lohi), q.build_ring_zeeman(lat, g, B, Jpm=0.05 if pairs else 0.0))
+    got = []
+    for kernel in (1, 0):
+        op.set_kernel(kernel)
+        out = []
+        for precision in ("f64", "mixed"):
+            ev, vec, rep = q.diagonalise(op, nev=2, ncv=12, tol=1e-10, seed=4, precision=precision)
+            assert rep.applies >= 50
+            out += [ev, vec]
+        out += list(q.eigval0(op, seed=3, max_iterations=60)[:2])
+        out += list(q.ftlm([op, op], [2, 4], M=44, seed=6, precision="f64")[1])
+        got.append(out)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
