@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
         const Word4 rw = lk.row_words(row, s);
-        double acc = valid ? (kFam ? fam_diag(P, s.x, s.y, 0) : P.diag[row]) * (double)x[row] : 0.0;
+        double acc = valid ? (kFam ? fam_diag(P, s.x, s.y, 0) : P.diag[row]) * widen(x[row]) : 0.0;
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
         tile_spin_words(s, P.nwords, lane, spinw);
         int cnt = 0;
@@ -460,11 +460,11 @@ __global__ void __launch_bounds__(256, LK::kMinBlocks) k_apply_tile(TileParams P
             for (int u = 0; u < kNB; ++u)
                 if (above_tol(xv[u])) {
                     const double cs = term_coeff(S, has_z, tt[u], s);
-                    acc += (kFam ? fam_coef(P, cs, 0) : cs) * (double)xv[u];
+                    acc += (kFam ? fam_coef(P, cs, 0) : cs) * widen<true>(xv[u]);
                 }
         }
         if (valid) {
-            if (accumulate) acc += (double)y[row];
+            if (accumulate) acc += widen(y[row]);
             y[row] = (YT)acc;
         }
         __syncwarp();
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK 
                             } else {
                                 dl = P.diag[rl];
                             }
-                            acc = dl * (double)xd;
+                            acc = dl * widen(xd);
                         }
                     }
                     for (int s0 = 0; s0 < steps; s0 += kU) {
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK 
                                 ff_fma(acc, ck.x, ck.y, (float)xv[u]);
                             } else {
                                 const double ck = hc[kb + s0 + u];
-                                acc += (kFam ? fam_coef(P, ck, c) : ck) * (double)xv[u];
+                                acc += (kFam ? fam_coef(P, ck, c) : ck) * widen<true>(xv[u]);
                             }
                         }
                     }
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK 
                             }
                             y[rl * R + c] = (XT)(acc.hi + acc.lo);
                         } else {
-                            if (accumulate) acc += (double)y[rl * R + c];
+                            if (accumulate) acc += widen(y[rl * R + c]);
                             y[rl * R + c] = (XT)acc;
                         }
                     }
@@ -902,7 +902,7 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK 
 #pragma unroll
                         for (int m = 0; m < KM; ++m) {
                             const int rr = r0 + lane + 32 * m;
-                            acc[m] = (rr < R) ? (kFam ? fam_diag(P, sl0, sl1, rr) : dl) * (double)x[rl * R + rr] : 0.0;
+                            acc[m] = (rr < R) ? (kFam ? fam_diag(P, sl0, sl1, rr) : dl) * widen(x[rl * R + rr]) : 0.0;
                         }
                         for (int k = b0; k < b0 + nl; k += 4) {
                             XT xv[4][KM];
@@ -922,14 +922,14 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK 
 #pragma unroll
                                 for (int m = 0; m < KM; ++m)
                                     if (above_tol(xv[u][m]))
-                                        acc[m] += (kFam ? fam_coef(P, ck[u], r0 + lane + 32 * m) : ck[u]) * (double)xv[u][m];
+                                        acc[m] += (kFam ? fam_coef(P, ck[u], r0 + lane + 32 * m) : ck[u]) * widen<true>(xv[u][m]);
                         }
 #pragma unroll
                         for (int m = 0; m < KM; ++m) {
                             const int rr = r0 + lane + 32 * m;
                             if (rr < R) {
                                 double v = acc[m];
-                                if (accumulate) v += (double)y[rl * R + rr];
+                                if (accumulate) v += widen(y[rl * R + rr]);
                                 y[rl * R + rr] = (XT)v;
                             }
                         }
@@ -1277,7 +1277,7 @@ __global__ void __launch_bounds__(256, kCachedBlocks) k_apply_cached(const doubl
         const bool valid = row < n;
         const uint64_t o0 = C.off[tile];
         const int width = (int)(C.off[tile + 1] - o0);
-        double acc = valid ? diag[row] * (double)x[row] : 0.0;
+        double acc = valid ? diag[row] * widen(x[row]) : 0.0;
         const uint32_t* cp = C.cols + o0 * 32 + lane;
         const TT* tp = tids + o0 * 32 + lane;
         constexpr int kU = 6;  // entries in flight per lane
@@ -1300,11 +1300,11 @@ __global__ void __launch_bounds__(256, kCachedBlocks) k_apply_cached(const doubl
                     // the FP64 pipe, GB300's bottleneck here, sees one multiply-add per hit
                     const double v = __longlong_as_double(__double_as_longlong(cs[t[u]]) ^
                                                           ((unsigned long long)(c[u] & kCacheNeg) << 32));
-                    acc += v * (double)xv[u];
+                    acc += v * widen<true>(xv[u]);
                 }
         }
         if (valid) {
-            if (accumulate) acc += (double)y[row];
+            if (accumulate) acc += widen(y[row]);
             y[row] = (YT)acc;
         }
     }

@@ -129,11 +129,7 @@ struct Vec32 {
     using W = float2;
     using Acc = DF;
     using Coef = float2;
-    __device__ static W from_apply(double y) {
-        float2 w;
-        df_split(y, w.x, w.y);
-        return w;
-    }
+    __device__ static W from_apply(double y) { return split_f64(y); }
     __device__ static Coef coef(double h) { return from_apply(h); }
     __device__ static Acc zero() { return DF{0.f, 0.f}; }
     __device__ static void dot(Acc& a, W w, V v) { df_fma(a, w.x, w.y, v); }

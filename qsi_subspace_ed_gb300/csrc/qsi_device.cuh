@@ -61,6 +61,47 @@ struct DiagSpec {
     double constant;  // -sum_k w_k * popcount(M_k)
 };
 
+// Conversions between FP32 and FP64 with integer instructions: the conversion instructions run on GB300's FP64 pipe, 17-20
+// cycles per warp each, where a materialised apply of an FP32 vector has one multiply-add per hit (64-spin Q=0 basis:
+// 178 us with them, 90 without).
+// (double)x exactly; kNormal: x is known to be neither zero nor subnormal.
+template <bool kNormal = false>
+__device__ __forceinline__ double widen(float x) {
+    const uint32_t b = __float_as_uint(x), m = b & 0x7FFFFFFFu;
+    uint32_t hi = (m >> 3) + 0x38000000u, lo = b << 29;  // exponent bias 127 -> 1023
+    if (m >= 0x7F800000u) {
+        hi += 0x38000000u;  // infinity, NaN
+    } else if (!kNormal && m < 0x00800000u) {  // m * 2^-149, m exact as a float
+        const uint32_t c = __float_as_uint((float)m);
+        hi = m ? (c >> 3) + 0x38000000u - (149u << 20) : 0u;
+        lo = c << 29;
+    }
+    return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+template <bool kNormal>
+__device__ __forceinline__ double widen(double x) {
+    return x;
+}
+
+// v as a (hi, lo) float pair: hi the nearest float, lo the nearest float to the rest.
+__device__ __forceinline__ float2 split_f64(double v) {
+    const uint64_t u = (uint64_t)__double_as_longlong(v);
+    const int e = (int)(u >> 52) & 0x7FF;
+    if ((uint32_t)(e - 960) > 180u) {  // zero; outside 2^-63 .. 2^118, where hi or lo may not be normal floats
+        if ((u << 1) == 0) return make_float2(__uint_as_float((uint32_t)(u >> 32)), 0.f);
+        const float h = (float)v;
+        return make_float2(h, (float)(v - (double)h));
+    }
+    const uint64_t m = (u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    const uint32_t q = (uint32_t)((m + 0x0FFFFFFF + ((m >> 29) & 1)) >> 29);  // to nearest, ties to even
+    const int rest = (int)((uint32_t)m - (q << 29));                         // m - q 2^29, at most 2^28
+    const uint32_t sign = (uint32_t)(u >> 32) & 0x80000000u;
+    const float h = __uint_as_float((((uint32_t)(e - 896) << 23) + (q - 0x800000u)) | sign);
+    const float l = (float)rest * __uint_as_float((uint32_t)(e - 948) << 23 | sign);  // 2^(e - 1075)
+    return make_float2(h, l);
+}
+
 // Sorted basis with a direct bucket table over the top `bits` bits below
 // `shift`: bucket(s) = s >> shift; tab[v] = {first, size} is the index range of
 // the states in bucket v ({0, 0} for an empty bucket), so one 8-byte load

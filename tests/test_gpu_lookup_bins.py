@@ -156,3 +156,33 @@ def test_pairs_that_leave_one_way(kept):
     i = np.arange(200_000)
     lohi = lohi[~(((i & 3) == 3 - kept) & ((i >> 10) % 3 == 0))]
     check(lohi, opsum(PAIRS[:2] + PAIRS[3:7]), (1, 9))
+
+
+@pytest.mark.parametrize("R", [1, 3, 20])
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("add", [False, True])
+def test_fp32_vectors_of_every_magnitude(R, special, add):
+    """FP32 vectors summed in FP64, widened by integer instructions: zeros of both signs, subnormals, the tolerance's
+    neighbours, the largest floats, infinities and NaN, bitwise as the row kernels' conversions."""
+    lat = workloads.lattice("pyro_1x2x1")
+    lohi = q.enumerate_basis(lat)
+    g, B = workloads.ring_zeeman_params(5)
+    op = q.LazyOpSum(q.ZBasis(lohi), q.build_ring_zeeman(lat, g, B))
+    rng = np.random.default_rng(R)
+    n = len(lohi)
+    x = np.ldexp(rng.standard_normal((n, R)), rng.integers(-160, 120, (n, R))).astype(np.float32)
+    pick = rng.integers(0, 12, (n, R))
+    for k, v in enumerate([0.0, -0.0, 1e-15, np.nextafter(np.float32(1e-15), np.float32(1)), 1e-45, -1e-39]):
+        x[pick == k] = v
+    y0 = np.ldexp(rng.standard_normal((n, R)), rng.integers(-160, 60, (n, R))).astype(np.float32)
+    if special:
+        x[5::97], x[7::89], x[9::83] = np.inf, -np.inf, np.nan
+    got = []
+    for kernel, cached in ((0, False), (1, False), (1, True)):
+        op.set_kernel(kernel, 3)  # batched sums in FP64 too
+        if cached:
+            op.materialise(True)
+        y = y0.copy()
+        op.apply_batched(x, y, accumulate=add)
+        got.append(y)
+    assert np.array_equal(got[0], got[1], equal_nan=True) and np.array_equal(got[0], got[2], equal_nan=True)
