@@ -59,7 +59,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 // every thread receives it.  One thread evaluates f: an FP64 square root and division by all threads of all blocks
 // took the FP64 pipe longer than the scaling they are for (27.8 us at 2.9 M rows).
 template <class F>
-__device__ __forceinline__ double of_partials(const double* __restrict__ partial, int count, double* sh, F&& f) {
+__device__ __forceinline__ double of_partials(const double* partial, int count, double* sh, F&& f) {
     if (threadIdx.x < 32) {
         double v[4] = {0.0, 0.0, 0.0, 0.0};
         for (int b = threadIdx.x; b < count; b += 128)
@@ -1446,40 +1446,63 @@ static qsi_status btrlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, 
 }
 
 // ------------------------------------------------------------------ eigval0 (mfeig0)
-// Lowest eigenvalue of the symmetric tridiagonal (a, b) by Sturm-count
-// multisection: each of the block's threads counts eigenvalues below one
-// point; the bracket shrinks by blockDim+1 per round.
-__global__ void k_tridiag_lowest(const double* __restrict__ a, const double* __restrict__ b, int m, double lo, double hi,
-                                 double* out) {
-    __shared__ int cnt[256];
-    __shared__ double bounds[2];
-    if (threadIdx.x == 0) bounds[0] = lo, bounds[1] = hi;
-    __syncthreads();
-    for (int round = 0; round < 12; ++round) {
-        double L = bounds[0], H = bounds[1];
-        double x = L + (H - L) * (threadIdx.x + 1) / (blockDim.x + 1);
-        int c = 0;
-        double d = 1.0;
-        for (int i = 0; i < m; ++i) {
-            double bb = (i > 0) ? b[i - 1] * b[i - 1] : 0.0;
-            d = (a[i] - x) - (i > 0 ? bb / d : 0.0);
-            if (d == 0.0) d = -1e-300;
-            c += (d < 0.0);
-        }
-        cnt[threadIdx.x] = c;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            // first point whose count >= 1 bounds the lowest eigenvalue from above
-            int t = 0;
-            while (t < (int)blockDim.x && cnt[t] < 1) ++t;
-            double nl = (t == 0) ? L : L + (H - L) * t / (blockDim.x + 1);
-            double nh = (t == (int)blockDim.x) ? H : L + (H - L) * (t + 1) / (blockDim.x + 1);
-            bounds[0] = nl;
-            bounds[1] = nh;
-        }
-        __syncthreads();
+// Lowest eigenvalue of the symmetric tridiagonal by multisection, one launch per round: thread j tests whether the
+// eigenvalue lies below point j of the bracket, and the next round's bracket is the interval that the points leave.
+// t[i] = {a_i, -b_{i-1}^2}, scaled to a spectrum of width 1..2.  The eigenvalue is above x while the leading minors
+// p_i = (a_i - x) p_{i-1} - b_{i-1}^2 p_{i-2} stay positive.
+//
+// A serial chain: the minors take one dependent multiply-add (64 cycles) per row, where the quotients p_i / p_{i-1} take a
+// division (446), and one warp per SM keeps the FP64 pipe (three instructions per row and warp) below that chain.
+// m = 5,000: 55 ms as quotients, twelve rounds of 256 points on one SM; 2.8 ms.
+constexpr int kSturmRounds = 5;  // 4,865^5 = 2.7e18: the bracket ends below the rounding of the tests
+constexpr int kSturmChunk = 512;
+struct Bracket {
+    double lo, hi;
+    // The interval before point `first` of n points (n: behind the last one).
+    __host__ __device__ double point(int j, int n) const { return lo + (hi - lo) * (double)(j + 1) / (double)(n + 1); }
+    __host__ __device__ void narrow(int first, int n) {
+        first = first < n ? first : n;
+        const double l = first == 0 ? lo : point(first - 1, n), h = first >= n ? hi : point(first, n);
+        lo = l, hi = h;
     }
-    if (threadIdx.x == 0) *out = 0.5 * (bounds[0] + bounds[1]);
+};
+__global__ void __launch_bounds__(32) k_sturm_round(const double2* __restrict__ t, int m, Bracket B, int round,
+                                                    int* __restrict__ first) {
+    __shared__ double2 chunk[kSturmChunk];
+    const int lane = threadIdx.x, n = gridDim.x * 32, j = blockIdx.x * 32 + lane;
+    for (int r = 0; r < round; ++r) B.narrow(first[r], n);
+    const double x = B.point(j, n);
+    double p = 1.0, pp = 0.0;
+    bool below = false;  // a minor was not positive: the eigenvalue is not above x
+    for (int i0 = 0; i0 < m && !__all_sync(0xffffffffu, below); i0 += kSturmChunk) {
+        __syncwarp();
+        for (int i = lane; i < kSturmChunk; i += 32) chunk[i] = i0 + i < m ? t[i0 + i] : make_double2(0.0, 0.0);
+        __syncwarp();
+        const int k = min(kSturmChunk, m - i0);
+        auto step = [&](const double2 c) {
+            const double q = fma(c.x - x, p, c.y * pp);
+            pp = p;
+            p = q;
+            below = below || __double_as_longlong(q) <= 0;
+        };
+        int i = 0;
+        for (; i + 8 <= k && !below; i += 8) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) step(chunk[i + u]);
+            // keep the pair in range by its exponents: a step at most triples it and seldom shrinks it far
+            int hp = __double2hiint(p), hq = __double2hiint(pp);
+            const int e = max(hp, hq) >> 20;
+            if (!below && (e > 1023 + 300 || e < 1023 - 300)) {
+                const int d = (1023 - e) << 20;
+                hp = max(hp + d, 1 << 20), hq = max(hq + d, 1 << 20);
+                p = __hiloint2double(hp, __double2loint(p));
+                pp = __hiloint2double(hq, __double2loint(pp));
+            }
+        }
+        for (; i < k && !below; ++i) step(chunk[i]);
+    }
+    const int f = __reduce_min_sync(0xffffffffu, below ? j : n);
+    if (lane == 0 && f < n) atomicMin(first + round, f);
 }
 
 // Eigenvector of the tridiagonal for eigenvalue lam by inverse iteration with
@@ -1607,6 +1630,120 @@ __global__ void __launch_bounds__(256) k_three_term_scale(double* __restrict__ u
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) u[r] *= inv;
 }
 
+
+constexpr unsigned long long kEmptySlot = ~0ull;
+// The three passes as one cooperative launch, the block's rows in registers, for vectors of at most kStepRows rows per
+// thread with one block on each SM: the passes of a short vector are launches and reductions rather than traffic.
+// 221,628 rows: an iteration of the recurrence takes 30 us with it and 34 with the three launches.
+constexpr int kStepRows = 4, kStepMaxGrid = 256;
+
+// Sum over all threads of a cooperative launch of kDotBlock threads per block, in the same order in every block, then f of
+// it: every thread receives it.  Inside a block by shared memory, so that the FP64 pipe (20 cycles per warp and add
+// however few lanes) sees 20 adds instead of the 85 of shuffles in every warp.  Between blocks each block's sum is its
+// own flag in its slot (an empty slot holds all ones, a NaN that no arithmetic produces): one round trip through L2,
+// without fences or atomics.  A wait that runs out (about a second) marks the run as failed and every block returns false.
+template <class F>
+__device__ __forceinline__ bool grid_sum(double v, unsigned long long* slots, double* sh, int* failed, double& out, F&& f) {
+    const int t = threadIdx.x;
+    __syncthreads();
+    sh[t] = v;
+    __syncthreads();
+    if (t < 128) v = (sh[t] + sh[t + 128]) + (sh[t + 256] + sh[t + 384]);
+    __syncthreads();
+    if (t < 128) sh[t] = v;
+    __syncthreads();
+    int ok = 1;
+    if (t < 32) {
+        v = (sh[t] + sh[t + 32]) + (sh[t + 64] + sh[t + 96]);
+        for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (t == 0) *(volatile unsigned long long*)(slots + blockIdx.x) = (unsigned long long)__double_as_longlong(v);
+        unsigned long long got[kStepMaxGrid / 32];
+        int tries = 1 << 20;
+        do {
+            ok = 1;
+#pragma unroll
+            for (int u = 0; u < kStepMaxGrid / 32; ++u) {
+                got[u] = 0;
+                if (t + 32 * u < gridDim.x) got[u] = *(volatile unsigned long long*)(slots + t + 32 * u);
+            }
+#pragma unroll
+            for (int u = 0; u < kStepMaxGrid / 32; ++u) ok = ok && got[u] != kEmptySlot;
+            ok = __all_sync(0xffffffffu, ok);
+        } while (!ok && --tries);
+        double w[kStepMaxGrid / 32];
+#pragma unroll
+        for (int u = 0; u < kStepMaxGrid / 32; ++u) w[u] = __longlong_as_double((long long)got[u]);
+        v = ((w[0] + w[1]) + (w[2] + w[3])) + ((w[4] + w[5]) + (w[6] + w[7]));
+        for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (t == 0) {
+            sh[0] = f(v);
+            if (!ok) *(volatile int*)failed = 1;
+        }
+    }
+    ok = __syncthreads_and(ok);
+    out = sh[0];
+    return ok;
+}
+
+__global__ void __launch_bounds__(kDotBlock, 1) k_three_term_step(const double* __restrict__ w, const double* __restrict__ v,
+                                                                  double* __restrict__ u, const double* __restrict__ beta_prev,
+                                                                  double* __restrict__ alpha, double* __restrict__ beta,
+                                                                  double* __restrict__ ev, double y, int64_t n,
+                                                                  unsigned long long* slots, unsigned long long* next,
+                                                                  int* failed) {
+    __shared__ double sh[kDotBlock];
+    // this launch's slots: dots, then norms; the next launch's are emptied
+    if (threadIdx.x < 2) next[threadIdx.x * kStepMaxGrid + blockIdx.x] = kEmptySlot;
+    const RowRange R(n);
+    const double nb = beta_prev ? -*beta_prev : 0.0;
+    double t[kStepRows], x[kStepRows], acc = 0.0, a, inv;
+#pragma unroll
+    for (int q = 0; q < kStepRows; ++q) {
+        const int64_t r = R.a + threadIdx.x + q * kDotBlock;
+        t[q] = x[q] = 0.0;
+        if (r < R.b) {
+            t[q] = w[r] + nb * u[r];
+            x[q] = v[r];
+            acc += x[q] * t[q];
+        }
+    }
+    if (!grid_sum(acc, slots, sh, failed, a, [](double z) { return z; })) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *alpha = a;
+    acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < kStepRows; ++q) {
+        const int64_t r = R.a + threadIdx.x + q * kDotBlock;
+        if (r < R.b) {
+            t[q] = t[q] - a * x[q];
+            acc += t[q] * t[q];
+            if (ev) ev[r] += y * x[q];
+        }
+    }
+    auto inverse = [&](double z) {
+        const double b = sqrt(z);
+        if (blockIdx.x == 0) *beta = b;
+        return 1.0 / b;
+    };
+    if (!grid_sum(acc, slots + kStepMaxGrid, sh, failed, inv, inverse)) return;
+#pragma unroll
+    for (int q = 0; q < kStepRows; ++q) {
+        const int64_t r = R.a + threadIdx.x + q * kDotBlock;
+        if (r < R.b) u[r] = t[q] * inv;
+    }
+}
+// Blocks of k_three_term_step for n rows, at least two rows per thread where there are as many; 0: too many rows for one
+// block on each SM, or no cooperative launch.
+static int step_blocks(int64_t n) {
+    int dev = 0, sms = 0, coop = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_three_term_step, kDotBlock, 0) != cudaSuccess)
+        return 0;
+    const int64_t most = std::min(sms, kStepMaxGrid), want = (n + 2 * kDotBlock - 1) / (2 * kDotBlock);
+    if (!coop || per_sm < 1 || n > most * kDotBlock * kStepRows) return 0;
+    return (int)std::max<int64_t>(1, std::min(most, want));
+}
+
 // y += a x
 __global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, double a, int64_t n) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) y[r] += a * x[r];
@@ -1621,13 +1758,30 @@ static qsi_status lowest_of_tridiag(const std::vector<double>& al, const std::ve
         lo = std::min(lo, al[i] - r);
         hi = std::max(hi, al[i] + r);
     }
-    DevBuf<double> d;
-    QSI_CUDA(d.alloc((size_t)2 * m + 1, st));
-    QSI_CUDA(cudaMemcpyAsync(d.p, al.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st));
-    if (m > 1) QSI_CUDA(cudaMemcpyAsync(d.p + m, be.data(), (size_t)(m - 1) * 8, cudaMemcpyHostToDevice, st));
-    k_tridiag_lowest<<<1, 256, 0, st>>>(d.p, d.p + m, m, lo - 1e-12 * std::fabs(lo) - 1e-300, hi, d.p + 2 * m);
-    QSI_CUDA(cudaMemcpyAsync(&e0, d.p + 2 * m, 8, cudaMemcpyDeviceToHost, st));
+    lo -= 1e-12 * std::fabs(lo) + 1e-300;
+    const int shift = hi - lo > 0 && std::isfinite(hi - lo) ? std::ilogb(hi - lo) : 0;
+    const double down = std::ldexp(1.0, -shift);
+    std::vector<double2> t(m);
+    for (int i = 0; i < m; ++i) {
+        const double b = i ? be[i - 1] * down : 0.0;
+        t[i] = make_double2(al[i] * down, -(b * b));
+    }
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    DevBuf<double2> d;
+    QSI_CUDA(d.alloc((size_t)m + 2, st));  // the terms, then the rounds' first points
+    int* first = reinterpret_cast<int*>(d.p + m);
+    QSI_CUDA(cudaMemsetAsync(first, 0x7F, kSturmRounds * sizeof(int), st));
+    QSI_CUDA(cudaMemcpyAsync(d.p, t.data(), (size_t)m * 16, cudaMemcpyHostToDevice, st));
+    Bracket B{lo * down, hi * down};
+    for (int r = 0; r < kSturmRounds; ++r) k_sturm_round<<<sms, 32, 0, st>>>(d.p, m, B, r, first);
+    QSI_CUDA(cudaGetLastError());
+    int found[kSturmRounds];
+    QSI_CUDA(cudaMemcpyAsync(found, first, sizeof(found), cudaMemcpyDeviceToHost, st));
     QSI_CUDA(cudaStreamSynchronize(st));
+    for (int r = 0; r < kSturmRounds; ++r) B.narrow(found[r], sms * 32);
+    e0 = std::ldexp(0.5 * (B.lo + B.hi), shift);
     return QSI_OK;
 }
 
@@ -1751,12 +1905,32 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
     QSI_CUDA(coef.alloc((size_t)2 * max_it + 2, st));
     double *d_al = coef.p, *d_be = coef.p + max_it;
     double *dot_partial = vx.partial, *norm_partial = vx.partial + kDotMaxGrid;
+    const int step_grid = step_blocks(n);
+    const bool one_launch = step_grid > 0;
+    DevBuf<unsigned long long> slots;  // two sets for k_three_term_step, then whether an exchange failed
+    int launched = 0;
+    QSI_CUDA(slots.alloc(4 * kStepMaxGrid + 1, st));
+    int* failed = reinterpret_cast<int*>(slots.p + 4 * kStepMaxGrid);
+    QSI_CUDA(cudaMemsetAsync(slots.p, 0xFF, 4 * kStepMaxGrid * 8, st));
+    QSI_CUDA(cudaMemsetAsync(failed, 0, 8, st));
     // Iterations [it, end) enqueued without waiting; before: iteration `it` starts from v, u and beta[it - 1].
     auto enqueue = [&](int it, int end, const std::vector<double>* ritz) -> qsi_status {
         for (; it < end; ++it) {
             const bool acc = ritz && it < (int)ritz->size();
             qsi_status ss = launch_apply(A.get(), v.p, w.p, 1, QSI_F64, 0, st);
             if (ss) return ss;
+            if (one_launch) {
+                const double* bp = it > 0 ? d_be + it - 1 : nullptr;
+                double *pa = d_al + it, *pb = d_be + it, *pe = acc ? ev.p : nullptr, y = acc ? (*ritz)[it] : 0.0;
+                unsigned long long *mine = slots.p + (launched & 1 ? 2 * kStepMaxGrid : 0),
+                                   *next = slots.p + (launched & 1 ? 0 : 2 * kStepMaxGrid);
+                ++launched;
+                int64_t rows = n;
+                void* args[] = {&w.p, &v.p, &u.p, &bp, &pa, &pb, &pe, &y, &rows, &mine, &next, &failed};
+                QSI_CUDA(cudaLaunchCooperativeKernel(k_three_term_step, step_grid, kDotBlock, args, 0, st));
+                std::swap(v.p, u.p);
+                continue;
+            }
             k_three_term_dot<<<vx.grid, kDotBlock, 0, st>>>(w.p, v.p, u.p, it > 0 ? d_be + it - 1 : nullptr, n, dot_partial);
             k_three_term_subtract<<<vx.grid, kDotBlock, 0, st>>>(v.p, u.p, dot_partial, vx.grid, d_al + it,
                                                                  acc ? ev.p : nullptr, acc ? (*ritz)[it] : 0.0, n, norm_partial);
@@ -1765,6 +1939,12 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         }
         QSI_CUDA(cudaGetLastError());
         return QSI_OK;
+    };
+    auto exchanged = [&]() -> qsi_status {  // waits for the stream
+        int timed_out = 0;
+        QSI_CUDA(cudaMemcpyAsync(&timed_out, failed, sizeof(int), cudaMemcpyDeviceToHost, st));
+        QSI_CUDA(cudaStreamSynchronize(st));
+        return timed_out ? fail(QSI_CUDA_ERROR, "eigval0: an exchange between blocks ran out of time") : QSI_OK;
     };
     std::vector<double> al, be, ritz;
     double eig = 1e308, e0_pass0 = 0.0;
@@ -1849,7 +2029,8 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
             be.resize(it + got);
             QSI_CUDA(cudaMemcpyAsync(al.data() + it, d_al + it, (size_t)got * 8, cudaMemcpyDeviceToHost, st));
             QSI_CUDA(cudaMemcpyAsync(be.data() + it, d_be + it, (size_t)got * 8, cudaMemcpyDeviceToHost, st));
-            QSI_CUDA(cudaStreamSynchronize(st));
+            s = exchanged();
+            if (s) return s;
             bool vanished = false;
             for (; it < end && !vanished; ++it)
                 if (be[it] < cfg->abs_tol) {
@@ -1906,6 +2087,8 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         if (s) return s;
         if (last < (int)ritz.size()) k_axpy<<<grid_for(n, 256), 256, 0, st>>>(ev.p, v.p, ritz[last], n);
     }
+    s = exchanged();
+    if (s) return s;
     *e0 = e0_pass0;
     if (iterations) *iterations = its;
     if (cfg->calc_eigenvector && eigvec) {

@@ -180,3 +180,30 @@ def test_solves_with_their_own_cache(pairs, n):
         got.append(out)
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("scale", [1e-120, 1.0, 1e120])
+@pytest.mark.parametrize("n", [300, 1025, 4097])
+def test_eigval0_levels_and_scales(n, scale):
+    """One to five blocks of rows, tridiagonals of one to several chunks, and spectra of any width: the lowest level of the
+    dense matrix, scaled, and its vector."""
+    bits = max(1, (n - 1).bit_length())
+    H = q.SymbolicOpSum()
+    for k in range(bits):
+        H.add_term(-scale * (1 + 0.01 * k), q.SymbolicPMROperator(f"{k}x"))
+        H.add_term(scale * 0.3 * (k + 1), q.SymbolicPMROperator(f"{k}z"))
+    lohi = np.zeros((n, 2), dtype=np.uint64)
+    lohi[:, 0] = np.arange(n)
+    op = q.LazyOpSum(q.ZBasis(lohi), H)
+    D = np.zeros((n, n))
+    r, c, v = op.triplets(tol=0.0)
+    np.add.at(D, (r, c), v / scale)
+    w, V = np.linalg.eigh(D)
+    its = min(n - 50, 700)
+    e, vec, got = q.eigval0(op, seed=4, abs_tol=scale * 1e-13, rel_tol=1e-16, min_iterations=10, max_iterations=its)
+    # 700 steps reach the lowest level to rounding (width below 150, multisection and recurrence of 1e-15 of it)
+    assert abs(e / scale - w[0]) < 1e-11
+    if scale < 1:
+        return  # the stop rule divides by at least 1e-10, so the second pass ends at min_iterations
+    # the second pass stops when the level moves by less than 1e-13: residual^2 <= about ten times that, times the width
+    assert np.linalg.norm(D @ vec - w[0] * vec) < 1e-4 * np.linalg.norm(vec)
