@@ -1349,6 +1349,119 @@ static qsi_status launch_cached(qsi_op* op, const void* x, void* y, int xdtype, 
 }
 
 
+// 4 .. 32 FP32 vectors of a materialised operator (vec4_ok): R / 4 lanes of four vectors each sum a row, 128 / R rows per
+// warp at once, reading the cache where it lies.  The diagonal, then the entries in cache order in double-float, as in
+// k_apply_tile_batched, so the results are bitwise its.
+//
+// k_apply_tile_batched reads the cache twice and passes every entry through its list in shared memory, whose size and
+// whose registers leave three blocks per SM; here it is four, waiting for gathers.  Against it, in us:
+//   vectors                  4             16             32             64
+//   64-spin Q=0              441 -> 187    716 -> 571     1086 -> 1074   1781 -> 2072
+//   96-spin 8.8.16.16        8545 -> 2993  12269 -> 9342  18289 -> 16578 28492 -> 31712
+// Each row's columns and terms are read by all its lanes, from 64 vectors on by too many.  Other depths: six entries in
+// flight and three blocks 186, 612, 1171 us at 4, 16, 32 vectors (64-spin), more blocks spill.
+constexpr int kCachedVecMax = 32;
+constexpr int kCachedVecBlocks = 4;
+template <typename TT>
+__global__ void __launch_bounds__(256, kCachedVecBlocks) k_apply_cached_vec4(const float2* __restrict__ coef, int n_off,
+                                                      const float2* __restrict__ diag_ff, CacheView C,
+                                                      const TT* __restrict__ tids, int64_t n, const float* __restrict__ x,
+                                                      float* __restrict__ y, int R, int accumulate,
+                                                      const float2* __restrict__ ycoef) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* cs = reinterpret_cast<float2*>(smem_raw);
+    for (int k = threadIdx.x; k < n_off; k += blockDim.x) cs[k] = coef[k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lpc = R / 4, cpw = 32 / lpc, g = lane / lpc, rr = 4 * (lane % lpc);
+    const int64_t ntiles = (n + 31) >> 5;
+    for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
+        const uint64_t o0 = C.off[tile];
+        const int width = (int)(C.off[tile + 1] - o0);
+        const float* xr = x + rr;
+        for (int l0 = 0; l0 < 32; l0 += cpw) {
+            const int64_t row = tile * 32 + l0 + g;
+            const bool valid = row < n;
+            const uint32_t* cp = C.cols + o0 * 32 + l0 + g;
+            const TT* tp = tids + o0 * 32 + l0 + g;
+            FF2 a0{0, 0}, a1{0, 0};
+            auto add = [&](float2 f, const float4 v, bool all) {
+                const uint64_t ch = pk2(f.x, f.x), cn = pk2(-f.x, -f.x), cl = pk2(f.y, f.y);
+                ff2_fma(a0, ch, cn, cl, pk2(tol_select(v.x, all), tol_select(v.y, all)));
+                ff2_fma(a1, ch, cn, cl, pk2(tol_select(v.z, all), tol_select(v.w, all)));
+            };
+            constexpr int kU = 4;  // entries in flight per lane, and as many columns read ahead
+            uint32_t c[kU];
+            TT t[kU];
+            auto fetch = [&](int k0) {
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const bool in = k0 + u < width;
+                    c[u] = in ? __ldg(cp + (uint64_t)(k0 + u) * 32) : kEmpty;
+                    t[u] = in ? __ldg(tp + (uint64_t)(k0 + u) * 32) : (TT)0;
+                }
+            };
+            fetch(0);
+            if (valid) add(diag_ff[row], *reinterpret_cast<const float4*>(xr + row * R), true);
+            for (int k0 = 0; k0 < width; k0 += kU) {
+                float4 v[kU];
+                float2 f[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    f[u] = make_float2(0.f, 0.f);
+                    if (c[u] == kEmpty) continue;
+                    v[u] = *reinterpret_cast<const float4*>(xr + (int64_t)(c[u] & ~kCacheNeg) * R);
+                    f[u] = cs[t[u]];
+                    if (c[u] & kCacheNeg) f[u] = make_float2(-f[u].x, -f[u].y);
+                }
+                fetch(k0 + kU);
+#pragma unroll
+                for (int u = 0; u < kU; ++u) add(f[u], v[u], false);
+            }
+            if (!valid) continue;
+            float4* yp = reinterpret_cast<float4*>(y + row * R + rr);
+            if (accumulate) {
+                const float4 yv = *yp;
+                if (ycoef) {
+                    const float4 ca = *reinterpret_cast<const float4*>(ycoef + rr);
+                    const float4 cb = *reinterpret_cast<const float4*>(ycoef + rr + 2);
+                    ff2_fma(a0, pk2(ca.x, ca.z), pk2(-ca.x, -ca.z), pk2(ca.y, ca.w), pk2(yv.x, yv.y));
+                    ff2_fma(a1, pk2(cb.x, cb.z), pk2(-cb.x, -cb.z), pk2(cb.y, cb.w), pk2(yv.z, yv.w));
+                } else {
+                    const uint64_t one = pk2(1.0f, 1.0f), mone = pk2(-1.0f, -1.0f), zero = pk2(0.f, 0.f);
+                    ff2_fma(a0, one, mone, zero, pk2(yv.x, yv.y));
+                    ff2_fma(a1, one, mone, zero, pk2(yv.z, yv.w));
+                }
+            }
+            const float2 a = unpk2(add2(a0.hi, a0.lo)), b = unpk2(add2(a1.hi, a1.lo));
+            *yp = make_float4(a.x, a.y, b.x, b.y);
+        }
+    }
+}
+
+static qsi_status launch_cached_vec4(qsi_op* op, const float* x, float* y, int R, int accumulate, const float2* ycoef,
+                                     cudaStream_t st) {
+    const int64_t n = op->basis->n, ntiles = (n + 31) / 32;
+    const qsi_tuning& T = op->tune[1];
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int bps = T.grid_bps > 0 ? T.grid_bps : 4 * kCachedVecBlocks;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + 7) / 8, (int64_t)sms * bps));
+    const size_t smem = (size_t)std::max(op->tile.n, 1) * 8;
+    auto go = [&](auto tt) {
+        using TT = decltype(tt);
+        k_apply_cached_vec4<TT><<<grid, 256, smem, st>>>(op->tile.ff, op->tile.n, op->d_diag_ff, cache_view(op),
+                                                        (const TT*)op->d_cache_tid, n, x, y, R, accumulate, ycoef);
+    };
+    if (op->cache_tid_bytes == 1) go(uint8_t{});
+    else go(uint16_t{});
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "cached apply launch: %s", cudaGetErrorString(e));
+    return QSI_OK;
+}
+
 // Admitted terms of the tile's widest row: the tile's number of cache lines.
 __global__ void __launch_bounds__(256) k_cache_widths(TileParams P, uint64_t* __restrict__ width) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1563,7 +1676,12 @@ qsi_status launch_family(qsi_op* tmpl, const double* x, double* y, int R, const 
 static qsi_status launch_tiles(qsi_op* op, const void* x, void* y, int R, int xdtype, int ydtype, int accumulate,
                                cudaStream_t st, bool batched, const float2* ycoef) {
     auto go = [&](auto lk) { return launch_tiles_lk(op, lk, x, y, R, xdtype, ydtype, accumulate, st, batched, ycoef); };
-    if (op->d_cache_cols) return go(LookupCache{cache_view(op)});
+    if (op->d_cache_cols) {
+        if (batched && xdtype == QSI_F32 && op->ff_accumulate && R <= kCachedVecMax && op->tune[1].vec_width < 8 &&
+            vec4_ok(op->basis->n, R, x, y))
+            return launch_cached_vec4(op, (const float*)x, (float*)y, R, accumulate, ycoef, st);
+        return go(LookupCache{cache_view(op)});
+    }
     if (op->basis->d_bins && op->tune[batched].use_hash) {
         if (op->closed) return go(LookupBins<true>{op->basis->bview()});
         return go(LookupBins<false>{op->basis->bview()});

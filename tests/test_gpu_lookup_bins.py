@@ -118,7 +118,7 @@ def test_long_lists_and_many_coefficients(n, most):
     check(integers(n), opsum(xor_terms(bits, most)), (1, 8), terms=most)
 
 
-@pytest.mark.parametrize("R", [1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 20, 33])
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 20, 32, 33])
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("pairs", [0, 2])
 def test_few_vectors(R, dtype, pairs):
