@@ -2490,19 +2490,34 @@ __global__ void __launch_bounds__(256) k_col_dots(const VT* __restrict__ a, cons
     col_block_sum<VW>(L, res, R, sh, partial);
 }
 
-// Sum over blocks of partial[b][r] in block order, sixteen loads ahead of the adds: the adds are a chain (their order
-// fixes the recurrences' rounding), the loads need not be.
-__device__ __forceinline__ double col_sum(const double* __restrict__ partial, int nblocks, int R, int r) {
-    double t = 0.0;
-    int b = 0;
-    for (; b + 16 <= nblocks; b += 16) {
-        double v[16];
+// Thread r < R: sum over blocks of partial[b][r] in block order, by a block of kColSumBlock threads, R a power of two up to
+// that.  The adds are a chain of 65 cycles each (their order fixes the recurrences' rounding), 33 us for 1,024 blocks; the
+// whole block loads the next chunk behind them.  With each column's thread loading for itself, sixteen ahead, R = 16:
+// 120 us against 52.
+constexpr int kColSumBlock = 256, kColSumPer = 8, kColChunk = kColSumBlock * kColSumPer;
+__device__ __forceinline__ double col_sum(const double* __restrict__ partial, int nblocks, int R, double* sh) {
+    const int total = nblocks * R, tid = threadIdx.x;
+    double next[kColSumPer], t = 0.0;
+    auto load = [&](int base) {
 #pragma unroll
-        for (int u = 0; u < 16; ++u) v[u] = __ldg(partial + (int64_t)(b + u) * R + r);
+        for (int u = 0; u < kColSumPer; ++u) {
+            const int i = base + u * kColSumBlock + tid;
+            next[u] = i < total ? __ldg(partial + i) : 0.0;
+        }
+    };
+    load(0);
+    for (int base = 0; base < total; base += kColChunk) {
+        __syncthreads();
 #pragma unroll
-        for (int u = 0; u < 16; ++u) t += v[u];
+        for (int u = 0; u < kColSumPer; ++u) sh[u * kColSumBlock + tid] = next[u];
+        __syncthreads();
+        load(base + kColChunk);
+        if (tid < R) {
+            const int rows = min(kColChunk, total - base) / R;
+#pragma unroll 8
+            for (int b = 0; b < rows; ++b) t += sh[b * R + tid];
+        }
     }
-    for (; b < nblocks; ++b) t += partial[(int64_t)b * R + r];
     return t;
 }
 
@@ -2511,8 +2526,10 @@ __device__ __forceinline__ double col_sum(const double* __restrict__ partial, in
 __global__ void k_col_reduce(const double* __restrict__ partial, int nblocks, int R, double* __restrict__ out,
                              int sqrt_out, double* __restrict__ inv = nullptr, float2* __restrict__ inv_ff = nullptr,
                              float2* __restrict__ neg_ff = nullptr) {
-    for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        const double t = col_sum(partial, nblocks, R, r);
+    __shared__ double sh[kColChunk];
+    const double t = col_sum(partial, nblocks, R, sh);
+    const int r = threadIdx.x;
+    if (r < R) {
         out[r] = sqrt_out ? sqrt(t) : t;
         if (inv) {
             const double v = out[r] > 0 ? 1.0 / out[r] : 1.0;
@@ -2706,9 +2723,11 @@ __global__ void k_ftlm_coef3(const double* __restrict__ partial, int nblocks, in
                              double* __restrict__ beta, double* __restrict__ inv, float2* __restrict__ inv_ff,
                              float2* __restrict__ neg_ff) {
     const int64_t stride = (int64_t)nblocks * R;
-    for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        const double cp = col_sum(partial, nblocks, R, r), pp = col_sum(partial + stride, nblocks, R, r),
-                     cc = col_sum(partial + 2 * stride, nblocks, R, r);
+    __shared__ double sh[kColChunk];
+    const double cp = col_sum(partial, nblocks, R, sh), pp = col_sum(partial + stride, nblocks, R, sh),
+                 cc = col_sum(partial + 2 * stride, nblocks, R, sh);
+    const int r = threadIdx.x;
+    if (r < R) {
         const double a = cp;
         const double b2 = pp - 2.0 * a * cp + a * a * cc;
         const double b = b2 > 0.0 ? sqrt(b2) : 0.0;
@@ -2906,7 +2925,7 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
                         const float* c = reinterpret_cast<const float*>(cur[s]);
                         float* p = reinterpret_cast<float*>(prev[s]);
                         k_col_dots3<VW><<<kColGrid, blk, 0, st>>>(c, p, F.n, F.R, F.partial.p);
-                        k_ftlm_coef3<<<1, 256, 0, st>>>(F.partial.p, kColGrid, F.R, dA + (size_t)j * F.R, beta,
+                        k_ftlm_coef3<<<1, kColSumBlock, 0, st>>>(F.partial.p, kColGrid, F.R, dA + (size_t)j * F.R, beta,
                                                         F.inv.p, F.inv_ff.p, F.nbeta_ff.p);
                         k_ftlm_update_scaled<VW><<<kColGrid, blk, 0, st>>>(p, c, dA + (size_t)j * F.R, F.inv_ff.p,
                                                                            F.n, F.R);
@@ -2914,14 +2933,14 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
                     }
                 }
                 k_col_dots<VT, VW><<<kColGrid, blk, 0, st>>>(cur[s], two ? prev[s] : F.W.p, F.n, F.R, F.partial.p);
-                k_col_reduce<<<1, 256, 0, st>>>(F.partial.p, kColGrid, F.R, dA + (size_t)j * F.R, 0);
+                k_col_reduce<<<1, kColSumBlock, 0, st>>>(F.partial.p, kColGrid, F.R, dA + (size_t)j * F.R, 0);
                 if (two)
                     k_ftlm_update<VT, VW, true><<<kColGrid, blk, 0, st>>>(prev[s], cur[s], nullptr, dA + (size_t)j * F.R,
                                                                           nullptr, F.n, F.R, F.partial.p);
                 else
                     k_ftlm_update<VT, VW><<<kColGrid, blk, 0, st>>>(prev[s], cur[s], F.W.p, dA + (size_t)j * F.R,
                                                                     bprev, F.n, F.R, F.partial.p);
-                k_col_reduce<<<1, 256, 0, st>>>(F.partial.p, kColGrid, F.R, beta, 1, F.inv.p, F.inv_ff.p,
+                k_col_reduce<<<1, kColSumBlock, 0, st>>>(F.partial.p, kColGrid, F.R, beta, 1, F.inv.p, F.inv_ff.p,
                                                 two ? F.nbeta_ff.p : nullptr);
                 k_col_scale<VT, VW><<<grid_for(F.n * F.R / VW, 256), 256, 0, st>>>(
                     prev[s], F.inv.p, F.inv_ff.p, F.n, F.R, (two && !ff[s]) ? cur[s] : nullptr, beta,
