@@ -169,10 +169,10 @@ qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t bucket_bits
 qsi_status qsi_basis_destroy(qsi_basis* b);
 qsi_status qsi_basis_dim(const qsi_basis* b, int64_t* dim);
 /* Rebuilds the lookup index: a top-bits bucket table with bucket_bits bits
- * (<= 0 keeps the current table) and, with use_hash, an open-addressing
- * hash index of the states (states of at most 96 bits).  Column lookups use
- * the hash index when present and enabled on the operator, else the bucket
- * table plus a binary search of the bucket. */
+ * (<= 0 keeps the current table) and, with use_hash, a hash index of the
+ * states in bins that belong to the buckets (states of at most 96 bits).
+ * Column lookups use the hash index when present and enabled on the operator,
+ * else the bucket table plus a binary search of the bucket. */
 qsi_status qsi_basis_index(qsi_basis* b, int32_t use_hash, int32_t bucket_bits);
 qsi_status qsi_basis_info(const qsi_basis* b, int32_t* bucket_bits, int32_t* has_hash,
                           int64_t* index_bytes);
@@ -256,7 +256,8 @@ qsi_status qsi_op_set_kernel(qsi_op* op, int32_t kernel, int32_t use_hash, int32
 /* Launch settings of the tile kernels, kept separately for single-vector
  * applies (which = 0) and batched applies (which = 1; -1 sets both):
  * grid_bps = blocks per SM (0 = built-in choice), vec_width = FP32 vectors
- * per lane of the batched kernel (0 or 4, 8, 16), vec_chunk = vectors per pass
+ * per lane of the batched kernel (4, 8, 16; 0 = built-in choice; a
+ * materialised operator takes 8 as 4), vec_chunk = vectors per pass
  * (0, 16, 32, 64, 128, 256 or 512; 0 = 32 lanes' worth).  qsi_op_get_tuning also
  * reports the kernel, use_hash (as qsi_op_set_kernel takes it) and list_cap
  * of that class.  No counterpart in the reference (its apply is an OpenMP

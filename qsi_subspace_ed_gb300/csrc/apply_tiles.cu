@@ -1,4 +1,4 @@
-// Bit-sliced tile kernels of the pull-gather apply, and the hash index.
+// Bit-sliced tile kernels of the pull-gather apply, the materialised operator's kernels, and the hash index.
 //
 // A warp owns a tile of 32 consecutive basis rows.  The tile's 32 states are
 // transposed with warp shuffles into one 32-bit word per spin (bit l = spin
@@ -11,8 +11,8 @@
 //
 // Single vector: each lane finds its own row's columns and gathers x.
 // Batched (R vectors, [row][R] layout): lanes first look up all columns of
-// the tile into a shared-memory hit list; then the warp walks the list row
-// by row and gathers each column's R values with coalesced loads.
+// the tile, term by term, into a shared-memory hit list; then the warp walks
+// the list row by row and gathers each column's R values with coalesced loads.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -548,6 +548,7 @@ constexpr int kVec16 = -2;
 constexpr int kGroup = -3;
 constexpr int kGroupMax = 16;
 constexpr uint32_t kDiagSlot = 0x80000000u;
+constexpr int kWideFrom = 32;
 inline bool vec4_ok(int64_t n, int R, const void* x, const void* y) {
     return n < (int64_t)kDiagSlot - 1 && R >= 4 && (R & 3) == 0 &&
            (R <= 128 ? (R & (R - 1)) == 0 : (R & 127) == 0) &&
@@ -561,7 +562,7 @@ inline bool vec16_ok(int64_t n, int R, const void* x, const void* y) {
 }
 
 template <typename XT, class LK, bool kFF, int KM, bool kFam = false>
-__global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
+__global__ void __launch_bounds__(256, KM == kVec8 || KM == kVec16 ? 2 : 3) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
                                                             XT* __restrict__ y, int R, int accumulate, int cap,
                                                             const float2* __restrict__ ycoef) {
     // accumulate: y <- H x + c y per column, c = 1, or the (hi, lo) float pair ycoef[column] (double-float paths)
@@ -724,12 +725,15 @@ __global__ void __launch_bounds__(256, 3) k_apply_tile_batched(TileParams P, LK 
                 // FP32 storage, double-float accumulation, no FP64 instruction.  The chunk's hit list
                 // is walked in order across row boundaries with kU column gathers in flight.
                 static_assert(std::is_same<XT, float>::value, "double-float accumulation is for FP32 vectors");
-                // Column gathers in flight per lane.  With 16-byte gathers 24 floats are in flight at 80 registers and
-                // three blocks per SM; bound by the gathers' latency, 64 vectors take, with the look-ups / materialised:
+                // Column gathers in flight per lane, bound by their latency.  64 vectors, with the look-ups / materialised,
+                // four vectors per lane and a list of 256:
                 //   floats, blocks          32, 2        32, 3        24, 3        20, 3        16, 3
                 //   96-spin 8.8.16.16 ms  40.1 / 38.9  40.4 / 30.2  37.7 / 28.5  38.5 / 29.8  45.9 / 31.4
                 //   64-spin Q=0 ms        2.48 / 2.30  2.62 / 1.87  2.38 / 1.78  2.38 / 1.84  2.73 / 1.91
-                constexpr int kU = v4 ? 24 / VPL : 8;
+                // eight vectors per lane and a list of 512, whose shared memory holds it to two blocks:
+                //   96-spin 8.8.16.16 ms  32.1 / 33.1               44.5 / 39.7
+                //   64-spin Q=0 ms        1.88 / 1.82               2.55 / 2.18
+                constexpr int kU = !v4 ? 8 : VPL == 4 ? 6 : 32 / VPL;
                 const int kbeg = __shfl_sync(0xffffffffu, base, row_start);
                 const int last = row_end - 1;
                 const int kend = __shfl_sync(0xffffffffu, base + pc, last);
@@ -1574,7 +1578,19 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
             else go(float{}, float{});
         }
     } else {
-        const TileLaunch L = tile_launch(op, 16, T.list_cap);
+        // Vectors per lane and list of the 16-byte gathers.  From kWideFrom vectors on eight per lane and a list of 512 (any
+        // other list was asked for), since a row's look-ups then cost less beside its gathers; a cache has no look-ups
+        // and does best with four and 256, or sixteen where they are asked for (figures at the kernel).
+        const bool cached = std::is_same<LK, LookupCache>::value;
+        int width = T.vec_width, want = T.list_cap;
+        if (xdtype == QSI_F32 && op->ff_accumulate) {
+            if (cached && width != 16) width = 4, want = std::min(want, 256);
+            else if (!cached && width == 0 && R >= kWideFrom && vec8_ok(P.B.n, R, x, y)) {
+                width = 8;
+                if (want == 256) want = 512;
+            }
+        }
+        const TileLaunch L = tile_launch(op, 16, want);
         const int block = L.block, cap = L.cap;
         const size_t smem = L.smem;
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "batched apply: %zu bytes of shared memory needed", smem);
@@ -1586,8 +1602,8 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
                 k<<<one_wave(k, block, smem, ntiles, T.grid_bps), block, smem, st>>>(P, lk, (const double*)x, (double*)y, R,
                                                                          accumulate, cap, ycoef);
             } else if (op->ff_accumulate) {
-                auto k = (T.vec_width == 16 && vec16_ok(P.B.n, R, x, y)) ? k_apply_tile_batched<float, LK, true, kVec16>
-                         : (T.vec_width == 8 && vec8_ok(P.B.n, R, x, y))  ? k_apply_tile_batched<float, LK, true, kVec8>
+                auto k = (width == 16 && vec16_ok(P.B.n, R, x, y)) ? k_apply_tile_batched<float, LK, true, kVec16>
+                         : (width == 8 && vec8_ok(P.B.n, R, x, y))        ? k_apply_tile_batched<float, LK, true, kVec8>
                          : vec4_ok(P.B.n, R, x, y)                        ? k_apply_tile_batched<float, LK, true, kVec4>
                                                                           : k_apply_tile_batched<float, LK, true, KM>;
                 set_smem(k, smem);

@@ -29,7 +29,7 @@ struct qsi_tuning {
     int list_cap = 256;  // hit-list entries per warp in the batched tile kernel
     int grid_bps = 0;    // tile-kernel blocks per SM (0: built-in choice)
     int vec_chunk = 0;   // vectors per pass of the 16-byte batched kernel (0: up to 32 lanes' worth)
-    int vec_width = 0;   // FP32 vectors per lane of the 16-byte batched kernel: 4 (0), 8 or 16
+    int vec_width = 0;   // FP32 vectors per lane of the 16-byte batched kernel: 4, 8 or 16 (0: built-in choice)
 };
 
 struct qsi_family;
