@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(256, KM == kVec8 || KM == kVec16 ? 2 : 3) k_ap
     static_assert(!v4 || kFF, "16-byte gathers are for FP32 vectors with double-float accumulation");
     int lpc = 32, cpw = 1;
     if constexpr (v4) {
-        const int vc = P.vchunk > 0 ? P.vchunk : 32 * VPL;
+        const int vc = P.vchunk > 0 ? min(P.vchunk, 32 * VPL) : 32 * VPL;  // the warp's lanes at most
         lpc = (R >= vc ? vc : R) / VPL;
         cpw = 32 / lpc;
     }

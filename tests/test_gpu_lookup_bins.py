@@ -186,3 +186,22 @@ def test_fp32_vectors_of_every_magnitude(R, special, add):
         op.apply_batched(x, y, accumulate=add)
         got.append(y)
     assert np.array_equal(got[0], got[1], equal_nan=True) and np.array_equal(got[0], got[2], equal_nan=True)
+
+
+@pytest.mark.parametrize("R,chunk,width", [(32, 16, 0), (64, 0, 16), (128, 128, 8), (256, 256, 0), (256, 256, 8), (512, 512, 0), (512, 512, 16)])
+def test_vectors_per_lane_and_pass(R, chunk, width):
+    """Built-in and asked-for vectors per lane with passes of up to all vectors, wider than a warp of four-vector lanes
+    too: bitwise the same, with the look-ups and materialised."""
+    lat = workloads.lattice("pyro_1x2x1")
+    g, B = workloads.ring_zeeman_params(5)
+    op = q.LazyOpSum(q.ZBasis(q.enumerate_basis(lat)), q.build_ring_zeeman(lat, g, B))
+    X = np.random.default_rng(R).standard_normal((op.rows(), R)).astype(np.float32)
+    ref = np.zeros((op.rows(), R), dtype=np.float32)
+    op.set_tuning(0, 0, which=1, vec_width=4)
+    op.apply_batched(X, ref)
+    op.set_tuning(0, chunk, which=1, vec_width=width)
+    for cached in (False, True):
+        op.materialise(cached)
+        Y = np.zeros_like(ref)
+        op.apply_batched(X, Y)
+        assert np.array_equal(Y, ref), cached
