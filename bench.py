@@ -498,7 +498,7 @@ def materialised_leg(args, q, op, n, h, x, y_host, peak, peak_kind, with_solves,
         torch.cuda.nvtx.range_pop()
         bpr = 16 + R * 4 * (h + 2) + 4 * h
         ach = n * bpr / (ms * 1e-3) / 1e9
-        kn = f"k_apply_tile_batched<float,LookupCache,FF,16-byte gathers x{op.tuning(1)['vec_width'] or 4}> R={R}"
+        kn = f"k_apply_tile_batched<float,LookupCache,FF,16-byte gathers x{16 if op.tuning(1)['vec_width'] == 16 else 4}> R={R}"
         out[f"batched_r{R}"] = {"value": n * R / (ms * 1e-3), "unit": "state-vectors/s", "ms_per_apply": ms,
                                 "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                                              "frac": ach / peak, "peak_kind": peak_kind, "bytes_per_row": bpr,
@@ -609,7 +609,7 @@ def run_ours(args):
     peak, peak_kind = measured_peaks()
     bytes_per_row = 16 + 8 + 8 * h + 8
     achieved = n * bytes_per_row / (ms * 1e-3) / 1e9
-    lookup = "LookupHash" if op.tuning(0)["use_hash"] and basis.index_info()["hash"] else "LookupTable"
+    lookup = "LookupBins" if op.tuning(0)["use_hash"] and basis.index_info()["hash"] else "LookupTable"
     kname = f"k_apply_tile<double,double,{lookup}>"
     traffic = measured_traffic(w.name, kname, n)
     # the timed steps' input and result, kept on the host for the whole-size parity check against the oracle
@@ -686,8 +686,8 @@ def run_ours(args):
             bval = n * R / (bms * 1e-3)
             bbytes = n * (16 + R * 4 * (h + 2))
             tb = op.tuning(1)
-            blk = "LookupHash" if tb["use_hash"] and basis.index_info()["hash"] else "LookupTable"
-            bk = f"k_apply_tile_batched<float,{blk},FF,16-byte gathers x{tb['vec_width'] or 4}> R={R}"
+            blk = "LookupBins" if tb["use_hash"] and basis.index_info()["hash"] else "LookupTable"
+            bk = f"k_apply_tile_batched<float,{blk},FF,16-byte gathers x{tb['vec_width'] or (8 if R >= 32 else 4)}> R={R}"
             bach = bbytes / (bms * 1e-3) / 1e9
             key = "batched_mixed" if R == Rs[0] else f"batched_mixed_r{R}"
             line[key] = {"value": bval, "unit": "state-vectors/s", "R": R, "ms_per_apply": bms,

@@ -145,7 +145,7 @@ extern "C" qsi_status qsi_op_autotune(qsi_op* op, const void* x, void* y, int32_
                           cfg.use_hash, cfg.grid_bps, cfg.vec_chunk, cfg.list_cap, best);
             T.log += line;
         }
-        // lookup: bisection over the bucket table or the regional hash, whose regions are the table's buckets
+        // lookup: bisection over the bucket table or the hash index, whose bins belong to the table's buckets
         // (QSI_TUNE_INDEX: both at widths around the current one; QSI_TUNE_LOOKUP: at the current width, leaving
         // the basis as it is).  code = 2 * bits + (1 for the hash).
         if (s == QSI_OK && (flags & (QSI_TUNE_INDEX | QSI_TUNE_LOOKUP))) {
