@@ -327,7 +327,11 @@ typedef struct qsi_report {
 
 /* Thick-restart Lanczos for the nev smallest eigenpairs with full
  * reorthogonalisation (the mfsparse path: compute_spectrum_iterative,
- * include/matrix_diag_bits.hpp:51-95).  evecs is dim x nev, vector-major. */
+ * include/matrix_diag_bits.hpp:51-95).  evecs is dim x nev, vector-major.  A
+ * vector's sign is the one that the rotations of the projected eigenproblem
+ * give it (cyclic Jacobi from the identity, pairs in the circle method's order
+ * with the first player in place): a seed and an operator determine it, except
+ * inside a degenerate level. */
 qsi_status qsi_lanczos_solve(qsi_op* op, const qsi_lanczos_cfg* cfg, double* evals,
                              double* evecs, qsi_report* report);
 
@@ -395,7 +399,8 @@ qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, const int32_t* 
  * (diagonals a[k*m..], off-diagonals b[k*m..], the first m-1 used), m <= 128:
  * ascending eigenvalues and the first component of each eigenvector — the
  * Ritz values and weights of FTLM (the dense tridiagonal solve of
- * components/linalg_routines/include/lapack_adapter.hpp:37-91, batched). */
+ * components/linalg_routines/include/lapack_adapter.hpp:37-91, batched).  Signs
+ * of the components: as for qsi_lanczos_solve's vectors. */
 qsi_status qsi_tridiag_ritz(const double* a, const double* b, int32_t m, int32_t n_mat,
                             double* evals, double* first);
 

@@ -438,15 +438,22 @@ __global__ void __launch_bounds__(128) k_ritz_vectors(const VT* __restrict__ V, 
 // ends the iteration: 6-9 sweeps.  (A test on the whole off-diagonal mass never
 // passed for elements that are left at rounding size: every call took all 60 sweeps, 5.6 ms for a 24 x 24 matrix
 // against 0.3 ms.)
-// Cosine and sine of a rotation that all but clears apq (to about 1e-7 of it; the next sweep finds the rest): the
-// tangent in FP32, from elements scaled into its range, and c = 1 / sqrt(1 + t^2) in FP64 by Newton's iteration from the
-// FP32 value, so the rotation is orthogonal to rounding whatever the tangent's error.  An FP64 division takes 446
-// cycles and a square root 691; three and two of them in a chain were most of a round.
+// The order of the pairs is part of the result: the columns come with the signs that the rotations from the identity
+// give them, and another order gives others.  It is the circle method with player 0 in place: in round r, position
+// i >= 1 holds player 1 + (i - 1 - r) mod (M - 1), and positions t and M - 1 - t meet.
+// Cosine and sine of a rotation that clears apq: the tangent from FP32, with elements scaled into its range, then one
+// Newton step in FP64 on apq t^2 + (aqq - app) t - apq, which squares FP32's relative error of 1e-7; c = 1 / sqrt(1 + t^2)
+// in FP64 by Newton's iteration from the FP32 value.  An FP64 division takes 446 cycles and a square root 691; three
+// and two of them in a chain were most of a round.
 __device__ __forceinline__ void rotation(double app, double aqq, double apq, double scale, double& c, double& s) {
-    const float d = (float)((aqq - app) * scale), o = (float)(apq * scale);
+    const double dd = (aqq - app) * scale, oo = apq * scale;
+    const float d = (float)dd, o = (float)oo;
     const float theta = d / (2.0f * o);
     const float tf = (theta >= 0.f ? 1.0f : -1.0f) / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
-    const double t = (double)tf, x = fma(t, t, 1.0);
+    double t = (double)tf;
+    const double ot = oo * t;
+    t -= fma(ot + dd, t, -oo) * (double)(1.0f / (float)(ot + ot + dd));
+    const double x = fma(t, t, 1.0);
     double y = (double)rsqrtf((float)x);  // 1 <= x <= 2
     y = fma(y, fma(-0.5 * x * y, y, 0.5), y);
     y = fma(y, fma(-0.5 * x * y, y, 0.5), y);
@@ -488,10 +495,9 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
         for (int round = 0; round < M - 1; ++round) {
             int any = 0;
             if (threadIdx.x < H) {
-                // round-robin: player M-1 stays, the others turn
                 const int t = threadIdx.x;
-                int p = (t == 0) ? M - 1 : (round + t) % (M - 1);
-                int q = (t == 0) ? round : (round + M - 1 - t) % (M - 1);
+                int p = (t == 0) ? 0 : 1 + (t - 1 - round + M - 1) % (M - 1);
+                int q = 1 + (2 * M - 3 - t - round) % (M - 1);
                 if (p > q) {
                     const int tmp = p;
                     p = q;
