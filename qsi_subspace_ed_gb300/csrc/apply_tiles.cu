@@ -1179,7 +1179,8 @@ __global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, Closure*
     const int64_t ntiles = (P.B.n + 31) >> 5;
     long long skew = 0;
     for (int64_t tile = (int64_t)blockIdx.x * nw + wid; tile < ntiles; tile += (int64_t)gridDim.x * nw) {
-        if (*(volatile int*)&out->missed) break;
+        // any block may set the flag at any time: one lane reads it for the warp, which then leaves or stays as a whole
+        if (__shfl_sync(0xffffffffu, lane == 0 ? *(volatile int*)&out->missed : 0, 0)) break;
         const int64_t row = tile * 32 + lane;
         const bool valid = row < P.B.n;
         const state2 s = valid ? P.B.states[row] : make_ulonglong2(0, 0);
@@ -1200,7 +1201,7 @@ __global__ void __launch_bounds__(256) k_find_miss(TileParams P, LK lk, Closure*
             __syncwarp();
             row_start = row_end;
         }
-        if (miss) *(volatile int*)&out->missed = 1;
+        if (__any_sync(0xffffffffu, miss) && lane == 0) *(volatile int*)&out->missed = 1;
     }
     if constexpr (kForward) {
 #pragma unroll
