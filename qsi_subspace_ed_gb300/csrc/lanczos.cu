@@ -441,24 +441,15 @@ __global__ void __launch_bounds__(128) k_ritz_vectors(const VT* __restrict__ V, 
 // The order of the pairs is part of the result: the columns come with the signs that the rotations from the identity
 // give them, and another order gives others.  It is the circle method with player 0 in place: in round r, position
 // i >= 1 holds player 1 + (i - 1 - r) mod (M - 1), and positions t and M - 1 - t meet.
-// Cosine and sine of a rotation that clears apq: the tangent from FP32, with elements scaled into its range, then one
-// Newton step in FP64 on apq t^2 + (aqq - app) t - apq, which squares FP32's relative error of 1e-7; c = 1 / sqrt(1 + t^2)
-// in FP64 by Newton's iteration from the FP32 value.  An FP64 division takes 446 cycles and a square root 691; three
-// and two of them in a chain were most of a round.
-__device__ __forceinline__ void rotation(double app, double aqq, double apq, double scale, double& c, double& s) {
-    const double dd = (aqq - app) * scale, oo = apq * scale;
-    const float d = (float)dd, o = (float)oo;
-    const float theta = d / (2.0f * o);
-    const float tf = (theta >= 0.f ? 1.0f : -1.0f) / (fabsf(theta) + sqrtf(theta * theta + 1.0f));
-    double t = (double)tf;
-    const double ot = oo * t;
-    t -= fma(ot + dd, t, -oo) * (double)(1.0f / (float)(ot + ot + dd));
-    const double x = fma(t, t, 1.0);
-    double y = (double)rsqrtf((float)x);  // 1 <= x <= 2
-    y = fma(y, fma(-0.5 * x * y, y, 0.5), y);
-    y = fma(y, fma(-0.5 * x * y, y, 0.5), y);
-    c = y;
-    s = t * y;
+// Cosine and sine of the rotation that clears apq, by FP64 divisions and square roots (446 and 691 cycles here, three and
+// two of them in a chain, most of a round).  A tangent from FP32 with a Newton step takes 8% off the 32-spin solve
+// (6.9 -> 6.4 ms with its vectors) but is good to 1e-14 only, and a block solve of FP32 vectors, whose residuals lie at
+// what they resolve, then ended at 1.016e-6 where its bound is 1e-6 (0.986e-6 as it is; 0.95 .. 1.2e-6 over seeds).
+__device__ __forceinline__ void rotation(double app, double aqq, double apq, double& c, double& s) {
+    const double theta = (aqq - app) / (2.0 * apq);
+    const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+    c = 1.0 / sqrt(t * t + 1.0);
+    s = t * c;
 }
 
 __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, int M, double* __restrict__ evals,
@@ -472,7 +463,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
     int* qq = pp + H;
     double* V = v_shared ? sn + H + H : evecs + (int64_t)blockIdx.x * M * M;  // 2 * H ints take H doubles
     __shared__ double red[32];
-    __shared__ double tau, inv_norm;
+    __shared__ double tau;
     const double* Ab = Ain + (int64_t)blockIdx.x * M * M;
     double* Vb = evecs + (int64_t)blockIdx.x * M * M;
     double* eb = evals + (int64_t)blockIdx.x * M;
@@ -483,12 +474,8 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
         nrm += Ab[i] * Ab[i];
     }
     nrm = block_sum(nrm, red);
-    if (threadIdx.x == 0) {
-        tau = nrm > 0.0 ? 1e-17 * sqrt(nrm) : 1e300;
-        inv_norm = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
-    }
+    if (threadIdx.x == 0) tau = nrm > 0.0 ? 1e-17 * sqrt(nrm) : 1e300;
     __syncthreads();
-    const double scale = inv_norm;
     const int nblk = H * (H + 1) / 2;  // blocks (t, u), t <= u
     for (int sweep = 0; sweep < max_sweeps; ++sweep) {
         int rotated = 0;
@@ -508,7 +495,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
                 const double apq = A[p * M + q];
                 double c = 1.0, s = 0.0;
                 if (fabs(apq) > tau) {
-                    rotation(A[p * M + p], A[q * M + q], apq, scale, c, s);
+                    rotation(A[p * M + p], A[q * M + q], apq, c, s);
                     any = 1;
                 }
                 cs[t] = c;
