@@ -1019,10 +1019,10 @@ __global__ void k_bins_check(BinView H, uint32_t* bins) {
         uint32_t offset, tag, w[kBinSlots];
         uint32_t* p = state_bin(H, bins, i, offset, tag);
         for (int k = 0; k < kBinSlots; ++k) w[k] = *(volatile uint32_t*)(p + k);
-        const uint32_t m = bin_match(w, tag);
-        if (m >= H.off_mask || m == offset) continue;
+        const uint32_t m = bin_match(w, tag), mark = H.off_mask - 1;
+        if (m >= mark || m == offset) continue;
         for (int k = 0; k < kBinSlots; ++k)
-            if (w[k] != kEmpty && (w[k] ^ tag) < H.off_mask) atomicOr(p + k, H.off_mask);
+            if ((w[k] ^ tag) < mark) *(volatile uint32_t*)(p + k) = tag | mark;
     }
 }
 
@@ -1049,7 +1049,7 @@ qsi_status build_hash(qsi_basis* b) {
             QSI_CUDA(cudaMalloc(&b->d_bins, b->n_bins * kBinSlots * sizeof(uint32_t)));
         }
         b->off_mask = 15;
-        while (b->off_mask < b->largest_bucket) b->off_mask = 2 * b->off_mask + 1;
+        while (b->off_mask <= b->largest_bucket) b->off_mask = 2 * b->off_mask + 1;  // offsets below the mark, off_mask - 1
         QSI_CUDA(cudaMemset(b->d_bins, 0xFF, b->n_bins * kBinSlots * sizeof(uint32_t)));
         k_bins_insert<<<grid_for(b->n, 256), 256>>>(b->bview(), b->d_bins);
         k_bins_check<<<grid_for(b->n, 256), 256>>>(b->bview(), b->d_bins);

@@ -180,10 +180,13 @@ __device__ __forceinline__ int64_t basis_find(const BasisView& B, uint64_t lo, u
 // lookup, with the rows' keys stored (8 bytes per state) and the terms' computed when they are staged.
 //
 // The bins decide nothing alone.  A state that finds its bin full is left out (few in a thousand), and
-// a state whose tag another state of its bin carries too has both slots marked with offset off_mask (k_bins_check),
+// a state whose tag another state of its bin carries too has both slots marked with offset off_mask - 1 (k_bins_check),
 // so for a state of the basis its first match is itself, marked, or absent with a full bin; the last two are settled
-// by bisecting the bucket.  (The all-ones tag meets the free slots' kEmpty as a mark.)  A state outside the basis may
-// match a tag by chance: callers that can meet one compare the state found (kClosed = false).
+// by bisecting the bucket.  Offset off_mask stays unused: with it a slot of the all-ones tag would be a free slot
+// (kEmpty), and its full bin one with room, whose left-out states no lookup would find.  The shorter the tags, the
+// likelier: a bucket of 2^24 states leaves eight bits, and every bucket is large where all states share their top
+// bits.  A state outside the basis may match a tag by chance: callers that can meet one compare the state found
+// (kClosed = false).
 //
 // Why bins: a table of 16-byte {state, index} slots with linear probing (load 1/2, 1.5 probes on average) made a
 // warp wait for its unluckiest lane, four to six dependent loads per lookup, and spent 340 warp instructions per 32
@@ -221,9 +224,9 @@ __device__ __forceinline__ void load_bin(const uint32_t* p, uint32_t (&w)[kBinSl
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
         : "l"(p));
 }
-// Smallest slot ^ tag of a bin: below off_mask it is the offset of the slot that carries the tag (an offset beyond the
-// bucket's size belongs to a neighbouring bucket that shares the bin), off_mask a marked slot, above it no slot
-// carries the tag.
+// Smallest slot ^ tag of a bin: below off_mask - 1 it is the offset of the slot that carries the tag (an offset beyond the
+// bucket's size belongs to a neighbouring bucket that shares the bin), off_mask - 1 a marked slot; from off_mask on
+// no slot carries the tag (off_mask itself: a free slot met by the all-ones tag).
 __device__ __forceinline__ uint32_t bin_match(const uint32_t (&w)[kBinSlots], uint32_t tag) {
     uint32_t m = w[0] ^ tag;
 #pragma unroll
@@ -298,7 +301,7 @@ struct LookupBins {
                     const state2 t = state(u), e = __ldg(H.B.states + J[u]);
                     if (e.x != t.x || e.y != t.y) J[u] = kEmpty;
                 }
-            } else if (kClosed || m == H.off_mask || w[u][kBinSlots - 1] != kEmpty) {
+            } else if (kClosed || m == H.off_mask - 1 || w[u][kBinSlots - 1] != kEmpty) {
                 const state2 t = state(u);
                 J[u] = (uint32_t)range_find(H.B.states, bucket[u].x, bucket[u].x + bucket[u].y, t.x, t.y);
             }

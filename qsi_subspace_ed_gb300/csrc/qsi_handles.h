@@ -18,7 +18,7 @@ struct qsi_basis {
     uint64_t n_bins = 0;
     uint2* d_keys = nullptr;         // ... and the states' keys
     uint32_t largest_bucket = 0;
-    uint32_t off_mask = 0;           // offset field of a slot: wide enough for the largest bucket
+    uint32_t off_mask = 0;           // offset field of a slot: wide enough for the largest bucket and two marks
     qsi::BasisView view() const { return qsi::BasisView{d_states, d_tab, n, shift, n_buckets}; }
     qsi::BinView bview() const { return qsi::BinView{view(), d_bins, d_keys, off_mask}; }
 };
