@@ -2039,7 +2039,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         s = lowest_of_tridiag(al, b2, eig, st);
         if (s) return s;
         e0_pass0 = eig;
-        if (cfg->calc_eigenvector) {
+        if (cfg->calc_eigenvector && !al.empty()) {
             const int m = (int)al.size();
             DevBuf<double> d, work, y;
             QSI_CUDA(d.alloc((size_t)2 * m, st));
@@ -2059,7 +2059,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         // rel_tol from min_iterations on, or the first pass's end.
         QSI_CUDA(A.alloc(ev, n));
         QSI_CUDA(cudaMemsetAsync(ev.p, 0, (size_t)n * 8, st));
-        int last = std::min(its, max_it - 1);
+        int last = std::min(its, max_it - 1);  // -1: no iterations were asked for
         eig = 1e308;
         for (int it = std::max(0, cfg->min_iterations); it < its; ++it) {
             const double old = eig;
@@ -2078,7 +2078,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         QSI_CUDA(cudaMemsetAsync(u.p, 0, (size_t)n * 8, st));
         s = enqueue(0, last, &ritz);
         if (s) return s;
-        if (last < (int)ritz.size()) k_axpy<<<grid_for(n, 256), 256, 0, st>>>(ev.p, v.p, ritz[last], n);
+        if (last >= 0 && last < (int)ritz.size()) k_axpy<<<grid_for(n, 256), 256, 0, st>>>(ev.p, v.p, ritz[last], n);
     }
     s = exchanged();
     if (s) return s;
