@@ -1871,6 +1871,7 @@ static qsi_status write_eigval0_checkpoint(const char* path, const double* d_v, 
 // checkpoint, the first pass resumes from it and writes it at the top of an
 // iteration (the state that iteration starts from).
 constexpr int kEig0Batch = 128;
+constexpr int kEig0Ring = 2 * kEig0Batch;  // coefficients kept on the device: a batch's and the one before it
 
 static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigval0Checkpoint* ck, double* e0,
                               double* eigvec, int32_t* iterations) {
@@ -1895,8 +1896,9 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
     QSI_CUDA(u.alloc(n, st));
     QSI_CUDA(w.alloc(n, st));
     const int max_it = std::max(0, cfg->max_iterations);
-    QSI_CUDA(coef.alloc((size_t)2 * max_it + 2, st));
-    double *d_al = coef.p, *d_be = coef.p + max_it;
+    QSI_CUDA(coef.alloc(2 * kEig0Ring, st));
+    auto d_al = [&](int it) { return coef.p + it % kEig0Ring; };
+    auto d_be = [&](int it) { return coef.p + kEig0Ring + it % kEig0Ring; };
     double *dot_partial = vx.partial, *norm_partial = vx.partial + kDotMaxGrid;
     const int step_grid = step_blocks(n);
     const bool one_launch = step_grid > 0;
@@ -1913,8 +1915,8 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
             qsi_status ss = launch_apply(A.get(), v.p, w.p, 1, QSI_F64, 0, st);
             if (ss) return ss;
             if (one_launch) {
-                const double* bp = it > 0 ? d_be + it - 1 : nullptr;
-                double *pa = d_al + it, *pb = d_be + it, *pe = acc ? ev.p : nullptr, y = acc ? (*ritz)[it] : 0.0;
+                const double* bp = it > 0 ? d_be(it - 1) : nullptr;
+                double *pa = d_al(it), *pb = d_be(it), *pe = acc ? ev.p : nullptr, y = acc ? (*ritz)[it] : 0.0;
                 unsigned long long *mine = slots.p + (launched & 1 ? 2 * kStepMaxGrid : 0),
                                    *next = slots.p + (launched & 1 ? 0 : 2 * kStepMaxGrid);
                 ++launched;
@@ -1924,10 +1926,10 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                 std::swap(v.p, u.p);
                 continue;
             }
-            k_three_term_dot<<<vx.grid, kDotBlock, 0, st>>>(w.p, v.p, u.p, it > 0 ? d_be + it - 1 : nullptr, n, dot_partial);
-            k_three_term_subtract<<<vx.grid, kDotBlock, 0, st>>>(v.p, u.p, dot_partial, vx.grid, d_al + it,
+            k_three_term_dot<<<vx.grid, kDotBlock, 0, st>>>(w.p, v.p, u.p, it > 0 ? d_be(it - 1) : nullptr, n, dot_partial);
+            k_three_term_subtract<<<vx.grid, kDotBlock, 0, st>>>(v.p, u.p, dot_partial, vx.grid, d_al(it),
                                                                  acc ? ev.p : nullptr, acc ? (*ritz)[it] : 0.0, n, norm_partial);
-            k_three_term_scale<<<scale_grid(n), 256, 0, st>>>(u.p, norm_partial, vx.grid, d_be + it, n);
+            k_three_term_scale<<<scale_grid(n), 256, 0, st>>>(u.p, norm_partial, vx.grid, d_be(it), n);
             std::swap(v.p, u.p);
         }
         QSI_CUDA(cudaGetLastError());
@@ -1978,7 +1980,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                 std::memcpy(&beta, dbeta.data.data(), 8);
                 QSI_CUDA(cudaMemcpyAsync(v.p, dv.data.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
                 QSI_CUDA(cudaMemcpyAsync(u.p, du.data.data(), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-                if (m > 0) QSI_CUDA(cudaMemcpyAsync(d_be + m - 1, &beta, 8, cudaMemcpyHostToDevice, st));
+                if (m > 0) QSI_CUDA(cudaMemcpyAsync(d_be((int)m - 1), &beta, 8, cudaMemcpyHostToDevice, st));
                 QSI_CUDA(cudaStreamSynchronize(st));
                 it0 = (int)itv;
             }
@@ -2008,22 +2010,27 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
                     return fail(QSI_TIMEOUT, "eigval0: stopped at iteration %d, checkpoint written to %s", it, ck->path);
                 }
             }
-            int end = std::min(max_it, it + kEig0Batch);
+            int64_t stop_at = std::min<int64_t>(max_it, (int64_t)it + kEig0Batch);
             if (ck) {
-                if (ck->wall_limit_s > 0) end = it + 1;
-                if (ck->every > 0) end = std::min(end, (it / ck->every + 1) * ck->every);
-                if (ck->stop_after > 0) end = std::min(end, it0 + ck->stop_after);
+                if (ck->wall_limit_s > 0) stop_at = it + 1;
+                if (ck->every > 0) stop_at = std::min<int64_t>(stop_at, (it / ck->every + 1) * ck->every);
+                if (ck->stop_after > 0) stop_at = std::min<int64_t>(stop_at, it0 + ck->stop_after);
             }
+            const int end = (int)stop_at;
             A.plan(it + (ck && ck->stop_after > 0 ? end - it : max_it - it));
             s = enqueue(it, end, nullptr);
             if (s) return s;
             const int got = end - it;
             al.resize(it + got);
             be.resize(it + got);
-            QSI_CUDA(cudaMemcpyAsync(al.data() + it, d_al + it, (size_t)got * 8, cudaMemcpyDeviceToHost, st));
-            QSI_CUDA(cudaMemcpyAsync(be.data() + it, d_be + it, (size_t)got * 8, cudaMemcpyDeviceToHost, st));
+            double ring[2 * kEig0Ring];
+            QSI_CUDA(cudaMemcpyAsync(ring, coef.p, sizeof(ring), cudaMemcpyDeviceToHost, st));
             s = exchanged();
             if (s) return s;
+            for (int i = it; i < end; ++i) {
+                al[i] = ring[i % kEig0Ring];
+                be[i] = ring[kEig0Ring + i % kEig0Ring];
+            }
             bool vanished = false;
             for (; it < end && !vanished; ++it)
                 if (be[it] < cfg->abs_tol) {

@@ -23,3 +23,22 @@ def test_no_iterations(most, vector):
     assert its == 0
     assert vec is None if not vector else not vec.any()
     assert np.isfinite(q.eigval0(op, max_iterations=30, calc_eigenvector=vector)[0])
+
+
+def test_an_open_number_of_iterations():
+    """As many iterations as there may be on a basis where the recurrence ends by itself: device memory for the
+    coefficients of a batch, not for all that were allowed."""
+    torch = pytest.importorskip("torch")
+    H = q.SymbolicOpSum()
+    for k in range(3):
+        H.add_term(1.0 + k, q.SymbolicPMROperator(f"{k}x"))
+    op = q.LazyOpSum(q.ZBasis(np.stack([np.arange(8, dtype=np.uint64), np.zeros(8, dtype=np.uint64)], axis=1)), H)
+    want = q.eigval0(op, max_iterations=40)
+    free, _ = torch.cuda.mem_get_info()
+    fill = torch.empty(max(0, free - (8 << 30)), dtype=torch.uint8, device="cuda")
+    try:
+        got = q.eigval0(op, max_iterations=2**31 - 1)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert got[0] == want[0] and got[2] == want[2] <= 8 and np.array_equal(got[1], want[1])
