@@ -2013,8 +2013,8 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
             int64_t stop_at = std::min<int64_t>(max_it, (int64_t)it + kEig0Batch);
             if (ck) {
                 if (ck->wall_limit_s > 0) stop_at = it + 1;
-                if (ck->every > 0) stop_at = std::min<int64_t>(stop_at, (it / ck->every + 1) * ck->every);
-                if (ck->stop_after > 0) stop_at = std::min<int64_t>(stop_at, it0 + ck->stop_after);
+                if (ck->every > 0) stop_at = std::min<int64_t>(stop_at, ((int64_t)it / ck->every + 1) * ck->every);
+                if (ck->stop_after > 0) stop_at = std::min<int64_t>(stop_at, (int64_t)it0 + ck->stop_after);
             }
             const int end = (int)stop_at;
             A.plan(it + (ck && ck->stop_after > 0 ? end - it : max_it - it));

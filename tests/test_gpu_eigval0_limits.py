@@ -42,3 +42,14 @@ def test_an_open_number_of_iterations():
         del fill
         torch.cuda.empty_cache()
     assert got[0] == want[0] and got[2] == want[2] <= 8 and np.array_equal(got[1], want[1])
+
+
+def test_a_stop_behind_the_last_iteration(tmp_path):
+    """After a resumption, stops and checkpoints so far off that the iteration to come to is no 32-bit number."""
+    op = operator()
+    path = str(tmp_path / "ck.h5")
+    want = q.eigval0(op, max_iterations=90)
+    with pytest.raises(q.QsiError):
+        q.eigval0(op, max_iterations=90, checkpoint=path, stop_after=37)
+    got = q.eigval0(op, max_iterations=90, checkpoint=path, stop_after=2**31 - 1, checkpoint_every=2**31 - 1)
+    assert got[0] == want[0] and got[2] == want[2] and np.array_equal(got[1], want[1])
