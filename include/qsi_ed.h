@@ -251,16 +251,19 @@ qsi_status qsi_op_info(const qsi_op* op, int32_t* n_offdiag, int32_t* n_pruned,
  * makes FP32 batched applies accumulate rows in FP64 instead of double-float
  * (two FP32 words, about 2^-48 relative; the default, since FP64 issue is
  * slow on this GPU);
- * list_cap (> 0) sets the per-warp hit-list size of the batched tile kernel. */
+ * list_cap (> 0) sets the per-warp hit-list size of the batched tile kernel
+ * (0 leaves it as it is; a built-in choice until one is set). */
 qsi_status qsi_op_set_kernel(qsi_op* op, int32_t kernel, int32_t use_hash, int32_t list_cap);
 /* Launch settings of the tile kernels, kept separately for single-vector
  * applies (which = 0) and batched applies (which = 1; -1 sets both):
  * grid_bps = blocks per SM (0 = built-in choice), vec_width = FP32 vectors
- * per lane of the batched kernel (4, 8, 16; 0 = built-in choice; a
- * materialised operator takes 8 as 4), vec_chunk = vectors per pass
- * (0, 16, 32, 64, 128, 256 or 512; 0 = 32 lanes' worth).  qsi_op_get_tuning also
- * reports the kernel, use_hash (as qsi_op_set_kernel takes it) and list_cap
- * of that class.  No counterpart in the reference (its apply is an OpenMP
+ * per lane of the batched kernel (4, 8, 16; 0 = built-in choice), vec_chunk =
+ * vectors per pass (0, 16, 32, 64, 128, 256 or 512; 0 = 32 lanes' worth).  For
+ * double-float sums a materialised operator, which has no look-ups to spread
+ * over more vectors, takes 8 per lane as 4 and, with 4, lists above 256 as 256;
+ * its blocks of 4 to 32 FP32 vectors take neither list nor vec_chunk.
+ * qsi_op_get_tuning also reports the kernel, use_hash (as qsi_op_set_kernel
+ * takes it) and list_cap (0 = built-in choice) of that class.  No counterpart in the reference (its apply is an OpenMP
  * loop with nothing to tune); results do not depend on these settings. */
 qsi_status qsi_op_set_tuning(qsi_op* op, int32_t which, int32_t grid_bps, int32_t vec_chunk,
                              int32_t vec_width);

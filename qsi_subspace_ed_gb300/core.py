@@ -399,7 +399,7 @@ class LazyOpSum:
         return dict(zip(("offdiag", "pruned", "diag_classes", "diag_generic"), (a.value for a in v)))
 
     def set_tuning(self, grid_bps: int = 0, vec_chunk: int = 0, which: int = -1, vec_width: int = 0) -> None:
-        """Blocks per SM of the tile kernels, vectors per pass and vectors per lane (4 or 8) of the FP32 batched
+        """Blocks per SM of the tile kernels, vectors per pass and vectors per lane (4, 8 or 16) of the FP32 batched
         kernel (0 = built-in) for single-vector (which=0), batched (1) or both (-1) applies."""
         call("qsi_op_set_tuning", self._h, int(which), int(grid_bps), int(vec_chunk), int(vec_width))
 

@@ -33,7 +33,7 @@ struct TileParams {
     const double* diag;  // per-row diagonal, precomputed with diag_value
     const float2* diag_ff;  // the same as (hi, lo) float pairs
     int nwords;
-    int vchunk;             // vectors per pass of the 16-byte batched kernel (16, 32, 64 or 128; 0 = 128)
+    int vchunk;             // vectors per pass of the 16-byte batched kernel (0: as many as 32 lanes hold)
     // operator families (family mode kernels only): the terms' coefficients encode their class as +-(class + 1)
     // and fcoef[class * fR + column] is the coefficient of that class in each column's operator
     const double* fcoef = nullptr;
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(256, RC <= 4 ? 4 : 2) k_apply_tile_cols(TilePa
     }
 }
 
-// KM values selecting 16-byte FP32 gathers of 4 (kVec4) or 8 (kVec8) vectors per lane (see batched_body), and
+// KM values selecting 16-byte FP32 gathers of 4 (kVec4) or 8 (kVec8) vectors per lane (see k_apply_tile_batched), and
 // the bases, vector counts and pointers each takes.  Their hit lists mark the diagonal slot with the top bit of
 // the row index.
 constexpr int kVec4 = 0;
@@ -1557,6 +1557,20 @@ static int tile_grid(int64_t ntiles, int block, int bps) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((ntiles + nw - 1) / nw, (int64_t)sms * (bps > 0 ? bps : 8)));
 }
 
+// From kWideFrom vectors on eight per lane and a list of 512, since a row's look-ups then cost less beside its gathers; a
+// cache has no look-ups and does best with four and at most 256, or sixteen where they are asked for (figures at the kernel).
+BatchedChoice batched_choice(const qsi_op* op, int R, int dtype, const void* x, const void* y) {
+    const qsi_tuning& T = op->tune[1];
+    const int64_t n = op->basis->n;
+    const bool gathers = dtype == QSI_F32 && op->ff_accumulate, cached = op->d_cache_cols != nullptr;
+    int width = 4;
+    if (gathers && T.vec_width == 16 && vec16_ok(n, R, x, y)) width = 16;
+    else if (gathers && !cached && (T.vec_width == 8 || (T.vec_width == 0 && R >= kWideFrom)) && vec8_ok(n, R, x, y)) width = 8;
+    int list = T.list_cap > 0 ? T.list_cap : width == 8 ? 512 : 256;
+    if (gathers && cached && width == 4) list = std::min(list, 256);
+    return {width, list};
+}
+
 template <class LK>
 static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int R, int xdtype, int ydtype,
                                   int accumulate, cudaStream_t st, bool batched, const float2* ycoef) {
@@ -1579,19 +1593,8 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
             else go(float{}, float{});
         }
     } else {
-        // Vectors per lane and list of the 16-byte gathers.  From kWideFrom vectors on eight per lane and a list of 512 (any
-        // other list was asked for), since a row's look-ups then cost less beside its gathers; a cache has no look-ups
-        // and does best with four and 256, or sixteen where they are asked for (figures at the kernel).
-        const bool cached = std::is_same<LK, LookupCache>::value;
-        int width = T.vec_width, want = T.list_cap;
-        if (xdtype == QSI_F32 && op->ff_accumulate) {
-            if (cached && width != 16) width = 4, want = std::min(want, 256);
-            else if (!cached && width == 0 && R >= kWideFrom && vec8_ok(P.B.n, R, x, y)) {
-                width = 8;
-                if (want == 256) want = 512;
-            }
-        }
-        const TileLaunch L = tile_launch(op, 16, want);
+        const BatchedChoice C = batched_choice(op, R, xdtype, x, y);
+        const TileLaunch L = tile_launch(op, 16, C.list);
         const int block = L.block, cap = L.cap;
         const size_t smem = L.smem;
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "batched apply: %zu bytes of shared memory needed", smem);
@@ -1603,10 +1606,11 @@ static qsi_status launch_tiles_lk(qsi_op* op, LK lk, const void* x, void* y, int
                 k<<<one_wave(k, block, smem, ntiles, T.grid_bps), block, smem, st>>>(P, lk, (const double*)x, (double*)y, R,
                                                                          accumulate, cap, ycoef);
             } else if (op->ff_accumulate) {
-                auto k = (width == 16 && vec16_ok(P.B.n, R, x, y)) ? k_apply_tile_batched<float, LK, true, kVec16>
-                         : (width == 8 && vec8_ok(P.B.n, R, x, y))        ? k_apply_tile_batched<float, LK, true, kVec8>
-                         : vec4_ok(P.B.n, R, x, y)                        ? k_apply_tile_batched<float, LK, true, kVec4>
-                                                                          : k_apply_tile_batched<float, LK, true, KM>;
+                auto k = C.width == 16             ? k_apply_tile_batched<float, LK, true, kVec16>
+                         : vec4_ok(P.B.n, R, x, y) ? k_apply_tile_batched<float, LK, true, kVec4>
+                                                   : k_apply_tile_batched<float, LK, true, KM>;
+                if constexpr (!std::is_same<LK, LookupCache>::value)
+                    if (C.width == 8) k = k_apply_tile_batched<float, LK, true, kVec8>;
                 set_smem(k, smem);
                 k<<<one_wave(k, block, smem, ntiles, T.grid_bps), block, smem, st>>>(P, lk, (const float*)x, (float*)y, R,
                                                                          accumulate, cap, ycoef);
@@ -1659,7 +1663,7 @@ static qsi_status launch_family_lk(qsi_op* tmpl, LK lk, const double* x, double*
         set_smem(k, L.smem);
         k<<<tile_grid(ntiles, L.block, 0), L.block, L.smem, st>>>(P, lk, x, y, accumulate, L.cap);
     } else {
-        const TileLaunch L = tile_launch(tmpl, 16, tmpl->tune[1].list_cap);
+        const TileLaunch L = tile_launch(tmpl, 16, batched_choice(tmpl, R, QSI_F64, x, y).list);
         const int block = L.block, cap = L.cap;
         const size_t smem = L.smem;
         if (smem > 227 * 1024) return fail(QSI_INVALID_ARG, "family apply: %zu bytes of shared memory needed", smem);
@@ -1694,7 +1698,7 @@ static qsi_status launch_tiles(qsi_op* op, const void* x, void* y, int R, int xd
                                cudaStream_t st, bool batched, const float2* ycoef) {
     auto go = [&](auto lk) { return launch_tiles_lk(op, lk, x, y, R, xdtype, ydtype, accumulate, st, batched, ycoef); };
     if (op->d_cache_cols) {
-        if (batched && xdtype == QSI_F32 && op->ff_accumulate && R <= kCachedVecMax && op->tune[1].vec_width < 8 &&
+        if (batched && xdtype == QSI_F32 && op->ff_accumulate && R <= kCachedVecMax &&
             vec4_ok(op->basis->n, R, x, y))
             return launch_cached_vec4(op, (const float*)x, (float*)y, R, accumulate, ycoef, st);
         return go(LookupCache{cache_view(op)});

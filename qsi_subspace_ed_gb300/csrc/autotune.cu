@@ -12,6 +12,7 @@
 //   list_cap    per-warp hit-list size of the batched kernel (rows per chunk)
 #include <algorithm>
 #include <cstdio>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -62,13 +63,21 @@ struct Trial {
         return QSI_OK;
     }
 
-    // Tries each value of one parameter, keeps the fastest (set(v) applies a value).
+    // Tries each value of one parameter, keeps the fastest (set(v) applies a value).  ran, where given: the kernel that
+    // the settings come to; a value that comes to a kernel timed before is left out.
     template <class Set>
-    qsi_status sweep(const char* name, const std::vector<int>& values, int& best_value, float& best_ms, Set set) {
+    qsi_status sweep(const char* name, const std::vector<int>& values, int& best_value, float& best_ms, Set set,
+                     const std::function<int()>& ran = {}) {
+        std::vector<int> seen;
+        if (ran) seen.push_back(ran());
         for (int v : values) {
             if (v == best_value) continue;
             qsi_status s = set(v);
             if (s != QSI_OK) return s;
+            if (ran) {
+                if (std::find(seen.begin(), seen.end(), ran()) != seen.end()) continue;
+                seen.push_back(ran());
+            }
             float ms = 0.f;
             s = time(ms);
             if (s != QSI_OK) return s;
@@ -179,10 +188,10 @@ extern "C" qsi_status qsi_op_autotune(qsi_op* op, const void* x, void* y, int32_
                 s = T.sweep("vec_width", widths, cur, best, [&](int v) {
                     cfg.vec_width = v;
                     return QSI_OK;
-                });
+                }, [&] { return batched_choice(op, R, dtype, T.x, T.y).width; });
             }
             std::vector<int> vcs;
-            const int vpl = cfg.vec_width >= 8 ? cfg.vec_width : 4;
+            const int vpl = batched_choice(op, R, dtype, T.x, T.y).width;
             for (int v : {16, 32, 64, 128, 256, 512})
                 if (v <= R && v >= vpl && v <= 32 * vpl) vcs.push_back(v);
             int cur = cfg.vec_chunk;
@@ -205,7 +214,7 @@ extern "C" qsi_status qsi_op_autotune(qsi_op* op, const void* x, void* y, int32_
             s = T.sweep("list_cap", {128, 192, 256, 384, 512}, cur, best, [&](int v) {
                 cfg.list_cap = v;
                 return QSI_OK;
-            });
+            }, [&] { return batched_choice(op, R, dtype, T.x, T.y).list; });
         }
         if (s == QSI_OK) {
             char line[128];

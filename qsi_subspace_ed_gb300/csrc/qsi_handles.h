@@ -26,7 +26,7 @@ struct qsi_basis {
 // Launch settings of one class of applies (single vector, batched).  None of them changes results.
 struct qsi_tuning {
     int use_hash = 1;    // look columns up through the basis hash index when it exists (else bucket table)
-    int list_cap = 256;  // hit-list entries per warp in the batched tile kernel
+    int list_cap = 0;    // hit-list entries per warp in the batched tile kernel (0: built-in choice)
     int grid_bps = 0;    // tile-kernel blocks per SM (0: built-in choice)
     int vec_chunk = 0;   // vectors per pass of the 16-byte batched kernel (0: up to 32 lanes' worth)
     int vec_width = 0;   // FP32 vectors per lane of the 16-byte batched kernel: 4, 8 or 16 (0: built-in choice)
@@ -134,6 +134,12 @@ qsi_status preload_apply_f64();
 // Looks the static staging arrays of qsi_op_apply_static up on the current device (once per device).
 qsi_status static_stage_prepare();
 qsi_status build_diag(qsi_op* op);
+// What a batched apply of R vectors runs with: FP32 vectors per lane of its 16-byte gathers (4, 8 or 16) and hit-list entries
+// per warp, as op->tune[1] asks for and R, the vectors' addresses and the operator's form allow.
+struct BatchedChoice {
+    int width, list;
+};
+BatchedChoice batched_choice(const qsi_op* op, int R, int dtype, const void* x, const void* y);
 // Y <- H X + c Y for R FP32 vectors [row][R] summed in double-float (the tile kernels, also for R = 1): c = 0
 // (accumulate = 0), 1, or per column the (hi, lo) float pair ycoef[column].
 qsi_status launch_apply_ff(qsi_op* op, const float* x, float* y, int R, int accumulate, const float2* ycoef,
