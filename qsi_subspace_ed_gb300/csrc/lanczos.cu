@@ -2245,8 +2245,9 @@ static qsi_status gram(const double* A, int ka, const double* C, int kc, int64_t
 
 // compute_all_expectations / compute_cross_correlation (src/expectation_eval.cpp:27-110) on the device:
 // expect[l][i][j] = psi_j . (O_l psi_i), cross[l][m][i][j] = (O_l psi_i) . (O_m psi_j).  The images W_{l,i} = O_l psi_i
-// of as many operators as a GiB holds (of all, for cross) come from one launch, those of operators with diagonal
-// terms from an apply each; their products with psi and with one another are Gram matrices, FP64 in a fixed order.
+// of as many operators and vectors as a GiB, or else half the free memory, holds (of all, for cross) come from one launch,
+// those of operators with diagonal terms from an apply each; their products with psi and with one another are Gram matrices,
+// FP64 in a fixed order.
 extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, const int32_t* op_offsets, int32_t n_ops,
                                        const double* psi, int32_t nvec, double* expect, double* cross) {
     return guarded([&]() -> qsi_status {
@@ -2295,14 +2296,30 @@ extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, cons
         QSI_CUDA(cudaMemcpyAsync(d_first.p, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         QSI_CUDA(P.alloc((size_t)n * nvec, st));
         QSI_CUDA(cudaMemcpyAsync(P.p, psi, (size_t)n * nvec * 8, cudaMemcpyHostToDevice, st));
-        const int per = cross ? n_ops : (int)std::max<int64_t>(1, std::min<int64_t>(n_ops, ((int64_t)1 << 27) / (n * nvec)));
-        QSI_CUDA(W.alloc((size_t)n * nvec * per, st));
+        // images at a time (without cross): of nv vectors, and of `per` operators where all vectors fit
+        int nv = nvec, per = n_ops;
+        auto share = [&](int64_t most) {
+            nv = (int)std::max<int64_t>(1, std::min<int64_t>(nvec, most / n));
+            per = (int)std::max<int64_t>(1, std::min<int64_t>(n_ops, most / (n * nv)));
+        };
+        if (!cross) share((int64_t)1 << 27);
+        cudaError_t we = W.alloc((size_t)n * nv * per, st);
+        if (we == cudaErrorMemoryAllocation && !cross) {
+            cudaGetLastError();
+            size_t free_b = 0, total_b = 0;
+            QSI_CUDA(cudaMemGetInfo(&free_b, &total_b));
+            share((int64_t)(free_b / 16));
+            we = W.alloc((size_t)n * nv * per, st);
+        }
+        QSI_CUDA(we);
         std::vector<double> h;
-        for (int l0 = 0; l0 < n_ops; l0 += per) {
-            const int nl = std::min(per, n_ops - l0);
+        for (int l0 = 0; l0 < n_ops; l0 += per)
+        for (int i0 = 0; i0 < nvec; i0 += nv) {
+            const int nl = std::min(per, n_ops - l0), ni = std::min(nv, nvec - i0);
+            const double* psi_i = P.p + (size_t)i0 * n;
             for (int y0 = 0; y0 < nl; y0 += 32768)
                 k_observables<<<dim3(grid_for(n, 256), std::min(32768, nl - y0)), 256, 0, st>>>(
-                    b->view(), d_pull.p, d_first.p + l0 + y0, P.p, nvec, W.p + (size_t)y0 * nvec * n);
+                    b->view(), d_pull.p, d_first.p + l0 + y0, psi_i, ni, W.p + (size_t)y0 * ni * n);
             QSI_CUDA(cudaGetLastError());
             for (int l = l0; l < l0 + nl; ++l) {
                 if (direct[l]) continue;
@@ -2310,15 +2327,16 @@ extern "C" qsi_status qsi_expectations(qsi_basis* b, const qsi_term* terms, cons
                 qsi_status s = create_op(b, terms + op_offsets[l], op_offsets[l + 1] - op_offsets[l], false, &op);
                 if (s) return s;
                 QSI_CUDA(cudaStreamSynchronize(st));
-                for (int i = 0; i < nvec && s == QSI_OK; ++i)
-                    s = launch_apply(op, P.p + (size_t)i * n, W.p + ((size_t)(l - l0) * nvec + i) * n, 1, QSI_F64, 0, op->stream);
+                for (int i = 0; i < ni && s == QSI_OK; ++i)
+                    s = launch_apply(op, psi_i + (size_t)i * n, W.p + ((size_t)(l - l0) * ni + i) * n, 1, QSI_F64, 0, op->stream);
                 if (s == QSI_OK && cudaStreamSynchronize(op->stream) != cudaSuccess) s = fail(QSI_CUDA_ERROR, "apply");
                 qsi_op_destroy(op);
                 if (s) return s;
             }
-            qsi_status s = gram(W.p, nl * nvec, P.p, nvec, n, st, h);
+            qsi_status s = gram(W.p, nl * ni, P.p, nvec, n, st, h);
             if (s) return s;
-            std::copy(h.begin(), h.end(), expect + (size_t)l0 * nvec * nvec);
+            for (int l = 0; l < nl; ++l)
+                std::copy_n(h.begin() + (size_t)l * ni * nvec, (size_t)ni * nvec, expect + ((size_t)(l0 + l) * nvec + i0) * nvec);
         }
         if (cross) {
             const int panel = std::max(1, 2048 / nvec);  // operators per Gram matrix: all of them (symmetric) or a panel
