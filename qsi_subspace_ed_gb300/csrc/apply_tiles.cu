@@ -14,8 +14,12 @@
 // the tile, term by term, into a shared-memory hit list; then the warp walks
 // the list row by row and gathers each column's R values with coalesced loads.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <vector>
 #include <type_traits>
 
@@ -1832,6 +1836,22 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes, size_t most) {
 constexpr int64_t kCacheMinRows = 8192;
 static int64_t applies_for_cache(int64_t n) { return n >= (1 << 20) ? 6 : 16; }
 
+// The solves that hold a cache, and how often memory was asked of them.
+struct SolveCaches {
+    struct Holder {
+        int device;
+        uint64_t asked;  // when the cache was built
+    };
+    std::mutex m;
+    std::condition_variable gone;
+    std::map<const SolveOp*, Holder> live;
+    std::atomic<uint64_t> asked{0};
+};
+static SolveCaches& solve_caches() {
+    static SolveCaches c;
+    return c;
+}
+
 void SolveOp::plan(int64_t applies) {
     const int64_t n = op_->basis->n;
     if (tried_ || op_->kernel != 1 || op_->family || op_->d_cache_cols || n < kCacheMinRows ||
@@ -1845,11 +1865,49 @@ void SolveOp::plan(int64_t applies) {
         materialise(&view_, true, nullptr, free_b / 4);
     }
     cudaGetLastError();  // without a cache the solve applies the operator as it is
+    if (view_.d_cache_cols) {
+        SolveCaches& c = solve_caches();
+        std::lock_guard<std::mutex> l(c.m);
+        asked_ = c.asked;
+        c.live[this] = {op_->device, asked_};
+    }
+}
+
+qsi_op* SolveOp::get() {
+    if (view_.d_cache_cols && solve_caches().asked.load(std::memory_order_relaxed) != asked_) drop();
+    return hold();
 }
 
 bool SolveOp::drop() {
     if (!view_.d_cache_cols) return false;
     drop_cache(&view_);
+    SolveCaches& c = solve_caches();
+    if (c.asked != asked_) {  // another thread waits for the memory: out of the pool, too
+        cudaMemPool_t pool;
+        cudaStreamSynchronize(op_->stream);
+        if (cudaDeviceGetDefaultMemPool(&pool, op_->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    }
+    std::lock_guard<std::mutex> l(c.m);
+    c.live.erase(this);
+    c.gone.notify_all();
+    return true;
+}
+
+bool reclaim_solve_caches() {
+    int dev = 0;
+    cudaGetLastError();
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    SolveCaches& c = solve_caches();
+    std::unique_lock<std::mutex> l(c.m);
+    const uint64_t mine = c.asked + 1;
+    auto none = [&] {
+        for (const auto& e : c.live)
+            if (e.second.device == dev && e.second.asked < mine) return false;
+        return true;
+    };
+    if (none()) return false;
+    c.asked = mine;
+    c.gone.wait(l, none);
     return true;
 }
 

@@ -2930,10 +2930,10 @@ static qsi_status ftlm_run(qsi_op** ops, int ns, const int32_t* Rs, int M, uint6
             // by -beta_prev on the way: inside the double-float apply, else by the previous step's column pass
             VT* out = two ? prev[s] : F.W.p;
             if (ff[s])
-                status = launch_apply_ff(A[s].get(), reinterpret_cast<const float*>(cur[s]), reinterpret_cast<float*>(out), F.R,
+                status = launch_apply_ff(A[s].hold(), reinterpret_cast<const float*>(cur[s]), reinterpret_cast<float*>(out), F.R,
                                          two ? 1 : 0, two ? F.nbeta_ff.p : nullptr, st);
             else
-                status = launch_apply(A[s].get(), cur[s], out, F.R, sizeof(VT) == 4 ? QSI_F32 : QSI_F64, two ? 1 : 0, st);
+                status = launch_apply(A[s].hold(), cur[s], out, F.R, sizeof(VT) == 4 ? QSI_F32 : QSI_F64, two ? 1 : 0, st);
             const double* bprev = j ? dB + (size_t)(j - 1) * F.R : nullptr;
             double* beta = dB + (size_t)j * F.R;
             auto col_step = [&](auto vw) {

@@ -66,7 +66,8 @@ qsi_status build_buckets(qsi_basis* b) {
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(&b->largest_bucket, d_largest, sizeof(uint32_t), cudaMemcpyDeviceToHost);
     cudaFree(d_largest);
-    if (e != cudaSuccess) return fail(QSI_CUDA_ERROR, "bucket table: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess)
+        return fail(e == cudaErrorMemoryAllocation ? QSI_OOM : QSI_CUDA_ERROR, "bucket table: %s", cudaGetErrorString(e));
     return QSI_OK;
 }
 
@@ -405,7 +406,9 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
         if (bad) return cleanup(fail(QSI_INVALID_ARG, "qsi_basis_create: basis states are not strictly increasing"));
         // hash index for states of at most 96 bits (skipped, not fatal, when it does not fit in memory)
         if (hb < 96) {
-            if (build_hash(b) != QSI_OK) {
+            qsi_status hs = build_hash(b);
+            if (hs == QSI_OOM && reclaim_solve_caches()) hs = build_hash(b);
+            if (hs != QSI_OK) {
                 drop_hash(b);
                 cudaGetLastError();
             }

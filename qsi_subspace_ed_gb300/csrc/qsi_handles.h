@@ -99,6 +99,8 @@ qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes, size_t most = SI
 // An operator as one solve applies it: with a lookup cache of the solve's own, in a copy of the handle, once enough
 // applies are known to use it and if it takes no more than a quarter of the free device memory; the results are
 // bitwise those of the operator without it.  A family's members apply in their family's batches and get none.
+// The cache is memory to spare: the solve gives it up for its own later allocations (alloc) and, at its next apply or its
+// end, for any call of another thread that ran out of memory (reclaim_solve_caches).
 class SolveOp {
    public:
     explicit SolveOp(qsi_op* op) : op_(op) {}
@@ -107,7 +109,9 @@ class SolveOp {
     SolveOp& operator=(const SolveOp&) = delete;
     // applies: those done so far and those sure to follow.
     void plan(int64_t applies);
-    qsi_op* get() { return view_.d_cache_cols ? &view_ : op_; }
+    // The operator for the next apply; for all applies of a graph: hold().
+    qsi_op* get();
+    qsi_op* hold() { return view_.d_cache_cols ? &view_ : op_; }
     // Frees the cache behind the applies enqueued on the operator's stream; whether there was one.
     bool drop();
     // An allocation on the operator's stream that comes before the cache when both don't fit.
@@ -126,6 +130,7 @@ class SolveOp {
     qsi_op* op_;
     qsi_op view_;
     bool tried_ = false;
+    uint64_t asked_ = 0;  // requests for memory when the cache was built
 };
 // Fills the bucket table of a basis at its current width (b->bits, b->shift, b->n_buckets).
 qsi_status build_buckets(qsi_basis* b);
