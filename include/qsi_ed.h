@@ -193,6 +193,11 @@ qsi_status qsi_op_destroy(qsi_op* op);
  * up; enable = 0 frees it.  Applies give bitwise the results of the matrix-free apply either way.  *bytes (may
  * be NULL): the cache's size. */
 qsi_status qsi_op_materialise(qsi_op* op, int32_t enable, int64_t* bytes);
+/* Solves of many applies (qsi_lanczos_solve, qsi_eigval0, qsi_ftlm_run) materialise the operator for themselves where
+ * that pays, in memory that they give back at their end, or when another call of the library runs out of it.  `most`
+ * limits those bytes for solves with this handle: 0 = none, negative (the default) = a quarter of the free device
+ * memory, which no larger limit exceeds either.  Results are the same.  Members of a family never do it. */
+qsi_status qsi_op_set_solve_cache(qsi_op* op, int64_t most);
 /* Operator families for serving many parameter points of one sector at once (the request loop that replaces
  * the reference's static phase-diagram plans, driver/ed_phasedia_plan.sh:21-25 with
  * driver/execute_asynchronous.sh:1-38; no counterpart in the operator code): the terms of qsi_op_create with a

@@ -387,6 +387,11 @@ class LazyOpSum:
         call("qsi_op_materialise", self._h, int(bool(enable)), C.byref(nb))
         return nb.value
 
+    def set_solve_cache(self, most: int = -1) -> None:
+        """Most bytes of device memory in which a solve with this operator materialises it for itself: 0 = it does not,
+        negative = a quarter of the free memory."""
+        call("qsi_op_set_solve_cache", self._h, int(most))
+
     def set_kernel(self, kernel: int = 1, use_hash: bool = True, list_cap: int = 0) -> None:
         """kernel 0: row per thread / warp per row; 1: bit-sliced 32-row tiles (default).  use_hash bit 0: hash
         index lookups; bit 1: FP64 instead of double-float accumulation of FP32 batched applies."""

@@ -1855,14 +1855,15 @@ static SolveCaches& solve_caches() {
 void SolveOp::plan(int64_t applies) {
     const int64_t n = op_->basis->n;
     if (tried_ || op_->kernel != 1 || op_->family || op_->d_cache_cols || n < kCacheMinRows ||
-        n >= ((int64_t)1 << 31) - 1 || applies < applies_for_cache(n))
+        n >= ((int64_t)1 << 31) - 1 || applies < applies_for_cache(n) || op_->solve_cache == 0)
         return;
     tried_ = true;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
         view_ = *op_;
         view_.cache_pooled = true;
-        materialise(&view_, true, nullptr, free_b / 4);
+        const size_t most = free_b / 4;
+        materialise(&view_, true, nullptr, op_->solve_cache < 0 ? most : std::min(most, (size_t)op_->solve_cache));
     }
     cudaGetLastError();  // without a cache the solve applies the operator as it is
     if (view_.d_cache_cols) {

@@ -637,6 +637,12 @@ extern "C" qsi_status qsi_op_materialise(qsi_op* op, int32_t enable, int64_t* by
     });
 }
 
+extern "C" qsi_status qsi_op_set_solve_cache(qsi_op* op, int64_t most) {
+    if (!op) return fail(QSI_INVALID_ARG, "qsi_op_set_solve_cache: null operator");
+    op->solve_cache = most;
+    return QSI_OK;
+}
+
 namespace qsi {
 
 qsi_status preload_apply_f64_rows() {

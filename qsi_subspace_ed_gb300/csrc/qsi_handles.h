@@ -62,6 +62,7 @@ struct qsi_op {
     int cache_tid_bytes = 1;
     size_t cache_entries = 0;
     bool cache_pooled = false;         // from the stream-ordered allocator (SolveOp)
+    int64_t solve_cache = -1;          // most bytes for a solve's own cache (negative: SolveOp's quarter)
     cudaStream_t stream = nullptr;
     int device = 0;        // the device current at qsi_op_create (owner of every buffer and of the stream)
     void* d_x = nullptr;   // staging for host-pointer applies
@@ -97,7 +98,7 @@ qsi_status find_closed(qsi_op* op);
 qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes, size_t most = SIZE_MAX);
 
 // An operator as one solve applies it: with a lookup cache of the solve's own, in a copy of the handle, once enough
-// applies are known to use it and if it takes no more than a quarter of the free device memory; the results are
+// applies are known to use it and if it takes no more than a quarter of the free device memory, or less if the handle says so; the results are
 // bitwise those of the operator without it.  A family's members apply in their family's batches and get none.
 // The cache is memory to spare: the solve gives it up for its own later allocations (alloc) and, at its next apply or its
 // end, for any call of another thread that ran out of memory (reclaim_solve_caches).

@@ -68,7 +68,8 @@ class Request:
 
 
 def solve_footprint(dim: int, nev: int, ncv: int) -> int:
-    """Device bytes one FP64 solve needs beyond the resident basis (Krylov basis, Ritz block, vectors, diagonal)."""
+    """Device bytes one FP64 solve needs beyond the resident basis (Krylov basis, Ritz block, vectors, diagonal); the
+    lookup cache that a plain solve may build for itself is admitted apart (RequestLoop._spare)."""
     return 8 * dim * (ncv + 1 + 2 * nev + 4) + (64 << 20)
 
 
@@ -91,6 +92,7 @@ class RequestLoop:
         self.batching = batching and solve is None
         self.min_batch_rows = min_batch_rows  # None: the family's default (small bases run their applies at once)
         self._solve = solve or self._solve_default
+        self._plain = solve is None and not self.batching
         self._make_basis = make_basis or ZBasis
         self._families: dict[str, OperatorFamily] = {}
         self._lock = threading.Condition()
@@ -150,6 +152,15 @@ class RequestLoop:
             need += basis_footprint(sec.dim, self.slots if self.batching else 0)
         return need
 
+    def _spare(self, req: Request) -> int:
+        """Bytes of the budget that no basis still to come and no solve like req on a free slot can want: what a plain
+        solve, once it and its basis are counted, may take for a lookup cache of its own."""
+        coming = sum(basis_footprint(s.dim) for k, s in self.sectors.items() if k not in self._bases)
+        left = self.budget - self._in_use - coming
+        other = max(solve_footprint(s.dim, req.nev, req.ncv) for s in self.sectors.values())
+        free_slots = self.slots - len(self._running)
+        return max(0, left - min(free_slots, max(0, left) // other) * other)
+
     def _pick(self) -> Request | None:
         """Next admissible request: a resident, running sector first, then the oldest that fits."""
         running_sectors = {r.sector for r in self._running.values()}
@@ -191,10 +202,15 @@ class RequestLoop:
                     # stays resident and accounted for
                     self._in_use += basis_footprint(sec.dim, self.slots if self.batching else 0)
                 family = self._families.get(req.sector)
+                cache = self._spare(req) if self._plain else 0
+                need += cache
+                self._in_use += cache
             req.start = time.perf_counter()
             try:
                 if family is not None:
                     req.evals = self._solve_member(req, family)
+                elif self._plain:
+                    req.evals = self._solve_default(req, basis, self.sectors[req.sector], cache)
                 else:
                     req.evals = self._solve(req, basis, self.sectors[req.sector])
             except Exception as e:  # a failed solve is reported with its request, the loop carries on
@@ -221,8 +237,9 @@ class RequestLoop:
         return ev
 
     @staticmethod
-    def _solve_default(req: Request, basis: ZBasis, sec: Sector) -> np.ndarray:
+    def _solve_default(req: Request, basis: ZBasis, sec: Sector, cache_bytes: int = -1) -> np.ndarray:
         op = LazyOpSum(basis, build_ring_zeeman(sec.lattice, req.g, req.B))
+        op.set_solve_cache(cache_bytes)
         try:
             ev, _, _ = diagonalise(op, nev=req.nev, ncv=req.ncv, tol=req.tol, seed=req.rid + 1, want_vectors=False)
         finally:

@@ -79,3 +79,17 @@ def test_another_solve_takes_the_memory(basis):
         torch.cuda.empty_cache()
     assert np.array_equal(got, want)
     assert out["result"][0] == level  # bit for bit, with the cache for a part of the iterations
+
+
+@pytest.mark.parametrize("most,cached", [(-1, True), (0, False), (100 * MB, False), (1 << 40, True)])
+def test_the_limit_of_a_solves_own_cache(basis, most, cached):
+    """The cache is built where the limit allows all of it; the results are the same."""
+    op = operator(basis, 4)
+    kw = dict(seed=2, max_iterations=2500, calc_eigenvector=False)
+    op.set_solve_cache(0)
+    want = q.eigval0(op, **kw)[0]
+    least = finish(*run(q.eigval0, op, **kw))["least"]
+    op.set_solve_cache(most)
+    out = finish(*run(q.eigval0, op, **kw))
+    assert out["result"][0] == want
+    assert (least - out["least"] > 150 * MB) == cached
