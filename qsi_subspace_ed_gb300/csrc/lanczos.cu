@@ -1447,7 +1447,8 @@ static qsi_status btrlan(qsi_op* op, const qsi_lanczos_cfg& cfg, double* evals, 
 // A serial chain: the minors take one dependent multiply-add (64 cycles) per row, where the quotients p_i / p_{i-1} take a
 // division (446), and one warp per SM keeps the FP64 pipe (three instructions per row and warp) below that chain.
 // m = 5,000: 55 ms as quotients, twelve rounds of 256 points on one SM; 2.8 ms.
-constexpr int kSturmRounds = 5;  // 4,865^5 = 2.7e18: the bracket ends below the rounding of the tests
+constexpr int kSturmBlocks = 152;  // a warp on each SM; the same points on a device with fewer
+constexpr int kSturmRounds = 5;    // 4,865^5 = 2.7e18: the bracket ends below the rounding of the tests
 constexpr int kSturmChunk = 512;
 struct Bracket {
     double lo, hi;
@@ -1759,21 +1760,18 @@ static qsi_status lowest_of_tridiag(const std::vector<double>& al, const std::ve
         const double b = i ? be[i - 1] * down : 0.0;
         t[i] = make_double2(al[i] * down, -(b * b));
     }
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     DevBuf<double2> d;
     QSI_CUDA(d.alloc((size_t)m + 2, st));  // the terms, then the rounds' first points
     int* first = reinterpret_cast<int*>(d.p + m);
     QSI_CUDA(cudaMemsetAsync(first, 0x7F, kSturmRounds * sizeof(int), st));
     QSI_CUDA(cudaMemcpyAsync(d.p, t.data(), (size_t)m * 16, cudaMemcpyHostToDevice, st));
     Bracket B{lo * down, hi * down};
-    for (int r = 0; r < kSturmRounds; ++r) k_sturm_round<<<sms, 32, 0, st>>>(d.p, m, B, r, first);
+    for (int r = 0; r < kSturmRounds; ++r) k_sturm_round<<<kSturmBlocks, 32, 0, st>>>(d.p, m, B, r, first);
     QSI_CUDA(cudaGetLastError());
     int found[kSturmRounds];
     QSI_CUDA(cudaMemcpyAsync(found, first, sizeof(found), cudaMemcpyDeviceToHost, st));
     QSI_CUDA(cudaStreamSynchronize(st));
-    for (int r = 0; r < kSturmRounds; ++r) B.narrow(found[r], sms * 32);
+    for (int r = 0; r < kSturmRounds; ++r) B.narrow(found[r], kSturmBlocks * 32);
     e0 = std::ldexp(0.5 * (B.lo + B.hi), shift);
     return QSI_OK;
 }
