@@ -546,8 +546,9 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
         }
         if (!rotated) break;
     }
-    // ascending order by counting, then the eigenvector columns in that order (row by row through the free A when
-    // they are in place in global memory)
+    // ascending order by counting, NaN before the numbers (a rank for everyone, so that every output is written, the
+    // padding's the last), then the eigenvector columns in that order (row by row through the free A when they are in
+    // place in global memory)
     int* perm = pp;  // M entries: pp and qq
     __syncthreads();
     for (int i = threadIdx.x; i < M; i += blockDim.x) {
@@ -555,7 +556,8 @@ __global__ void __launch_bounds__(256) k_jacobi(const double* __restrict__ Ain, 
         int rank = 0;
         for (int j = 0; j < M; ++j) {
             const double e = A[j * M + j];
-            rank += (e < d || (!(e > d) && j < i)) ? 1 : 0;
+            const bool before = e < d || (isnan(e) && !isnan(d)), behind = d < e || (isnan(d) && !isnan(e));
+            rank += before || (!behind && j < i);
         }
         perm[i] = rank;
         eb[rank] = d;
