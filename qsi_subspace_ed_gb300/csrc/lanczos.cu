@@ -2,13 +2,14 @@
 // reorthogonalisation (the mfsparse path), the plain three-term Lanczos of
 // projED::lanczos::eigval0 (the mfeig0 path) and batched FTLM recurrences.
 //
-// All dot products, norms and reorthogonalisation coefficients are FP64 and
-// reduced in a fixed order (per-block partial sums, then one block), so a solve
-// is deterministic for a given seed.  With precision QSI_F32 the stored Krylov
-// vectors are FP32 and the operator gathers FP32, while the working vector w,
-// every coefficient and the projected eigenproblem stay FP64 (sums over FP32
-// vectors run in double-float on the FP32 pipe, about 2^-46 relative); the
-// Ritz pairs are then polished by FP64 Rayleigh-Ritz steps with FP64 applies.
+// Dot products, norms and coefficients are reduced in a fixed order (per-block
+// partial sums, then a fixed tree), so a solve is deterministic for a given
+// seed.  With precision QSI_F32 the stored Krylov vectors are FP32 and the
+// operator gathers FP32 into FP64 sums; the working vector w is a pair of
+// floats per row, the sums over rows run in double-float on the FP32 pipe
+// (about 2^-46 relative) up to each thread's, and the coefficients and the
+// projected eigenproblem are FP64.  The Ritz pairs are then polished by FP64
+// Rayleigh-Ritz steps with FP64 applies.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -370,12 +371,6 @@ __global__ void k_randn(double* __restrict__ w, int64_t n, uint64_t seed, int ra
         double rad = sqrt(-2.0 * log(u1));
         w[r] = rad * cospi(2.0 * u2);
     }
-}
-
-template <typename VT>
-__global__ void k_to_f64(const VT* __restrict__ v, double* __restrict__ w, int64_t n) {
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        w[r] = (double)v[r];
 }
 
 // V[:, 0..k) <- V[:, 0..m) * Y[0..m, 0..k) in place, row chunk by row chunk.  FP32 vectors: each sum in
@@ -1941,7 +1936,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
         QSI_CUDA(cudaStreamSynchronize(st));
         return timed_out ? fail(QSI_CUDA_ERROR, "eigval0: an exchange between blocks ran out of time") : QSI_OK;
     };
-    std::vector<double> al, be, ritz;
+    std::vector<double> al, be, ritz, ring(2 * kEig0Ring);
     double eig = 1e308, e0_pass0 = 0.0;
     int its = 0;
     const auto t_start = std::chrono::steady_clock::now();
@@ -2023,8 +2018,7 @@ static qsi_status eigval0_run(qsi_op* op, const qsi_eigval0_cfg* cfg, const Eigv
             const int got = end - it;
             al.resize(it + got);
             be.resize(it + got);
-            double ring[2 * kEig0Ring];
-            QSI_CUDA(cudaMemcpyAsync(ring, coef.p, sizeof(ring), cudaMemcpyDeviceToHost, st));
+            QSI_CUDA(cudaMemcpyAsync(ring.data(), coef.p, ring.size() * 8, cudaMemcpyDeviceToHost, st));
             s = exchanged();
             if (s) return s;
             for (int i = it; i < end; ++i) {
