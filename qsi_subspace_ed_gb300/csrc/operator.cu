@@ -37,6 +37,7 @@ __global__ void k_fill_buckets(BasisView B, uint2* tab) {
     for (; i < B.n; i += (int64_t)gridDim.x * blockDim.x) {
         bool ok;
         const uint64_t cur = bucket_of(B, B.states[i].x, B.states[i].y, ok);
+        if (!ok) continue;  // states that are not in order (k_check_sorted), above the last one
         if (i == 0 || bucket_of(B, B.states[i - 1].x, B.states[i - 1].y, ok) != cur) tab[cur].x = (uint32_t)i;
     }
 }
@@ -47,6 +48,7 @@ __global__ void k_size_buckets(BasisView B, uint2* tab, uint32_t* largest) {
     for (; i < B.n; i += (int64_t)gridDim.x * blockDim.x) {
         bool ok;
         const uint64_t cur = bucket_of(B, B.states[i].x, B.states[i].y, ok);
+        if (!ok) continue;
         if (i + 1 != B.n && bucket_of(B, B.states[i + 1].x, B.states[i + 1].y, ok) == cur) continue;
         const uint32_t m = (uint32_t)(i + 1) - tab[cur].x;
         tab[cur].y = m;
