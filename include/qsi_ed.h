@@ -161,14 +161,14 @@ qsi_status qsi_partition_basis_h5(const char* in_path, const char* dataset, cons
                                   const uint64_t* sl_masks, int32_t n_sl);
 
 /* ---------------------------------------------------------------- device basis */
-/* Copies a sorted basis to the device and builds its top-bits bucket table.
+/* Copies a sorted basis to the device and builds its bucket table (over the highest bits in which the states differ).
  * bucket_bits <= 0 picks a size automatically.  The caller keeps its buffer
  * (LazyOpSum holds a non-owning basis reference, operator_matrix.hpp:116). */
 qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t bucket_bits,
                             qsi_basis** out);
 qsi_status qsi_basis_destroy(qsi_basis* b);
 qsi_status qsi_basis_dim(const qsi_basis* b, int64_t* dim);
-/* Rebuilds the lookup index: a top-bits bucket table with bucket_bits bits
+/* Rebuilds the lookup index: a bucket table over the bucket_bits highest bits in which the states differ
  * (<= 0 keeps the current table) and, with use_hash, a hash index of the
  * states in bins that belong to the buckets (states of at most 96 bits).
  * Column lookups use the hash index when present and enabled on the operator,

@@ -166,7 +166,7 @@ extern "C" qsi_status qsi_op_autotune(qsi_op* op, const void* x, void* y, int32_
             std::vector<int> codes;
             for (int d = -4; d <= 4; d += 2) {
                 const int bits = b0 + d;
-                if (!((flags & QSI_TUNE_INDEX) || d == 0) || bits < 8 || bits > std::min(31, b->hb + 1)) continue;
+                if (!((flags & QSI_TUNE_INDEX) || d == 0) || bits < 8 || bits > std::min(31, b->vb + 1)) continue;
                 codes.push_back(2 * bits);
                 if (can_hash) codes.push_back(2 * bits + 1);
             }

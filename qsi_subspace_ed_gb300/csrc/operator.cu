@@ -378,10 +378,16 @@ extern "C" qsi_status qsi_basis_create(const uint64_t* lohi, int64_t n, int32_t 
             const bool bins = hb < 96 && n < ((int64_t)1 << 31);
             bits = std::min(28, std::max(8, bins ? lg - 1 : lg + 1));
         }
-        bits = std::min(bits, std::min(31, hb + 1));
+        // the states differ nowhere above the highest bit in which the first and the last do
+        const uint64_t dlo = lo ^ lohi[0], dhi = hi ^ lohi[1];
+        const int vb = dhi ? 64 + 63 - __builtin_clzll(dhi) : (dlo ? 63 - __builtin_clzll(dlo) : 0);
+        b->top0 = vb >= 63 ? 0 : lo >> (vb + 1) << (vb + 1);
+        b->top1 = vb >= 127 ? 0 : vb < 64 ? hi : hi >> (vb - 63) << (vb - 63);
+        bits = std::min(bits, std::min(31, vb + 1));
         b->bits = bits;
         b->hb = hb;
-        b->shift = hb + 1 - bits;
+        b->vb = vb;
+        b->shift = vb + 1 - bits;
         b->n_buckets = 1u << bits;
         cudaError_t e = cudaMalloc(&b->d_states, (size_t)n * sizeof(state2));
         if (e == cudaSuccess) e = cudaMalloc(&b->d_tab, (size_t)b->n_buckets * sizeof(uint2));
@@ -837,13 +843,13 @@ extern "C" qsi_status qsi_basis_index(qsi_basis* b, int32_t use_hash, int32_t bu
     return guarded([&]() -> qsi_status {
         if (!b) return fail(QSI_INVALID_ARG, "qsi_basis_index: null basis");
         if (bucket_bits > 0 && bucket_bits != b->bits) {
-            int bits = std::min<int>(bucket_bits, std::min(31, b->hb + 1));
+            int bits = std::min<int>(bucket_bits, std::min(31, b->vb + 1));
             uint2* nt = nullptr;
             QSI_CUDA(cudaMalloc(&nt, ((size_t)1 << bits) * sizeof(uint2)));
             cudaFree(b->d_tab);
             b->d_tab = nt;
             b->bits = bits;
-            b->shift = b->hb + 1 - bits;
+            b->shift = b->vb + 1 - bits;
             b->n_buckets = 1u << bits;
             qsi_status bs = build_buckets(b);
             if (bs != QSI_OK) return bs;

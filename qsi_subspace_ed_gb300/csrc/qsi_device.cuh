@@ -102,16 +102,20 @@ __device__ __forceinline__ float2 split_f64(double v) {
     return make_float2(h, l);
 }
 
-// Sorted basis with a direct bucket table over the top `bits` bits below
-// `shift`: bucket(s) = s >> shift; tab[v] = {first, size} is the index range of
-// the states in bucket v ({0, 0} for an empty bucket), so one 8-byte load
-// gives a lookup both bounds.
+// Sorted basis with a direct bucket table over the `bits` highest bits in which
+// its states differ: bucket(s) = (s ^ top) >> shift, top the bits above them that
+// all states share (spins that are up everywhere; with those in the bucket
+// number all states of such a basis were in one bucket: 16 flips on 2^24
+// patterns with spin 64 up took 7.1 ms, 1.2 without); tab[v] = {first, size} is the
+// index range of the states in bucket v ({0, 0} for an empty bucket), so one
+// 8-byte load gives a lookup both bounds.
 struct BasisView {
     const state2* states;
     const uint2* tab;
     int64_t n;
     int shift;
     uint32_t n_buckets;
+    uint64_t top0, top1;
 };
 
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
@@ -121,6 +125,8 @@ __device__ __forceinline__ bool less128(uint64_t alo, uint64_t ahi, uint64_t blo
 }
 
 __device__ __forceinline__ uint64_t bucket_of(const BasisView& B, uint64_t lo, uint64_t hi, bool& in_range) {
+    lo ^= B.top0;
+    hi ^= B.top1;
     uint64_t v;
     if (B.shift >= 64) {
         v = hi >> (B.shift - 64);
@@ -133,6 +139,12 @@ __device__ __forceinline__ uint64_t bucket_of(const BasisView& B, uint64_t lo, u
     }
     in_range = v < B.n_buckets;
     return v;
+}
+
+// The 32 bits from `shift` on, linear over XOR: that of a state of the basis XOR that of the shared bits is its bucket.
+__device__ __forceinline__ uint32_t bucket_word(const BasisView& B, uint64_t lo, uint64_t hi) {
+    if (B.shift >= 64) return (uint32_t)(hi >> (B.shift - 64));
+    return (uint32_t)(B.shift == 0 ? lo : (hi << (64 - B.shift)) | (lo >> B.shift));
 }
 
 // Exact index of state (lo, hi) in [a, b), or -1: lower-bound bisection.  The state at the final position was loaded
@@ -184,8 +196,8 @@ __device__ __forceinline__ int64_t basis_find(const BasisView& B, uint64_t lo, u
 // so for a state of the basis its first match is itself, marked, or absent with a full bin; the last two are settled
 // by bisecting the bucket.  Offset off_mask stays unused: with it a slot of the all-ones tag would be a free slot
 // (kEmpty), and its full bin one with room, whose left-out states no lookup would find.  The shorter the tags, the
-// likelier: a bucket of 2^24 states leaves eight bits, and every bucket is large where all states share their top
-// bits.  A state outside the basis may match a tag by chance: callers that can meet one compare the state found
+// likelier: a bucket of 2^24 states leaves eight bits, and so many are in one bucket where a few others lie far above
+// them.  A state outside the basis may match a tag by chance: callers that can meet one compare the state found
 // (kClosed = false).
 //
 // Why bins: a table of 16-byte {state, index} slots with linear probing (load 1/2, 1.5 probes on average) made a
@@ -263,7 +275,7 @@ struct LookupTable {
 };
 
 // kClosed: every state looked up is in the basis (qsi_op::closed), so a match needs no comparison.  Terms that flip a
-// bit above the basis's highest never land in it and are pruned before they get here.
+// bit which all states share never land in the basis and are pruned before they get here.
 template <bool kClosed>
 struct LookupBins {
     BinView H;
@@ -271,15 +283,13 @@ struct LookupBins {
     // registers), 317 with three and 342 with four at three resident blocks
     static constexpr int kNB = 2, kMinBlocks = 4;
     __device__ __forceinline__ Word4 row_words(int64_t row, const state2 s) const {
-        bool ok;
         const uint2 k = row < H.B.n ? __ldg(H.keys + row) : make_uint2(0, 0);
-        return Word4{(uint32_t)bucket_of(H.B, s.x, s.y, ok), k.x, k.y, 0};
+        return Word4{bucket_word(H.B, s.x, s.y), k.x, k.y, 0};
     }
     __device__ __forceinline__ uint4 term_words(const uint4 x) const {
-        bool ok;
         const uint64_t lo = (uint64_t)x.y << 32 | x.x, hi = (uint64_t)x.w << 32 | x.z;
         const uint2 k = state_key(lo, hi);
-        return make_uint4((uint32_t)bucket_of(H.B, lo, hi, ok), k.x, k.y, 0);
+        return make_uint4(bucket_word(H.B, lo ^ H.B.top0, hi ^ H.B.top1), k.x, k.y, 0);  // the shared bits taken out here
     }
     template <int NB, class F>
     __device__ __forceinline__ void find_batch(const Word4 (&s)[NB], int n, uint32_t (&J)[NB], F&& state) const {

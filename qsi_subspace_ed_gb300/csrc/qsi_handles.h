@@ -14,12 +14,14 @@ struct qsi_basis {
     qsi::state2* d_states = nullptr;
     uint2* d_tab = nullptr;
     int hb = 0;                      // highest bit used by any state
+    int vb = 0;                      // highest bit in which two states differ
+    uint64_t top0 = 0, top1 = 0;     // the bits above vb, which all states share
     uint32_t* d_bins = nullptr;      // optional hash index over the bucket table (states <= 96 bits)
     uint64_t n_bins = 0;
     uint2* d_keys = nullptr;         // ... and the states' keys
     uint32_t largest_bucket = 0;
     uint32_t off_mask = 0;           // offset field of a slot: wide enough for the largest bucket and two marks
-    qsi::BasisView view() const { return qsi::BasisView{d_states, d_tab, n, shift, n_buckets}; }
+    qsi::BasisView view() const { return qsi::BasisView{d_states, d_tab, n, shift, n_buckets, top0, top1}; }
     qsi::BinView bview() const { return qsi::BinView{view(), d_bins, d_keys, off_mask}; }
 };
 
