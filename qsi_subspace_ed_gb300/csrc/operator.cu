@@ -253,11 +253,15 @@ __global__ void k_count_connectivity(BasisView B, const PushTerm* __restrict__ o
 
 // hit[t] = 1 when transposed term t maps some row's state onto a basis state.  A block stops once every term
 // is known to hit (terms that hit usually do so within the first rows); terms that never hit are tested on
-// every row they admit.  Rows 0, stride, 2 stride, ... are tested.
-__global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms, int n, int64_t stride,
+// every row they admit.  Rows 0, stride, 2 stride, ... are tested, for the share of the terms that is blockIdx.y's.
+__global__ void k_pull_term_hits(BasisView B, const PullTerm* __restrict__ terms, int n_terms, int64_t stride,
                                  int* __restrict__ hit) {
     extern __shared__ int known[];
     __shared__ int n_known;
+    const int first = (int)((int64_t)blockIdx.y * n_terms / gridDim.y);
+    const int n = (int)((int64_t)(blockIdx.y + 1) * n_terms / gridDim.y) - first;
+    terms += first;
+    hit += first;
     if (threadIdx.x == 0) n_known = 0;
     __syncthreads();
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
@@ -300,10 +304,18 @@ static qsi_status prune_pull_terms(qsi_basis* b, std::vector<PullTerm>& pull) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         // A sample of rows first: every block of a launch finds each term by itself, so a full grid repeats that
         // work thousands of times; after the sample its blocks mostly have nothing left to find (64-spin Q=0 basis:
-        // 311 -> 78 us, 96-spin 8.8.16.16 sector: 946 -> 147 us).
+        // 311 -> 78 us, 96-spin 8.8.16.16 sector: 946 -> 147 us).  A thread tests its terms one after another, those
+        // that never hit to the last, so where the rows are few the terms are shared out over more blocks (512 terms,
+        // most without a hit, on the 64-spin 8.8.8.8 sector with a pair: the sample 1.0 ms with all terms per thread,
+        // 0.09 with 32, beside 1.07 for the 443,256 rows).
+        auto launch = [&](int64_t rows, int64_t stride) {
+            const int blocks = grid_for(rows, 256);
+            const int shares = std::max(1, std::min({16, 2 * 152 * 8 / blocks, (n + 31) / 32}));
+            k<<<dim3(blocks, shares), 256, smem>>>(b->view(), d_terms, n, stride, d_hit);
+        };
         const int64_t stride = b->n / kSampleRows;
-        if (stride > 1) k<<<kSampleRows / 256, 256, smem>>>(b->view(), d_terms, n, stride, d_hit);
-        k<<<grid_for(b->n, 256), 256, smem>>>(b->view(), d_terms, n, 1, d_hit);
+        if (stride > 1) launch(kSampleRows, stride);
+        launch(b->n, 1);
         e = cudaGetLastError();
     }
     std::vector<int> hit(n, 1);
