@@ -498,7 +498,9 @@ def materialised_leg(args, q, op, n, h, x, y_host, peak, peak_kind, with_solves,
         torch.cuda.nvtx.range_pop()
         bpr = 16 + R * 4 * (h + 2) + 4 * h
         ach = n * bpr / (ms * 1e-3) / 1e9
-        kn = f"k_apply_tile_batched<float,LookupCache,FF,16-byte gathers x{16 if op.tuning(1)['vec_width'] == 16 else 4}> R={R}"
+        width = 16 if op.tuning(1)["vec_width"] == 16 else 4
+        kn = (f"k_apply_cached_vec4<uint8> R={R}" if R in (4, 8, 16, 32) else
+              f"k_apply_tile_batched<float,LookupCache,FF,16-byte gathers x{width}> R={R}")
         out[f"batched_r{R}"] = {"value": n * R / (ms * 1e-3), "unit": "state-vectors/s", "ms_per_apply": ms,
                                 "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                                              "frac": ach / peak, "peak_kind": peak_kind, "bytes_per_row": bpr,

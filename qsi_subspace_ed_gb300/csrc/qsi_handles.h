@@ -100,8 +100,9 @@ qsi_status find_closed(qsi_op* op);
 qsi_status materialise(qsi_op* op, bool enable, int64_t* bytes, size_t most = SIZE_MAX);
 
 // An operator as one solve applies it: with a lookup cache of the solve's own, in a copy of the handle, once enough
-// applies are known to use it and if it takes no more than a quarter of the free device memory, or less if the handle says so; the results are
-// bitwise those of the operator without it.  A family's members apply in their family's batches and get none.
+// applies are known to use it and if it takes no more than a quarter of the free device memory, or less if the handle
+// says so; the results are bitwise those of the operator without it.  A family's members apply in their family's
+// batches and get none.
 // The cache is memory to spare: the solve gives it up for its own later allocations (alloc) and, at its next apply or its
 // end, for any call of another thread that ran out of memory (reclaim_solve_caches).
 class SolveOp {

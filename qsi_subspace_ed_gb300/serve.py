@@ -74,8 +74,8 @@ def solve_footprint(dim: int, nev: int, ncv: int) -> int:
 
 
 def basis_footprint(dim: int, batch_cols: int = 0) -> int:
-    """Bytes admitted for a basis: states, bucket table and hash index with room to spare (together they take at most
-    32 B/state at the automatic size), and with batching the family's two [dim][batch_cols] FP64 batch blocks."""
+    """Bytes admitted for a basis: states, bucket table, bins and keys with room to spare (together they take at most
+    48 B/state at the automatic size), and with batching the family's two [dim][batch_cols] FP64 batch blocks."""
     return dim * (16 + 4 + 64 + 16 * batch_cols)
 
 
