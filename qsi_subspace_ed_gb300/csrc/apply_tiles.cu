@@ -609,6 +609,7 @@ __global__ void __launch_bounds__(256, KM == kVec8 || KM == kVec16 || (KM == 4 &
         if constexpr (kCached) {  // the row's entries are read from the cache, misses left out
             cur = lk.cursor(tile, lane);
             width = (int)((lk.cursor(tile + 1, lane) - cur) >> 5);
+#pragma unroll 8
             for (int k = 0; k < width; ++k) cnt += __ldg(lk.C.cols + cur + (uint64_t)k * 32) != kEmpty;
             if constexpr (kFam) s = valid ? P.B.states[row] : s;
         } else {
@@ -641,10 +642,19 @@ __global__ void __launch_bounds__(256, KM == kVec8 || KM == kVec16 || (KM == 4 &
             if constexpr (kCached) {
                 if (in_chunk) {
                     int k = base + (v4 ? 1 : 0);
-                    for (int e = 0; e < width; ++e) {
-                        const uint64_t at = cur + (uint64_t)e * 32;
-                        const uint32_t c = __ldg(lk.C.cols + at);
-                        if (c != kEmpty) put(k++, c & ~kCacheNeg, lk.term(at), c & kCacheNeg);
+                    constexpr int kE = KM == kGroup ? 4 : 8;  // entries read at once (the group's kernel has registers for four)
+                    for (int e0 = 0; e0 < width; e0 += kE) {
+                        uint32_t c[kE], t[kE];
+#pragma unroll
+                        for (int u = 0; u < kE; ++u) {
+                            const uint64_t at = cur + (uint64_t)(e0 + u) * 32;
+                            const bool in = e0 + u < width;
+                            c[u] = in ? __ldg(lk.C.cols + at) : kEmpty;
+                            t[u] = in ? lk.term(at) : 0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < kE; ++u)
+                            if (c[u] != kEmpty) put(k++, c[u] & ~kCacheNeg, t[u], c[u] & kCacheNeg);
                     }
                 }
             } else {
