@@ -566,7 +566,8 @@ inline bool vec16_ok(int64_t n, int R, const void* x, const void* y) {
 }
 
 // Blocks per SM: two where a lane sums four FP32 vectors without 16-byte gathers (KM = 4), which spill at three (100 vectors on
-// the 64-spin Q=0 basis 6,100 -> 4,620 us, 388 to 36,056 rows 59-125 -> 44-92; FP64 sums have no more than fit at three).
+// the 64-spin Q=0 basis 6,100 -> 4,620 us, 388 to 36,056 rows 59-125 -> 44-92); FP64 sums stay at three (8,260 us there, 8,480
+// at two).
 template <typename XT, class LK, bool kFF, int KM, bool kFam = false>
 __global__ void __launch_bounds__(256, KM == kVec8 || KM == kVec16 || (KM == 4 && kFF) ? 2 : 3) k_apply_tile_batched(TileParams P, LK lk, const XT* __restrict__ x,
                                                             XT* __restrict__ y, int R, int accumulate, int cap,
